@@ -183,6 +183,17 @@ __device__ __forceinline__ double rcp_pos(double x) {
     return fma(r, e, r);
 }
 
+// n / x for a positive, finite, normal x: the hardware approximation r0 of 1/x
+// (relative error e <= 2^-23) corrected by 1/x = r0 (1 + e + e^2 + O(e^3)),
+// e = 1 - x r0, applied to n r0: four FP64 operations, within about one ulp.
+__device__ __forceinline__ double quot_pos(double n, double x) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    const double e = __fma_rn(-x, r, 1.0);
+    const double q = __dmul_rn(n, r);
+    return __fma_rn(q, __fma_rn(e, e, e), q);
+}
+
 // Copies nc components of one cell, src and dst component strides ss and ds,
 // four components' loads issued before their stores (the caller guarantees
 // the two do not overlap and src is not written meanwhile), so a thread keeps

@@ -663,67 +663,84 @@ __device__ __forceinline__ void update_body(const RhsBox& B, int stage, double d
 // ---------------------------------------------------------------------------
 // WENO5 column sweep (order 5 with Navier-Stokes terms, one-division mode):
 // one thread walks a segment of faces along d for one component, keeping the
-// per-cell parts of the reconstruction in registers.
+// per-cell parts of the reconstruction in registers.  FP64 issue bounds it
+// (GB300 issues 2 FP64 operations per SM and cycle), so the form below is the
+// one with the fewest FP64 operations: about 75 per (face, component).
 //
-// The six smoothness indicators and six candidate polynomials of a face's two
-// WENO5-JS edges (flux_schemes.H:373-446) are functions of the three cells
-// centred on f-2, f-1, f, f+1; per centre y with neighbours (x, y, z) there
-// are three distinct indicators, K1 t^2 + A with t = x - 2y + z and
-// A = (3x-4y+z)^2/4, (x-4y+3z)^2/4 or (x-z)^2/4, and four distinct
-// polynomials.  Computing them once per cell instead of once per face use
-// (six uses) and rebuilding each cell's Euler flux once instead of six times
-// removes most of the per-face FP64 work; each face then only combines the
-// nonlinear weights.  The left edge uses (B, C, A) at centres (f-2, f-1, f),
-// the right edge (A, C, B) at (f+1, f, f-1).  Results differ from the
-// per-face form by rounding only (the mirrored edge evaluates the same
-// polynomials with operands in the other order).
+// The WENO5-JS edges (flux_schemes.H:373-446) in second differences.  With
+// cell differences D and t_m = v_{m-1} - 2 v_m + v_{m+1}, the linear weights
+// 1 : 6 : 3 and the nonlinear weights w2 + w1 + w0 = 1, both edges of face f
+// are the mean of its two cells less a correction,
+//   left  = (v_{f-1} + v_f)/2 - (w2 (3 t_{f-1} - 2 t_{f-2}) + w1 t_{f-1} + w0 t_f)/6,
+//   right = the same mirrored,
+// (each candidate polynomial written about the mean, with w2 + w1 + w0 = 1),
+// so the local Lax-Friedrichs flux needs the fluxes' mean and the corrections
+// only: the state's mean cancels.  Rounding errors of the reconstruction then
+// scale with the differences instead of the values (three to five times
+// smaller against 80-bit arithmetic than the candidate form on smooth, noisy
+// and discontinuous data).
+//   Indicators: with D-, D+ the differences on both sides of a cell, t = D+ -
+// D-, q = D+ + D-, four times eps + beta is s_C = 4 eps + (13/3) t^2 + q^2
+// for the central candidate and s_A = s_C - 8 t D-, s_B = s_C + 8 t D+ for the
+// one-sided ones (the squares' differences factor; the cancellation is mild,
+// s_C <= 2.2 s_A and 2.2 s_B).  Scaling all of them by 4 leaves the weights.
+//   The right edge of face m and the left edge of face m + 1 lie in cell m and
+// see the same five cells, so they share the three weight products
+//   X = C_m A_{m+1}, Y = B_{m-1} A_{m+1}, Z = B_{m-1} C_m   (A, B, C = s^2):
+// left edge: numerator X (3 t_m - 2 t_{m-1}) + 6 Y t_m + 3 Z t_{m+1} over
+// X + 6 Y + 3 Z, right edge with X and Z and the neighbours exchanged.
+//   The two corrections of a face are added as one fraction (one division for
+// the fluxes, one for the states).
+// 64^3 box, 10 components: 1.29 ms of fluxes per right-hand side, against
+// 2.34 ms in the candidate form (130 FP64 operations per face and component,
+// one division per edge).
 // ---------------------------------------------------------------------------
 constexpr int SWEEP_SEG = 32;  // longest face segment per thread (batched launches)
 
-// Per stencil centre: the three smoothness indicators already in the form the
-// weights use, (eps + beta)^2 (each is needed by one left and one right edge),
-// and the candidate polynomials.
-struct WenoCell {
-    double dA, dB, dC, p1, p2, p3, p4;
+// Per stencil centre: the second difference and the three (4 (eps + beta))^2.
+struct WenoCtr {
+    double t, dA, dB, dC;
 };
 
 // The sweep and the per-face form must round identically, so every operation
 // of the per-cell and per-face parts is an explicit intrinsic (the compiler
 // may neither contract nor reorder them differently in the two contexts).
-__device__ __forceinline__ WenoCell weno_cell(double x, double y, double z) {
-    WenoCell r;
-    // t = x - 2y + z, tA = 3x - 4y + z, tB = x - 4y + 3z = 4t - tA, q = x - z
-    const double t = __dadd_rn(__fma_rn(-2.0, y, x), z);
-    const double m4y = __dmul_rn(-4.0, y);
-    const double tA = __dadd_rn(__fma_rn(3.0, x, m4y), z);
-    const double tB = __fma_rn(4.0, t, -tA);
-    const double q = __dsub_rn(x, z);
-    // eps + K1 t^2 + u^2/4 for the three u, with eps folded into the shared term
-    const double kte = __fma_rn(__dmul_rn(13.0 / 12.0, t), t, kEpsWeno);
-    const double sA = __fma_rn(__dmul_rn(0.25, tA), tA, kte);
-    const double sB = __fma_rn(__dmul_rn(0.25, tB), tB, kte);
-    const double sC = __fma_rn(__dmul_rn(0.25, q), q, kte);
+__device__ __forceinline__ WenoCtr weno_ctr(double Dm, double Dp) {
+    WenoCtr r;
+    r.t = __dsub_rn(Dp, Dm);
+    const double q = __dadd_rn(Dp, Dm);
+    const double kte = __fma_rn(__dmul_rn(13.0 / 3.0, r.t), r.t, 4.0 * kEpsWeno);
+    const double sC = __fma_rn(q, q, kte);
+    const double t8 = __dmul_rn(8.0, r.t);
+    const double sA = __fma_rn(-t8, Dm, sC);
+    const double sB = __fma_rn(t8, Dp, sC);
     r.dA = __dmul_rn(sA, sA);
     r.dB = __dmul_rn(sB, sB);
     r.dC = __dmul_rn(sC, sC);
-    // candidates (times 6): 2x - 7y + 11z, -x + 5y + 2z, 2x + 5y - z, 11x - 7y + 2z
-    const double m7y = __dmul_rn(-7.0, y), y5 = __dmul_rn(5.0, y);
-    r.p1 = __fma_rn(11.0, z, __fma_rn(2.0, x, m7y));
-    r.p2 = __fma_rn(2.0, z, __dsub_rn(y5, x));
-    r.p3 = __fma_rn(2.0, x, __dsub_rn(y5, z));
-    r.p4 = __fma_rn(11.0, x, __fma_rn(2.0, z, m7y));
     return r;
 }
 
-// Nonlinear combination of one edge: (eps + beta)^2 of the three candidates
-// d2, d1, d0 with linear weights 1, 6, 3 and candidates v2, v1, v0 (divided
-// by 6).  The weight sum is a positive normal number, so a Newton-refined
-// reciprocal replaces the division.
-__device__ __forceinline__ double weno_comb(double d2, double d1, double d0, double v2, double v1, double v0) {
-    const double e2 = __dmul_rn(d1, d0), e1 = __dmul_rn(6.0, __dmul_rn(d2, d0)), e0 = __dmul_rn(3.0, __dmul_rn(d2, d1));
-    const double num = __fma_rn(e0, v0, __fma_rn(e1, v1, __dmul_rn(e2, v2)));
-    const double den = __dadd_rn(__dadd_rn(e2, e1), e0);
-    return __dmul_rn(num, rcp_pos(__dmul_rn(6.0, den)));
+// The corrections' fractions (a third of the numerators) of the two edges in
+// cell m from the centres m-1 (t, dB), m (t, dC), m+1 (t, dA): nL / dL of the
+// left edge of face m+1, nR / dR of the right edge of face m.
+__device__ __forceinline__ void weno_pair(double tm, double dBm, double t0, double dC0, double tp, double dAp,
+                                          double& nL, double& dL, double& nR, double& dR) {
+    const double X = __dmul_rn(dC0, dAp), Y = __dmul_rn(dBm, dAp), Z = __dmul_rn(dBm, dC0);
+    const double p = __fma_rn(2.0, Y, X), q = __fma_rn(2.0, Y, Z);
+    dL = __fma_rn(3.0, q, X);  // X + 6Y + 3Z
+    dR = __fma_rn(3.0, p, Z);
+    const double a = __dmul_rn(X, tm), b = __dmul_rn(Z, tp);
+    nL = __fma_rn(t0, p, __fma_rn(-2.0 / 3.0, a, b));
+    nR = __fma_rn(t0, q, __fma_rn(-2.0 / 3.0, b, a));
+}
+
+// nl/dl + nr/dr as one fraction.  dl, dr > 0; past 2^460 (jumps beyond 1e17)
+// the products could overflow and the fractions are added apart.
+__device__ __forceinline__ double frac_sum(double nl, double dl, double nr, double dr) {
+    constexpr int kBig = (1023 + 460) << 20;
+    if (__double2hiint(dl) < kBig && __double2hiint(dr) < kBig)
+        return quot_pos(__fma_rn(nl, dr, __dmul_rn(nr, dl)), __dmul_rn(dl, dr));
+    return __dadd_rn(quot_pos(nl, dl), quot_pos(nr, dr));
 }
 
 // Transverse directions of a sweep along d (the first one is x when d != 0,
@@ -744,135 +761,199 @@ __host__ __device__ __forceinline__ int64_t sweep_items(const RhsBox& B, int d, 
     return (int64_t)(B.hi[a] - B.lo[a] + 1) * (B.hi[b] - B.lo[b] + 1) * sweep_nseg(B, d, seg);
 }
 
-// Raw values of one cell for component c: the state and its Euler flux along d.
-__device__ __forceinline__ void sweep_raw(const RhsBox& B, int d, int c, int sc, int64_t os, int64_t ox, double& u,
-                                          double& f) {
-    const Fab& S = B.sb;
-    const Fab& X = B.aux;
-    u = S.p[os + sc * S.ns];
-    const double va = (c >= 1 && c <= 3) ? X.p[ox + (AUX_VX + c - 1) * X.ns] : 0.0;
-    f = euler_flux(c, d, u, S.p[os + RHO * S.ns], va, X.p[ox + (AUX_VX + d) * X.ns], X.p[ox + AUX_PF * X.ns],
-                   S.p[os + RHOE * S.ns]);
+// What the WENO5 flux of component c along d reads and writes, as plain
+// pointers and strides held in registers (the batched launches take the box
+// from device memory, which the stores would have the compiler read again).
+struct Flux5Ctx {
+    const double *u, *m, *v, *p, *vf;  // state component; momentum, velocity along d; pressure; volume fraction
+    const double* fs;                  // face scalars (component stride fns)
+    int64_t fns;
+    double* out;    // flux
+    double* reg;    // flux array of the caller (component 0), or null
+    int64_t rns, rsc;
+    int kind;       // 0 density, 1 energy, 2 momentum along d, 3 other
+    int c;
+    double idx;
+};
+
+__device__ __forceinline__ Flux5Ctx flux5_ctx(const RhsBox& B, int d, int c) {
+    Flux5Ctx x;
+    const Fab &S = B.sb, &X = B.aux, &F = B.fs[d], &O = B.flx[d], &U = B.uflux[d];
+    const int sc = (c < NCONS) ? c : c + (NFLO - NCONS);
+    x.u = S.p + sc * S.ns;
+    x.m = S.p + (RHOU + d) * S.ns;
+    x.vf = S.p + VFRAC * S.ns;
+    x.v = X.p + (AUX_VX + d) * X.ns;
+    x.p = X.p + AUX_PF * X.ns;
+    x.fs = F.p;
+    x.fns = F.ns;
+    x.out = O.p + c * O.ns;
+    x.reg = U.p;
+    x.rns = U.ns;
+    x.rsc = sc * U.ns;
+    x.kind = (c == RHO) ? 0 : (c == RHOE) ? 1 : (c == 1 + d) ? 2 : 3;
+    x.c = c;
+    x.idx = B.idx[d];
+    return x;
+}
+
+// State and Euler flux of one cell (state offset os, scratch offset ox;
+// consprim_funcs.H:48-81 with a unit normal): the density flux is the momentum
+// itself, the others the conserved value times the normal velocity, plus the
+// pressure.
+__device__ __forceinline__ void flux5_cell(const Flux5Ctx& x, int64_t os, int64_t ox, double& u, double& f) {
+    u = x.u[os];
+    if (x.kind == 0)
+        f = x.m[os];
+    else if (x.kind == 1)
+        f = __dmul_rn(__dadd_rn(u, x.p[ox]), x.v[ox]);
+    else if (x.kind == 2)
+        f = __fma_rn(u, x.v[ox], x.p[ox]);
+    else
+        f = __dmul_rn(u, x.v[ox]);
+}
+
+// Local Lax-Friedrichs flux of a regular face from its corrections' fractions
+// (f: of the Euler flux, u: of the state) and fsum = f_L + f_R.
+__device__ __forceinline__ double weno_llf(double lam, double fsum, double nLf, double dLf, double nRf, double dRf,
+                                           double nLu, double dLu, double nRu, double dRu) {
+    const double pf = frac_sum(nLf, dLf, nRf, dRf), pu = frac_sum(nLu, dLu, -nRu, dRu);
+    return __fma_rn(-0.25, __fma_rn(lam, pu, pf), __dmul_rn(0.5, fsum));
 }
 
 // First-order stencil near the immersed boundary (compute_flux_3d.H:233-249):
-// the six cells collapse to (L, L, L, R, R, R).  Both edges then have the
-// indicators 0, (K1 + 1/4) D^2 and (K1 + 9/4) D^2 with D = R - L, hence the
-// same nonlinear weights, and the candidates 6L, 4L + 2R, 2L + 4R (left edge)
-// and their mirror images (right edge).
-__device__ __forceinline__ void weno_collapsed(double L, double R, double& up, double& um) {
-    const double D = __dsub_rn(R, L), D2 = __dmul_rn(D, D);
-    const double s2 = kEpsWeno, s1 = __fma_rn(13.0 / 12.0 + 0.25, D2, kEpsWeno),
-                 s0 = __fma_rn(13.0 / 12.0 + 2.25, D2, kEpsWeno);
-    const double d2 = __dmul_rn(s2, s2), d1 = __dmul_rn(s1, s1), d0 = __dmul_rn(s0, s0);
-    const double e2 = __dmul_rn(d1, d0), e1 = __dmul_rn(6.0, __dmul_rn(d2, d0)), e0 = __dmul_rn(3.0, __dmul_rn(d2, d1));
-    const double r = rcp_pos(__dmul_rn(6.0, __dadd_rn(__dadd_rn(e2, e1), e0)));
-    const double vl1 = __fma_rn(2.0, R, __dmul_rn(4.0, L)), vl0 = __fma_rn(4.0, R, __dmul_rn(2.0, L));
-    const double vr1 = __fma_rn(2.0, L, __dmul_rn(4.0, R)), vr0 = __fma_rn(4.0, L, __dmul_rn(2.0, R));
-    up = __dmul_rn(__fma_rn(e0, vl0, __fma_rn(e1, vl1, __dmul_rn(e2, __dmul_rn(6.0, L)))), r);
-    um = __dmul_rn(__fma_rn(e0, vr0, __fma_rn(e1, vr1, __dmul_rn(e2, __dmul_rn(6.0, R)))), r);
+// the six cells collapse to (L, L, L, R, R, R).  Of the second differences
+// only t_{f-1} = D and t_f = -D with D = R - L remain, both edges have the
+// same weight products, the corrections of the Euler flux cancel and those of
+// the state add up: flux = (f_L + f_R)/2 - lam D (X + 2Y - Z) / (2 (X + 6Y + 3Z)).
+__device__ __forceinline__ double weno_llf_collapsed(double lam, double fsum, double D) {
+    const double D2 = __dmul_rn(D, D);
+    const double sC = __fma_rn(16.0 / 3.0, D2, 4.0 * kEpsWeno), sA = __fma_rn(8.0, D2, sC);
+    const double dB = (4.0 * kEpsWeno) * (4.0 * kEpsWeno), dC = __dmul_rn(sC, sC), dA = __dmul_rn(sA, sA);
+    const double X = __dmul_rn(dC, dA), Y = __dmul_rn(dB, dA), Z = __dmul_rn(dB, dC);
+    const double p = __fma_rn(2.0, Y, X), q = __fma_rn(2.0, Y, Z);
+    const double w = quot_pos(__dsub_rn(p, Z), __fma_rn(3.0, q, X));
+    return __dmul_rn(0.5, __fma_rn(-__dmul_rn(lam, D), w, fsum));
 }
 
-// The four cells of a face's stencil (centres f-2 .. f+1) for the state and
-// for the Euler flux of one component.
-struct WenoWindow {
-    WenoCell u0, u1, u2, u3, f0, f1, f2, f3;
-};
-
-// Flux of component c through one face (the sweep and the per-face form share
-// it, so they agree bitwise): uL/uR and fL/fR are the state and Euler flux of
-// the two cells next to the face, vfL/vfR their volume fractions.
-__device__ __forceinline__ double flux5_face(const RhsBox& B, int d, int c, const Fab& FS, int64_t qf,
-                                             const WenoWindow& w, double uL, double uR, double fL, double fR,
-                                             double vfL, double vfR, bool hyper = true) {
+// Complete flux of one face (the sweep and the per-face form share it, so
+// they agree bitwise), stored: fh is the hyperbolic flux where active, D = u_R
+// - u_L, oL/oR the face's cells, qf, qo, qr its offsets in the face scalars,
+// the flux scratch and the caller's flux array.
+__device__ __forceinline__ void flux5_finish(const Flux5Ctx& x, bool active, double fh, double D, int64_t oL,
+                                             int64_t oR, int64_t qf, int64_t qo, int64_t qr) {
     const DevParams& P = c_P;
-    const int flags = (int)__double_as_longlong(FS.p[qf + FS_FLAGS * FS.ns]);
+    const int c = x.c;
     double F = 0.0;
-    if (hyper && (flags & 1)) {
-        const double lam = FS.p[qf + FS_LAMBDA * FS.ns];
-        double fp, fm, up, um;
-        if (!(flags & 2)) {
-            fp = weno_comb(w.f0.dB, w.f1.dC, w.f2.dA, w.f0.p1, w.f1.p2, w.f2.p3);
-            fm = weno_comb(w.f3.dA, w.f2.dC, w.f1.dB, w.f3.p4, w.f2.p3, w.f1.p2);
-            up = weno_comb(w.u0.dB, w.u1.dC, w.u2.dA, w.u0.p1, w.u1.p2, w.u2.p3);
-            um = weno_comb(w.u3.dA, w.u2.dC, w.u1.dB, w.u3.p4, w.u2.p3, w.u1.p2);
-        } else {
-            weno_collapsed(fL, fR, fp, fm);
-            weno_collapsed(uL, uR, up, um);
-        }
-        const double fh = __fma_rn(0.5, __fma_rn(lam, up, fp), __dmul_rn(0.5, __fma_rn(-lam, um, fm)));
+    if (active) {
         F = (c < NCONS) ? fh : __dmul_rn(P.advect_flag[c - NCONS], fh);
-        if (c >= RHOU && c <= RHOW) F = __dsub_rn(F, FS.p[qf + (FS_VIS + c - 1) * FS.ns]);
+        if (c >= RHOU && c <= RHOW) F = __dsub_rn(F, x.fs[qf + (FS_VIS + c - 1) * x.fns]);
         if (c == RHOE) {
-            F = __dsub_rn(F, FS.p[qf + (FS_VISE + 0) * FS.ns]);
-            F = __dsub_rn(F, FS.p[qf + (FS_VISE + 1) * FS.ns]);
-            F = __dsub_rn(F, FS.p[qf + (FS_VISE + 2) * FS.ns]);
+            F = __dsub_rn(F, x.fs[qf + (FS_VISE + 0) * x.fns]);
+            F = __dsub_rn(F, x.fs[qf + (FS_VISE + 1) * x.fns]);
+            F = __dsub_rn(F, x.fs[qf + (FS_VISE + 2) * x.fns]);
         }
     }
-    if (c == RHOE) F = __dsub_rn(F, FS.p[qf + FS_THERM * FS.ns]);
+    if (c == RHOE) F = __dsub_rn(F, x.fs[qf + FS_THERM * x.fns]);
     if (c >= NCONS) {  // species diffusion (compute_flux_3d.H:425-428)
         const int s = c - NCONS;
         double Dh = P.diff_hm[s];
         if (P.diff_mode[s] != MFG_TRANSPORT_CONST) {  // harmonic mean of gas vf + solid (1 - vf)
             const double g = P.diff_gas[s], so = P.diff_solid[s];
+            const double vfL = x.vf[oL], vfR = x.vf[oR];
             const double dl = __fma_rn(g, vfL, __dmul_rn(so, __dsub_rn(1.0, vfL)));
             const double dr = __fma_rn(g, vfR, __dmul_rn(so, __dsub_rn(1.0, vfR)));
             Dh = __ddiv_rn(__dmul_rn(__dmul_rn(2.0, dl), dr), __dadd_rn(__dadd_rn(dl, dr), 1e-30));
         }
-        F = __fma_rn(-__dmul_rn(Dh, __dsub_rn(uR, uL)), B.idx[d], F);
+        F = __fma_rn(-__dmul_rn(Dh, D), x.idx, F);
     }
-    return F;
-}
-
-__device__ __forceinline__ void flux5_store(const RhsBox& B, int d, int c, int sc, const Idx3& f, double F) {
-    const Fab& O = B.flx[d];
-    O.p[O.off(f.i, f.j, f.k) + c * O.ns] = F;
-    if (B.uflux[d].p) {
-        const Fab& U = B.uflux[d];
-        const int64_t qu = U.off(f.i, f.j, f.k);
-        U.p[qu + sc * U.ns] = F;
+    x.out[qo] = F;
+    if (x.reg) {
+        x.reg[qr + x.rsc] = F;
         if (c == 0)
-            for (int z = NCONS; z < NFLO; ++z) U.p[qu + z * U.ns] = 0.0;
+            for (int z = NCONS; z < NFLO; ++z) x.reg[qr + z * x.rns] = 0.0;
     }
 }
 
 // Per-face form (for launches too small to fill the GPU with column
-// segments): one thread per (face, component) builds the four cells itself.
+// segments): one thread per (face, component) builds its stencil itself.
 __device__ __forceinline__ void flux5_face_body(const RhsBox& B, int d, int c, int64_t t) {
     int len[3];
     for (int e = 0; e < 3; ++e) len[e] = B.hi[e] - B.lo[e] + 1 + (e == d);
     if (t >= (int64_t)len[0] * len[1] * len[2]) return;
     const Idx3 f = delinear(t, B.lo, len);
-    const Fab& S = B.sb;
-    const Fab& X = B.aux;
-    const int sc = (c < NCONS) ? c : c + (NFLO - NCONS);
-    const int64_t sd = (d == 0) ? 1 : (d == 1) ? S.js : S.ks;
-    const int64_t xd = (d == 0) ? 1 : (d == 1) ? X.js : X.ks;
-    const int64_t oR = S.off(f.i, f.j, f.k), xR = X.off(f.i, f.j, f.k);
-    const double* vfp = S.p + VFRAC * S.ns;
-    const Fab& FS = B.fs[d];
-    if (c >= NCONS && c_P.advect_flag[c - NCONS] == 0.0) {  // not advected: diffusion only
-        const WenoWindow w0 = {};
-        const double F = flux5_face(B, d, c, FS, FS.off(f.i, f.j, f.k), w0, S.p[oR - sd + sc * S.ns],
-                                    S.p[oR + sc * S.ns], 0.0, 0.0, vfp[oR - sd], vfp[oR], false);
-        flux5_store(B, d, c, sc, f, F);
-        return;
-    }
-    double ru[6], rf[6];
+    const Flux5Ctx x = flux5_ctx(B, d, c);
+    const int64_t sd = (d == 0) ? 1 : (d == 1) ? B.sb.js : B.sb.ks;
+    const int64_t xd = (d == 0) ? 1 : (d == 1) ? B.aux.js : B.aux.ks;
+    const int64_t oR = B.sb.off(f.i, f.j, f.k), xR = B.aux.off(f.i, f.j, f.k);
+    const int64_t qf = B.fs[d].off(f.i, f.j, f.k);
+    const bool advected = c < NCONS || c_P.advect_flag[c - NCONS] != 0.0;  // else diffusion only
+    const int flags = advected ? (int)__double_as_longlong(x.fs[qf + FS_FLAGS * x.fns]) & 3 : 0;
+    double fh = 0.0, D;
+    if (flags == 1) {
+        double ru[6], rf[6];
 #pragma unroll
-    for (int q = 0; q < 6; ++q) sweep_raw(B, d, c, sc, oR + (q - 3) * sd, xR + (q - 3) * xd, ru[q], rf[q]);
-    WenoWindow w;
-    w.u0 = weno_cell(ru[0], ru[1], ru[2]);
-    w.u1 = weno_cell(ru[1], ru[2], ru[3]);
-    w.u2 = weno_cell(ru[2], ru[3], ru[4]);
-    w.u3 = weno_cell(ru[3], ru[4], ru[5]);
-    w.f0 = weno_cell(rf[0], rf[1], rf[2]);
-    w.f1 = weno_cell(rf[1], rf[2], rf[3]);
-    w.f2 = weno_cell(rf[2], rf[3], rf[4]);
-    w.f3 = weno_cell(rf[3], rf[4], rf[5]);
-    const double F = flux5_face(B, d, c, FS, FS.off(f.i, f.j, f.k), w, ru[2], ru[3], rf[2], rf[3], vfp[oR - sd],
-                                vfp[oR]);
-    flux5_store(B, d, c, sc, f, F);
+        for (int q = 0; q < 6; ++q) flux5_cell(x, oR + (q - 3) * sd, xR + (q - 3) * xd, ru[q], rf[q]);
+        double n[2][2], e[2][2];  // fractions nL/dL, nR/dR of the flux and of the state
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const double* r = h ? ru : rf;
+            double dd[5];
+#pragma unroll
+            for (int q = 0; q < 5; ++q) dd[q] = __dsub_rn(r[q + 1], r[q]);
+            const WenoCtr c0 = weno_ctr(dd[0], dd[1]), c1 = weno_ctr(dd[1], dd[2]), c2 = weno_ctr(dd[2], dd[3]),
+                          c3 = weno_ctr(dd[3], dd[4]);
+            double un, ud;
+            weno_pair(c0.t, c0.dB, c1.t, c1.dC, c2.t, c2.dA, n[h][0], e[h][0], un, ud);
+            weno_pair(c1.t, c1.dB, c2.t, c2.dC, c3.t, c3.dA, un, ud, n[h][1], e[h][1]);
+            if (h) D = dd[2];
+        }
+        fh = weno_llf(x.fs[qf + FS_LAMBDA * x.fns], __dadd_rn(rf[2], rf[3]), n[0][0], e[0][0], n[0][1], e[0][1],
+                      n[1][0], e[1][0], n[1][1], e[1][1]);
+    } else if (flags & 1) {
+        double uL, uR, fL, fR;
+        flux5_cell(x, oR - sd, xR - xd, uL, fL);
+        flux5_cell(x, oR, xR, uR, fR);
+        D = __dsub_rn(uR, uL);
+        fh = weno_llf_collapsed(x.fs[qf + FS_LAMBDA * x.fns], __dadd_rn(fL, fR), D);
+    } else {
+        D = __dsub_rn(x.u[oR], x.u[oR - sd]);
+    }
+    flux5_finish(x, flags & 1, fh, D, oR - sd, oR, qf, B.flx[d].off(f.i, f.j, f.k),
+                 x.reg ? B.uflux[d].off(f.i, f.j, f.k) : 0);
+}
+
+// Carried from face to face for one of the two reconstructed quantities (the
+// state or its Euler flux): v0, v1 = cells f, f+1; D = v1 - v0; centres f-1
+// (t, dB) and f (t, dB, dC); the left edge's fraction of this face.
+struct WenoRun {
+    double v0, v1, D;
+    double tm, dBm, t0, dB0, dC0, nL, dL;
+};
+
+// Starts the run at face f: va .. vL = cells f-3, f-2, f-1.
+__device__ __forceinline__ void weno_prime(WenoRun& r, double va, double vb, double vL) {
+    const double d0 = __dsub_rn(vb, va), d1 = __dsub_rn(vL, vb), d2 = __dsub_rn(r.v0, vL);
+    const WenoCtr c0 = weno_ctr(d0, d1), c1 = weno_ctr(d1, d2), c2 = weno_ctr(d2, r.D);
+    double un, ud;
+    weno_pair(c0.t, c0.dB, c1.t, c1.dC, c2.t, c2.dA, r.nL, r.dL, un, ud);
+    r.tm = c1.t;
+    r.dBm = c1.dB;
+    r.t0 = c2.t;
+    r.dB0 = c2.dB;
+    r.dC0 = c2.dC;
+}
+
+// Adds centre f+1 (Dn = v_{f+2} - v_{f+1}): the right edge's fraction of face
+// f, and the state of the run moved to face f+1.
+__device__ __forceinline__ void weno_next(WenoRun& r, double Dn, double& nR, double& dR) {
+    const WenoCtr c = weno_ctr(r.D, Dn);
+    weno_pair(r.tm, r.dBm, r.t0, r.dC0, c.t, c.dA, r.nL, r.dL, nR, dR);
+    r.tm = r.t0;
+    r.dBm = r.dB0;
+    r.t0 = c.t;
+    r.dB0 = c.dB;
+    r.dC0 = c.dC;
 }
 
 __device__ __forceinline__ void flux5_sweep_body(const RhsBox& B, int d, int c, int64_t t, int seglen = SWEEP_SEG) {
@@ -889,91 +970,76 @@ __device__ __forceinline__ void flux5_sweep_body(const RhsBox& B, int d, int c, 
     const int f0 = B.lo[d] + seg * per;
     const int f1 = min(B.lo[d] + nf - 1, f0 + per - 1);
     if (f0 > f1) return;
-    int iv[3];
-    iv[ta] = B.lo[ta] + (int)(col % na);
-    iv[tb] = B.lo[tb] + (int)(col / na);
-    iv[d] = f0;
-    const Fab& S = B.sb;
-    const Fab& X = B.aux;
-    const Fab& FS = B.fs[d];
-    const int sc = (c < NCONS) ? c : c + (NFLO - NCONS);
-    const int64_t sd = (d == 0) ? 1 : (d == 1) ? S.js : S.ks;
-    const int64_t xd = (d == 0) ? 1 : (d == 1) ? X.js : X.ks;
-    const int64_t fd = (d == 0) ? 1 : (d == 1) ? FS.js : FS.ks;
-    int64_t oR = S.off(iv[0], iv[1], iv[2]);  // right cell of the current face
-    int64_t xR = X.off(iv[0], iv[1], iv[2]);
-    int64_t qf = FS.off(iv[0], iv[1], iv[2]);
-    const double* vfp = S.p + VFRAC * S.ns;
+    const int ia = B.lo[ta] + (int)(col % na), ib = B.lo[tb] + (int)(col / na);
+    const int i = (d == 0) ? f0 : ia, j = (d == 0) ? ia : (d == 1) ? f0 : ib, k = (d == 2) ? f0 : ib;
+    const Flux5Ctx x = flux5_ctx(B, d, c);
+    const int64_t sd = (d == 0) ? 1 : (d == 1) ? B.sb.js : B.sb.ks;
+    const int64_t xd = (d == 0) ? 1 : (d == 1) ? B.aux.js : B.aux.ks;
+    // the face scalars and the flux scratch have the same extents
+    const int64_t fd = (d == 0) ? 1 : (d == 1) ? B.fs[d].js : B.fs[d].ks;
+    const int64_t rd = (d == 0) ? 1 : (d == 1) ? B.uflux[d].js : B.uflux[d].ks;
+    int64_t oR = B.sb.off(i, j, k);  // right cell of the current face
+    int64_t xR = B.aux.off(i, j, k);
+    int64_t qf = B.fs[d].off(i, j, k);
+    int64_t qr = x.reg ? B.uflux[d].off(i, j, k) : 0;
     if (c >= NCONS && c_P.advect_flag[c - NCONS] == 0.0) {  // not advected: diffusion only
-        const WenoWindow w0 = {};
-        for (int f = f0; f <= f1; ++f, oR += sd, qf += fd, ++iv[d]) {
-            const double F = flux5_face(B, d, c, FS, qf, w0, S.p[oR - sd + sc * S.ns], S.p[oR + sc * S.ns], 0.0, 0.0,
-                                        vfp[oR - sd], vfp[oR], false);
-            Idx3 fi;
-            fi.i = iv[0];
-            fi.j = iv[1];
-            fi.k = iv[2];
-            flux5_store(B, d, c, sc, fi, F);
-        }
+        for (int fc = f0; fc <= f1; ++fc, oR += sd, qf += fd, qr += rd)
+            flux5_finish(x, false, 0.0, __dsub_rn(x.u[oR], x.u[oR - sd]), oR - sd, oR, qf, qf, qr);
         return;
     }
-    // raw values of cells f-3 .. f+2; the per-cell WENO parts of the four
-    // stencil centres f-2 .. f+1 are built only when a face needs them: faces
-    // on the solid side of the immersed boundary (no hyperbolic flux) and
-    // first-order fallback faces use the raw values alone, so columns through
-    // solid regions skip the reconstruction's per-cell work (bitwise the same
-    // numbers: each centre is the same weno_cell of the same three values)
-    double ru[6], rf[6];
-#pragma unroll
-    for (int q = 0; q < 6; ++q) sweep_raw(B, d, c, sc, oR + (q - 3) * sd, xR + (q - 3) * xd, ru[q], rf[q]);
-    WenoWindow w;
-    unsigned have = 0;  // bit q: centre f-2+q built
-    for (int f = f0;; ++f) {
-        const int flags = (int)__double_as_longlong(FS.p[qf + FS_FLAGS * FS.ns]);
-        if ((flags & 3) == 1) {
-            if (!(have & 1u)) {
-                w.u0 = weno_cell(ru[0], ru[1], ru[2]);
-                w.f0 = weno_cell(rf[0], rf[1], rf[2]);
+    // Cells f-1 .. f+1 to start with; the WENO parts are built only when a
+    // face needs them: faces on the solid side of the immersed boundary (no
+    // hyperbolic flux) and first-order fallback faces use the cell values
+    // alone, and the run starts again (three centres) at the next regular face.
+    WenoRun u, f;
+    double uL, fL;
+    flux5_cell(x, oR - sd, xR - xd, uL, fL);
+    flux5_cell(x, oR, xR, u.v0, f.v0);
+    flux5_cell(x, oR + sd, xR + xd, u.v1, f.v1);
+    double Du = __dsub_rn(u.v0, uL);  // u_f - u_{f-1}
+    u.D = __dsub_rn(u.v1, u.v0);
+    f.D = __dsub_rn(f.v1, f.v0);
+    bool primed = false;
+    for (int fc = f0;; ++fc) {
+        double un, fn;  // cell f+2, loaded before this face's arithmetic
+        flux5_cell(x, oR + 2 * sd, xR + 2 * xd, un, fn);
+        const int flags = (int)__double_as_longlong(x.fs[qf + FS_FLAGS * x.fns]) & 3;
+        const double Dun = __dsub_rn(un, u.v1), Dfn = __dsub_rn(fn, f.v1);
+        double fh = 0.0;
+        if (flags == 1) {
+            if (!primed) {
+                double ua, fa, ub, fb;
+                flux5_cell(x, oR - 3 * sd, xR - 3 * xd, ua, fa);
+                flux5_cell(x, oR - 2 * sd, xR - 2 * xd, ub, fb);
+                weno_prime(u, ua, ub, uL);
+                weno_prime(f, fa, fb, fL);
+                primed = true;
             }
-            if (!(have & 2u)) {
-                w.u1 = weno_cell(ru[1], ru[2], ru[3]);
-                w.f1 = weno_cell(rf[1], rf[2], rf[3]);
-            }
-            if (!(have & 4u)) {
-                w.u2 = weno_cell(ru[2], ru[3], ru[4]);
-                w.f2 = weno_cell(rf[2], rf[3], rf[4]);
-            }
-            if (!(have & 8u)) {
-                w.u3 = weno_cell(ru[3], ru[4], ru[5]);
-                w.f3 = weno_cell(rf[3], rf[4], rf[5]);
-            }
-            have = 15u;
+            const double nLu = u.nL, dLu = u.dL, nLf = f.nL, dLf = f.dL;
+            double nRu, dRu, nRf, dRf;
+            weno_next(f, Dfn, nRf, dRf);
+            weno_next(u, Dun, nRu, dRu);
+            fh = weno_llf(x.fs[qf + FS_LAMBDA * x.fns], __dadd_rn(fL, f.v0), nLf, dLf, nRf, dRf, nLu, dLu, nRu, dRu);
+        } else {
+            primed = false;
+            if (flags & 1) fh = weno_llf_collapsed(x.fs[qf + FS_LAMBDA * x.fns], __dadd_rn(fL, f.v0), Du);
         }
-        const double F = flux5_face(B, d, c, FS, qf, w, ru[2], ru[3], rf[2], rf[3], vfp[oR - sd], vfp[oR]);
-        Idx3 fi;
-        fi.i = iv[0];
-        fi.j = iv[1];
-        fi.k = iv[2];
-        flux5_store(B, d, c, sc, fi, F);
-        if (f == f1) break;
-        // advance one face: load cell f+3, shift the window
-        ++iv[d];
+        flux5_finish(x, flags & 1, fh, Du, oR - sd, oR, qf, qf, qr);
+        if (fc == f1) break;
+        // advance one face
         oR += sd;
         xR += xd;
         qf += fd;
-#pragma unroll
-        for (int q = 0; q < 5; ++q) {
-            ru[q] = ru[q + 1];
-            rf[q] = rf[q + 1];
-        }
-        sweep_raw(B, d, c, sc, oR + 2 * sd, xR + 2 * xd, ru[5], rf[5]);
-        w.u0 = w.u1;
-        w.u1 = w.u2;
-        w.u2 = w.u3;
-        w.f0 = w.f1;
-        w.f1 = w.f2;
-        w.f2 = w.f3;
-        have = (have >> 1) & 7u;
+        qr += rd;
+        uL = u.v0;
+        fL = f.v0;
+        Du = u.D;
+        u.v0 = u.v1;
+        f.v0 = f.v1;
+        u.v1 = un;
+        f.v1 = fn;
+        u.D = Dun;
+        f.D = Dfn;
     }
 }
 
