@@ -99,14 +99,16 @@ __global__ void __launch_bounds__(TPB) flux_kernel(RhsBox B, int d) {
     flux_body<FAST>(B, d, blockIdx.y, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 constexpr int SWEEP_TPB = 128;
-// Four blocks per SM (128 registers, 20 bytes spilled): the dependent FP64
-// chains of 16 warps keep the FP64 pipe busier than those of 12 (146
-// registers): 42.3 against 43.0 ms per 128^3 Taylor-Green step.
+// Four blocks per SM (128 registers, 20 bytes spilled): 16 warps keep the FP64
+// and integer pipes busier than 12 (168 registers): 24.6 against 25.7 ms per
+// 128^3 Taylor-Green step.
 __global__ void __launch_bounds__(SWEEP_TPB, 4) flux5_sweep_kernel(RhsBox B, int d, int seg) {
-    flux5_sweep_body(B, d, blockIdx.y, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, seg);
+    const Fp fp;
+    flux5_sweep_body(fp, B, d, blockIdx.y, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, seg);
 }
 __global__ void __launch_bounds__(SWEEP_TPB, 2) flux5_face_kernel(RhsBox B, int d) {
-    flux5_face_body(B, d, blockIdx.y, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
+    const Fp fp;
+    flux5_face_body(fp, B, d, blockIdx.y, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 // One box's column segments must fill the GPU: segments of 32, 16 or 8 faces
 // (longer ones share more per-cell work), else the per-face form of the same

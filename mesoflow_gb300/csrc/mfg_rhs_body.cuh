@@ -5,6 +5,7 @@
 #pragma once
 #include "mfg_internal.h"
 #include "mfg_physics.cuh"
+#include "mfg_weno_weights.cuh"
 
 namespace mfg {
 namespace {
@@ -665,82 +666,53 @@ __device__ __forceinline__ void update_body(const RhsBox& B, int stage, double d
 // one thread walks a segment of faces along d for one component, keeping the
 // per-cell parts of the reconstruction in registers.  FP64 issue bounds it
 // (GB300 issues 2 FP64 operations per SM and cycle), so the form below is the
-// one with the fewest FP64 operations: about 75 per (face, component).
+// one with the fewest FP64 operations, about 23 per (face, component).
 //
 // The WENO5-JS edges (flux_schemes.H:373-446) in second differences.  With
 // cell differences D and t_m = v_{m-1} - 2 v_m + v_{m+1}, the linear weights
 // 1 : 6 : 3 and the nonlinear weights w2 + w1 + w0 = 1, both edges of face f
-// are the mean of its two cells less a correction,
-//   left  = (v_{f-1} + v_f)/2 - (w2 (3 t_{f-1} - 2 t_{f-2}) + w1 t_{f-1} + w0 t_f)/6,
+// are the mean of its two cells less a sixth of a correction,
+//   left  P = w2 (3 t_{f-1} - 2 t_{f-2}) + w1 t_{f-1} + w0 t_f
+//           = t_{f-1} + 2 w2 (t_{f-1} - t_{f-2}) + w0 (t_f - t_{f-1}),
 //   right = the same mirrored,
 // (each candidate polynomial written about the mean, with w2 + w1 + w0 = 1),
 // so the local Lax-Friedrichs flux needs the fluxes' mean and the corrections
 // only: the state's mean cancels.  Rounding errors of the reconstruction then
-// scale with the differences instead of the values (three to five times
-// smaller against 80-bit arithmetic than the candidate form on smooth, noisy
-// and discontinuous data).
-//   Indicators: with D-, D+ the differences on both sides of a cell, t = D+ -
-// D-, q = D+ + D-, four times eps + beta is s_C = 4 eps + (13/3) t^2 + q^2
-// for the central candidate and s_A = s_C - 8 t D-, s_B = s_C + 8 t D+ for the
-// one-sided ones (the squares' differences factor; the cancellation is mild,
-// s_C <= 2.2 s_A and 2.2 s_B).  Scaling all of them by 4 leaves the weights.
+// scale with the differences instead of the values (two to five times smaller
+// against 80-bit arithmetic than the candidate form on smooth, noisy and
+// discontinuous data).
 //   The right edge of face m and the left edge of face m + 1 lie in cell m and
-// see the same five cells, so they share the three weight products
-//   X = C_m A_{m+1}, Y = B_{m-1} A_{m+1}, Z = B_{m-1} C_m   (A, B, C = s^2):
-// left edge: numerator X (3 t_m - 2 t_{m-1}) + 6 Y t_m + 3 Z t_{m+1} over
-// X + 6 Y + 3 Z, right edge with X and Z and the neighbours exchanged.
-//   The two corrections of a face are added as one fraction (one division for
-// the fluxes, one for the states).
-// 64^3 box, 10 components: 1.29 ms of fluxes per right-hand side, against
-// 2.34 ms in the candidate form (130 FP64 operations per face and component,
-// one division per edge).
+// see the same five cells, so they share the products of their weights.
+//   The weights are ratios of positive numbers: mfg_weno_weights.cuh forms
+// them in 64-bit fixed point on the integer pipe (560 cycles per warp, cell
+// and quantity, in the shadow of about 800 on the FP64 pipe).
+// Fluxes of a 64^3 box with 10 components, per right-hand side: 2.34 ms in the
+// candidate form (130 FP64 operations per face and component, one division per
+// edge), 1.29 ms in second differences with FP64 weights (75 operations),
+// 0.57 ms with the fixed-point weights (23 operations).
 // ---------------------------------------------------------------------------
 constexpr int SWEEP_SEG = 32;  // longest face segment per thread (batched launches)
 
-// Per stencil centre: the second difference and the three (4 (eps + beta))^2.
-struct WenoCtr {
-    double t, dA, dB, dC;
+// FP64 sums and products as fused multiply-adds with 1 and -0 in registers:
+// bitwise the add and the multiply, at the fused multiply-add's rate (a warp
+// holds the FP64 pipe for 70 cycles; DADD and DMUL, and fused multiply-adds
+// with an operand from the constant bank or an immediate, for 82).  The two
+// constants pass through a shuffle so that they stay in registers; every lane
+// of the warp constructs it.
+struct Fp {
+    double one, nz;
+    __device__ __forceinline__ Fp() {
+        one = __hiloint2double(__shfl_sync(0xffffffffu, 0x3ff00000, 0), 0);
+        nz = __hiloint2double(__shfl_sync(0xffffffffu, (int)0x80000000, 0), 0);
+    }
+    __device__ __forceinline__ double add(double a, double b) const { return __fma_rn(a, one, b); }
+    __device__ __forceinline__ double sub(double a, double b) const { return __fma_rn(b, -one, a); }
+    __device__ __forceinline__ double mul(double a, double b) const { return __fma_rn(a, b, nz); }
 };
 
-// The sweep and the per-face form must round identically, so every operation
-// of the per-cell and per-face parts is an explicit intrinsic (the compiler
-// may neither contract nor reorder them differently in the two contexts).
-__device__ __forceinline__ WenoCtr weno_ctr(double Dm, double Dp) {
-    WenoCtr r;
-    r.t = __dsub_rn(Dp, Dm);
-    const double q = __dadd_rn(Dp, Dm);
-    const double kte = __fma_rn(__dmul_rn(13.0 / 3.0, r.t), r.t, 4.0 * kEpsWeno);
-    const double sC = __fma_rn(q, q, kte);
-    const double t8 = __dmul_rn(8.0, r.t);
-    const double sA = __fma_rn(-t8, Dm, sC);
-    const double sB = __fma_rn(t8, Dp, sC);
-    r.dA = __dmul_rn(sA, sA);
-    r.dB = __dmul_rn(sB, sB);
-    r.dC = __dmul_rn(sC, sC);
-    return r;
-}
-
-// The corrections' fractions (a third of the numerators) of the two edges in
-// cell m from the centres m-1 (t, dB), m (t, dC), m+1 (t, dA): nL / dL of the
-// left edge of face m+1, nR / dR of the right edge of face m.
-__device__ __forceinline__ void weno_pair(double tm, double dBm, double t0, double dC0, double tp, double dAp,
-                                          double& nL, double& dL, double& nR, double& dR) {
-    const double X = __dmul_rn(dC0, dAp), Y = __dmul_rn(dBm, dAp), Z = __dmul_rn(dBm, dC0);
-    const double p = __fma_rn(2.0, Y, X), q = __fma_rn(2.0, Y, Z);
-    dL = __fma_rn(3.0, q, X);  // X + 6Y + 3Z
-    dR = __fma_rn(3.0, p, Z);
-    const double a = __dmul_rn(X, tm), b = __dmul_rn(Z, tp);
-    nL = __fma_rn(t0, p, __fma_rn(-2.0 / 3.0, a, b));
-    nR = __fma_rn(t0, q, __fma_rn(-2.0 / 3.0, b, a));
-}
-
-// nl/dl + nr/dr as one fraction.  dl, dr > 0; past 2^460 (jumps beyond 1e17)
-// the products could overflow and the fractions are added apart.
-__device__ __forceinline__ double frac_sum(double nl, double dl, double nr, double dr) {
-    constexpr int kBig = (1023 + 460) << 20;
-    if (__double2hiint(dl) < kBig && __double2hiint(dr) < kBig)
-        return quot_pos(__fma_rn(nl, dr, __dmul_rn(nr, dl)), __dmul_rn(dl, dr));
-    return __dadd_rn(quot_pos(nl, dl), quot_pos(nr, dr));
+__device__ __forceinline__ double weight_of(uint64_t bits) { return __longlong_as_double((long long)bits); }
+__device__ __forceinline__ WenoInd weno_ind(double Dm, double Dp) {
+    return weno_ind(weno_diff((uint64_t)__double_as_longlong(Dm)), weno_diff((uint64_t)__double_as_longlong(Dp)));
 }
 
 // Transverse directions of a sweep along d (the first one is x when d != 0,
@@ -801,24 +773,25 @@ __device__ __forceinline__ Flux5Ctx flux5_ctx(const RhsBox& B, int d, int c) {
 // consprim_funcs.H:48-81 with a unit normal): the density flux is the momentum
 // itself, the others the conserved value times the normal velocity, plus the
 // pressure.
-__device__ __forceinline__ void flux5_cell(const Flux5Ctx& x, int64_t os, int64_t ox, double& u, double& f) {
+__device__ __forceinline__ void flux5_cell(const Fp& fp, const Flux5Ctx& x, int64_t os, int64_t ox, double& u,
+                                           double& f) {
     u = x.u[os];
     if (x.kind == 0)
         f = x.m[os];
     else if (x.kind == 1)
-        f = __dmul_rn(__dadd_rn(u, x.p[ox]), x.v[ox]);
+        f = fp.mul(fp.add(u, x.p[ox]), x.v[ox]);
     else if (x.kind == 2)
         f = __fma_rn(u, x.v[ox], x.p[ox]);
     else
-        f = __dmul_rn(u, x.v[ox]);
+        f = fp.mul(u, x.v[ox]);
 }
 
-// Local Lax-Friedrichs flux of a regular face from its corrections' fractions
-// (f: of the Euler flux, u: of the state) and fsum = f_L + f_R.
-__device__ __forceinline__ double weno_llf(double lam, double fsum, double nLf, double dLf, double nRf, double dRf,
-                                           double nLu, double dLu, double nRu, double dRu) {
-    const double pf = frac_sum(nLf, dLf, nRf, dRf), pu = frac_sum(nLu, dLu, -nRu, dRu);
-    return __fma_rn(-0.25, __fma_rn(lam, pu, pf), __dmul_rn(0.5, fsum));
+// Local Lax-Friedrichs flux of a regular face from the corrections of its two
+// edges (f: of the Euler flux, u: of the state) and fsum = f_L + f_R.
+__device__ __forceinline__ double weno_llf(const Fp& fp, double lam, double fsum, double pLf, double pRf, double pLu,
+                                           double pRu) {
+    const double S = __fma_rn(lam, fp.sub(pLu, pRu), fp.add(pLf, pRf));
+    return __fma_rn(-1.0 / 12.0, S, __dmul_rn(0.5, fsum));
 }
 
 // First-order stencil near the immersed boundary (compute_flux_3d.H:233-249):
@@ -840,21 +813,21 @@ __device__ __forceinline__ double weno_llf_collapsed(double lam, double fsum, do
 // they agree bitwise), stored: fh is the hyperbolic flux where active, D = u_R
 // - u_L, oL/oR the face's cells, qf, qo, qr its offsets in the face scalars,
 // the flux scratch and the caller's flux array.
-__device__ __forceinline__ void flux5_finish(const Flux5Ctx& x, bool active, double fh, double D, int64_t oL,
-                                             int64_t oR, int64_t qf, int64_t qo, int64_t qr) {
+__device__ __forceinline__ void flux5_finish(const Fp& fp, const Flux5Ctx& x, bool active, double fh, double D,
+                                             int64_t oL, int64_t oR, int64_t qf, int64_t qo, int64_t qr) {
     const DevParams& P = c_P;
     const int c = x.c;
     double F = 0.0;
     if (active) {
         F = (c < NCONS) ? fh : __dmul_rn(P.advect_flag[c - NCONS], fh);
-        if (c >= RHOU && c <= RHOW) F = __dsub_rn(F, x.fs[qf + (FS_VIS + c - 1) * x.fns]);
+        if (c >= RHOU && c <= RHOW) F = fp.sub(F, x.fs[qf + (FS_VIS + c - 1) * x.fns]);
         if (c == RHOE) {
-            F = __dsub_rn(F, x.fs[qf + (FS_VISE + 0) * x.fns]);
-            F = __dsub_rn(F, x.fs[qf + (FS_VISE + 1) * x.fns]);
-            F = __dsub_rn(F, x.fs[qf + (FS_VISE + 2) * x.fns]);
+            F = fp.sub(F, x.fs[qf + (FS_VISE + 0) * x.fns]);
+            F = fp.sub(F, x.fs[qf + (FS_VISE + 1) * x.fns]);
+            F = fp.sub(F, x.fs[qf + (FS_VISE + 2) * x.fns]);
         }
     }
-    if (c == RHOE) F = __dsub_rn(F, x.fs[qf + FS_THERM * x.fns]);
+    if (c == RHOE) F = fp.sub(F, x.fs[qf + FS_THERM * x.fns]);
     if (c >= NCONS) {  // species diffusion (compute_flux_3d.H:425-428)
         const int s = c - NCONS;
         double Dh = P.diff_hm[s];
@@ -865,7 +838,7 @@ __device__ __forceinline__ void flux5_finish(const Flux5Ctx& x, bool active, dou
             const double dr = __fma_rn(g, vfR, __dmul_rn(so, __dsub_rn(1.0, vfR)));
             Dh = __ddiv_rn(__dmul_rn(__dmul_rn(2.0, dl), dr), __dadd_rn(__dadd_rn(dl, dr), 1e-30));
         }
-        F = __fma_rn(-__dmul_rn(Dh, D), x.idx, F);
+        F = __fma_rn(-fp.mul(Dh, D), x.idx, F);
     }
     x.out[qo] = F;
     if (x.reg) {
@@ -877,7 +850,7 @@ __device__ __forceinline__ void flux5_finish(const Flux5Ctx& x, bool active, dou
 
 // Per-face form (for launches too small to fill the GPU with column
 // segments): one thread per (face, component) builds its stencil itself.
-__device__ __forceinline__ void flux5_face_body(const RhsBox& B, int d, int c, int64_t t) {
+__device__ __forceinline__ void flux5_face_body(const Fp& fp, const RhsBox& B, int d, int c, int64_t t) {
     int len[3];
     for (int e = 0; e < 3; ++e) len[e] = B.hi[e] - B.lo[e] + 1 + (e == d);
     if (t >= (int64_t)len[0] * len[1] * len[2]) return;
@@ -893,70 +866,88 @@ __device__ __forceinline__ void flux5_face_body(const RhsBox& B, int d, int c, i
     if (flags == 1) {
         double ru[6], rf[6];
 #pragma unroll
-        for (int q = 0; q < 6; ++q) flux5_cell(x, oR + (q - 3) * sd, xR + (q - 3) * xd, ru[q], rf[q]);
-        double n[2][2], e[2][2];  // fractions nL/dL, nR/dR of the flux and of the state
+        for (int q = 0; q < 6; ++q) flux5_cell(fp, x, oR + (q - 3) * sd, xR + (q - 3) * xd, ru[q], rf[q]);
+        double pL[2], pR[2];  // corrections of the flux and of the state
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const double* r = h ? ru : rf;
-            double dd[5];
+            double dd[5], tt[4];
 #pragma unroll
-            for (int q = 0; q < 5; ++q) dd[q] = __dsub_rn(r[q + 1], r[q]);
-            const WenoCtr c0 = weno_ctr(dd[0], dd[1]), c1 = weno_ctr(dd[1], dd[2]), c2 = weno_ctr(dd[2], dd[3]),
-                          c3 = weno_ctr(dd[3], dd[4]);
-            double un, ud;
-            weno_pair(c0.t, c0.dB, c1.t, c1.dC, c2.t, c2.dA, n[h][0], e[h][0], un, ud);
-            weno_pair(c1.t, c1.dB, c2.t, c2.dC, c3.t, c3.dA, un, ud, n[h][1], e[h][1]);
+            for (int q = 0; q < 5; ++q) dd[q] = fp.sub(r[q + 1], r[q]);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) tt[q] = fp.sub(dd[q + 1], dd[q]);
+            const double g0 = fp.sub(tt[1], tt[0]), g1 = fp.sub(tt[2], tt[1]), g2 = fp.sub(tt[3], tt[2]);
+            const WenoInd i0 = weno_ind(dd[0], dd[1]), i1 = weno_ind(dd[1], dd[2]), i2 = weno_ind(dd[2], dd[3]),
+                          i3 = weno_ind(dd[3], dd[4]);
+            const WenoWeights wl = weno_weights(i0.dB, i0.eB, i1.dC, i1.eC, i2.dA, i2.eA);
+            const WenoWeights wr = weno_weights(i1.dB, i1.eB, i2.dC, i2.eC, i3.dA, i3.eA);
+            pL[h] = __fma_rn(weight_of(wl.nearL), g1, __fma_rn(weight_of(wl.farL2), g0, tt[1]));
+            pR[h] = __fma_rn(-weight_of(wr.nearR), g1, __fma_rn(-weight_of(wr.farR2), g2, tt[2]));
             if (h) D = dd[2];
         }
-        fh = weno_llf(x.fs[qf + FS_LAMBDA * x.fns], __dadd_rn(rf[2], rf[3]), n[0][0], e[0][0], n[0][1], e[0][1],
-                      n[1][0], e[1][0], n[1][1], e[1][1]);
+        fh = weno_llf(fp, x.fs[qf + FS_LAMBDA * x.fns], fp.add(rf[2], rf[3]), pL[0], pR[0], pL[1], pR[1]);
     } else if (flags & 1) {
         double uL, uR, fL, fR;
-        flux5_cell(x, oR - sd, xR - xd, uL, fL);
-        flux5_cell(x, oR, xR, uR, fR);
-        D = __dsub_rn(uR, uL);
-        fh = weno_llf_collapsed(x.fs[qf + FS_LAMBDA * x.fns], __dadd_rn(fL, fR), D);
+        flux5_cell(fp, x, oR - sd, xR - xd, uL, fL);
+        flux5_cell(fp, x, oR, xR, uR, fR);
+        D = fp.sub(uR, uL);
+        fh = weno_llf_collapsed(x.fs[qf + FS_LAMBDA * x.fns], fp.add(fL, fR), D);
     } else {
-        D = __dsub_rn(x.u[oR], x.u[oR - sd]);
+        D = fp.sub(x.u[oR], x.u[oR - sd]);
     }
-    flux5_finish(x, flags & 1, fh, D, oR - sd, oR, qf, B.flx[d].off(f.i, f.j, f.k),
+    flux5_finish(fp, x, flags & 1, fh, D, oR - sd, oR, qf, B.flx[d].off(f.i, f.j, f.k),
                  x.reg ? B.uflux[d].off(f.i, f.j, f.k) : 0);
 }
 
 // Carried from face to face for one of the two reconstructed quantities (the
-// state or its Euler flux): v0, v1 = cells f, f+1; D = v1 - v0; centres f-1
-// (t, dB) and f (t, dB, dC); the left edge's fraction of this face.
+// state or its Euler flux): v0, v1 = cells f, f+1; D = v1 - v0; t_f and g =
+// t_f - t_{f-1}; the indicators of the centres f-1 (B) and f (B, C); the left
+// edge's correction at this face.
 struct WenoRun {
     double v0, v1, D;
-    double tm, dBm, t0, dB0, dC0, nL, dL;
+    double t0, g, pL;
+    uint64_t dBm, dB0, dC0;
+    int eBm, eB0, eC0;
 };
 
-// Starts the run at face f: va .. vL = cells f-3, f-2, f-1.
-__device__ __forceinline__ void weno_prime(WenoRun& r, double va, double vb, double vL) {
-    const double d0 = __dsub_rn(vb, va), d1 = __dsub_rn(vL, vb), d2 = __dsub_rn(r.v0, vL);
-    const WenoCtr c0 = weno_ctr(d0, d1), c1 = weno_ctr(d1, d2), c2 = weno_ctr(d2, r.D);
-    double un, ud;
-    weno_pair(c0.t, c0.dB, c1.t, c1.dC, c2.t, c2.dA, r.nL, r.dL, un, ud);
-    r.tm = c1.t;
-    r.dBm = c1.dB;
-    r.t0 = c2.t;
-    r.dB0 = c2.dB;
-    r.dC0 = c2.dC;
-}
-
-// Adds centre f+1 (Dn = v_{f+2} - v_{f+1}): the right edge's fraction of face
-// f, and the state of the run moved to face f+1.
-__device__ __forceinline__ void weno_next(WenoRun& r, double Dn, double& nR, double& dR) {
-    const WenoCtr c = weno_ctr(r.D, Dn);
-    weno_pair(r.tm, r.dBm, r.t0, r.dC0, c.t, c.dA, r.nL, r.dL, nR, dR);
-    r.tm = r.t0;
+// Adds centre f+1 (Dn = v_{f+2} - v_{f+1}): returns the right edge's
+// correction at face f and moves the indicators, t, g and the left edge's
+// correction of the run to face f+1.
+__device__ __forceinline__ double weno_next(const Fp& fp, WenoRun& r, double D, double Dn) {
+    const WenoInd c = weno_ind(D, Dn);
+    const WenoWeights w = weno_weights(r.dBm, r.eBm, r.dC0, r.eC0, c.dA, c.eA);
+    const double t = fp.sub(Dn, D), gp = fp.sub(t, r.t0);
+    r.pL = __fma_rn(weight_of(w.nearL), gp, __fma_rn(weight_of(w.farL2), r.g, r.t0));
+    const double pR = __fma_rn(-weight_of(w.nearR), r.g, __fma_rn(-weight_of(w.farR2), gp, r.t0));
+    r.t0 = t;
+    r.g = gp;
     r.dBm = r.dB0;
-    r.t0 = c.t;
+    r.eBm = r.eB0;
     r.dB0 = c.dB;
+    r.eB0 = c.eB;
     r.dC0 = c.dC;
+    r.eC0 = c.eC;
+    return pR;
 }
 
-__device__ __forceinline__ void flux5_sweep_body(const RhsBox& B, int d, int c, int64_t t, int seglen = SWEEP_SEG) {
+// Starts the run at face f: va .. vL = cells f-3, f-2, f-1.
+__device__ __forceinline__ void weno_prime(const Fp& fp, WenoRun& r, double va, double vb, double vL) {
+    const double d0 = fp.sub(vb, va), d1 = fp.sub(vL, vb), d2 = fp.sub(r.v0, vL);
+    const WenoInd c0 = weno_ind(d0, d1), c1 = weno_ind(d1, d2);
+    const double ta = fp.sub(d1, d0);
+    r.t0 = fp.sub(d2, d1);
+    r.g = fp.sub(r.t0, ta);
+    r.dBm = c0.dB;
+    r.eBm = c0.eB;
+    r.dB0 = c1.dB;
+    r.eB0 = c1.eB;
+    r.dC0 = c1.dC;
+    r.eC0 = c1.eC;
+    weno_next(fp, r, d2, r.D);
+}
+
+__device__ __forceinline__ void flux5_sweep_body(const Fp& fp, const RhsBox& B, int d, int c, int64_t t,
+                                                 int seglen = SWEEP_SEG) {
     if (t >= sweep_items(B, d, seglen)) return;
     int ta, tb;
     sweep_dirs(d, ta, tb);
@@ -984,7 +975,7 @@ __device__ __forceinline__ void flux5_sweep_body(const RhsBox& B, int d, int c, 
     int64_t qr = x.reg ? B.uflux[d].off(i, j, k) : 0;
     if (c >= NCONS && c_P.advect_flag[c - NCONS] == 0.0) {  // not advected: diffusion only
         for (int fc = f0; fc <= f1; ++fc, oR += sd, qf += fd, qr += rd)
-            flux5_finish(x, false, 0.0, __dsub_rn(x.u[oR], x.u[oR - sd]), oR - sd, oR, qf, qf, qr);
+            flux5_finish(fp, x, false, 0.0, fp.sub(x.u[oR], x.u[oR - sd]), oR - sd, oR, qf, qf, qr);
         return;
     }
     // Cells f-1 .. f+1 to start with; the WENO parts are built only when a
@@ -993,38 +984,36 @@ __device__ __forceinline__ void flux5_sweep_body(const RhsBox& B, int d, int c, 
     // alone, and the run starts again (three centres) at the next regular face.
     WenoRun u, f;
     double uL, fL;
-    flux5_cell(x, oR - sd, xR - xd, uL, fL);
-    flux5_cell(x, oR, xR, u.v0, f.v0);
-    flux5_cell(x, oR + sd, xR + xd, u.v1, f.v1);
-    double Du = __dsub_rn(u.v0, uL);  // u_f - u_{f-1}
-    u.D = __dsub_rn(u.v1, u.v0);
-    f.D = __dsub_rn(f.v1, f.v0);
+    flux5_cell(fp, x, oR - sd, xR - xd, uL, fL);
+    flux5_cell(fp, x, oR, xR, u.v0, f.v0);
+    flux5_cell(fp, x, oR + sd, xR + xd, u.v1, f.v1);
+    double Du = fp.sub(u.v0, uL);  // u_f - u_{f-1}
+    u.D = fp.sub(u.v1, u.v0);
+    f.D = fp.sub(f.v1, f.v0);
     bool primed = false;
     for (int fc = f0;; ++fc) {
         double un, fn;  // cell f+2, loaded before this face's arithmetic
-        flux5_cell(x, oR + 2 * sd, xR + 2 * xd, un, fn);
+        flux5_cell(fp, x, oR + 2 * sd, xR + 2 * xd, un, fn);
         const int flags = (int)__double_as_longlong(x.fs[qf + FS_FLAGS * x.fns]) & 3;
-        const double Dun = __dsub_rn(un, u.v1), Dfn = __dsub_rn(fn, f.v1);
+        const double Dun = fp.sub(un, u.v1), Dfn = fp.sub(fn, f.v1);
         double fh = 0.0;
         if (flags == 1) {
             if (!primed) {
                 double ua, fa, ub, fb;
-                flux5_cell(x, oR - 3 * sd, xR - 3 * xd, ua, fa);
-                flux5_cell(x, oR - 2 * sd, xR - 2 * xd, ub, fb);
-                weno_prime(u, ua, ub, uL);
-                weno_prime(f, fa, fb, fL);
+                flux5_cell(fp, x, oR - 3 * sd, xR - 3 * xd, ua, fa);
+                flux5_cell(fp, x, oR - 2 * sd, xR - 2 * xd, ub, fb);
+                weno_prime(fp, u, ua, ub, uL);
+                weno_prime(fp, f, fa, fb, fL);
                 primed = true;
             }
-            const double nLu = u.nL, dLu = u.dL, nLf = f.nL, dLf = f.dL;
-            double nRu, dRu, nRf, dRf;
-            weno_next(f, Dfn, nRf, dRf);
-            weno_next(u, Dun, nRu, dRu);
-            fh = weno_llf(x.fs[qf + FS_LAMBDA * x.fns], __dadd_rn(fL, f.v0), nLf, dLf, nRf, dRf, nLu, dLu, nRu, dRu);
+            const double pLu = u.pL, pLf = f.pL;
+            const double pRf = weno_next(fp, f, f.D, Dfn), pRu = weno_next(fp, u, u.D, Dun);
+            fh = weno_llf(fp, x.fs[qf + FS_LAMBDA * x.fns], fp.add(fL, f.v0), pLf, pRf, pLu, pRu);
         } else {
             primed = false;
-            if (flags & 1) fh = weno_llf_collapsed(x.fs[qf + FS_LAMBDA * x.fns], __dadd_rn(fL, f.v0), Du);
+            if (flags & 1) fh = weno_llf_collapsed(x.fs[qf + FS_LAMBDA * x.fns], fp.add(fL, f.v0), Du);
         }
-        flux5_finish(x, flags & 1, fh, Du, oR - sd, oR, qf, qf, qr);
+        flux5_finish(fp, x, flags & 1, fh, Du, oR - sd, oR, qf, qf, qr);
         if (fc == f1) break;
         // advance one face
         oR += sd;

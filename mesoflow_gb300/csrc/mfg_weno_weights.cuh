@@ -1,0 +1,175 @@
+// Nonlinear WENO5-JS weights (flux_schemes.H:373-446) in 64-bit fixed point.
+//
+// GB300 issues 2 FP64 operations per SM and cycle and 64 to 128 integer ones:
+// a warp's FP64 add or multiply holds its scheduler's FP64 pipe for 82 cycles,
+// a fused multiply-add for 70, while the high half of a 64 x 64-bit product
+// takes 18 cycles of the integer pipe, which the order-5 flux kernels leave
+// idle.  The weights are ratios of positive numbers, so they need no signs, no
+// special values and no rounding modes, and fixed point gives them with errors
+// of 2^-50 or less relative to their sum (the FP64 form reached 2^-50 at best,
+// since it formed the indicators from rounded second differences): indicators,
+// squares, products, sums and reciprocals run here, beside the FP64 pipe that
+// forms the differences and applies the weights.
+//
+// Everything is integer arithmetic but the 23-bit seed of the reciprocal, so
+// every kernel that uses it gets the same bits.
+#pragma once
+#include <stdint.h>
+#include <string.h>
+
+#ifdef __CUDACC__
+#define MFG_HD __host__ __device__ __forceinline__
+#else
+#define MFG_HD inline
+#endif
+
+namespace mfg {
+
+MFG_HD uint64_t umulhi64(uint64_t a, uint64_t b) {
+#ifdef __CUDA_ARCH__
+    return __umul64hi(a, b);
+#else
+    return (uint64_t)(((unsigned __int128)a * b) >> 64);
+#endif
+}
+
+MFG_HD int clz32(uint32_t x) {  // x != 0
+#ifdef __CUDA_ARCH__
+    return __clz((int)x);
+#else
+    return __builtin_clz(x);
+#endif
+}
+
+// Bits of the float32 1/f, f in (1, 2), relative error below 2^-22.
+MFG_HD uint32_t rcp_seed_bits(uint32_t fbits) {
+#ifdef __CUDA_ARCH__
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint_as_float(fbits)));
+    return __float_as_uint(r);
+#else
+    float f;
+    memcpy(&f, &fbits, 4);
+    f = 1.0f / f;
+    uint32_t b;
+    memcpy(&b, &f, 4);
+    return b;
+#endif
+}
+
+MFG_HD int imin(int a, int b) { return a < b ? a : b; }
+MFG_HD int imax(int a, int b) { return a > b ? a : b; }
+
+// A cell difference split: |D| = m 2^(e - 1083), 2^60 <= m < 2^61 (zero and
+// denormals read as about 2^-1023, far below the exponent floor).
+struct WenoDiff {
+    uint64_t m;
+    int e;
+    uint32_t sign;  // bit 31
+};
+
+MFG_HD WenoDiff weno_diff(uint64_t bits) {
+    WenoDiff r;
+    const uint32_t hi = (uint32_t)(bits >> 32);
+    r.e = (int)((hi >> 20) & 0x7ffu);
+    r.m = ((bits & 0x000fffffffffffffull) | 0x0010000000000000ull) << 8;
+    r.sign = hi;
+    return r;
+}
+
+// (eps + beta)^2 of a centre's three candidates up to one common factor:
+// normalised 62 to 64-bit mantissas and the exponents of their square roots.
+struct WenoInd {
+    uint64_t dA, dB, dC;
+    int eA, eB, eC;
+};
+
+// Exponent below which differences count as this one (2^-10: their squares are
+// below eps = 1e-6), and 3 eps there in the units of the squares, 2^(2e - 2102).
+constexpr int kWenoExpFloor = 1012;
+constexpr uint64_t kWenoEps3 = 906694364710971881ull;  // 3e-6 * 2^78
+
+// With D-, D+ the differences on both sides of the centre, 3 (eps + beta) is
+// 3 eps + 4 D-^2 - 5 D- D+ + 4 D+^2 for the central candidate and, for the
+// one-sided ones, that plus 6 D- (D- - D+) and 6 D+ (D+ - D-).  All three are
+// at least 0.73 max(D-^2, D+^2), so the fixed point relative to the larger
+// difference keeps them to 2^-50 at worst.
+MFG_HD WenoInd weno_ind(const WenoDiff& a, const WenoDiff& b) {
+    const int E = imax(imax(a.e, b.e), kWenoExpFloor);
+    const uint64_t ma = a.m >> imin(E - a.e, 63), mb = b.m >> imin(E - b.e, 63);
+    const uint64_t E1 = umulhi64(ma, ma), E2 = umulhi64(mb, mb);
+    uint64_t X = umulhi64(ma, mb);
+    if ((a.sign ^ b.sign) >> 31) X = 0 - X;
+    const uint64_t sC = ((E1 + E2) << 2) - 5 * X + (kWenoEps3 >> imin(2 * (E - kWenoExpFloor), 63));
+    const uint64_t sA = sC + 6 * (E1 - X), sB = sC + 6 * (E2 - X);
+    // each is at least 2^55: the high words are not zero
+    const int zA = clz32((uint32_t)(sA >> 32)), zB = clz32((uint32_t)(sB >> 32)), zC = clz32((uint32_t)(sC >> 32));
+    const uint64_t nA = sA << zA, nB = sB << zB, nC = sC << zC;
+    WenoInd r;
+    r.dA = umulhi64(nA, nA);
+    r.dB = umulhi64(nB, nB);
+    r.dC = umulhi64(nC, nC);
+    r.eA = 2 * E - zA;
+    r.eB = 2 * E - zB;
+    r.eC = 2 * E - zC;
+    return r;
+}
+
+// 2^126 / d for a normalised d (top bit set), relative error below 2^-59: the
+// float32 seed r0 (e = 1 - x r0, |e| < 2^-21) corrected by r0 (1 + e + e^2).
+MFG_HD uint64_t rcp_fixed(uint64_t d) {
+    const uint32_t dh = (uint32_t)(d >> 32), dl = (uint32_t)d;
+    uint32_t rb = rcp_seed_bits(0x3f800000u | ((dh & 0x7fffffffu) >> 8) | 1u);
+    rb = rb < 0x3f000000u ? 0x3f000000u : rb > 0x3f7fffffu ? 0x3f7fffffu : rb;  // in [1/2, 1)
+    const uint32_t R0 = ((rb & 0x7fffffu) | 0x800000u) << 7;                     // r0 2^31
+    const uint64_t T = (uint64_t)dh * R0 + (((uint64_t)dl * R0) >> 32);          // (1 - e) 2^62
+    const int64_t e = (int64_t)((1ull << 62) - T);
+    const int32_t es = (int32_t)(e >> 18);
+    const int64_t g = e + (((int64_t)es * es) >> 26);  // (e + e^2) 2^62
+    const int32_t gh = (int32_t)(g >> 32);
+    const uint32_t gl = (uint32_t)g;
+    return ((uint64_t)R0 << 32) + (uint64_t)(((int64_t)gh * (int32_t)R0) << 2) + (((uint64_t)R0 * gl) >> 30);
+}
+
+// w 2^-62 2^k as the bits of a double, truncated (0 reads as 2^(k-62)).
+MFG_HD uint64_t weight_bits(uint64_t w, int k) {
+    uint32_t hi = (uint32_t)(w >> 32), lo = (uint32_t)w | 1u;
+    int e = 1023 + 1 + k;
+    if (hi == 0) {
+        hi = lo;
+        lo = 0;
+        e -= 32;
+    }
+    const int z = clz32(hi);
+    const uint64_t n = (((uint64_t)hi << 32) | lo) << z;  // top bit set: adds one to the exponent below
+    return ((uint64_t)(uint32_t)(e - z - 1) << 52) + (n >> 11);
+}
+
+// Weights of the two edges in cell m from the centres m-1 (dB), m (dC), m+1
+// (dA).  With X = C A, Y = B A, Z = B C the left edge of face m+1 has the
+// weights X, 6 Y, 3 Z over their sum for the far, middle and near candidate,
+// the right edge of face m has Z, 6 Y, 3 X.  Returned: twice the far weight
+// and the near weight of each edge, as double bits.
+struct WenoWeights {
+    uint64_t farL2, nearL, farR2, nearR;
+};
+
+MFG_HD WenoWeights weno_weights(uint64_t dB, int eB, uint64_t dC, int eC, uint64_t dA, int eA) {
+    const int em = imin(imin(eA, eB), eC);
+    // common exponent of the three products; four bits of headroom for the sums
+    const uint64_t X = umulhi64(dC, dA) >> imin(2 * (eB - em) + 4, 63);
+    const uint64_t Y = umulhi64(dB, dA) >> imin(2 * (eC - em) + 4, 63);
+    const uint64_t Z = umulhi64(dB, dC) >> imin(2 * (eA - em) + 4, 63);
+    const uint64_t X3 = 3 * X, Z3 = 3 * Z, Y6 = 6 * Y;
+    const uint64_t sL = X + Y6 + Z3, sR = Z + Y6 + X3;
+    const int zL = clz32((uint32_t)(sL >> 32)), zR = clz32((uint32_t)(sR >> 32));
+    const uint64_t rL = rcp_fixed(sL << zL), rR = rcp_fixed(sR << zR);
+    WenoWeights w;
+    w.farL2 = weight_bits(umulhi64(X << zL, rL), 1);
+    w.nearL = weight_bits(umulhi64(Z3 << zL, rL), 0);
+    w.farR2 = weight_bits(umulhi64(Z << zR, rR), 1);
+    w.nearR = weight_bits(umulhi64(X3 << zR, rR), 0);
+    return w;
+}
+
+}  // namespace mfg
