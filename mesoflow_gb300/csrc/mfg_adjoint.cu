@@ -618,15 +618,16 @@ __global__ void __launch_bounds__(AT) adj_face_kernel(AdjBox A, int d) {
     for (int s = 0; s < NS; ++s) specL[s] = (s < ns) ? S.p[oL + (NFLO + s) * S.ns] : 0.0;
     const double rhoR = S.p[oR + RHO * S.ns];
     const double reigR = X.p[xR + AUX_REIG * X.ns];
-    const double gamR = X.p[xR + AUX_GAM * X.ns];
-    const double pRp = thermo_p<NS>(reigR, rhoR, specL);
+    const double gamR = 1.0 + X.p[xR + AUX_KAP * X.ns];
+    const double kapL = X.p[xL + AUX_KAP * X.ns];
+    const double pRp = kapL * reigR;
     const double qR = (gamR * pRp) / rhoR;
-    const double aR = sqrt(qR);
+    const double aR = eig_speed(gamR, kapL, reigR, rcp_pos(rhoR));  // as the forward face pass
     if (aL >= aR) {
         aadd(&GA.p[xL + AUX_AOWN * GA.ns], lamb);
     } else {
         const double qb = lamb / (2.0 * aR);
-        aadd(&GA.p[xR + AUX_GAM * GA.ns], qb * pRp / rhoR);
+        aadd(&GA.p[xR + AUX_KAP * GA.ns], qb * pRp / rhoR);
         const double pb = qb * gamR / rhoR;
         aadd(&G.p[oR + RHO * G.ns], -qb * qR / rhoR);
         double dpr, dpc[NS];
@@ -687,7 +688,7 @@ __global__ void __launch_bounds__(AT) adj_aux_kernel(AdjBox A) {
 #pragma unroll
     for (int s = 0; s < NS; ++s) sb[s] = 0.0;
     double vb[3] = {ab[AUX_VX], ab[AUX_VY], ab[AUX_VZ]};
-    double gb = ab[AUX_GAM], reb = ab[AUX_REIG];
+    double gb = ab[AUX_KAP], reb = ab[AUX_REIG];
     if (ab[AUX_AOWN] != 0.0) {  // a = sqrt(gamma p_eig / rho)
         const double qb = ab[AUX_AOWN] * (0.5 / aown);
         gb += qb * peig * irho;

@@ -7,7 +7,7 @@
 namespace mfg {
 
 // Per-cell scalars of prim_kernel (scratch over grow(bx, 3)).
-enum AuxComp { AUX_VX = 0, AUX_VY, AUX_VZ, AUX_PF, AUX_REIG, AUX_AOWN, AUX_GAM, NAUX };
+enum AuxComp { AUX_VX = 0, AUX_VY, AUX_VZ, AUX_PF, AUX_REIG, AUX_AOWN, AUX_KAP /* gamma - 1 */, NAUX };
 
 // Per-face scalars of face_kernel (scratch over growHi(bx, d, 1)).
 enum FsComp {
@@ -19,9 +19,9 @@ enum FsComp {
     FS_PL,         // AUSM left pressure
     FS_PR,         // AUSM right pressure
     FS_VIS,        // 3: viscous momentum terms tau_{d,a}
-    FS_VISE = FS_VIS + 3,   // 3: viscous work terms tau_{d,a} * facevel_a
-    FS_THERM = FS_VISE + 3, // heat-conduction term k dT/dn
-    NFS
+    FS_VISE = FS_VIS + 3,   // viscous work sum_a tau_{d,a} * facevel_a
+    FS_THERM = FS_VISE + 1, // heat-conduction term k dT/dn
+    NFS = 14                // two spare: the box-size limit of the allocation-free entry point follows from it
 };
 
 // Kernel kinds of the launch counter / event profiler (mfg_prof.cu).

@@ -132,6 +132,13 @@ __device__ __forceinline__ void muscl(double uim2, double uL, double uR, double 
     uRh = uR - half;
 }
 
+// Sound speed sqrt(gamma p / rho), p = kap rho e (get_max_eigenvalue,
+// flux_schemes.H:21-43).  Explicit roundings: equal states give equal speeds
+// wherever it is compiled (the adjoint compares the two sides of a face).
+__device__ __forceinline__ double eig_speed(double gam, double kap, double rhoe, double irho) {
+    return sqrt_nonneg(__dmul_rn(__dmul_rn(gam, __dmul_rn(kap, rhoe)), irho));
+}
+
 // ---------------------------------------------------------------------------
 // prim_kernel: per-cell scalars over grow(bx, 3)
 // ---------------------------------------------------------------------------
@@ -158,12 +165,11 @@ __device__ __forceinline__ void prim_body(const RhsBox& B, int64_t t) {
     const double irho = rcp_pos(rho);
     const double vx = m0 * irho, vy = m1 * irho, vz = m2 * irho;
     const double rhoe = E - (0.5 * rho) * ((vx * vx + vy * vy) + vz * vz);
-    const double pf = thermo_p<NS>(rhoe, rho, spec);
+    const double kap = thermo_kappa<NS>(rho, spec);
+    const double pf = rhoe * kap;
     // get_max_eigenvalue's own-species terms (flux_schemes.H:21-43)
     const double reig = E - (0.5 * ((m0 * m0 + m1 * m1) + m2 * m2)) * irho;
-    const double peig = thermo_p<NS>(reig, rho, spec);
-    const double gam = thermo_gamma<NS>(rho, spec);
-    const double aown = sqrt((gam * peig) * irho);
+    const double aown = eig_speed(1.0 + kap, kap, reig, irho);
     const Fab& X = B.aux;
     const int64_t q = X.off(c.i, c.j, c.k);
     X.p[q + AUX_VX * X.ns] = vx;
@@ -172,7 +178,7 @@ __device__ __forceinline__ void prim_body(const RhsBox& B, int64_t t) {
     X.p[q + AUX_PF * X.ns] = pf;
     X.p[q + AUX_REIG * X.ns] = reig;
     X.p[q + AUX_AOWN * X.ns] = aown;
-    X.p[q + AUX_GAM * X.ns] = gam;
+    X.p[q + AUX_KAP * X.ns] = kap;
 }
 
 // ---------------------------------------------------------------------------
@@ -227,7 +233,6 @@ __device__ __forceinline__ void face_body_at(const RhsBox& B, int d, const Idx3&
     for (int q = 0; q < NFS; ++q) fs[q] = 0.0;
     fs[FS_FLAGS] = __longlong_as_double((active ? 1 : 0) | ((P.do_ns && fallback) ? 2 : 0));  // bit pattern
     double uL[NCONS + NS], uR[NCONS + NS];  // AUSM+-up face states (orders 1, 2)
-    double vise = 0.0;                      // viscous work of the energy flux (orders 1, 2)
 
     if (active) {
         const int ord = P.order_hyp;
@@ -240,13 +245,18 @@ __device__ __forceinline__ void face_body_at(const RhsBox& B, int d, const Idx3&
             const double aL = X.p[qL + AUX_AOWN * X.ns];
             double aR;
             if (ord == 5) {
-                // presR is evaluated with the left cell's species (flux_schemes.H:33)
-                double specL[NS];
-#pragma unroll
-                for (int s = 0; s < NS; ++s) specL[s] = (s < P.nspec) ? S.p[oL + (NFLO + s) * S.ns] : 0.0;
+                // presR is evaluated with the left cell's species (flux_schemes.H:33):
+                // kappa of the left cell, but for the background-gas family, whose
+                // kappa depends on the density too
                 const double rhoR = S.p[oR + RHO * S.ns];
-                const double pR = thermo_p<NS>(X.p[qR + AUX_REIG * X.ns], rhoR, specL);
-                aR = sqrt((X.p[qR + AUX_GAM * X.ns] * pR) / rhoR);
+                double kapL = X.p[qL + AUX_KAP * X.ns];
+                if (P.thermo_kind == MFG_THERMO_BG_GAS) {
+                    double specL[NS];
+#pragma unroll
+                    for (int s = 0; s < NS; ++s) specL[s] = (s < P.nspec) ? S.p[oL + (NFLO + s) * S.ns] : 0.0;
+                    kapL = thermo_kappa<NS>(rhoR, specL);
+                }
+                aR = eig_speed(1.0 + X.p[qR + AUX_KAP * X.ns], kapL, X.p[qR + AUX_REIG * X.ns], rcp_pos(rhoR));
             } else {
                 aR = X.p[qR + AUX_AOWN * X.ns];
             }
@@ -274,24 +284,25 @@ __device__ __forceinline__ void face_body_at(const RhsBox& B, int d, const Idx3&
             // normal velocity (the transverse velocities are not needed)
             const double hkL = (0.5 * ((uL[RHOU] * uL[RHOU] + uL[RHOV] * uL[RHOV]) + uL[RHOW] * uL[RHOW])) * irL;
             const double hkR = (0.5 * ((uR[RHOU] * uR[RHOU] + uR[RHOV] * uR[RHOV]) + uR[RHOW] * uR[RHOW])) * irR;
-            const double pL = thermo_p<NS>(uL[RHOE] - hkL, rL, uL + NCONS);
-            const double pR = thermo_p<NS>(uR[RHOE] - hkR, rR, uR + NCONS);
-            const double gL = thermo_gamma<NS>(rL, uL + NCONS), gR = thermo_gamma<NS>(rR, uR + NCONS);
+            // kappa = gamma - 1 of both states as one division each, or as its
+            // numerator and denominator: 2 (gamma - 1)/(gamma + 1) = 2 n/(2 d + n)
+            double kL = P.gm1_single, kR = P.gm1_single, afL = P.astar_fac, afR = P.astar_fac;
+            if (P.thermo_kind != MFG_THERMO_MASS_SINGLE) {
+                double n, dn;
+                thermo_ratio<NS>(rL, uL + NCONS, n, dn);
+                kL = quot_pos(n, dn);
+                afL = quot_pos(2.0 * n, fma(2.0, dn, n));
+                thermo_ratio<NS>(rR, uR + NCONS, n, dn);
+                kR = quot_pos(n, dn);
+                afR = quot_pos(2.0 * n, fma(2.0, dn, n));
+            }
+            const double pL = (uL[RHOE] - hkL) * kL, pR = (uR[RHOE] - hkR) * kR;
             const double vL = ((d == 0) ? uL[RHOU] : (d == 1) ? uL[RHOV] : uL[RHOW]) * irL;
             const double vR = ((d == 0) ? uR[RHOU] : (d == 1) ? uR[RHOV] : uR[RHOW]) * irR;
-            const bool cg = P.thermo_kind == MFG_THERMO_MASS_SINGLE;
-            // gamma/(gamma-1) and 2(gamma-1)/(gamma+1): constants of the single-gas
-            // family, else per face state with reciprocals of the positive gamma +- 1
-            double gfL = P.g_gm1, gfR = P.g_gm1, afL = P.astar_fac, afR = P.astar_fac;
-            if (!cg) {
-                gfL = gL * rcp_pos(gL - 1.0);
-                gfR = gR * rcp_pos(gR - 1.0);
-                afL = (2.0 * (gL - 1.0)) * rcp_pos(gL + 1.0);
-                afR = (2.0 * (gR - 1.0)) * rcp_pos(gR + 1.0);
-            }
-            // total enthalpy gamma/(gamma-1) p/rho + |v|^2/2 = (gf p + |m|^2/(2 rho)) / rho
-            const double HL = fma(gfL, pL, hkL) * irL;
-            const double HR = fma(gfR, pR, hkR) * irR;
+            // total enthalpy gamma/(gamma-1) p/rho + |v|^2/2 = (E + p) / rho; E + p
+            // is also what the energy flux advects
+            const double epL = uL[RHOE] + pL, epR = uR[RHOE] + pR;
+            const double HL = epL * irL, HR = epR * irR;
             const double rsum = rL + rR;
             // a_hat = a*^2 / max(a*, |v|) per side, a_1/2 = min(a_hat_L, a_hat_R)
             // and its reciprocal.  On a subsonic side (a* >= |v|, tested as
@@ -342,8 +353,8 @@ __device__ __forceinline__ void face_body_at(const RhsBox& B, int d, const Idx3&
             fs[FS_MH] = Mh;
             fs[FS_MODM] = modM;
             fs[FS_PH] = ph;
-            fs[FS_PL] = pL;
-            fs[FS_PR] = pR;
+            fs[FS_PL] = epL;
+            fs[FS_PR] = epR;
         }
         // viscous stress (compute_flux_3d.H:293-367); lagged primitive velocities
         const double* V0 = S.p + VELX * S.ns;
@@ -384,12 +395,9 @@ __device__ __forceinline__ void face_body_at(const RhsBox& B, int d, const Idx3&
             const double tn = (a == d) ? mu * (2.0 * gnd - kTwo3rd * delu)
                                        : mu * fma(dn[a], ids, (a == t1) ? d_t1 : d_t2);
             fs[FS_VIS + a] = tn;
-            if (ord >= 4) fs[FS_VISE + a] = tn * (0.5 * fv2[a]);
         }
-        // orders 1, 2: the viscous work sum_a tau_{d a} v_a of the energy flux
-        // with fused multiply-adds (the face thread assembles that flux itself)
-        if (ord <= 2)
-            vise = 0.5 * fma(fs[FS_VIS + 0], fv2[0], fma(fs[FS_VIS + 1], fv2[1], fs[FS_VIS + 2] * fv2[2]));
+        // the viscous work sum_a tau_{d a} v_a of the energy flux
+        fs[FS_VISE] = 0.5 * fma(fs[FS_VIS + 0], fv2[0], fma(fs[FS_VIS + 1], fv2[1], fs[FS_VIS + 2] * fv2[2]));
     }
     if (P.do_ns) {
         // heat conduction (compute_flux_3d.H:373-374), conductivity from (i,j,k),(i-1,j,k)
@@ -421,14 +429,14 @@ __device__ __forceinline__ void face_body_at(const RhsBox& B, int d, const Idx3&
             if (active) {
                 double fL = uL[c], fR = uR[c];
                 if (c == RHOE) {
-                    fL = uL[c] + fs[FS_PL];
-                    fR = uR[c] + fs[FS_PR];
+                    fL = fs[FS_PL];
+                    fR = fs[FS_PR];
                 }
                 double fh = fma(wR, fR, wL * fL);
                 if (c == 1 + d) fh += fs[FS_PH];
                 F = (c < NCONS) ? fh : P.advect_flag[c - NCONS] * fh;
                 if (c >= RHOU && c <= RHOW) F -= fs[FS_VIS + c - 1];
-                if (c == RHOE) F -= vise;
+                if (c == RHOE) F -= fs[FS_VISE];
             }
             if (c == RHOE) F -= fs[FS_THERM];
             if (c >= NCONS) {
@@ -446,10 +454,18 @@ __device__ __forceinline__ void face_body_at(const RhsBox& B, int d, const Idx3&
             for (int z = NCONS; z < NFLO; ++z) U.p[qu + z * U.ns] = 0.0;
         return;
     }
+    // what the flux pass of this face reads: the AUSM+-up scalars only for
+    // orders 1/2; lambda and the viscous terms only where active.  FS_MH is
+    // zero for orders 4/5 (the adjoint sums the eigenvalue's adjoint there).
     const Fab& F = B.fs[d];
     const int64_t q = F.off(f.i, f.j, f.k);
+    const bool ausm = P.order_hyp <= 2;
 #pragma unroll
-    for (int c = 0; c < NFS; ++c) F.p[q + c * F.ns] = fs[c];
+    for (int c = 0; c < NFS; ++c) {
+        if (!(c == FS_FLAGS || c == FS_MH || c == FS_THERM) && !active) continue;
+        if (c >= FS_MODM && c <= FS_PR && !ausm) continue;
+        F.p[q + c * F.ns] = fs[c];
+    }
 }
 
 // Face t (linear index over growHi(bx, d, 1)) of direction d.
@@ -530,19 +546,15 @@ __device__ __forceinline__ void flux_body(const RhsBox& B, int d, int c, int64_t
                 const double ah = FS.p[qf + FS_LAMBDA * FS.ns];
                 double fL = uLh, fR = uRh;
                 if (c == RHOE) {
-                    fL = uLh + FS.p[qf + FS_PL * FS.ns];
-                    fR = uRh + FS.p[qf + FS_PR * FS.ns];
+                    fL = FS.p[qf + FS_PL * FS.ns];
+                    fR = FS.p[qf + FS_PR * FS.ns];
                 }
                 fh = ((0.5 * Mh) * (fL + fR) - (0.5 * modM) * (fR - fL)) * ah;
                 if (c == 1 + d) fh += FS.p[qf + FS_PH * FS.ns];
             }
             F = (c < NCONS) ? fh : P.advect_flag[c - NCONS] * fh;
             if (c >= RHOU && c <= RHOW) F -= FS.p[qf + (FS_VIS + c - 1) * FS.ns];
-            if (c == RHOE) {
-                F -= FS.p[qf + (FS_VISE + 0) * FS.ns];
-                F -= FS.p[qf + (FS_VISE + 1) * FS.ns];
-                F -= FS.p[qf + (FS_VISE + 2) * FS.ns];
-            }
+            if (c == RHOE) F -= FS.p[qf + FS_VISE * FS.ns];
         }
         if (c == RHOE) F -= FS.p[qf + FS_THERM * FS.ns];
     } else if (c >= NCONS) {
@@ -821,11 +833,7 @@ __device__ __forceinline__ void flux5_finish(const Fp& fp, const Flux5Ctx& x, bo
     if (active) {
         F = (c < NCONS) ? fh : __dmul_rn(P.advect_flag[c - NCONS], fh);
         if (c >= RHOU && c <= RHOW) F = fp.sub(F, x.fs[qf + (FS_VIS + c - 1) * x.fns]);
-        if (c == RHOE) {
-            F = fp.sub(F, x.fs[qf + (FS_VISE + 0) * x.fns]);
-            F = fp.sub(F, x.fs[qf + (FS_VISE + 1) * x.fns]);
-            F = fp.sub(F, x.fs[qf + (FS_VISE + 2) * x.fns]);
-        }
+        if (c == RHOE) F = fp.sub(F, x.fs[qf + FS_VISE * x.fns]);
     }
     if (c == RHOE) F = fp.sub(F, x.fs[qf + FS_THERM * x.fns]);
     if (c >= NCONS) {  // species diffusion (compute_flux_3d.H:425-428)

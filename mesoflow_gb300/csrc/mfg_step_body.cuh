@@ -414,20 +414,19 @@ __device__ __forceinline__ unsigned prims_cell(double* u, const double* spec) {
     // on the integer pipe (the FP64 pipe bounds this kernel)
     if (is_one(vf)) {
         const double rho = u[RHO];
-        // one Newton-refined reciprocal of the (positive) density for the three
+        // one refined reciprocal of the (positive) density for the three
         // velocities and the mass-single temperature instead of four divisions
         const double irho = rcp_pos(rho);
         const double vx = u[RHOU] * irho, vy = u[RHOV] * irho, vz = u[RHOW] * irho;
         const double rhoe = u[RHOE] - (0.5 * rho) * ((vx * vx + vy * vy) + vz * vz);
-        const double p = thermo_p<NS>(rhoe, rho, spec);
+        double p, T;
+        thermo_pt<NS>(rhoe, rho, irho, spec, p, T);
         u[DENS] = rho;
         u[VELX] = vx;
         u[VELY] = vy;
         u[VELZ] = vz;
         u[PRES] = p;
-        // p / R / rho of the mass-single family as (p / rho) / R with the
-        // reciprocals above and from mfg_init (a few ulp from the two divisions)
-        u[TEMP] = (P.thermo_kind == MFG_THERMO_MASS_SINGLE) ? (p * irho) * P.inv_gas_R : thermo_t<NS>(rho, p, spec);
+        u[TEMP] = T;
         wrote = (1u << DENS) | (1u << VELX) | (1u << VELY) | (1u << VELZ) | (1u << PRES) | (1u << TEMP);
     } else if (P.conj_ht && is_zero_bits(vf)) {
         u[TEMP] = P.solid_temp;
