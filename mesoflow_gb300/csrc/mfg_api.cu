@@ -151,6 +151,9 @@ RhsBox make_rhs_box(const mfg_box& b, const mfg_geom& g, double* base) {
         B.hi[d] = b.hi[d];
         B.dx[d] = g.dx[d];
         B.idx[d] = 1.0 / g.dx[d];
+        B.iq[d] = 0.25 * B.idx[d];
+        B.i43[d] = (4.0 / 3.0) * B.idx[d];
+        B.iq23[d] = -kTwo3rd * B.iq[d];
         n[d] = b.hi[d] - b.lo[d] + 1;
     }
     B.sb = make_fab(b.sborder);

@@ -530,8 +530,9 @@ __global__ void __launch_bounds__(BT) bk_prim(const RhsBox* __restrict__ B, cons
 
 template <int NS>
 __global__ void __launch_bounds__(BT) bk_face(const RhsBox* __restrict__ B, const Tile* __restrict__ tiles, int ntiles) {
+    const Fp fp;
     TILE_LOOP
-    face_body<NS>(B[tl.box], tl.part, t);
+    face_body<NS>(fp, B[tl.box], tl.part, t);
     TILE_END
 }
 

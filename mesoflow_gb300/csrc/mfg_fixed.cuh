@@ -1,0 +1,178 @@
+// Reciprocals, reciprocal square roots and the limiter's harmonic half of
+// FP64 numbers on the integer pipe.
+//
+// GB300 issues 2 FP64 operations per SM and cycle: a warp's FP64 add or
+// multiply holds its scheduler's FP64 pipe for 70 to 82 cycles, a reciprocal
+// refined there for 210, a reciprocal square root for 385.  The high half of a
+// 64 x 64-bit product takes 18 cycles of the integer pipe, so a 62-bit
+// fixed-point evaluation takes 75 to 150 cycles of a pipe that the FP64-bound
+// kernels leave idle, and its result is rounded once, from 59 or more correct
+// bits (the FP64 sequences round three to five times).
+#pragma once
+#include <stdint.h>
+#include <string.h>
+
+#ifdef __CUDACC__
+#define MFG_HD __host__ __device__ __forceinline__
+#else
+#define MFG_HD inline
+#endif
+
+namespace mfg {
+
+MFG_HD uint64_t umulhi64(uint64_t a, uint64_t b) {
+#ifdef __CUDA_ARCH__
+    return __umul64hi(a, b);
+#else
+    return (uint64_t)(((unsigned __int128)a * b) >> 64);
+#endif
+}
+
+MFG_HD int clz32(uint32_t x) {  // x != 0
+#ifdef __CUDA_ARCH__
+    return __clz((int)x);
+#else
+    return __builtin_clz(x);
+#endif
+}
+
+MFG_HD uint64_t bits_of(double x) {
+#ifdef __CUDA_ARCH__
+    return (uint64_t)__double_as_longlong(x);
+#else
+    uint64_t u;
+    memcpy(&u, &x, 8);
+    return u;
+#endif
+}
+
+MFG_HD double double_of(uint64_t u) {
+#ifdef __CUDA_ARCH__
+    return __longlong_as_double((long long)u);
+#else
+    double x;
+    memcpy(&x, &u, 8);
+    return x;
+#endif
+}
+
+// Bits of the float32 1/f, f in (1, 2), and 1/sqrt(f), f in (1, 4), relative
+// error below 2^-22.
+MFG_HD uint32_t rcp_seed_bits(uint32_t fbits) {
+#ifdef __CUDA_ARCH__
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint_as_float(fbits)));
+    return __float_as_uint(r);
+#else
+    float f;
+    memcpy(&f, &fbits, 4);
+    f = 1.0f / f;
+    uint32_t b;
+    memcpy(&b, &f, 4);
+    return b;
+#endif
+}
+MFG_HD uint32_t rsqrt_seed_bits(uint32_t fbits) {
+#ifdef __CUDA_ARCH__
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint_as_float(fbits)));
+    return __float_as_uint(r);
+#else
+    float f;
+    memcpy(&f, &fbits, 4);
+    f = 1.0f / __builtin_sqrtf(f);
+    uint32_t b;
+    memcpy(&b, &f, 4);
+    return b;
+#endif
+}
+
+MFG_HD int imin(int a, int b) { return a < b ? a : b; }
+MFG_HD int imax(int a, int b) { return a > b ? a : b; }
+
+// 2^126 / d for a normalised d (top bit set), relative error below 2^-59: the
+// float32 seed r0 (e = 1 - x r0, |e| < 2^-21) corrected by r0 (1 + e + e^2).
+MFG_HD uint64_t rcp_fixed(uint64_t d) {
+    const uint32_t dh = (uint32_t)(d >> 32), dl = (uint32_t)d;
+    uint32_t rb = rcp_seed_bits(0x3f800000u | ((dh & 0x7fffffffu) >> 8) | 1u);
+    rb = rb < 0x3f000000u ? 0x3f000000u : rb > 0x3f7fffffu ? 0x3f7fffffu : rb;  // in [1/2, 1)
+    const uint32_t R0 = ((rb & 0x7fffffu) | 0x800000u) << 7;                     // r0 2^31
+    const uint64_t T = (uint64_t)dh * R0 + (((uint64_t)dl * R0) >> 32);          // (1 - e) 2^62
+    const int64_t e = (int64_t)((1ull << 62) - T);
+    const int32_t es = (int32_t)(e >> 18);
+    const int64_t g = e + (((int64_t)es * es) >> 26);  // (e + e^2) 2^62
+    const int32_t gh = (int32_t)(g >> 32);
+    const uint32_t gl = (uint32_t)g;
+    return ((uint64_t)R0 << 32) + (uint64_t)(((int64_t)gh * (int32_t)R0) << 2) + (((uint64_t)R0 * gl) >> 30);
+}
+
+constexpr uint64_t kMantMask = 0x000fffffffffffffull, kMantOne = 0x0010000000000000ull;
+
+// Whether x is positive with an exponent away from the ends of the range (the
+// integer forms below; everything else takes the FP64 sequences).
+MFG_HD bool mid_positive(double x) {
+    return (uint32_t)(bits_of(x) >> 32) - (40u << 20) < (1960u << 20);
+}
+
+// 1 / x for mid_positive(x).
+MFG_HD double rcp_mid(double x) {
+    const uint64_t b = bits_of(x);
+    const uint64_t r = rcp_fixed(((b & kMantMask) | kMantOne) << 11);  // (2^62, 2^63]
+    const uint32_t e = 2044u - (uint32_t)(b >> 52);
+    return double_of(((uint64_t)e << 52) + ((r + 512) >> 10));  // r's top bit adds one to e
+}
+
+// 1 / sqrt(x) for mid_positive(x): x = m 2^(2h) with m in [1, 4), seed y0 =
+// 1/sqrt(m) (1 + O(2^-21)), corrected by y0 (1 + e/2 + 3 e^2/8), e = 1 - m y0^2.
+MFG_HD double rsqrt_mid(double x) {
+    const uint64_t b = bits_of(x);
+    const uint32_t ex = (uint32_t)(b >> 52);
+    const uint32_t odd = (ex ^ 1u) & 1u;                                        // exponent ex - 1023 odd: m in [2, 4)
+    const uint64_t m = ((b & kMantMask) | kMantOne) << (9 + odd);               // m 2^61
+    const uint32_t mh = (uint32_t)(m >> 32), ml = (uint32_t)m;                  // m 2^29
+    const uint32_t f = (0x3f800000u + (odd << 23)) | (uint32_t)((b >> 29) & 0x7fffffu) | 1u;
+    uint32_t yb = rsqrt_seed_bits(f);                                           // 1/sqrt(m) in (1/2, 1)
+    yb = yb < 0x3f000000u ? 0x3f000000u : yb > 0x3f7fffffu ? 0x3f7fffffu : yb;
+    const uint32_t y0 = ((yb & 0x7fffffu) | 0x800000u) << 7;                    // y0 2^31
+    const uint64_t p = (uint64_t)y0 * y0;                                       // y0^2 2^62, exact
+    const uint32_t ph = (uint32_t)(p >> 32), pl = (uint32_t)p;
+    // m y0^2 2^59 = m 2^61 * p 2^62 / 2^64
+    const uint64_t q = (uint64_t)mh * ph + (((uint64_t)mh * pl) >> 32) + (((uint64_t)ml * ph) >> 32);
+    const int64_t e = (int64_t)((1ull << 62) - (q << 3));                       // e 2^62
+    const int32_t es = (int32_t)(e >> 18);
+    const int64_t g = (e >> 1) + 3 * (((int64_t)es * es) >> 29);               // (e/2 + 3 e^2/8) 2^62
+    const int32_t gh = (int32_t)(g >> 32);
+    const uint32_t gl = (uint32_t)g;
+    // y 2^63 in [2^62, 2^63]
+    const uint64_t y =
+        ((uint64_t)y0 << 32) + (uint64_t)(((int64_t)gh * (int32_t)y0) << 2) + (((uint64_t)y0 * gl) >> 30);
+    const uint32_t h = (ex - 1023u - odd) >> 1;  // arithmetic halving of an even number, modulo 2^32
+    const uint32_t e2 = 1021u - ((h & 0x40000000u) ? h | 0x80000000u : h);
+    return double_of(((uint64_t)e2 << 52) + ((y + 512) >> 10));
+}
+
+// d1 d2 / (d1 + d2) for differences of the same sign, 0 otherwise: half the
+// limited slope of the Tatsumi-Martinelli-Jameson limiter (compute_flux_3d.H:
+// 33-65) in closed form, as the smaller difference times the larger one's
+// share of the sum.  A non-finite difference gives NaN.
+MFG_HD double limited_half(double d1, double d2) {
+    const uint64_t b1 = bits_of(d1), b2 = bits_of(d2);
+    const uint64_t a1 = b1 & 0x7fffffffffffffffull, a2 = b2 & 0x7fffffffffffffffull;
+    const uint64_t hi = a1 > a2 ? a1 : a2, lo = a1 > a2 ? a2 : a1;
+    const int eh = (int)(hi >> 52), el = (int)(lo >> 52);
+    const uint64_t mh = ((hi & kMantMask) | kMantOne) << 10, ml = ((lo & kMantMask) | kMantOne) << 10;  // top bit 62
+    uint64_t s = mh + (ml >> imin(eh - el, 63));
+    const int k = (int)(~s >> 63);  // 1 when the sum stays below 2^63
+    s <<= k;
+    const uint64_t q = umulhi64(mh << k, rcp_fixed(s));  // share 2^62, in [2^61, 2^62]
+    uint64_t r = umulhi64(ml << 1, q << 1);              // half 2^(...), in [2^61, 2^62 + 1]
+    const int n = (int)((~r >> 62) & 1);
+    r <<= n;
+    uint64_t h = ((uint64_t)(uint32_t)(el - 1 - n) << 52) + ((r + 512) >> 10);
+    h |= b1 & 0x8000000000000000ull;
+    if ((int64_t)(b1 ^ b2) < 0 || el < 2) h = 0;
+    if (eh == 0x7ff) h = 0x7ff8000000000000ull;
+    return double_of(h);
+}
+
+}  // namespace mfg

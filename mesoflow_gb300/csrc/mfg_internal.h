@@ -9,19 +9,15 @@ namespace mfg {
 // Per-cell scalars of prim_kernel (scratch over grow(bx, 3)).
 enum AuxComp { AUX_VX = 0, AUX_VY, AUX_VZ, AUX_PF, AUX_REIG, AUX_AOWN, AUX_KAP /* gamma - 1 */, NAUX };
 
-// Per-face scalars of face_kernel (scratch over growHi(bx, d, 1)).
+// Per-face scalars of face_kernel for orders 4 and 5 (scratch over growHi(bx, d, 1)).
 enum FsComp {
     FS_FLAGS = 0,  // bit0: hyperbolic + viscous flux active, bit1: first-order IB fallback
-    FS_LAMBDA,     // LLF eigenvalue (orders 4, 5) or AUSM a_half (orders 1, 2)
-    FS_MH,         // AUSM M_half
-    FS_MODM,       // AUSM |M_half| with the entropy fix
-    FS_PH,         // AUSM p_half
-    FS_PL,         // AUSM left pressure
-    FS_PR,         // AUSM right pressure
+    FS_LAMBDA,     // LLF eigenvalue
+    FS_MH,         // zero; the adjoint sums the eigenvalue's adjoint here
     FS_VIS,        // 3: viscous momentum terms tau_{d,a}
     FS_VISE = FS_VIS + 3,   // viscous work sum_a tau_{d,a} * facevel_a
     FS_THERM = FS_VISE + 1, // heat-conduction term k dT/dn
-    NFS = 14                // two spare: the box-size limit of the allocation-free entry point follows from it
+    NFS = 14                // the rest is spare: the box-size limit of the allocation-free entry point follows from it
 };
 
 // Kernel kinds of the launch counter / event profiler (mfg_prof.cu).
@@ -56,6 +52,9 @@ struct RhsBox {
     int lo[3], hi[3];
     double dx[3];
     double idx[3];  // 1/dx
+    // geometry factors of the viscous stresses: 1/(4 dx) of a transverse
+    // difference of two-cell sums, 4/(3 dx) and -1/(6 dx) on the diagonal
+    double iq[3], i43[3], iq23[3];
     Fab sb, dsdt, sold, snew;
     Fab uflux[3];
     Fab aux;

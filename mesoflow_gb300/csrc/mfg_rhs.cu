@@ -47,7 +47,8 @@ __global__ void __launch_bounds__(TPB) prim_kernel(RhsBox B) {
 }
 template <int NS>
 __global__ void __launch_bounds__(TPB) face_kernel(RhsBox B, int d) {
-    face_body<NS>(B, d, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
+    const Fp fp;
+    face_body<NS>(fp, B, d, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 // Orders 1 and 2 with Navier-Stokes terms: the inactive faces (solid side,
 // conduction and diffusion only) of all three directions are written here
@@ -63,6 +64,7 @@ __device__ __forceinline__ int64_t face_list_off(const RhsBox& B, int d) {
 }
 template <int NS>
 __global__ void __launch_bounds__(TPB) face_split_kernel(RhsBox B) {
+    const Fp fp;
     const int d = blockIdx.y;
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     bool act = false;
@@ -71,7 +73,7 @@ __global__ void __launch_bounds__(TPB) face_split_kernel(RhsBox B) {
     if (t < (int64_t)len[0] * len[1] * len[2]) {
         const Idx3 f = delinear(t, lo, len);  // once for the test and the body
         act = face_active(B, d, f);
-        if (!act) face_body_at<NS, true>(B, d, f);
+        if (!act) face_body_at<NS, true>(fp, B, d, f);
     }
     const unsigned m = __ballot_sync(0xffffffffu, act);
     if (!m) return;
@@ -83,16 +85,15 @@ __global__ void __launch_bounds__(TPB) face_split_kernel(RhsBox B) {
 }
 // The direction is the block's (blockIdx.y), uniform as in face_kernel, so
 // the compiler forms the same multiply-adds in both.
-// 128-thread blocks at 4 per SM (120 registers, no spills): after the FP64
-// operation cuts the body fits without spilling at 16 resident warps, which
-// measured 0.8% faster than 5 blocks at 96 registers with 80 bytes spilled
-// (and 6 blocks at 80 registers 1% slower).
+// 128-thread blocks.  One or two species: 5 per SM (96 registers), 1% faster
+// than 4; more species need 128 registers (5 per SM spill: 8% slower with ten).
 constexpr int LIST_TPB = 128;
 template <int NS>
-__global__ void __launch_bounds__(LIST_TPB, 4) face_list_kernel(RhsBox B) {
+__global__ void __launch_bounds__(LIST_TPB, NS <= 2 ? 5 : 4) face_list_kernel(RhsBox B) {
     const int d = blockIdx.y;
     const unsigned w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w < B.fcount[d]) face_body<NS>(B, d, B.flist[face_list_off(B, d) + w]);
+    const Fp fp;
+    if (w < B.fcount[d]) face_body<NS>(fp, B, d, B.flist[face_list_off(B, d) + w]);
 }
 template <bool FAST>
 __global__ void __launch_bounds__(TPB) flux_kernel(RhsBox B, int d) {

@@ -12,6 +12,23 @@ namespace {
 
 constexpr double kEpsWeno = 1e-6;
 
+// FP64 sums and products as fused multiply-adds with 1 and -0 in registers:
+// bitwise the add and the multiply, at the fused multiply-add's rate (a warp
+// holds the FP64 pipe for 70 cycles; DADD and DMUL, and fused multiply-adds
+// with an operand from the constant bank or an immediate, for 82).  The two
+// constants pass through a shuffle so that they stay in registers; every lane
+// of the warp constructs it.
+struct Fp {
+    double one, nz;
+    __device__ __forceinline__ Fp() {
+        one = __hiloint2double(__shfl_sync(0xffffffffu, 0x3ff00000, 0), 0);
+        nz = __hiloint2double(__shfl_sync(0xffffffffu, (int)0x80000000, 0), 0);
+    }
+    __device__ __forceinline__ double add(double a, double b) const { return __fma_rn(a, one, b); }
+    __device__ __forceinline__ double sub(double a, double b) const { return __fma_rn(b, -one, a); }
+    __device__ __forceinline__ double mul(double a, double b) const { return __fma_rn(a, b, nz); }
+};
+
 // ---------------------------------------------------------------------------
 // index helpers
 // ---------------------------------------------------------------------------
@@ -87,51 +104,6 @@ __device__ __forceinline__ void weno_face(const double s[6], double& up, double&
     um = weno_edge<true, FAST>(s[5], s[4], s[3], s[2], s[1]);
 }
 
-// AUSM+-up split functions (flux_schemes.H:107-181), beta = 1/8.  The
-// supersonic branches of the pressure splits, (M + |M|)/(2M) and
-// (M - |M|)/(2M), are exactly 1 or 0 (with a zero's sign that no later
-// operation keeps), and those of the Mach splits, (M + |M|)/2 and
-// (M - |M|)/2, exactly M or +0 (2M and its halving are exact), so all four
-// are selects; the |M| <= 1 tests run on the integer pipe.
-__device__ __forceinline__ double split_mach_p(double M) {
-    return abs_le(M, 1.0) ? (0.25 * (M + 1.0)) * (M + 1.0) + (0.125 * (M * M - 1.0)) * (M * M - 1.0)
-                          : (is_positive(M) ? M : 0.0);
-}
-__device__ __forceinline__ double split_mach_m(double M) {
-    return abs_le(M, 1.0) ? (-0.25 * (M - 1.0)) * (M - 1.0) - (0.125 * (M * M - 1.0)) * (M * M - 1.0)
-                          : (is_negative(M) ? M : 0.0);
-}
-__device__ __forceinline__ double split_pres_p(double M, double alpha) {
-    return abs_le(M, 1.0)
-               ? ((0.25 * (M + 1.0)) * (M + 1.0)) * (2.0 - M) + ((alpha * M) * (M * M - 1.0)) * (M * M - 1.0)
-               : (is_positive(M) ? 1.0 : 0.0);
-}
-__device__ __forceinline__ double split_pres_m(double M, double alpha) {
-    return abs_le(M, 1.0)
-               ? ((0.25 * (M - 1.0)) * (M - 1.0)) * (2.0 + M) - ((alpha * M) * (M * M - 1.0)) * (M * M - 1.0)
-               : (is_positive(M) ? 0.0 : 1.0);
-}
-
-// MUSCL state of component c with the Tatsumi-Martinelli-Jameson limiter
-// (compute_flux_3d.H:33-65): uL + L/2 and uR - L/2 with
-// L = psi (d1 + d2) / 2, psi = 1 - q^2, q = |d1 - d2| / (|d1| + |d2| + 1e-20),
-// d1 = u_{i+1} - u_R, d2 = u_L - u_{i-2}.  In closed form L/2 = d1 d2 / (d1 + d2)
-// when d1 and d2 have the same sign (then 1 - q^2 = 4 d1 d2 / (d1 + d2)^2) and
-// 0 otherwise (q = 1): the reference's expression equals this up to rounding
-// and terms of the order of its 1e-20 guard, and the closed form needs one
-// reciprocal and four fewer FP64 operations.  The same-sign test is on the
-// integer pipe (d1 d2 > 0).
-__device__ __forceinline__ void muscl(double uim2, double uL, double uR, double uip1, double& uLh, double& uRh) {
-    const double delt1 = uip1 - uR;
-    const double delt2 = uL - uim2;
-    const double p = delt1 * delt2;
-    const double s = delt1 + delt2;
-    // p > 0 implies s != 0; otherwise the reciprocal's value is not used
-    const double half = is_positive(p) ? p * rcp_nonzero(s) : 0.0;
-    uLh = uL + half;
-    uRh = uR - half;
-}
-
 // Sound speed sqrt(gamma p / rho), p = kap rho e (get_max_eigenvalue,
 // flux_schemes.H:21-43).  Explicit roundings: equal states give equal speeds
 // wherever it is compiled (the adjoint compares the two sides of a face).
@@ -203,13 +175,50 @@ __device__ __forceinline__ bool face_active(const RhsBox& B, int d, const Idx3& 
     return c_P.do_ns && nonneg_ge(vf[oR - sd] + vf[oR], 1.0);
 }
 
+// 1/x and 1/sqrt(x) of a positive x: fixed point on the integer pipe, or the
+// FP64 forms at the ends of the exponent range.
+__device__ __forceinline__ double face_rcp(double x) { return mid_positive(x) ? rcp_mid(x) : rcp_pos(x); }
+__device__ __forceinline__ double face_rsqrt(double x) { return mid_positive(x) ? rsqrt_mid(x) : rsqrt(x); }
+
+// Whether |v| < a for v and a^2, both of moderate size, by their exponents
+// alone (true when |v| < 0.7 a; false when undecided).
+__device__ __forceinline__ bool surely_below(double v, double a2) {
+    const int ev = (__double2hiint(v) >> 20) & 0x7ff, ea = __double2hiint(a2) >> 20;
+    return ea > 0 && 2 * (ev + 1 - 1023) < ea - 1023;  // |v|^2 < 2^(2 (ev + 1)) <= 2^ea <= a^2
+}
+
+// The two sides' shares of an AUSM+-up face (flux_schemes.H:107-181, beta =
+// 1/8) at the Mach number M, sign = +1 for the left side and -1 for the right:
+// four times the Mach split, sign ((M + sign)^2 + (M^2 - 1)^2/2) below |M| = 1
+// and 2 (M + sign |M|) above, and the pressure split, (M + sign)^2 (2 - sign M)/4
+// + sign alpha M (M^2 - 1)^2 below and (M + sign |M|)/(2 M) above.  q = M^2 - 1.
+// The supersonic branches are exactly 4 M or 0, and 1 or 0; the |M| <= 1 tests
+// run on the integer pipe.
+__device__ __forceinline__ void ausm_split(const Fp& fp, double M, double sign, double q, double& m4, double& g,
+                                           double& mq2) {
+    const double a = __fma_rn(sign, fp.one, M);
+    const double sq = fp.mul(a, a), q2 = fp.mul(q, q);
+    const bool sub = abs_le(M, 1.0), on = sign > 0.0 ? is_positive(M) : is_negative(M);
+    m4 = sub ? __fma_rn(0.5, q2, sq) : (on ? __dmul_rn(4.0 * sign, M) : 0.0);
+    g = sub ? fp.mul(sq, __fma_rn(-sign, M, 2.0)) : (on ? 4.0 : 0.0);
+    mq2 = sub ? fp.mul(M, q2) : 0.0;
+}
+
 // Face f of direction d.  SOLID_SIDE: the caller knows the face is not
 // active and the pass is the split form of orders 1/2 with Navier-Stokes
 // terms (face_split_kernel); the flux branch and the first-order fallback
 // test (used only by the flux branch and the stored face scalars of orders
 // 4/5) are compiled out, the remaining arithmetic is the same.
+//
+// FP64 issue bounds the flux branch of orders 1/2.  Its reciprocals, square
+// roots and limiters run in fixed point on the integer pipe (mfg_fixed.cuh),
+// its sums and products as register-operand multiply-adds (Fp), and every
+// rounding is explicit, so the one-pass and the listed form agree bitwise.
+// About 170 FP64 operations per face of one species at 70 cycles (205 at 82
+// with the refined reciprocals there): face passes of a 256^3 sphere-pack step
+// 50.4 -> 38.0 ms; the listed form keeps the FP64 pipe 83% busy.
 template <int NS, bool SOLID_SIDE = false>
-__device__ __forceinline__ void face_body_at(const RhsBox& B, int d, const Idx3& f) {
+__device__ __forceinline__ void face_body_at(const Fp& fp, const RhsBox& B, int d, const Idx3& f) {
     const DevParams& P = c_P;
     const Fab& S = B.sb;
     const int64_t sd = (d == 0) ? 1 : (d == 1) ? S.js : S.ks;
@@ -219,6 +228,7 @@ __device__ __forceinline__ void face_body_at(const RhsBox& B, int d, const Idx3&
     const int64_t oR = S.off(f.i, f.j, f.k);  // right cell: face i separates i-1 and i
     const int64_t oL = oR - sd;
     const double* vf = S.p + VFRAC * S.ns;
+    const int ord = P.order_hyp;
 
     bool fallback = false;
     if (!SOLID_SIDE) {
@@ -226,16 +236,15 @@ __device__ __forceinline__ void face_body_at(const RhsBox& B, int d, const Idx3&
         for (int q = -3; q <= 2; ++q) fallback |= below_one(vf[oR + q * sd]);
     }
     // face volume fraction 0.5 (a + b) >= 0.5, i.e. a + b >= 1 (the halving is exact)
-    const bool active = !SOLID_SIDE && P.do_ns && nonneg_ge(vf[oL] + vf[oR], 1.0);
+    const bool active = !SOLID_SIDE && P.do_ns && nonneg_ge(fp.add(vf[oL], vf[oR]), 1.0);
 
-    double fs[NFS];
-#pragma unroll
-    for (int q = 0; q < NFS; ++q) fs[q] = 0.0;
-    fs[FS_FLAGS] = __longlong_as_double((active ? 1 : 0) | ((P.do_ns && fallback) ? 2 : 0));  // bit pattern
-    double uL[NCONS + NS], uR[NCONS + NS];  // AUSM+-up face states (orders 1, 2)
+    double lam = 0.0;                        // orders 4, 5: LLF eigenvalue
+    double uL[NCONS + NS], uR[NCONS + NS];   // orders 1, 2: advected face states, E + p for the energy
+    double wL = 0.0, wR = 0.0, ph = 0.0;     // orders 1, 2: mass-flux weights, interface pressure
+    double vis[3] = {0.0, 0.0, 0.0}, vise2 = 0.0;  // viscous stresses; twice the viscous work
+    double therm = 0.0;                      // heat conduction
 
     if (active) {
-        const int ord = P.order_hyp;
         if (ord == 5 || ord == 4) {
             const Fab& X = B.aux;
             const int64_t qL = X.off(f.i, f.j, f.k) - ((d == 0) ? 1 : (d == 1) ? X.js : X.ks);
@@ -260,30 +269,30 @@ __device__ __forceinline__ void face_body_at(const RhsBox& B, int d, const Idx3&
             } else {
                 aR = X.p[qR + AUX_AOWN * X.ns];
             }
-            fs[FS_LAMBDA] = max_nonneg(aL, aR) + veln;
+            lam = fp.add(max_nonneg(aL, aR), veln);
         } else {
             // AUSM+-up (flux_schemes.H:185-310) on first- or second-order states
+            // (MUSCL: u_L + h and u_R - h with h the limited half slope)
             const int nc = NCONS + P.nspec;
 #pragma unroll
             for (int c = 0; c < NCONS + NS; ++c) {
                 if (c >= nc) { uL[c] = uR[c] = 0.0; continue; }
-                const int sc = (c < NCONS) ? c : c + (NFLO - NCONS);
-                double ul = S.p[oL + sc * S.ns], ur = S.p[oR + sc * S.ns];
-                if (ord == 2) {
-                    double ulm1 = fallback ? ul : S.p[oL - sd + sc * S.ns];
-                    double urp1 = fallback ? ur : S.p[oR + sd + sc * S.ns];
-                    muscl(ulm1, ul, ur, urp1, uL[c], uR[c]);
-                } else {
-                    uL[c] = ul;
-                    uR[c] = ur;
+                const double* u = S.p + ((c < NCONS) ? c : c + (NFLO - NCONS)) * S.ns;
+                uL[c] = u[oL];
+                uR[c] = u[oR];
+                if (ord == 2 && !fallback) {
+                    const double h = limited_half(fp.sub(u[oR + sd], uR[c]), fp.sub(uL[c], u[oL - sd]));
+                    uL[c] = fp.add(uL[c], h);
+                    uR[c] = fp.sub(uR[c], h);
                 }
             }
             const double rL = uL[RHO], rR = uR[RHO];
-            const double irL = rcp_pos(rL), irR = rcp_pos(rR);
-            // kinetic energy density |m|^2 / (2 rho) from the momenta and the
-            // normal velocity (the transverse velocities are not needed)
-            const double hkL = (0.5 * ((uL[RHOU] * uL[RHOU] + uL[RHOV] * uL[RHOV]) + uL[RHOW] * uL[RHOW])) * irL;
-            const double hkR = (0.5 * ((uR[RHOU] * uR[RHOU] + uR[RHOV] * uR[RHOV]) + uR[RHOW] * uR[RHOW])) * irR;
+            const double irL = face_rcp(rL), irR = face_rcp(rR);
+            // internal energy rho e = E - |m|^2 / (2 rho) from the momenta
+            const double k2L = fp.mul(
+                __fma_rn(uL[RHOU], uL[RHOU], __fma_rn(uL[RHOV], uL[RHOV], fp.mul(uL[RHOW], uL[RHOW]))), irL);
+            const double k2R = fp.mul(
+                __fma_rn(uR[RHOU], uR[RHOU], __fma_rn(uR[RHOV], uR[RHOV], fp.mul(uR[RHOW], uR[RHOW]))), irR);
             // kappa = gamma - 1 of both states as one division each, or as its
             // numerator and denominator: 2 (gamma - 1)/(gamma + 1) = 2 n/(2 d + n)
             double kL = P.gm1_single, kR = P.gm1_single, afL = P.astar_fac, afR = P.astar_fac;
@@ -291,113 +300,111 @@ __device__ __forceinline__ void face_body_at(const RhsBox& B, int d, const Idx3&
                 double n, dn;
                 thermo_ratio<NS>(rL, uL + NCONS, n, dn);
                 kL = quot_pos(n, dn);
-                afL = quot_pos(2.0 * n, fma(2.0, dn, n));
+                afL = quot_pos(2.0 * n, __fma_rn(2.0, dn, n));
                 thermo_ratio<NS>(rR, uR + NCONS, n, dn);
                 kR = quot_pos(n, dn);
-                afR = quot_pos(2.0 * n, fma(2.0, dn, n));
+                afR = quot_pos(2.0 * n, __fma_rn(2.0, dn, n));
             }
-            const double pL = (uL[RHOE] - hkL) * kL, pR = (uR[RHOE] - hkR) * kR;
-            const double vL = ((d == 0) ? uL[RHOU] : (d == 1) ? uL[RHOV] : uL[RHOW]) * irL;
-            const double vR = ((d == 0) ? uR[RHOU] : (d == 1) ? uR[RHOV] : uR[RHOW]) * irR;
-            // total enthalpy gamma/(gamma-1) p/rho + |v|^2/2 = (E + p) / rho; E + p
-            // is also what the energy flux advects
-            const double epL = uL[RHOE] + pL, epR = uR[RHOE] + pR;
-            const double HL = epL * irL, HR = epR * irR;
-            const double rsum = rL + rR;
+            const double pL = fp.mul(__fma_rn(-0.5, k2L, uL[RHOE]), kL), pR = fp.mul(__fma_rn(-0.5, k2R, uR[RHOE]), kR);
+            const double vL = fp.mul((d == 0) ? uL[RHOU] : (d == 1) ? uL[RHOV] : uL[RHOW], irL);
+            const double vR = fp.mul((d == 0) ? uR[RHOU] : (d == 1) ? uR[RHOV] : uR[RHOW], irR);
+            // E + p: what the energy flux advects, and rho times the total enthalpy
+            // gamma/(gamma-1) p/rho + |v|^2/2
+            uL[RHOE] = fp.add(uL[RHOE], pL);
+            uR[RHOE] = fp.add(uR[RHOE], pR);
+            const double rsum = fp.add(rL, rR);
             // a_hat = a*^2 / max(a*, |v|) per side, a_1/2 = min(a_hat_L, a_hat_R)
-            // and its reciprocal.  On a subsonic side (a* >= |v|, tested as
-            // a*^2 >= v^2) a_hat = a*, so when both sides are subsonic a_1/2 is
-            // the square root of the smaller a*^2: a_1/2 = m rsqrt(m) and
-            // 1/a_1/2 = rsqrt(m), one reciprocal square root and no reciprocal.
-            // Otherwise each side as a* or a*^2/|v| (and |v|/a*^2), the smaller.
-            const double as2L = afL * HL, as2R = afR * HR;
+            // and its reciprocal.  On a subsonic side (a* >= |v|) a_hat = a*, so
+            // when both sides are subsonic a_1/2 is the square root of the smaller
+            // a*^2: a_1/2 = m rsqrt(m) and 1/a_1/2 = rsqrt(m).  Otherwise each
+            // side as a* or a*^2/|v| (and |v|/a*^2), the smaller.
+            const double as2L = fp.mul(afL, fp.mul(uL[RHOE], irL)), as2R = fp.mul(afR, fp.mul(uR[RHOE], irR));
             double ah, iah;
-            if (nonneg_ge(as2L, vL * vL) && nonneg_ge(as2R, vR * vR)) {
+            if ((surely_below(vL, as2L) || nonneg_ge(as2L, fp.mul(vL, vL))) &&
+                (surely_below(vR, as2R) || nonneg_ge(as2R, fp.mul(vR, vR)))) {
                 const double m = min_nonneg(as2L, as2R);
-                iah = rsqrt(m);
-                ah = m * iah;
+                iah = face_rsqrt(m);
+                ah = fp.mul(m, iah);
             } else {
-                double irs = rsqrt(as2L);
-                double ahL = as2L * irs, iahL = irs;
+                double irs = face_rsqrt(as2L);
+                double ahL = fp.mul(as2L, irs), iahL = irs;
                 if (!nonneg_ge(ahL, fabs(vL))) {
-                    ahL = as2L * rcp_pos(fabs(vL));
-                    iahL = fabs(vL) * rcp_pos(as2L);
+                    ahL = fp.mul(as2L, rcp_pos(fabs(vL)));
+                    iahL = fp.mul(fabs(vL), rcp_pos(as2L));
                 }
-                irs = rsqrt(as2R);
-                double ahR = as2R * irs, iahR = irs;
+                irs = face_rsqrt(as2R);
+                double ahR = fp.mul(as2R, irs), iahR = irs;
                 if (!nonneg_ge(ahR, fabs(vR))) {
-                    ahR = as2R * rcp_pos(fabs(vR));
-                    iahR = fabs(vR) * rcp_pos(as2R);
+                    ahR = fp.mul(as2R, rcp_pos(fabs(vR)));
+                    iahR = fp.mul(fabs(vR), rcp_pos(as2R));
                 }
                 const bool left = nonneg_le(ahL, ahR);
                 ah = left ? ahL : ahR;
                 iah = left ? iahL : iahR;
             }
-            const double ML = vL * iah, MR = vR * iah;
-            double Mh = split_mach_p(ML) + split_mach_m(MR);
-            const double Mb2 = 0.5 * (ML * ML + MR * MR);
+            const double ML = fp.mul(vL, iah), MR = fp.mul(vR, iah);
+            const double qL = __fma_rn(ML, ML, -fp.one), qR = __fma_rn(MR, MR, -fp.one);
+            double m4L, m4R, gL, gR, mqL, mqR;
+            ausm_split(fp, ML, 1.0, qL, m4L, gL, mqL);
+            ausm_split(fp, MR, -1.0, qR, m4R, gR, mqR);
+            // mean Mach number Mb^2 = (ML^2 + MR^2)/2 = 1 + (qL + qR)/2
+            const double qs = fp.add(qL, qR);
             // M_o = sqrt(min(1, max(Mb^2, 0.3^2))) as x rsqrt(x) on the clamped x
-            const double xmo = min_nonneg(1.0, max_nonneg(Mb2, 0.3 * 0.3));
-            const double Mo = xmo * rsqrt(xmo);
-            const double fa = Mo * (2.0 - Mo);
-            // pressure diffusion term (p_R - p_L) / (fa rho_1/2 a_1/2^2) / 4, rho_1/2 = (rho_L + rho_R) / 2
-            Mh = Mh - ((pos_part(1.0 - Mb2) * (pR - pL)) * (iah * iah)) * (0.5 * rcp_pos(fa * rsum));
+            const double xmo = min_nonneg(1.0, max_nonneg(pos_part(__fma_rn(0.5, qs, 1.0)), 0.3 * 0.3));
+            const double Mo = fp.mul(xmo, face_rsqrt(xmo));
+            const double fa = fp.mul(Mo, __fma_rn(-Mo, fp.one, 2.0));
+            const double fr = fp.mul(fa, rsum);
+            // pressure diffusion: M_1/2 less (1 - Mb^2)^+ (p_R - p_L) / (4 fa rho_1/2
+            // a_1/2^2) with rho_1/2 = (rho_L + rho_R)/2, as 4 M_1/2 less
+            // (-qs)^+ (p_R - p_L) / (fa (rho_L + rho_R) a_1/2^2)
+            const double pd = fp.mul(fp.mul(pos_part(-qs), fp.sub(pR, pL)), fp.mul(iah, iah));
+            const double Mh = __dmul_rn(0.25, __fma_rn(-pd, face_rcp(fr), fp.sub(m4L, m4R)));
             double modM = fabs(Mh);
-            if (nonneg_le(modM, 0.3)) modM = (Mh * Mh + 0.3 * 0.3) * (1.0 / (2.0 * 0.3));
+            if (nonneg_le(modM, 0.3)) modM = __dmul_rn(__fma_rn(Mh, Mh, 0.3 * 0.3), 1.0 / (2.0 * 0.3));
             // alpha = 3/16 (-4 + 5 fa^2) as (15/16 fa) fa - 3/4
-            const double alpha = fma((15.0 / 16.0) * fa, fa, -0.75);
-            const double PLp = split_pres_p(ML, alpha), PRm = split_pres_m(MR, alpha);
-            double ph = PLp * pL + PRm * pR;
-            ph = ph - ((((0.75 * PLp) * PRm) * rsum) * (fa * ah)) * (vR - vL);
-            fs[FS_LAMBDA] = ah;
-            fs[FS_MH] = Mh;
-            fs[FS_MODM] = modM;
-            fs[FS_PH] = ph;
-            fs[FS_PL] = epL;
-            fs[FS_PR] = epR;
+            const double alpha = __fma_rn(__dmul_rn(15.0 / 16.0, fa), fa, -0.75);
+            const double PLp = __fma_rn(alpha, mqL, __dmul_rn(0.25, gL)), PRm = __fma_rn(-alpha, mqR, __dmul_rn(0.25, gR));
+            const double pu = fp.mul(fp.mul(fp.mul(PLp, PRm), fp.mul(fr, ah)), fp.sub(vR, vL));
+            ph = __fma_rn(-0.75, pu, __fma_rn(PLp, pL, fp.mul(PRm, pR)));
+            // mass-flux weights with the wave speed folded in: the flux of a
+            // component (M/2 (fL + fR) - |M|/2 (fR - fL)) a_half is wL fL + wR fR
+            // with wL = (M + |M|) a_half / 2, wR = (M - |M|) a_half / 2
+            const double ahh = __dmul_rn(0.5, ah);
+            const double cmh = fp.mul(Mh, ahh), cmod = fp.mul(modM, ahh);
+            wL = fp.add(cmh, cmod);
+            wR = fp.sub(cmh, cmod);
         }
-        // viscous stress (compute_flux_3d.H:293-367); lagged primitive velocities
+        // Viscous stress (compute_flux_3d.H:293-367), lagged primitive
+        // velocities.  Only the row of the face normal is needed: off the diagonal
+        // mu (dV_a/dx_d + dV_d/dx_a), on it mu (2 dV_d/dx_d - 2/3 div V), where
+        // the divergence needs the two transverse diagonal derivatives, so
+        // mu (4/3 dV_d/dx_d - 2/3 (dV_t1/dx_t1 + dV_t2/dx_t2)): 7 of the 9
+        // gradients.  A transverse derivative is ((a + b) - (c + d)) / (4 dx);
+        // all scales sit in multiply-adds.
         const double* V0 = S.p + VELX * S.ns;
         const double* V1 = S.p + VELY * S.ns;
         const double* V2 = S.p + VELZ * S.ns;
-        // transverse derivatives (0.5 (a + b) - 0.5 (c + d)) / (2 dx) formed as
-        // ((a + b) - (c + d)) / (4 dx)
-        const double ids = B.idx[d], iq1 = 0.25 * B.idx[t1], iq2 = 0.25 * B.idx[t2];
-        // Only the stress row of the face normal is needed: tau_{d a} uses the
-        // normal derivatives of all three velocities, the two transverse
-        // derivatives of the normal velocity, and the divergence's two other
-        // diagonal terms (7 of the 9 gradients, 3 of the 9 stresses).
         const double* Vd = (d == 0) ? V0 : (d == 1) ? V1 : V2;
         const double* Vt1 = (t1 == 0) ? V0 : (t1 == 1) ? V1 : V2;
         const double* Vt2 = (t2 == 0) ? V0 : (t2 == 1) ? V1 : V2;
-        // normal differences; the derivative (x 1/dx) is formed only where the
-        // divergence needs it, the shear terms fold the scale into an FMA
-        const double dn[3] = {V0[oR] - V0[oL], V1[oR] - V1[oL], V2[oR] - V2[oL]};
-        const double gnd = dn[d] * ids;
-        const double d_t1 = ((Vd[oL + st1] + Vd[oR + st1]) - (Vd[oL - st1] + Vd[oR - st1])) * iq1;
-        const double d_t2 = ((Vd[oL + st2] + Vd[oR + st2]) - (Vd[oL - st2] + Vd[oR - st2])) * iq2;
-        // the divergence's two transverse diagonal terms, each scaled inside
-        // the FMA that adds it: div V = dV_d/dx_d + dV_t1/dx_t1 + dV_t2/dx_t2
-        const double s1 = (Vt1[oL + st1] + Vt1[oR + st1]) - (Vt1[oL - st1] + Vt1[oR - st1]);
-        const double s2 = (Vt2[oL + st2] + Vt2[oR + st2]) - (Vt2[oL - st2] + Vt2[oR - st2]);
+        const double vdL = Vd[oL], vdR = Vd[oR], v1L = Vt1[oL], v1R = Vt1[oR], v2L = Vt2[oL], v2R = Vt2[oR];
+        const double e1 = fp.sub(fp.add(Vd[oL + st1], Vd[oR + st1]), fp.add(Vd[oL - st1], Vd[oR - st1]));
+        const double e2 = fp.sub(fp.add(Vd[oL + st2], Vd[oR + st2]), fp.add(Vd[oL - st2], Vd[oR - st2]));
+        const double s1 = fp.sub(fp.add(Vt1[oL + st1], Vt1[oR + st1]), fp.add(Vt1[oL - st1], Vt1[oR - st1]));
+        const double s2 = fp.sub(fp.add(Vt2[oL + st2], Vt2[oR + st2]), fp.add(Vt2[oL - st2], Vt2[oR - st2]));
         // viscosity always from cells (i,j,k) and (i-1,j,k) (compute_flux_3d.H:179)
         const double mu = (P.visc_mode == MFG_TRANSPORT_CONST)
                               ? P.visc_hm
                               : harmonic_mean(blend(P.visc_mode, P.visc_gas, P.visc_solid, vf[oR]),
                                               blend(P.visc_mode, P.visc_gas, P.visc_solid, vf[oR - 1]));
-        const double delu = fma(s2, iq2, fma(s1, iq1, gnd));
-        // face velocities times 2 (the halving moves to the work sum)
-        const double fv2[3] = {V0[oL] + V0[oR], V1[oL] + V1[oR], V2[oL] + V2[oR]};
+        const double taud = fp.mul(mu, __fma_rn(fp.sub(vdR, vdL), B.i43[d],
+                                                __fma_rn(s1, B.iq23[t1], fp.mul(s2, B.iq23[t2]))));
+        const double tau1 = fp.mul(mu, __fma_rn(fp.sub(v1R, v1L), B.idx[d], fp.mul(e1, B.iq[t1])));
+        const double tau2 = fp.mul(mu, __fma_rn(fp.sub(v2R, v2L), B.idx[d], fp.mul(e2, B.iq[t2])));
+        // twice the viscous work sum_a tau_{d a} v_a of the energy flux
+        vise2 = __fma_rn(taud, fp.add(vdL, vdR), __fma_rn(tau1, fp.add(v1L, v1R), fp.mul(tau2, fp.add(v2L, v2R))));
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            // tau_{d a}: mu (2 dV_d/dx_d - 2/3 div V) on the diagonal, else
-            // mu (dV_d/dx_a + dV_a/dx_d)
-            const double tn = (a == d) ? mu * (2.0 * gnd - kTwo3rd * delu)
-                                       : mu * fma(dn[a], ids, (a == t1) ? d_t1 : d_t2);
-            fs[FS_VIS + a] = tn;
-        }
-        // the viscous work sum_a tau_{d a} v_a of the energy flux
-        fs[FS_VISE] = 0.5 * fma(fs[FS_VIS + 0], fv2[0], fma(fs[FS_VIS + 1], fv2[1], fs[FS_VIS + 2] * fv2[2]));
+        for (int a = 0; a < 3; ++a) vis[a] = (a == d) ? taud : (a == t1) ? tau1 : tau2;
     }
     if (P.do_ns) {
         // heat conduction (compute_flux_3d.H:373-374), conductivity from (i,j,k),(i-1,j,k)
@@ -406,46 +413,35 @@ __device__ __forceinline__ void face_body_at(const RhsBox& B, int d, const Idx3&
                               : harmonic_mean(blend(P.cond_mode, P.cond_gas, P.cond_solid, vf[oR]),
                                               blend(P.cond_mode, P.cond_gas, P.cond_solid, vf[oR - 1]));
         const double* T = S.p + TEMP * S.ns;
-        fs[FS_THERM] = kc * ((T[oR] - T[oL]) * B.idx[d]);
+        therm = fp.mul(kc, fp.mul(fp.sub(T[oR], T[oL]), B.idx[d]));
     }
-    if (SOLID_SIDE || (P.do_ns && P.order_hyp <= 2)) {
+    if (SOLID_SIDE || (P.do_ns && ord <= 2)) {
         // AUSM+-up: the face thread holds the face states and the scheme scalars,
         // so it writes every component's complete flux (no per-component pass).
         const Fab& O = B.flx[d];
         const int64_t qo = O.off(f.i, f.j, f.k);
         const Fab& U = B.uflux[d];
         const int64_t qu = U.p ? U.off(f.i, f.j, f.k) : 0;
-        // AUSM+-up mass-flux weights of the face, the wave speed folded in:
-        // fh = (M/2 (fL + fR) - |M|/2 (fR - fL)) a_half per component, as
-        // wL fL + wR fR with wL = (M + |M|) a_half / 2, wR = (M - |M|) a_half / 2
-        // (two FP64 operations per component instead of four)
-        const double cmh = (0.5 * fs[FS_MH]) * fs[FS_LAMBDA], cmod = (0.5 * fs[FS_MODM]) * fs[FS_LAMBDA];
-        const double wL = cmh + cmod, wR = cmh - cmod;
 #pragma unroll
         for (int c = 0; c < NCONS + NS; ++c) {
             if (c >= NCONS + P.nspec) break;
             const int sc = (c < NCONS) ? c : c + (NFLO - NCONS);
             double F = 0.0;
             if (active) {
-                double fL = uL[c], fR = uR[c];
-                if (c == RHOE) {
-                    fL = fs[FS_PL];
-                    fR = fs[FS_PR];
-                }
-                double fh = fma(wR, fR, wL * fL);
-                if (c == 1 + d) fh += fs[FS_PH];
-                F = (c < NCONS) ? fh : P.advect_flag[c - NCONS] * fh;
-                if (c >= RHOU && c <= RHOW) F -= fs[FS_VIS + c - 1];
-                if (c == RHOE) F -= fs[FS_VISE];
+                F = __fma_rn(wR, uR[c], fp.mul(wL, uL[c]));
+                if (c == 1 + d) F = fp.add(F, ph);
+                if (c >= NCONS && !is_one(P.advect_flag[c - NCONS])) F = fp.mul(P.advect_flag[c - NCONS], F);
+                if (c >= RHOU && c <= RHOW) F = fp.sub(F, vis[c - 1]);
+                if (c == RHOE) F = __fma_rn(-0.5, vise2, F);
             }
-            if (c == RHOE) F -= fs[FS_THERM];
+            if (c == RHOE) F = fp.sub(F, therm);
             if (c >= NCONS) {
                 const int s = c - NCONS;
                 const double Dh = (P.diff_mode[s] == MFG_TRANSPORT_CONST)
                                       ? P.diff_hm[s]
                                       : harmonic_mean(blend(P.diff_mode[s], P.diff_gas[s], P.diff_solid[s], vf[oL]),
                                                       blend(P.diff_mode[s], P.diff_gas[s], P.diff_solid[s], vf[oR]));
-                F -= (Dh * (S.p[oR + sc * S.ns] - S.p[oL + sc * S.ns])) * B.idx[d];
+                F = __fma_rn(-fp.mul(Dh, fp.sub(S.p[oR + sc * S.ns], S.p[oL + sc * S.ns])), B.idx[d], F);
             }
             O.p[qo + c * O.ns] = F;
             if (U.p) U.p[qu + sc * U.ns] = F;
@@ -454,28 +450,28 @@ __device__ __forceinline__ void face_body_at(const RhsBox& B, int d, const Idx3&
             for (int z = NCONS; z < NFLO; ++z) U.p[qu + z * U.ns] = 0.0;
         return;
     }
-    // what the flux pass of this face reads: the AUSM+-up scalars only for
-    // orders 1/2; lambda and the viscous terms only where active.  FS_MH is
-    // zero for orders 4/5 (the adjoint sums the eigenvalue's adjoint there).
+    // orders 4, 5: what the flux pass of this face reads
     const Fab& F = B.fs[d];
-    const int64_t q = F.off(f.i, f.j, f.k);
-    const bool ausm = P.order_hyp <= 2;
+    double* q = F.p + F.off(f.i, f.j, f.k);
+    q[FS_FLAGS * F.ns] = __longlong_as_double((active ? 1 : 0) | ((P.do_ns && fallback) ? 2 : 0));  // bit pattern
+    q[FS_MH * F.ns] = 0.0;
+    q[FS_THERM * F.ns] = therm;
+    if (active) {
+        q[FS_LAMBDA * F.ns] = lam;
 #pragma unroll
-    for (int c = 0; c < NFS; ++c) {
-        if (!(c == FS_FLAGS || c == FS_MH || c == FS_THERM) && !active) continue;
-        if (c >= FS_MODM && c <= FS_PR && !ausm) continue;
-        F.p[q + c * F.ns] = fs[c];
+        for (int a = 0; a < 3; ++a) q[(FS_VIS + a) * F.ns] = vis[a];
+        q[FS_VISE * F.ns] = __dmul_rn(0.5, vise2);
     }
 }
 
 // Face t (linear index over growHi(bx, d, 1)) of direction d.
 template <int NS>
-__device__ __forceinline__ void face_body(const RhsBox& B, int d, int64_t t) {
+__device__ __forceinline__ void face_body(const Fp& fp, const RhsBox& B, int d, int64_t t) {
     int lo[3] = {B.lo[0], B.lo[1], B.lo[2]}, len[3];
     for (int e = 0; e < 3; ++e) len[e] = B.hi[e] - B.lo[e] + 1 + (e == d);
     const int64_t nf = (int64_t)len[0] * len[1] * len[2];
     if (t >= nf) return;
-    face_body_at<NS>(B, d, delinear(t, lo, len));
+    face_body_at<NS>(fp, B, d, delinear(t, lo, len));
 }
 
 // ---------------------------------------------------------------------------
@@ -502,10 +498,10 @@ __device__ __forceinline__ void flux_body(const RhsBox& B, int d, int c, int64_t
 
     double F = 0.0;
     if (P.do_ns) {
-        if (active) {
+        if (active) {  // orders 4 and 5 (the face kernels write the fluxes of orders 1 and 2)
             const int ord = P.order_hyp;
             double fh;
-            if (ord == 5 || ord == 4) {
+            {
                 const Fab& X = B.aux;
                 const int64_t xd = (d == 0) ? 1 : (d == 1) ? X.js : X.ks;
                 const int64_t xR = X.off(f.i, f.j, f.k);
@@ -534,23 +530,6 @@ __device__ __forceinline__ void flux_body(const RhsBox& B, int d, int c, int64_t
                     fh = kTwelveth * (((7.0 * fl[3] + 7.0 * fl[2]) - fl[1]) - fl[4]);
                     fh -= ((kTwelveth * (((3.0 * us[3] - 3.0 * us[2]) - us[4]) + us[3])) * lam) * P.dissfactor;
                 }
-            } else {
-                double ul = u[oL], ur = u[oR], uLh = ul, uRh = ur;
-                if (ord == 2) {
-                    const double ulm1 = fallback ? ul : u[oL - sd];
-                    const double urp1 = fallback ? ur : u[oR + sd];
-                    muscl(ulm1, ul, ur, urp1, uLh, uRh);
-                }
-                const double Mh = FS.p[qf + FS_MH * FS.ns];
-                const double modM = FS.p[qf + FS_MODM * FS.ns];
-                const double ah = FS.p[qf + FS_LAMBDA * FS.ns];
-                double fL = uLh, fR = uRh;
-                if (c == RHOE) {
-                    fL = FS.p[qf + FS_PL * FS.ns];
-                    fR = FS.p[qf + FS_PR * FS.ns];
-                }
-                fh = ((0.5 * Mh) * (fL + fR) - (0.5 * modM) * (fR - fL)) * ah;
-                if (c == 1 + d) fh += FS.p[qf + FS_PH * FS.ns];
             }
             F = (c < NCONS) ? fh : P.advect_flag[c - NCONS] * fh;
             if (c >= RHOU && c <= RHOW) F -= FS.p[qf + (FS_VIS + c - 1) * FS.ns];
@@ -704,23 +683,6 @@ __device__ __forceinline__ void update_body(const RhsBox& B, int stage, double d
 // 0.57 ms with the fixed-point weights (23 operations).
 // ---------------------------------------------------------------------------
 constexpr int SWEEP_SEG = 32;  // longest face segment per thread (batched launches)
-
-// FP64 sums and products as fused multiply-adds with 1 and -0 in registers:
-// bitwise the add and the multiply, at the fused multiply-add's rate (a warp
-// holds the FP64 pipe for 70 cycles; DADD and DMUL, and fused multiply-adds
-// with an operand from the constant bank or an immediate, for 82).  The two
-// constants pass through a shuffle so that they stay in registers; every lane
-// of the warp constructs it.
-struct Fp {
-    double one, nz;
-    __device__ __forceinline__ Fp() {
-        one = __hiloint2double(__shfl_sync(0xffffffffu, 0x3ff00000, 0), 0);
-        nz = __hiloint2double(__shfl_sync(0xffffffffu, (int)0x80000000, 0), 0);
-    }
-    __device__ __forceinline__ double add(double a, double b) const { return __fma_rn(a, one, b); }
-    __device__ __forceinline__ double sub(double a, double b) const { return __fma_rn(b, -one, a); }
-    __device__ __forceinline__ double mul(double a, double b) const { return __fma_rn(a, b, nz); }
-};
 
 __device__ __forceinline__ double weight_of(uint64_t bits) { return __longlong_as_double((long long)bits); }
 __device__ __forceinline__ WenoInd weno_ind(double Dm, double Dp) {

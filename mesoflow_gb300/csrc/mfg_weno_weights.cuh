@@ -14,51 +14,9 @@
 // Everything is integer arithmetic but the 23-bit seed of the reciprocal, so
 // every kernel that uses it gets the same bits.
 #pragma once
-#include <stdint.h>
-#include <string.h>
-
-#ifdef __CUDACC__
-#define MFG_HD __host__ __device__ __forceinline__
-#else
-#define MFG_HD inline
-#endif
+#include "mfg_fixed.cuh"
 
 namespace mfg {
-
-MFG_HD uint64_t umulhi64(uint64_t a, uint64_t b) {
-#ifdef __CUDA_ARCH__
-    return __umul64hi(a, b);
-#else
-    return (uint64_t)(((unsigned __int128)a * b) >> 64);
-#endif
-}
-
-MFG_HD int clz32(uint32_t x) {  // x != 0
-#ifdef __CUDA_ARCH__
-    return __clz((int)x);
-#else
-    return __builtin_clz(x);
-#endif
-}
-
-// Bits of the float32 1/f, f in (1, 2), relative error below 2^-22.
-MFG_HD uint32_t rcp_seed_bits(uint32_t fbits) {
-#ifdef __CUDA_ARCH__
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint_as_float(fbits)));
-    return __float_as_uint(r);
-#else
-    float f;
-    memcpy(&f, &fbits, 4);
-    f = 1.0f / f;
-    uint32_t b;
-    memcpy(&b, &f, 4);
-    return b;
-#endif
-}
-
-MFG_HD int imin(int a, int b) { return a < b ? a : b; }
-MFG_HD int imax(int a, int b) { return a > b ? a : b; }
 
 // A cell difference split: |D| = m 2^(e - 1083), 2^60 <= m < 2^61 (zero and
 // denormals read as about 2^-1023, far below the exponent floor).
@@ -113,22 +71,6 @@ MFG_HD WenoInd weno_ind(const WenoDiff& a, const WenoDiff& b) {
     r.eB = 2 * E - zB;
     r.eC = 2 * E - zC;
     return r;
-}
-
-// 2^126 / d for a normalised d (top bit set), relative error below 2^-59: the
-// float32 seed r0 (e = 1 - x r0, |e| < 2^-21) corrected by r0 (1 + e + e^2).
-MFG_HD uint64_t rcp_fixed(uint64_t d) {
-    const uint32_t dh = (uint32_t)(d >> 32), dl = (uint32_t)d;
-    uint32_t rb = rcp_seed_bits(0x3f800000u | ((dh & 0x7fffffffu) >> 8) | 1u);
-    rb = rb < 0x3f000000u ? 0x3f000000u : rb > 0x3f7fffffu ? 0x3f7fffffu : rb;  // in [1/2, 1)
-    const uint32_t R0 = ((rb & 0x7fffffu) | 0x800000u) << 7;                     // r0 2^31
-    const uint64_t T = (uint64_t)dh * R0 + (((uint64_t)dl * R0) >> 32);          // (1 - e) 2^62
-    const int64_t e = (int64_t)((1ull << 62) - T);
-    const int32_t es = (int32_t)(e >> 18);
-    const int64_t g = e + (((int64_t)es * es) >> 26);  // (e + e^2) 2^62
-    const int32_t gh = (int32_t)(g >> 32);
-    const uint32_t gl = (uint32_t)g;
-    return ((uint64_t)R0 << 32) + (uint64_t)(((int64_t)gh * (int32_t)R0) << 2) + (((uint64_t)R0 * gl) >> 30);
 }
 
 // w 2^-62 2^k as the bits of a double, truncated (0 reads as 2^(k-62)).
