@@ -1296,6 +1296,7 @@ struct Work {
     CopyTab* d_tab = nullptr;  // [nbox] -> lam, [nbox] -> lamOld
     AdjBox* d_adj = nullptr;   // the stage's AdjBox views of every box (batched adjoint flux)
     double* d_scratch = nullptr;
+    bool grouped = true;  // d_scratch holds a group of boxes (rhs_group_count)
     int* d_list = nullptr;
     unsigned* d_count = nullptr;
     double* d_g = nullptr;  // [J, d/du_in, d/dlog A_r ...]
@@ -1421,10 +1422,7 @@ int fwd_step(Work& W, double dt, const Snap* snap, cudaStream_t st) {
     const int N = W.N;
     Fab none;
     memset(&none, 0, sizeof(none));
-    for (int b = 0; b < W.nbox; ++b)
-        ADJ_TRY(launch_axpy_valid(W.boxes[b], make_fab(W.boxes[b].s_old), none, 0.0, true,
-                                  make_fab(W.boxes[b].s_new), N, st),
-                "forward: phi_old copy");
+    ADJ_TRY(launch_copy_old(W.boxes.data(), W.nbox, N, st), "forward: phi_old copy");
     for (int stage = 1; stage <= 3; ++stage) {
         ADJ_TRY(launch_fill_patch(W.boxes.data(), W.nbox, W.g, stage == 1 ? 0 : 1, 0.0, st), "forward: fill patch");
         // the level-wide pass of mfg_cutcells, else box by box (bitwise the same)
@@ -1433,22 +1431,31 @@ int fwd_step(Work& W, double dt, const Snap* snap, cudaStream_t st) {
         if (lv == 0)
             for (int b = 0; b < W.nbox; ++b)
                 ADJ_TRY(launch_cutcells_box(W.boxes[b], W.g, nullptr, W.d_list, W.d_count, st), "forward: cut cells");
-        for (int b = 0; b < W.nbox; ++b) {
-            const mfg_box& x = W.boxes[b];
-            if (snap) {
-                const int lo[3] = {x.lo[0] - 3, x.lo[1] - 3, x.lo[2] - 3};
-                const int hi[3] = {x.hi[0] + 3, x.hi[1] + 3, x.hi[2] + 3};
-                ADJ_TRY(copy_region(W.gfab(snap->sb[stage - 1], b, N), make_fab(x.sborder), lo, hi, N, st),
-                        "forward: stage snapshot");
+        for (int b = 0; b < W.nbox;) {
+            const int n = W.grouped ? rhs_group_count(W.boxes.data() + b, W.nbox - b) : 1;
+            RhsBox B[kRhsGroup];
+            double* scratch = W.d_scratch;
+            for (int q = 0; q < n; ++q) {
+                const mfg_box& x = W.boxes[b + q];
+                if (snap) {
+                    const int lo[3] = {x.lo[0] - 3, x.lo[1] - 3, x.lo[2] - 3};
+                    const int hi[3] = {x.hi[0] + 3, x.hi[1] + 3, x.hi[2] + 3};
+                    ADJ_TRY(copy_region(W.gfab(snap->sb[stage - 1], b + q, N), make_fab(x.sborder), lo, hi, N, st),
+                            "forward: stage snapshot");
+                }
+                B[q] = layout_rhs_box(x, W.g, scratch);
+                scratch += rhs_box_scratch_doubles(x);
+                if (snap) snap_views(W, B[q], *snap, stage, b + q);  // keep the stage's primitives and face scalars
             }
-            RhsBox B = layout_rhs_box(x, W.g, W.d_scratch);
-            if (snap) snap_views(W, B, *snap, stage, b);  // keep the stage's primitives and face scalars
-            ADJ_TRY(launch_rhs_box(B, stage, dt, weno_fast_mode(), st), "forward: right-hand side");
+            ADJ_TRY(launch_rhs_boxes(B, n, stage, dt, weno_fast_mode(), st), "forward: right-hand side");
+            b += n;
         }
     }
     if (!snap) {  // no intermediates kept: the bookends in one pass, as mfg_advance_level
-        for (int b = 0; b < W.nbox; ++b)
-            ADJ_TRY(launch_post_step(W.boxes[b], dt, true, true, nullptr, nullptr, st), "forward: bookends");
+        for (int b = 0; b < W.nbox; b += kRhsGroup)
+            ADJ_TRY(launch_post_step(W.boxes.data() + b, std::min(kRhsGroup, W.nbox - b), dt, true, true, nullptr, nullptr,
+                                     st),
+                    "forward: bookends");
         return MFG_OK;
     }
     for (int b = 0; b < W.nbox; ++b) {
@@ -1661,7 +1668,7 @@ extern "C" int mfg_adjoint_objective(const mfg_box* boxes, int nbox, const mfg_g
     W.N = NFLO + P.nspec;
     W.vcell.resize(nbox);
     W.gcell.resize(nbox);
-    size_t maxcells = 0, maxscr = 0;
+    size_t maxcells = 0;
     for (int b = 0; b < nbox; ++b) {
         int n[3];
         for (int d = 0; d < 3; ++d) n[d] = boxes[b].hi[d] - boxes[b].lo[d] + 1;
@@ -1674,9 +1681,13 @@ extern "C" int mfg_adjoint_objective(const mfg_box* boxes, int nbox, const mfg_g
         W.vtot += (size_t)n[0] * n[1] * n[2];
         W.gtot += (size_t)(n[0] + 6) * (n[1] + 6) * (n[2] + 6);
         maxcells = std::max(maxcells, (size_t)n[0] * n[1] * n[2]);
-        maxscr = std::max(maxscr, rhs_box_scratch_doubles(n));
     }
-    ADJ_TRY(cudaMalloc(&W.d_scratch, maxscr * sizeof(double)), "allocation");
+    // scratch for the forward's groups of boxes, or box by box where memory is short for that
+    if (cudaMalloc(&W.d_scratch, rhs_list_scratch_doubles(boxes, nbox, true) * sizeof(double)) != cudaSuccess) {
+        cudaGetLastError();
+        W.grouped = false;
+        ADJ_TRY(cudaMalloc(&W.d_scratch, rhs_list_scratch_doubles(boxes, nbox, false) * sizeof(double)), "allocation");
+    }
     ADJ_TRY(cudaMalloc(&W.d_list, maxcells * sizeof(int)), "allocation");
     ADJ_TRY(cudaMalloc(&W.d_count, 256), "allocation");
     ADJ_TRY(cudaMalloc(&W.d_g, (2 + MAXR) * sizeof(double)), "allocation");

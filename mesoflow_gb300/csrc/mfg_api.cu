@@ -179,18 +179,37 @@ RhsBox make_rhs_box(const mfg_box& b, const mfg_geom& g, double* base) {
     return B;
 }
 
+// Lays the boxes of a group out one after the other from base.
+void make_rhs_group(const mfg_box* boxes, int n, const mfg_geom& g, double* base, RhsBox* out) {
+    for (int b = 0; b < n; ++b) {
+        out[b] = make_rhs_box(boxes[b], g, base);
+        base += rhs_box_scratch_doubles(boxes[b]);
+    }
+}
+
+// Reserves the pool for the right-hand sides of a list plus `more` doubles:
+// for groups of boxes, or box by box where memory is short for that.
+cudaError_t reserve_rhs(const mfg_box* boxes, int nbox, size_t more, cudaStream_t st, size_t* need, bool* grouped) {
+    *grouped = true;
+    *need = rhs_list_scratch_doubles(boxes, nbox, true);
+    cudaError_t e = pool_reserve((*need + more) * sizeof(double), st);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    *grouped = false;
+    *need = rhs_list_scratch_doubles(boxes, nbox, false);
+    return pool_reserve((*need + more) * sizeof(double), st);
+}
+
 int run_rhs(const mfg_box* boxes, int nbox, const mfg_geom* geom, int stage, double dt, cudaStream_t st) {
     size_t need = 0;
-    for (int b = 0; b < nbox; ++b) {
-        int n[3];
-        for (int d = 0; d < 3; ++d) n[d] = boxes[b].hi[d] - boxes[b].lo[d] + 1;
-        need = std::max(need, rhs_scratch_doubles(n));
-    }
-    cudaError_t e = pool_reserve(need * sizeof(double), st);
-    if (e != cudaSuccess) return MFG_ERR_CUDA;
-    for (int b = 0; b < nbox; ++b) {
-        RhsBox B = make_rhs_box(boxes[b], *geom, reinterpret_cast<double*>(g_pool.p));
-        if ((e = launch_rhs_box(B, stage, dt, g_fast_weno, st)) != cudaSuccess) return MFG_ERR_CUDA;
+    bool grouped = true;
+    if (reserve_rhs(boxes, nbox, 0, st, &need, &grouped) != cudaSuccess) return MFG_ERR_CUDA;
+    RhsBox B[kRhsGroup];
+    for (int b = 0; b < nbox;) {
+        const int n = grouped ? rhs_group_count(boxes + b, nbox - b) : 1;
+        make_rhs_group(boxes + b, n, *geom, reinterpret_cast<double*>(g_pool.p), B);
+        if (launch_rhs_boxes(B, n, stage, dt, g_fast_weno, st) != cudaSuccess) return MFG_ERR_CUDA;
+        b += n;
     }
     return MFG_OK;
 }
@@ -208,6 +227,22 @@ int validate_boxes(const mfg_box* boxes, int nbox, bool need_sb, bool need_dsdt,
     return check_boxes(boxes, nbox, need_sb, need_dsdt, need_old, need_new);
 }
 size_t rhs_box_scratch_doubles(const int n[3]) { return rhs_scratch_doubles(n); }
+size_t rhs_box_scratch_doubles(const mfg_box& b) {
+    int n[3];
+    for (int d = 0; d < 3; ++d) n[d] = b.hi[d] - b.lo[d] + 1;
+    return rhs_scratch_doubles(n);
+}
+size_t rhs_list_scratch_doubles(const mfg_box* boxes, int nbox, bool grouped) {
+    size_t need = 0;
+    for (int b = 0; b < nbox;) {
+        const int n = grouped ? rhs_group_count(boxes + b, nbox - b) : 1;
+        size_t s = 0;
+        for (int q = 0; q < n; ++q) s += rhs_box_scratch_doubles(boxes[b + q]);
+        need = std::max(need, s);
+        b += n;
+    }
+    return need;
+}
 RhsBox layout_rhs_box(const mfg_box& b, const mfg_geom& g, double* base) { return make_rhs_box(b, g, base); }
 bool weno_fast_mode() { return g_fast_weno; }
 
@@ -504,8 +539,7 @@ int mfg_est_timestep(const mfg_box* boxes, int nbox, const mfg_geom* geom, doubl
     if (pool_reserve(2 * sizeof(double), st) != cudaSuccess) return MFG_ERR_CUDA;
     double* acc = reinterpret_cast<double*>(g_pool.p);
     if (cudaMemsetAsync(acc, 0, 2 * sizeof(double), st) != cudaSuccess) return MFG_ERR_CUDA;
-    for (int b = 0; b < nbox; ++b)
-        if (launch_timestep(boxes[b], acc, st) != cudaSuccess) return MFG_ERR_CUDA;
+    if (launch_timestep(boxes, nbox, acc, st) != cudaSuccess) return MFG_ERR_CUDA;
     double h[2];
     if (cudaMemcpyAsync(h, acc, sizeof(h), cudaMemcpyDeviceToHost, st) != cudaSuccess) return MFG_ERR_CUDA;
     if (cudaStreamSynchronize(st) != cudaSuccess) return MFG_ERR_CUDA;
@@ -521,23 +555,18 @@ int mfg_est_timestep(const mfg_box* boxes, int nbox, const mfg_geom* geom, doubl
 // One coarse step of a single level: the swap, three RK3 stages (fill patch,
 // cut cells, fused RHS + stage algebra), the Strang chemistry sub-step, the
 // primitive refresh, species clipping and residual norms
-// (Source/mflo_evolve.cpp:251-318, 470-493, 33-58).  The bookends of box b
-// run right after its stage-3 update (the box's state is still in L2, and no
-// other box's stage 3 reads it: every box reads its own filled Sborder), in
-// box order, so the residual-norm sums run in the same order as a separate
-// pass.  With h_state, each box's phi_new is copied in from the host first and
-// copied back on the copy stream as soon as its bookends are done.
+// (Source/mflo_evolve.cpp:251-318, 470-493, 33-58).  The bookends of a group of
+// boxes run right after its stage-3 update (the boxes' states are still in L2,
+// and no other box's stage 3 reads them: every box reads its own filled
+// Sborder), in box order, so the residual-norm sums run in the same order as a
+// separate pass.  With h_state, each box's phi_new is copied in from the host
+// first and copied back on the copy stream as soon as its group's bookends are
+// done.
 static int advance_level(const mfg_box* boxes, int nbox, const mfg_geom* geom, double time, double dt,
                          int only_flow, int clip, double* resnorms, const mfg_array4* h_state, cudaStream_t st) {
     int rc;
     const int N = ncomp_total();
-    size_t need = 0;
-    for (int b = 0; b < nbox; ++b) {
-        int n[3];
-        for (int d = 0; d < 3; ++d) n[d] = boxes[b].hi[d] - boxes[b].lo[d] + 1;
-        need = std::max(need, rhs_scratch_doubles(n));
-    }
-    const size_t npart = (size_t)N * 1024;
+    const size_t npart = (size_t)kRhsGroup * N * 1024;
     cudaStream_t cs = nullptr;
     cudaEvent_t ev = nullptr;
     // every return after copies were queued on the copy stream first makes
@@ -559,12 +588,8 @@ static int advance_level(const mfg_box* boxes, int nbox, const mfg_geom* geom, d
                                 cudaMemcpyHostToDevice, st) != cudaSuccess)
                 return MFG_ERR_CUDA;
     }
-    Fab none;
-    memset(&none, 0, sizeof(none));
-    for (int b = 0; b < nbox; ++b)  // phi_old <- phi_new (std::swap of the reference)
-        if (launch_axpy_valid(boxes[b], make_fab(boxes[b].s_old), none, 0.0, true, make_fab(boxes[b].s_new), N, st) !=
-            cudaSuccess)
-            return MFG_ERR_CUDA;
+    // phi_old <- phi_new (std::swap of the reference)
+    if (launch_copy_old(boxes, nbox, N, st) != cudaSuccess) return MFG_ERR_CUDA;
     double* acc = nullptr;
     for (int stage = 1; stage <= 3; ++stage) {
         if ((rc = mfg_fill_patch(boxes, nbox, geom, stage == 1 ? 0 : 1, stage == 1 ? time : time + dt, st)))
@@ -573,26 +598,32 @@ static int advance_level(const mfg_box* boxes, int nbox, const mfg_geom* geom, d
         // the pool after the cut-cell pass (whose per-box form uses it too):
         // RHS scratch first, then the residual-norm partials and sums, which
         // must survive the later boxes' RHS launches of stage 3
-        if (pool_reserve((need + npart + N) * sizeof(double), st) != cudaSuccess) return MFG_ERR_CUDA;
+        size_t need = 0;
+        bool grouped = true;
+        if (reserve_rhs(boxes, nbox, npart + N, st, &need, &grouped) != cudaSuccess) return MFG_ERR_CUDA;
         double* scratch = reinterpret_cast<double*>(g_pool.p);
         double* part = (resnorms && stage == 3) ? scratch + need : nullptr;
         acc = part ? part + npart : nullptr;
         if (acc && cudaMemsetAsync(acc, 0, N * sizeof(double), st) != cudaSuccess) return MFG_ERR_CUDA;
-        for (int b = 0; b < nbox; ++b) {
-            RhsBox B = make_rhs_box(boxes[b], *geom, scratch);
-            if (launch_rhs_box(B, stage, dt, g_fast_weno, st) != cudaSuccess) return MFG_ERR_CUDA;
-            if (stage < 3) continue;
+        RhsBox B[kRhsGroup];
+        for (int b = 0; b < nbox;) {
+            const int n = grouped ? rhs_group_count(boxes + b, nbox - b) : 1;
+            make_rhs_group(boxes + b, n, *geom, scratch, B);
+            if (launch_rhs_boxes(B, n, stage, dt, g_fast_weno, st) != cudaSuccess) return MFG_ERR_CUDA;
             // the bookends in one pass: phi_old <- phi_new and the chemistry
             // sub-step (unless only_flow), primitive refresh, clipping, norms
-            if (launch_post_step(boxes[b], dt, !only_flow, clip != 0, part, acc, st) != cudaSuccess)
+            if (stage == 3 && launch_post_step(boxes + b, n, dt, !only_flow, clip != 0, part, acc, st) != cudaSuccess)
                 return MFG_ERR_CUDA;
-            if (h_state) {
-                if (cudaEventRecord(ev, st) != cudaSuccess || cudaStreamWaitEvent(cs, ev, 0) != cudaSuccess ||
-                    cudaMemcpyAsync(h_state[b].p, boxes[b].s_new.p,
-                                    view_span_doubles(boxes[b].s_new) * sizeof(double), cudaMemcpyDeviceToHost,
-                                    cs) != cudaSuccess)
+            if (stage == 3 && h_state) {
+                if (cudaEventRecord(ev, st) != cudaSuccess || cudaStreamWaitEvent(cs, ev, 0) != cudaSuccess)
                     return MFG_ERR_CUDA;
+                for (int q = b; q < b + n; ++q)
+                    if (cudaMemcpyAsync(h_state[q].p, boxes[q].s_new.p,
+                                        view_span_doubles(boxes[q].s_new) * sizeof(double), cudaMemcpyDeviceToHost,
+                                        cs) != cudaSuccess)
+                        return MFG_ERR_CUDA;
             }
+            b += n;
         }
     }
     if (h_state) {

@@ -523,8 +523,9 @@ __global__ void __launch_bounds__(BT) bk_cut(const CutBox* __restrict__ cb, cons
 
 template <int NS>
 __global__ void __launch_bounds__(BT) bk_prim(const RhsBox* __restrict__ B, const Tile* __restrict__ tiles, int ntiles) {
+    const Fp fp;
     TILE_LOOP
-    prim_body<NS>(B[tl.box], t);
+    prim_body<NS>(fp, B[tl.box], t);
     TILE_END
 }
 
@@ -532,7 +533,15 @@ template <int NS>
 __global__ void __launch_bounds__(BT) bk_face(const RhsBox* __restrict__ B, const Tile* __restrict__ tiles, int ntiles) {
     const Fp fp;
     TILE_LOOP
-    face_body<NS>(fp, B[tl.box], tl.part, t);
+    face_body<NS, false>(fp, B[tl.box], tl.part, t);
+    TILE_END
+}
+template <int NS>  // orders 4 and 5
+__global__ void __launch_bounds__(BT) bk_face_high(const RhsBox* __restrict__ B, const Tile* __restrict__ tiles,
+                                                   int ntiles) {
+    const Fp fp;
+    TILE_LOOP
+    face_body<NS, true>(fp, B[tl.box], tl.part, t);
     TILE_END
 }
 
@@ -568,8 +577,9 @@ bool flux_sweep_mode() {
 __global__ void __launch_bounds__(BT) bk_update(const RhsBox* __restrict__ B, const Tile* __restrict__ tiles,
                                                 int ntiles, int stage, double dt, const double* __restrict__ dtp) {
     if (dtp) dt = *dtp;
+    const Fp fp;
     TILE_LOOP
-    update_body(B[tl.box], stage, dt, tl.part, t);
+    update_body(fp, B[tl.box], stage, dt, tl.part, t);
     TILE_END
 }
 
@@ -991,7 +1001,11 @@ void b_rhs(mfg_boxlist& L, const TSet& TS, int stage, double dt, cudaStream_t st
     {
         const PhaseTiles& T = TS[PH_FACE];
         ProfScope ps(K_FACE, st);
-        NS_DISPATCH(bk_face, (T.grid, BT, 0, st), (L.d_rhs, T.d, T.n));
+        if (ord >= 4) {
+            NS_DISPATCH(bk_face_high, (T.grid, BT, 0, st), (L.d_rhs, T.d, T.n));
+        } else {
+            NS_DISPATCH(bk_face, (T.grid, BT, 0, st), (L.d_rhs, T.d, T.n));
+        }
     }
     if (!(c_host_params().do_ns && ord <= 2)) {
         const PhaseTiles& T = TS[PH_FLUX];

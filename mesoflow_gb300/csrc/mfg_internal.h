@@ -70,6 +70,9 @@ const DevParams& c_host_params();
 // Box validation, scratch size and scratch layout of the RHS (mfg_api.cu).
 int validate_boxes(const mfg_box* boxes, int nbox, bool need_sb, bool need_dsdt, bool need_old, bool need_new);
 size_t rhs_box_scratch_doubles(const int n[3]);
+size_t rhs_box_scratch_doubles(const mfg_box& b);
+// Scratch of the largest group (grouped) or of the largest box of a list.
+size_t rhs_list_scratch_doubles(const mfg_box* boxes, int nbox, bool grouped);
 struct RhsBox;
 RhsBox layout_rhs_box(const mfg_box& b, const mfg_geom& g, double* base);
 bool weno_fast_mode();
@@ -80,6 +83,17 @@ cudaError_t read_status(unsigned* v, bool clear);
 // Records the description of a failed CUDA call for mfg_last_error (mfg_api.cu).
 void note_cuda_error(cudaError_t e, const char* where);
 cudaError_t launch_rhs_box(const RhsBox& B, int stage, double dt, bool fast, cudaStream_t st);
+
+// Boxes that share the launches of one right-hand side: up to kRhsGroup
+// consecutive ones of together at most kRhsGroupCells cells (one 64^3 box:
+// larger ones fill the GPU by themselves), each with scratch of its own.
+constexpr int kRhsGroup = 8;
+constexpr int64_t kRhsGroupCells = 64 * 64 * 64;
+// Number of the leading boxes of the list that form a group (at least 1).
+int rhs_group_count(const mfg_box* boxes, int nbox);
+cudaError_t launch_rhs_boxes(const RhsBox* boxes, int n, int stage, double dt, bool fast, cudaStream_t st);
+cudaError_t launch_rhs_group(const RhsBox* boxes, int n, int stage, double dt, bool fast, bool split_on,
+                             cudaStream_t st);
 
 // Scratch sizes (doubles) for a box of the given valid extent.
 inline size_t aux_doubles(const int n[3]) {
@@ -102,9 +116,10 @@ cudaError_t launch_axpy_valid(const mfg_box& b, const Fab& dst, const Fab& src, 
 cudaError_t launch_update_prims(const mfg_box& b, double* minp_slot, cudaStream_t st);
 cudaError_t launch_split_chem(const mfg_box& b, int kind, double dt, int bg, cudaStream_t st);
 cudaError_t launch_clip_species(const mfg_box& b, cudaStream_t st);
-cudaError_t launch_post_step(const mfg_box& b, double dt, bool chem, bool clip, double* partial, double* acc,
+cudaError_t launch_post_step(const mfg_box* boxes, int n, double dt, bool chem, bool clip, double* partial, double* acc,
                              cudaStream_t st);
-cudaError_t launch_timestep(const mfg_box& b, double* acc2, cudaStream_t st);
+cudaError_t launch_timestep(const mfg_box* boxes, int nbox, double* acc2, cudaStream_t st);
+cudaError_t launch_copy_old(const mfg_box* boxes, int nbox, int ncomp, cudaStream_t st);
 
 cudaError_t launch_fill_patch(const mfg_box* boxes, int nbox, const mfg_geom& g, int s_src, double time,
                               cudaStream_t st);

@@ -115,7 +115,7 @@ __device__ __forceinline__ double eig_speed(double gam, double kap, double rhoe,
 // prim_kernel: per-cell scalars over grow(bx, 3)
 // ---------------------------------------------------------------------------
 template <int NS>
-__device__ __forceinline__ void prim_body(const RhsBox& B, int64_t t) {
+__device__ __forceinline__ void prim_body(const Fp& fp, const RhsBox& B, int64_t t) {
     int lo[3], len[3];
     for (int d = 0; d < 3; ++d) {
         lo[d] = B.lo[d] - MFG_NGROW;
@@ -135,12 +135,14 @@ __device__ __forceinline__ void prim_body(const RhsBox& B, int64_t t) {
     // cons_to_prim (consprim_funcs.H:9-23); one Newton-refined reciprocal of
     // the density replaces the reference's five divisions by it
     const double irho = rcp_pos(rho);
-    const double vx = m0 * irho, vy = m1 * irho, vz = m2 * irho;
-    const double rhoe = E - (0.5 * rho) * ((vx * vx + vy * vy) + vz * vz);
+    const double vx = fp.mul(m0, irho), vy = fp.mul(m1, irho), vz = fp.mul(m2, irho);
+    const double k2 = __fma_rn(vx, vx, __fma_rn(vy, vy, fp.mul(vz, vz)));
+    const double rhoe = __fma_rn(-__dmul_rn(0.5, rho), k2, E);
     const double kap = thermo_kappa<NS>(rho, spec);
-    const double pf = rhoe * kap;
+    const double pf = fp.mul(rhoe, kap);
     // get_max_eigenvalue's own-species terms (flux_schemes.H:21-43)
-    const double reig = E - (0.5 * ((m0 * m0 + m1 * m1) + m2 * m2)) * irho;
+    const double mm = __fma_rn(m0, m0, __fma_rn(m1, m1, fp.mul(m2, m2)));
+    const double reig = __fma_rn(-__dmul_rn(0.5, mm), irho, E);
     const double aown = eig_speed(1.0 + kap, kap, reig, irho);
     const Fab& X = B.aux;
     const int64_t q = X.off(c.i, c.j, c.k);
@@ -166,13 +168,13 @@ __device__ __forceinline__ int64_t face_count(const RhsBox& B, int d) {
 // Whether face f of direction d takes the flux branch of face_body
 // (Navier-Stokes terms on and face volume fraction >= 1/2), by the same
 // arithmetic.
-__device__ __forceinline__ bool face_active(const RhsBox& B, int d, const Idx3& f) {
+__device__ __forceinline__ bool face_active(const Fp& fp, const RhsBox& B, int d, const Idx3& f) {
     const Fab& S = B.sb;
     const int64_t sd = (d == 0) ? 1 : (d == 1) ? S.js : S.ks;
     const int64_t oR = S.off(f.i, f.j, f.k);
     const double* vf = S.p + VFRAC * S.ns;
     // 0.5 (a + b) >= 0.5 exactly when a + b >= 1 (the halving is exact)
-    return c_P.do_ns && nonneg_ge(vf[oR - sd] + vf[oR], 1.0);
+    return c_P.do_ns && nonneg_ge(fp.add(vf[oR - sd], vf[oR]), 1.0);
 }
 
 // 1/x and 1/sqrt(x) of a positive x: fixed point on the integer pipe, or the
@@ -217,7 +219,10 @@ __device__ __forceinline__ void ausm_split(const Fp& fp, double M, double sign, 
 // About 170 FP64 operations per face of one species at 70 cycles (205 at 82
 // with the refined reciprocals there): face passes of a 256^3 sphere-pack step
 // 50.4 -> 38.0 ms; the listed form keeps the FP64 pipe 83% busy.
-template <int NS, bool SOLID_SIDE = false>
+//
+// HIGH: orders 4 and 5, else 1 and 2 (the caller has the order from the host,
+// so each kernel holds the registers of its own branch).
+template <int NS, bool HIGH, bool SOLID_SIDE = false>
 __device__ __forceinline__ void face_body_at(const Fp& fp, const RhsBox& B, int d, const Idx3& f) {
     const DevParams& P = c_P;
     const Fab& S = B.sb;
@@ -245,7 +250,7 @@ __device__ __forceinline__ void face_body_at(const Fp& fp, const RhsBox& B, int 
     double therm = 0.0;                      // heat conduction
 
     if (active) {
-        if (ord == 5 || ord == 4) {
+        if (HIGH) {
             const Fab& X = B.aux;
             const int64_t qL = X.off(f.i, f.j, f.k) - ((d == 0) ? 1 : (d == 1) ? X.js : X.ks);
             const int64_t qR = X.off(f.i, f.j, f.k);
@@ -415,7 +420,7 @@ __device__ __forceinline__ void face_body_at(const Fp& fp, const RhsBox& B, int 
         const double* T = S.p + TEMP * S.ns;
         therm = fp.mul(kc, fp.mul(fp.sub(T[oR], T[oL]), B.idx[d]));
     }
-    if (SOLID_SIDE || (P.do_ns && ord <= 2)) {
+    if (!HIGH && (SOLID_SIDE || P.do_ns)) {
         // AUSM+-up: the face thread holds the face states and the scheme scalars,
         // so it writes every component's complete flux (no per-component pass).
         const Fab& O = B.flx[d];
@@ -450,7 +455,8 @@ __device__ __forceinline__ void face_body_at(const Fp& fp, const RhsBox& B, int 
             for (int z = NCONS; z < NFLO; ++z) U.p[qu + z * U.ns] = 0.0;
         return;
     }
-    // orders 4, 5: what the flux pass of this face reads
+    // orders 4, 5 (and the species-only branch of orders 1, 2): what the flux
+    // pass of this face reads
     const Fab& F = B.fs[d];
     double* q = F.p + F.off(f.i, f.j, f.k);
     q[FS_FLAGS * F.ns] = __longlong_as_double((active ? 1 : 0) | ((P.do_ns && fallback) ? 2 : 0));  // bit pattern
@@ -465,13 +471,13 @@ __device__ __forceinline__ void face_body_at(const Fp& fp, const RhsBox& B, int 
 }
 
 // Face t (linear index over growHi(bx, d, 1)) of direction d.
-template <int NS>
+template <int NS, bool HIGH>
 __device__ __forceinline__ void face_body(const Fp& fp, const RhsBox& B, int d, int64_t t) {
     int lo[3] = {B.lo[0], B.lo[1], B.lo[2]}, len[3];
     for (int e = 0; e < 3; ++e) len[e] = B.hi[e] - B.lo[e] + 1 + (e == d);
     const int64_t nf = (int64_t)len[0] * len[1] * len[2];
     if (t >= nf) return;
-    face_body_at<NS>(fp, B, d, delinear(t, lo, len));
+    face_body_at<NS, HIGH>(fp, B, d, delinear(t, lo, len));
 }
 
 // ---------------------------------------------------------------------------
@@ -575,7 +581,7 @@ __device__ __forceinline__ void flux_body(const RhsBox& B, int d, int c, int64_t
 // ---------------------------------------------------------------------------
 // One component n of the valid cell x (volume fraction vfrac): the body of
 // both launch shapes below, so they round identically.
-__device__ __forceinline__ void update_one(const RhsBox& B, int stage, double dt, int n, const Idx3& x,
+__device__ __forceinline__ void update_one(const Fp& fp, const RhsBox& B, int stage, double dt, int n, const Idx3& x,
                                            double vfrac) {
     const DevParams& P = c_P;
     const bool advected = (n < NCONS) || (n >= NFLO);
@@ -590,11 +596,11 @@ __device__ __forceinline__ void update_one(const RhsBox& B, int stage, double dt
             B.snew(x.i, x.j, x.k, n) = plus_zero(B.sb(x.i, x.j, x.k, n));
         } else if (stage == 2) {
             double v = plus_zero(B.snew(x.i, x.j, x.k, n));
-            v = add(v, mul(3.0, B.sold(x.i, x.j, x.k, n)));
+            v = fp.add(v, mul(3.0, B.sold(x.i, x.j, x.k, n)));
             B.snew(x.i, x.j, x.k, n) = mul(v, 0.25);
         } else if (stage == 3) {
             double v = plus_zero(B.snew(x.i, x.j, x.k, n));
-            v = add(B.sold(x.i, x.j, x.k, n), mul(2.0, v));
+            v = fp.add(B.sold(x.i, x.j, x.k, n), mul(2.0, v));
             B.snew(x.i, x.j, x.k, n) = mul(v, kThird);
         }
         return;
@@ -607,8 +613,9 @@ __device__ __forceinline__ void update_one(const RhsBox& B, int stage, double dt
         const int64_t oy = Fy.off(x.i, x.j, x.k) + c * Fy.ns;
         const int64_t oz = Fz.off(x.i, x.j, x.k) + c * Fz.ns;
         // explicit FMAs: every compiled copy of this body rounds the same way
-        ds = __fma_rn(Fz.p[oz] - Fz.p[oz + Fz.ks], B.idx[2],
-                      __fma_rn(Fy.p[oy] - Fy.p[oy + Fy.js], B.idx[1], mul(Fx.p[ox] - Fx.p[ox + 1], B.idx[0])));
+        ds = __fma_rn(fp.sub(Fz.p[oz], Fz.p[oz + Fz.ks]), B.idx[2],
+                      __fma_rn(fp.sub(Fy.p[oy], Fy.p[oy + Fy.js]), B.idx[1],
+                               mul(fp.sub(Fx.p[ox], Fx.p[ox + 1]), B.idx[0])));
         ds = plus_zero(ds);  // + source (compute_fluid_source is zero)
     }
     const int nnull = (P.species_in_solid == 1) ? NFLO : NFLO + P.nspec;
@@ -640,7 +647,7 @@ __device__ __forceinline__ void update_one(const RhsBox& B, int stage, double dt
     }
 }
 
-__device__ __forceinline__ void update_body(const RhsBox& B, int stage, double dt, int n, int64_t t) {
+__device__ __forceinline__ void update_body(const Fp& fp, const RhsBox& B, int stage, double dt, int n, int64_t t) {
     int lo[3] = {B.lo[0], B.lo[1], B.lo[2]}, len[3];
     for (int e = 0; e < 3; ++e) len[e] = B.hi[e] - B.lo[e] + 1;
     const int64_t nc = (int64_t)len[0] * len[1] * len[2];
@@ -648,7 +655,7 @@ __device__ __forceinline__ void update_body(const RhsBox& B, int stage, double d
     const Idx3 x = delinear(t, lo, len);
     const bool advected = (n < NCONS) || (n >= NFLO);
     // the flux-less components' fast path reads no volume fraction
-    update_one(B, stage, dt, n, x, advected ? B.sb(x.i, x.j, x.k, VFRAC) : 0.0);
+    update_one(fp, B, stage, dt, n, x, advected ? B.sb(x.i, x.j, x.k, VFRAC) : 0.0);
 }
 
 

@@ -71,18 +71,34 @@ __global__ void resnorm_kernel(Valid v, Fab Sn, Fab So, double a, double b, doub
 // change can be non-zero); the block then sums them by warp shuffles and one
 // warp adds the warps' sums in a fixed order, so the partials are
 // deterministic.
+//
+// One launch serves a group of boxes (blockIdx.y): a small box alone leaves
+// most of the GPU idle.  Every box keeps its own partials, reduced over its own
+// blocks, and the final sum adds the boxes in order: the norms' bits do not
+// depend on the grouping.
 constexpr int PTPB = 128;
+constexpr int PARTIALS = 1024;  // per box and component
+
+struct PostGroup {
+    Valid v[kRhsGroup];
+    Fab so[kRhsGroup], sn[kRhsGroup];
+    int nblk[kRhsGroup];
+};
 
 template <int NS, int CHEM, bool NORMS>
-__global__ void __launch_bounds__(PTPB) post_step_kernel(Valid v, Fab So, Fab Sn, double dt, int clip, double a,
-                                                         double b, double* partial, int nblk) {
+__global__ void __launch_bounds__(PTPB) post_step_kernel(const __grid_constant__ PostGroup g, double dt, int clip,
+                                                         double a, double b, double* partial) {
     constexpr int NM = NFLO + NS;
     const int N = NFLO + c_P.nspec;
+    const int q = blockIdx.y, nblk = g.nblk[q];
+    if (blockIdx.x >= nblk) return;
+    const Valid& v = g.v[q];
+    const Fab &So = g.so[q], &Sn = g.sn[q];
     double acc[NM];
 #pragma unroll
     for (int n = 0; n < NM; ++n) acc[n] = 0.0;
     bool nonfinite = false;
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < v.n; t += (int64_t)gridDim.x * blockDim.x) {
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < v.n; t += (int64_t)nblk * blockDim.x) {
         int i, j, k;
         cell_of(v, t, i, j, k);
         post_cell<NS, CHEM, NORMS>(So, Sn, i, j, k, dt, clip != 0, a, b, acc, nonfinite);
@@ -108,11 +124,11 @@ __global__ void __launch_bounds__(PTPB) post_step_kernel(Valid v, Fab So, Fab Sn
             x = 0.0;
             for (int w = 0; w < PTPB / 32; ++w) x += ws[w][n];
         }
-        partial[(int64_t)n * nblk + blockIdx.x] = x;
+        partial[((int64_t)q * N + n) * PARTIALS + blockIdx.x] = x;
     }
 }
 
-// Fixed-order final sum of the block partials, accumulated into acc[n].
+// Fixed-order final sum of the block partials of one box, accumulated into acc[n].
 __global__ void resnorm_final_kernel(const double* partial, int nblk, double* acc) {
     const int n = blockIdx.x;
     double x = 0.0;
@@ -120,17 +136,36 @@ __global__ void resnorm_final_kernel(const double* partial, int nblk, double* ac
     for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
     if (threadIdx.x == 0) acc[n] += x;
 }
-
+// The same for a group's boxes, box after box.
+__global__ void post_final_kernel(const __grid_constant__ PostGroup g, int nbox, const double* partial, double* acc) {
+    const int n = blockIdx.x, N = gridDim.x;
+    double sum = acc[n];
+    for (int q = 0; q < nbox; ++q) {
+        double x = 0.0;
+        for (int b = threadIdx.x; b < g.nblk[q]; b += 32) x += partial[((int64_t)q * N + n) * PARTIALS + b];
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+        sum += x;  // lane 0's is the box's sum
+    }
+    if (threadIdx.x == 0) acc[n] = sum;
+}
 
 // max wavespeed and max species diffusivity (Source/mflo_timestep.cpp:83-133)
+// over a group of boxes (blockIdx.y)
+constexpr int STEP_GROUP = 16;
+struct StepGroup {
+    Valid v[STEP_GROUP];
+    Fab s[STEP_GROUP];
+};
 template <int NS>
-__global__ void timestep_kernel(Valid v, Fab S, double* acc2) {
+__global__ void timestep_kernel(const __grid_constant__ StepGroup g, double* acc2) {
+    const Valid& v = g.v[blockIdx.y];
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t - threadIdx.x >= v.n) return;  // whole block past this box
     double ws = 0.0, md = 0.0;
     if (t < v.n) {
         int i, j, k;
         cell_of(v, t, i, j, k);
-        timestep_cell<NS>(S, i, j, k, ws, md);
+        timestep_cell<NS>(g.s[blockIdx.y], i, j, k, ws, md);
     }
     for (int o = 16; o > 0; o >>= 1) {
         ws = fmax(ws, __shfl_down_sync(0xffffffffu, ws, o));
@@ -140,6 +175,26 @@ __global__ void timestep_kernel(Valid v, Fab S, double* acc2) {
         atomic_max_nonneg(acc2, ws);
         atomic_max_nonneg(acc2 + 1, md);
     }
+}
+
+// Contiguous copies of several arrays in one launch (blockIdx.y = array), four
+// loads in flight per thread.
+constexpr int COPY_GROUP = 32;
+struct CopyList {
+    const double* src[COPY_GROUP];
+    double* dst[COPY_GROUP];
+    int64_t n[COPY_GROUP];
+};
+__global__ void __launch_bounds__(TPB) copy_list_kernel(const __grid_constant__ CopyList g) {
+    const double* __restrict__ src = g.src[blockIdx.y];
+    double* __restrict__ dst = g.dst[blockIdx.y];
+    const int64_t n = g.n[blockIdx.y], base = (int64_t)blockIdx.x * (4 * TPB) + threadIdx.x;
+    double v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = (base + u * TPB < n) ? src[base + u * TPB] : 0.0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+        if (base + u * TPB < n) dst[base + u * TPB] = v[u];
 }
 
 // dst = (copy_first ? base : dst) + a*src over the valid box, all components.
@@ -241,11 +296,10 @@ cudaError_t launch_resnorm_box(const mfg_box& b, double dt, double* partial, dou
     return cudaGetLastError();
 }
 
-// partial: scratch of (ncomp * 1024) doubles, acc: ncomp doubles (device), or
-// both null (no residual norms).
-cudaError_t launch_post_step(const mfg_box& b, double dt, bool chem, bool clip, double* partial, double* acc,
+// The bookends of n <= kRhsGroup boxes.  partial: scratch of (n * ncomp * 1024)
+// doubles, acc: ncomp doubles (device), or both null (no residual norms).
+cudaError_t launch_post_step(const mfg_box* boxes, int n, double dt, bool chem, bool clip, double* partial, double* acc,
                              cudaStream_t st) {
-    Valid v = valid_of(b);
     const int ns = c_host_params().nspec, nc = NFLO + ns;
     // one cell per thread up to one wave of blocks (4 of 128 threads resident
     // per SM at the kernel's ~115 registers), then a grid-stride loop: every
@@ -257,22 +311,29 @@ cudaError_t launch_post_step(const mfg_box& b, double dt, bool chem, bool clip, 
         int dev = 0, sms = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        wave = std::max(1, std::min(1024, 4 * sms));
+        wave = std::max(1, std::min(PARTIALS, 4 * sms));
     }
-    const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>(wave, (v.n + PTPB - 1) / PTPB));
+    PostGroup g;
+    int most = 1;
+    for (int q = 0; q < kRhsGroup; ++q) {
+        const mfg_box& b = boxes[q < n ? q : 0];
+        g.v[q] = valid_of(b);
+        g.so[q] = make_fab(b.s_old);
+        g.sn[q] = make_fab(b.s_new);
+        g.nblk[q] = (int)std::max<int64_t>(1, std::min<int64_t>(wave, (g.v[q].n + PTPB - 1) / PTPB));
+        if (q < n) most = std::max(most, g.nblk[q]);
+    }
+    const dim3 grid(most, n);
     const double a = 1.0 / dt, bb = -1.0 / dt;
-    const size_t smem = 0;
     const DevParams& P = c_host_params();
     // the sub-step of a zero source (no reactions, explicit integrator) is s + 0
     const int kind = !chem ? 0 : (P.chem_kind == 0 && (!P.chem_on || P.nreact == 0)) ? 1 : 2;
     ProfScope ps(K_POST, st, partial ? 2 : 1);
-#define MFG_POST_K(NSB, K)                                                                               \
-    if (partial)                                                                                         \
-        post_step_kernel<NSB, K, true><<<nblk, PTPB, smem, st>>>(v, make_fab(b.s_old), make_fab(b.s_new), dt, \
-                                                                 clip, a, bb, partial, nblk);            \
-    else                                                                                                 \
-        post_step_kernel<NSB, K, false><<<nblk, PTPB, smem, st>>>(v, make_fab(b.s_old), make_fab(b.s_new), dt, \
-                                                                  clip, a, bb, partial, nblk)
+#define MFG_POST_K(NSB, K)                                                                    \
+    if (partial)                                                                              \
+        post_step_kernel<NSB, K, true><<<grid, PTPB, 0, st>>>(g, dt, clip, a, bb, partial);   \
+    else                                                                                      \
+        post_step_kernel<NSB, K, false><<<grid, PTPB, 0, st>>>(g, dt, clip, a, bb, partial)
 #define MFG_POST(NSB)                     \
     if (kind == 0) MFG_POST_K(NSB, 0);    \
     else if (kind == 1) MFG_POST_K(NSB, 1); \
@@ -284,20 +345,30 @@ cudaError_t launch_post_step(const mfg_box& b, double dt, bool chem, bool clip, 
     else { MFG_POST(16) }
 #undef MFG_POST
 #undef MFG_POST_K
-    if (partial) resnorm_final_kernel<<<nc, 32, 0, st>>>(partial, nblk, acc);
+    if (partial) post_final_kernel<<<nc, 32, 0, st>>>(g, n, partial, acc);
     return cudaGetLastError();
 }
 
-cudaError_t launch_timestep(const mfg_box& b, double* acc2, cudaStream_t st) {
-    Valid v = valid_of(b);
-    Fab S = make_fab(b.s_new);
+cudaError_t launch_timestep(const mfg_box* boxes, int nbox, double* acc2, cudaStream_t st) {
     const int ns = c_host_params().nspec;
-    ProfScope ps(K_TIMESTEP, st);
-    if (ns <= 1) timestep_kernel<1><<<nblocks(v.n), TPB, 0, st>>>(v, S, acc2);
-    else if (ns <= 2) timestep_kernel<2><<<nblocks(v.n), TPB, 0, st>>>(v, S, acc2);
-    else if (ns <= 4) timestep_kernel<4><<<nblocks(v.n), TPB, 0, st>>>(v, S, acc2);
-    else if (ns <= 8) timestep_kernel<8><<<nblocks(v.n), TPB, 0, st>>>(v, S, acc2);
-    else timestep_kernel<16><<<nblocks(v.n), TPB, 0, st>>>(v, S, acc2);
+    for (int b = 0; b < nbox; b += STEP_GROUP) {
+        const int n = std::min(STEP_GROUP, nbox - b);
+        StepGroup g;
+        int64_t most = 0;
+        for (int q = 0; q < STEP_GROUP; ++q) {
+            const mfg_box& x = boxes[b + (q < n ? q : 0)];
+            g.v[q] = valid_of(x);
+            g.s[q] = make_fab(x.s_new);
+            most = std::max(most, g.v[q].n);
+        }
+        const dim3 grid(nblocks(most), n);
+        ProfScope ps(K_TIMESTEP, st);
+        if (ns <= 1) timestep_kernel<1><<<grid, TPB, 0, st>>>(g, acc2);
+        else if (ns <= 2) timestep_kernel<2><<<grid, TPB, 0, st>>>(g, acc2);
+        else if (ns <= 4) timestep_kernel<4><<<grid, TPB, 0, st>>>(g, acc2);
+        else if (ns <= 8) timestep_kernel<8><<<grid, TPB, 0, st>>>(g, acc2);
+        else timestep_kernel<16><<<grid, TPB, 0, st>>>(g, acc2);
+    }
     return cudaGetLastError();
 }
 
@@ -336,6 +407,43 @@ cudaError_t launch_axpy_valid(const mfg_box& b, const Fab& dst, const Fab& src, 
     dim3 g(nblocks(v.n), ncomp);
     ProfScope ps(K_COPY, st);
     axpy_kernel<<<g, TPB, 0, st>>>(v, dst, src, a, copy_first ? 1 : 0, base, ncomp);
+    return cudaGetLastError();
+}
+
+// phi_old <- phi_new of every box (not for stream capture): dense arrays, in
+// the same layout and apart from each other, by copy_list_kernel, the others
+// box by box.
+cudaError_t launch_copy_old(const mfg_box* boxes, int nbox, int ncomp, cudaStream_t st) {
+    Fab none;
+    memset(&none, 0, sizeof(none));
+    CopyList g;
+    int n = 0;
+    int64_t most = 0;
+    auto flush = [&]() {
+        if (!n) return;
+        ProfScope ps(K_COPY, st);
+        copy_list_kernel<<<dim3((unsigned)((most + 4 * TPB - 1) / (4 * TPB)), n), TPB, 0, st>>>(g);
+        n = 0;
+        most = 0;
+    };
+    for (int b = 0; b < nbox; ++b) {
+        const Fab d = make_fab(boxes[b].s_old), s = make_fab(boxes[b].s_new);
+        const int64_t cnt = (int64_t)ncomp * d.ns;
+        const bool apart = d.p + cnt <= s.p || s.p + cnt <= d.p;
+        if (d.p == s.p && dense_over(d, boxes[b]) && dense_over(s, boxes[b])) continue;
+        if (!apart || !dense_over(d, boxes[b]) || !dense_over(s, boxes[b])) {
+            flush();
+            const cudaError_t e = launch_axpy_valid(boxes[b], d, none, 0.0, true, s, ncomp, st);
+            if (e != cudaSuccess) return e;
+            continue;
+        }
+        g.src[n] = s.p;
+        g.dst[n] = d.p;
+        g.n[n++] = cnt;
+        most = std::max(most, cnt);
+        if (n == COPY_GROUP) flush();
+    }
+    flush();
     return cudaGetLastError();
 }
 
