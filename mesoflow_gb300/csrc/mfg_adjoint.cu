@@ -1856,6 +1856,7 @@ extern "C" int mfg_adjoint_objective(const mfg_box* boxes, int nbox, const mfg_g
     double h[2 + MAXR];
     ADJ_TRY(cudaMemcpyAsync(h, W.d_g, sizeof(h), cudaMemcpyDeviceToHost, st), "result copy");
     ADJ_TRY(cudaStreamSynchronize(st), "synchronize");
+    cutcache_sweep();
     unsigned status = 0;
     ADJ_TRY(read_status(&status, false), "status");
     if (status & MFG_STATUS_NAN) return MFG_ERR_NAN;

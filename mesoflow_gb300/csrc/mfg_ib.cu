@@ -26,12 +26,19 @@
 // often), with each fluid neighbour's offset and weights laid out so that a
 // warp's loads of one neighbour entry are contiguous.  Every later call first
 // compares the volume fraction with the copy on the device (exact, bit
-// patterns): the cut-cell kernel uses the stored entries when nothing
-// changed; otherwise it rebuilds the list and recomputes on the fly, so a
-// changed geometry is never served stale weights and no host round trip is
-// needed.  All paths give bitwise equal results.  Entries whose volume
-// fraction changed are dropped by cutcache_sweep (called where the host
-// synchronizes anyway) and rebuilt by the next call.
+// patterns) and brings the copy up to date:
+//   unchanged: the stored entries are applied;
+//   changed values, but the same gas, cut and solid cells (the ulp drift, or
+//   another state of the same geometry): the entries' weights are recomputed
+//   in place, then applied;
+//   another gas, cut or solid cell anywhere: the list is rebuilt and the
+//   weights computed on the fly in the same call, and the entry is out of use
+//   until cutcache_sweep (called where the host synchronizes anyway) drops it
+//   and the next call builds it anew.
+// No host round trip is needed, no stale weight is ever applied, and all paths
+// give bitwise equal results.  (Dropping an entry at every drift cost a host
+// sort and a dozen allocations per box in each of a state's first steps: the
+// second step of a 256^3 sphere pack took 165 ms, 67 ms now.)
 #include <algorithm>
 #include <cstring>
 #include <unordered_map>
@@ -46,6 +53,10 @@ __constant__ double c_wdir[125];
 namespace {
 
 constexpr int TPB = 128;
+// An entry's flag.  VF_MOVED: some value differs from the copy in this call;
+// VF_OTHER: since the entry was built some cell changed between gas, cut and
+// solid (kept until the entry is dropped).
+constexpr unsigned VF_MOVED = 1u, VF_OTHER = 2u;
 
 // Conjugate heat transfer: mean temperature of the 26 neighbours, read before
 // any cut cell is updated (ib_utils.H:345-364).
@@ -65,10 +76,10 @@ __global__ void cht_avg_kernel(CutBox c) {
 }
 
 // Appends the linear index of every cut cell (0 < vfrac < 1) of the box to
-// list; with a non-null flag, only when *flag is set.
+// list; with a non-null flag, only when it has VF_OTHER.
 __global__ void cut_list_kernel(CutBox c, int* __restrict__ list, unsigned* __restrict__ count,
                                 const unsigned* __restrict__ flag) {
-    if (flag && !*flag) return;
+    if (flag && !(*flag & VF_OTHER)) return;
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     bool cut = false;
     if (t < c.n) {
@@ -86,31 +97,57 @@ __global__ void cut_list_kernel(CutBox c, int* __restrict__ list, unsigned* __re
     if (cut) list[base + __popc(m & ((1u << lane) - 1u))] = (int)t;
 }
 
+// The on-the-fly form over the lists of several boxes (blockIdx.y); a box whose
+// list is empty costs one load.  The cache-off path and the changed boxes of
+// the cached one both run it, so they agree by construction.
+constexpr int CUT_GROUP = 16;
+struct CutGroup {
+    CutBox c[CUT_GROUP];
+    const int* list[CUT_GROUP];
+    const unsigned* count[CUT_GROUP];
+};
 template <int NS>
-__global__ void __launch_bounds__(TPB) cutcell_kernel(CutBox c, const int* __restrict__ list,
-                                                      const unsigned* __restrict__ count) {
-    const unsigned n = *count;
+__global__ void __launch_bounds__(TPB) cutcell_kernel(const __grid_constant__ CutGroup g) {
+    const unsigned n = *g.count[blockIdx.y];
+    const int* __restrict__ list = g.list[blockIdx.y];
+    const CutBox& c = g.c[blockIdx.y];
     for (unsigned w = blockIdx.x * blockDim.x + threadIdx.x; w < n; w += gridDim.x * blockDim.x)
         cutcell_one<NS>(c, list[w]);
 }
 
-// Grown-box volume fraction: copy (mode 0) or compare with the copy (mode 1,
-// sets *dirty on any difference of bit patterns).
+__device__ __forceinline__ int vf_kind(double v) { return is_one(v) ? 2 : (v > 0.0 && v < 1.0) ? 1 : 0; }
+
+// One grown cell's volume fraction against the copy, which takes the new value;
+// the warp's flag bits are raised by one lane.
+__device__ __forceinline__ void vf_compare(bool in, double v, double* copy, unsigned* flag) {
+    unsigned f = 0;
+    if (in) {
+        const double old = *copy;
+        if (__double_as_longlong(v) != __double_as_longlong(old)) {
+            f = VF_MOVED | (vf_kind(v) != vf_kind(old) ? VF_OTHER : 0u);
+            *copy = v;
+        }
+    }
+    f = __reduce_or_sync(0xffffffffu, f);
+    if (f && (threadIdx.x & 31) == 0) atomicOr(flag, f);
+}
+
+// Grown-box volume fraction: copy (mode 0) or compare with the copy (mode 1).
 __global__ void cut_vf_kernel(Fab S, int lo0, int lo1, int lo2, int l0, int l1, int l2, double* __restrict__ vf,
-                              unsigned* __restrict__ dirty, int mode) {
+                              unsigned* __restrict__ flag, int mode) {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    bool diff = false;
-    if (t < (int64_t)l0 * l1 * l2) {
+    const bool in = t < (int64_t)l0 * l1 * l2;
+    double v = 0.0;
+    if (in) {
         int i, j, k;
         split3(t, l0, l1, i, j, k);
-        const double v = S(lo0 + i, lo1 + j, lo2 + k, VFRAC);
-        if (mode == 0)
-            vf[t] = v;
-        else
-            diff = __double_as_longlong(v) != __double_as_longlong(vf[t]);
+        v = S(lo0 + i, lo1 + j, lo2 + k, VFRAC);
+        if (mode == 0) vf[t] = v;
     }
-    if (mode == 1 && __any_sync(0xffffffffu, diff) && (threadIdx.x & 31) == 0) atomicOr(dirty, 1u);
+    if (mode == 1) vf_compare(in, v, vf + t, flag);
 }
+
+__global__ void cut_flag_reset_kernel(unsigned* flag) { *flag &= VF_OTHER; }
 
 __global__ void cut_count_kernel(CutBox c, const int* __restrict__ list, unsigned n, int* __restrict__ kc) {
     const unsigned w = blockIdx.x * blockDim.x + threadIdx.x;
@@ -123,20 +160,21 @@ __global__ void cut_entries_kernel(CutBox c, CutCacheView cc, unsigned n, int* o
     if (w < n) cut_entries_one(c, (int)w, cc, off, wn, wd, scal);
 }
 
-// Stored entries when the volume fraction is unchanged (*dirty == 0), else
-// the on-the-fly form over the freshly built list.  The grid stride is a
+// The weights of the stored entries recomputed where values moved and the
+// geometry did not (same list, neighbours and layout).
+__global__ void cut_refresh_kernel(CutBox c, CutCacheView cc, unsigned n, const unsigned* __restrict__ flag) {
+    if (*flag != VF_MOVED) return;
+    for (unsigned w = blockIdx.x * blockDim.x + threadIdx.x; w < n; w += gridDim.x * blockDim.x)
+        cut_entries_one(c, (int)w, cc, const_cast<int*>(cc.off), const_cast<double*>(cc.wn), const_cast<double*>(cc.wd),
+                        const_cast<double*>(cc.scal));
+}
+
+// Stored entries, unless the entry is out of use.  The grid stride is a
 // multiple of 32, so a warp always holds one group of 32 list positions.
 template <int NS>
 __global__ void __launch_bounds__(TPB) cutcell_cached_kernel(CutBox c, CutCacheView cc, unsigned ncut,
-                                                             const unsigned* __restrict__ dirty,
-                                                             const int* __restrict__ list,
-                                                             const unsigned* __restrict__ count) {
-    if (*dirty) {
-        const unsigned n = *count;
-        for (unsigned w = blockIdx.x * blockDim.x + threadIdx.x; w < n; w += gridDim.x * blockDim.x)
-            cutcell_one<NS>(c, list[w]);
-        return;
-    }
+                                                             const unsigned* __restrict__ flag) {
+    if (*flag & VF_OTHER) return;
     for (unsigned w = blockIdx.x * blockDim.x + threadIdx.x; w < ncut; w += gridDim.x * blockDim.x)
         cutcell_cached<NS>(c, (int)w, cc);
 }
@@ -153,11 +191,11 @@ struct LevelCutBox {
     int glo[3], glen[3];  // grown box
 };
 
-// Clears every box's change flag and rebuilt-list count.
+// Clears every box's VF_MOVED and rebuilt-list count.
 __global__ void cut_level_reset_kernel(const LevelCutBox* __restrict__ tab, int nbox, unsigned* __restrict__ cnt) {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b < nbox) {
-        *tab[b].dirty = 0;
+        *tab[b].dirty &= VF_OTHER;
         cnt[b] = 0;
     }
 }
@@ -166,23 +204,31 @@ __global__ void cut_level_reset_kernel(const LevelCutBox* __restrict__ tab, int 
 __global__ void cut_level_vf_kernel(const LevelCutBox* __restrict__ tab) {
     const LevelCutBox& L = tab[blockIdx.y];
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t n = (int64_t)L.glen[0] * L.glen[1] * L.glen[2];
-    bool diff = false;
-    if (t < n) {
+    const bool in = t < (int64_t)L.glen[0] * L.glen[1] * L.glen[2];
+    double v = 0.0;
+    if (in) {
         int i, j, k;
         split3(t, L.glen[0], L.glen[1], i, j, k);
-        const double v = L.c.S(L.glo[0] + i, L.glo[1] + j, L.glo[2] + k, VFRAC);
-        diff = __double_as_longlong(v) != __double_as_longlong(L.vf[t]);
+        v = L.c.S(L.glo[0] + i, L.glo[1] + j, L.glo[2] + k, VFRAC);
     }
-    if (__any_sync(0xffffffffu, diff) && (threadIdx.x & 31) == 0) atomicOr(L.dirty, 1u);
+    vf_compare(in, v, L.vf + t, L.dirty);
 }
 
-// For a box whose volume fraction changed: its cut cells listed afresh
+// cut_refresh_kernel for every box of the level (blockIdx.y).
+__global__ void __launch_bounds__(TPB) cut_level_refresh_kernel(const LevelCutBox* __restrict__ tab) {
+    const LevelCutBox& L = tab[blockIdx.y];
+    if (*L.dirty != VF_MOVED) return;
+    for (unsigned w = blockIdx.x * blockDim.x + threadIdx.x; w < L.ncut; w += gridDim.x * blockDim.x)
+        cut_entries_one(L.c, (int)w, L.v, const_cast<int*>(L.v.off), const_cast<double*>(L.v.wn),
+                        const_cast<double*>(L.v.wd), const_cast<double*>(L.v.scal));
+}
+
+// For a box whose entry is out of use: its cut cells listed afresh
 // (grid-stride over the box; one atomic per warp).
 __global__ void cut_level_list_kernel(const LevelCutBox* __restrict__ tab, unsigned* __restrict__ cnt,
                                       int* __restrict__ lists, int64_t cap) {
     const LevelCutBox& L = tab[blockIdx.y];
-    if (!*L.dirty) return;
+    if (!(*L.dirty & VF_OTHER)) return;
     const CutBox& c = L.c;
     int* list = lists + (int64_t)blockIdx.y * cap;
     for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < c.n; base += (int64_t)gridDim.x * blockDim.x) {
@@ -204,7 +250,7 @@ __global__ void cut_level_list_kernel(const LevelCutBox* __restrict__ tab, unsig
     }
 }
 
-// Stored entries of every unchanged box: one warp per group of 32 list
+// Stored entries of every box in use: one warp per group of 32 list
 // positions, box after box (a box's Sborder stays in L2 while its groups
 // run), each box's groups in its own sorted order.
 template <int NS>
@@ -214,7 +260,7 @@ __global__ void __launch_bounds__(TPB) cutcell_level_kernel(const LevelCutBox* _
     if (gw >= ngroups) return;
     const int2 bg = groups[gw];
     const LevelCutBox& L = tab[bg.x];
-    if (*L.dirty) return;
+    if (*L.dirty & VF_OTHER) return;
     const unsigned w = 32u * (unsigned)bg.y + (threadIdx.x & 31);
     if (w < L.ncut) cutcell_cached<NS>(L.c, (int)w, L.v);
 }
@@ -316,6 +362,7 @@ int new_slot(cudaStream_t st) {
         unsigned* d = nullptr;
         if (cudaMalloc(&d, cap * sizeof(unsigned)) != cudaSuccess) return -1;
         if (cudaStreamSynchronize(st) != cudaSuccess) return -1;
+        if (cudaMemset(d, 0, cap * sizeof(unsigned)) != cudaSuccess) return -1;
         if (g_cache.dirty) {
             cudaMemcpy(d, g_cache.dirty, g_cache.cap * sizeof(unsigned), cudaMemcpyDeviceToDevice);
             cudaFree(g_cache.dirty);
@@ -384,6 +431,7 @@ bool build_entry(const mfg_box& b, const CutBox& c, const mfg_geom& g, CutEntry&
     if (cudaMalloc(&e.wd, nent * sizeof(double)) != cudaSuccess) return false;
     if (cudaMalloc(&e.scal, std::max<unsigned>(n, 1) * 2 * sizeof(double)) != cudaSuccess) return false;
     if ((e.slot = new_slot(st)) < 0) return false;
+    if (cudaMemsetAsync(g_cache.dirty + e.slot, 0, sizeof(unsigned), st) != cudaSuccess) return false;  // a reused slot's flag
     if (n) {
         if (cudaMemcpyAsync(e.list, sl.data(), n * sizeof(int), cudaMemcpyHostToDevice, st) != cudaSuccess ||
             cudaMemcpyAsync(e.kc, sk.data(), n * sizeof(int), cudaMemcpyHostToDevice, st) != cudaSuccess ||
@@ -418,14 +466,14 @@ CutEntry* find_entry(const mfg_box& b, const CutBox& c, const mfg_geom& g, cudaS
 
 }  // namespace
 
-// Drops the entries whose volume fraction changed in the last call; the host
-// has synchronized the stream before.
+// Drops the entries that are out of use (another geometry); the host has
+// synchronized the stream before.
 void cutcache_sweep() {
     if (g_cache.map.empty() || !g_cache.dirty) return;
     std::vector<unsigned> h(g_cache.nslots);
     if (cudaMemcpy(h.data(), g_cache.dirty, h.size() * sizeof(unsigned), cudaMemcpyDeviceToHost) != cudaSuccess) return;
     for (auto it = g_cache.map.begin(); it != g_cache.map.end();) {
-        if (it->second.slot >= 0 && h[it->second.slot]) {
+        if (it->second.slot >= 0 && (h[it->second.slot] & VF_OTHER)) {
             free_entry(it->second);
             it = g_cache.map.erase(it);
         } else {
@@ -545,16 +593,17 @@ CutLevelTable* level_prepare(const std::vector<LevelCutBox>& tab) {
 
 }  // namespace
 
-// All boxes of a level in four launches (change flags cleared, volume
-// fractions checked, lists of changed boxes rebuilt, stored entries applied)
-// plus one on-the-fly launch per box that does work only where the box's
-// volume fraction changed (the cache-off kernel itself, so those boxes give
-// that path's results by construction).  Returns 1 when done, -1 on a CUDA
-// error, and 0, having launched nothing, where the per-box path must run:
-// cache off, conjugate heat transfer (its neighbour-temperature scratch is
-// per box), a box without an entry, or a table to build during capture.
+// All boxes of a level in five launches (flags cleared, volume fractions
+// compared, moved boxes' weights refreshed, lists of boxes out of use rebuilt,
+// stored entries applied) plus the on-the-fly launch for sixteen boxes at a
+// time, which works only where a box is out of use (the cache-off kernel
+// itself, so those boxes give that path's results by construction).  Returns 1
+// when done, -1 on a CUDA error, and 0, having launched nothing, where the
+// per-box path must run: cache off, conjugate heat transfer (its
+// neighbour-temperature scratch is per box), a box without an entry, or a
+// table to build during capture.
 int launch_cutcells_level(const mfg_box* boxes, int nbox, const mfg_geom& g, cudaStream_t st) {
-    if (nbox < 2 || !g_cache.enabled || c_host_params().conj_ht) return 0;
+    if (nbox < 1 || !g_cache.enabled || c_host_params().conj_ht) return 0;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return 0;
     const double dxmin = fmin(g.dx[0], fmin(g.dx[1], g.dx[2]));
@@ -584,17 +633,27 @@ int launch_cutcells_level(const mfg_box* boxes, int nbox, const mfg_geom& g, cud
         return 0;
     }
     const int ns = c_host_params().nspec;
-    ProfScope ps(K_CUT, st, 4 + nbox);
+    ProfScope ps(K_CUT, st, 5 + (nbox + CUT_GROUP - 1) / CUT_GROUP);
     cut_level_reset_kernel<<<(nbox + 127) / 128, 128, 0, st>>>(T->d_tab, nbox, g_level.d_cnt);
     cut_level_vf_kernel<<<dim3((unsigned)((T->maxgrown + 255) / 256), (unsigned)nbox), 256, 0, st>>>(T->d_tab);
+    const unsigned per = (unsigned)std::max<int64_t>(1, std::min<int64_t>((T->cap + TPB - 1) / TPB, 152));
+    cut_level_refresh_kernel<<<dim3(per, (unsigned)nbox), TPB, 0, st>>>(T->d_tab);
     cut_level_list_kernel<<<dim3(8, (unsigned)nbox), TPB, 0, st>>>(T->d_tab, g_level.d_cnt, g_level.d_lists, T->cap);
     const unsigned nb = std::max(1u, (unsigned)(((uint64_t)T->ngroups * 32 + TPB - 1) / TPB));
 #define MFG_LEVEL_LAUNCH(K)                                                                                 \
     do {                                                                                                    \
         cutcell_level_kernel<K><<<nb, TPB, 0, st>>>(T->d_tab, T->d_groups, T->ngroups);                   \
-        for (int b = 0; b < nbox; ++b)                                                                      \
-            cutcell_kernel<K><<<152, TPB, 0, st>>>(tab[b].c, g_level.d_lists + (int64_t)b * T->cap,         \
-                                                   g_level.d_cnt + b);                                      \
+        for (int b = 0; b < nbox; b += CUT_GROUP) {                                                         \
+            const int n = std::min(CUT_GROUP, nbox - b);                                                    \
+            CutGroup cg;                                                                                    \
+            for (int q = 0; q < CUT_GROUP; ++q) {                                                           \
+                const int w = b + (q < n ? q : 0);                                                          \
+                cg.c[q] = tab[w].c;                                                                         \
+                cg.list[q] = g_level.d_lists + (int64_t)w * T->cap;                                         \
+                cg.count[q] = g_level.d_cnt + w;                                                            \
+            }                                                                                               \
+            cutcell_kernel<K><<<dim3(152, n), TPB, 0, st>>>(cg);                                            \
+        }                                                                                                   \
     } while (0)
     if (ns <= 1) MFG_LEVEL_LAUNCH(1);
     else if (ns <= 2) MFG_LEVEL_LAUNCH(2);
@@ -613,35 +672,41 @@ cudaError_t launch_cutcells_box(const mfg_box& b, const mfg_geom& g, double* tch
     const unsigned nb = (unsigned)((c.n + TPB - 1) / TPB);
     const int ns = c_host_params().nspec;
     CutEntry* ce = find_entry(b, c, g, st);
-    ProfScope ps(K_CUT, st, (ce ? 3 : 2) + (c_host_params().conj_ht ? 1 : 0));
+    ProfScope ps(K_CUT, st, (ce ? 6 : 2) + (c_host_params().conj_ht ? 1 : 0));
     if (c_host_params().conj_ht) cht_avg_kernel<<<nb, TPB, 0, st>>>(c);
     cudaMemsetAsync(count, 0, sizeof(unsigned), st);
+    const unsigned ng = (unsigned)std::min<int64_t>(std::max<int64_t>(nb, 1), 152 * 8);
+    unsigned* flag = nullptr;
     if (ce) {
-        unsigned* dirty = g_cache.dirty + ce->slot;
+        flag = g_cache.dirty + ce->slot;
         const int l0 = c.len[0] + 6, l1 = c.len[1] + 6, l2 = c.len[2] + 6;
         const int64_t ngc = (int64_t)l0 * l1 * l2;
-        cudaMemsetAsync(dirty, 0, sizeof(unsigned), st);
+        cut_flag_reset_kernel<<<1, 1, 0, st>>>(flag);
         cut_vf_kernel<<<(unsigned)((ngc + 255) / 256), 256, 0, st>>>(c.S, b.lo[0] - 3, b.lo[1] - 3, b.lo[2] - 3, l0,
-                                                                      l1, l2, ce->vf, dirty, 1);
-        cut_list_kernel<<<nb, TPB, 0, st>>>(c, list, count, dirty);
-        const unsigned ng = (unsigned)std::min<int64_t>(std::max<int64_t>(nb, 1), 152 * 8);
-#define MFG_CUT_ARGS c, ce->view(), ce->ncut, dirty, list, count
+                                                                      l1, l2, ce->vf, flag, 1);
+        cut_refresh_kernel<<<ng, TPB, 0, st>>>(c, ce->view(), ce->ncut, flag);
+#define MFG_CUT_ARGS c, ce->view(), ce->ncut, flag
         if (ns <= 1) cutcell_cached_kernel<1><<<ng, TPB, 0, st>>>(MFG_CUT_ARGS);
         else if (ns <= 2) cutcell_cached_kernel<2><<<ng, TPB, 0, st>>>(MFG_CUT_ARGS);
         else if (ns <= 4) cutcell_cached_kernel<4><<<ng, TPB, 0, st>>>(MFG_CUT_ARGS);
         else if (ns <= 8) cutcell_cached_kernel<8><<<ng, TPB, 0, st>>>(MFG_CUT_ARGS);
         else cutcell_cached_kernel<16><<<ng, TPB, 0, st>>>(MFG_CUT_ARGS);
 #undef MFG_CUT_ARGS
-        return cudaGetLastError();
     }
-    cut_list_kernel<<<nb, TPB, 0, st>>>(c, list, count, nullptr);
-    // a fixed grid walks the list (its length stays on the device)
-    const unsigned ng = (unsigned)std::min<int64_t>(nb, 152 * 8);
-    if (ns <= 1) cutcell_kernel<1><<<ng, TPB, 0, st>>>(c, list, count);
-    else if (ns <= 2) cutcell_kernel<2><<<ng, TPB, 0, st>>>(c, list, count);
-    else if (ns <= 4) cutcell_kernel<4><<<ng, TPB, 0, st>>>(c, list, count);
-    else if (ns <= 8) cutcell_kernel<8><<<ng, TPB, 0, st>>>(c, list, count);
-    else cutcell_kernel<16><<<ng, TPB, 0, st>>>(c, list, count);
+    // the on-the-fly form: without an entry, or where the entry is out of use
+    // (a fixed grid walks the list, whose length stays on the device)
+    cut_list_kernel<<<nb, TPB, 0, st>>>(c, list, count, flag);
+    CutGroup cg;
+    for (int q = 0; q < CUT_GROUP; ++q) {
+        cg.c[q] = c;
+        cg.list[q] = list;
+        cg.count[q] = count;
+    }
+    if (ns <= 1) cutcell_kernel<1><<<ng, TPB, 0, st>>>(cg);
+    else if (ns <= 2) cutcell_kernel<2><<<ng, TPB, 0, st>>>(cg);
+    else if (ns <= 4) cutcell_kernel<4><<<ng, TPB, 0, st>>>(cg);
+    else if (ns <= 8) cutcell_kernel<8><<<ng, TPB, 0, st>>>(cg);
+    else cutcell_kernel<16><<<ng, TPB, 0, st>>>(cg);
     return cudaGetLastError();
 }
 

@@ -7,7 +7,8 @@
 // each fluid neighbour in neighbourhood order, its offset and both weights
 // (plus 1/den and 1/sum w per cut cell) and cutcell_cached applies them.
 // Both accumulate in the same neighbour order and finish with the same
-// multiplications, so they give bitwise equal results.
+// multiplications, every rounding explicit, so they give bitwise equal results
+// in whichever kernels they are compiled.
 #pragma once
 #include "mfg_internal.h"
 #include "mfg_physics.cuh"
@@ -64,7 +65,7 @@ __device__ __forceinline__ void cut_geometry(const CutBox& c, int64_t o, double&
     const double gx = add(mul(V[o - 1], -hx), mul(V[o + 1], hx));
     const double gy = add(mul(V[o - S.js], -hy), mul(V[o + S.js], hy));
     const double gz = add(mul(V[o - S.ks], -hz), mul(V[o + S.ks], hz));
-    const double mag = sqrt((gx * gx + gy * gy) + gz * gz);
+    const double mag = sqrt(__fma_rn(gz, gz, __fma_rn(gy, gy, mul(gx, gx))));
     double xp[3] = {0.0, 0.0, 0.0};
     dist = 0.0;
     if (mag > kTiny) {
@@ -79,12 +80,19 @@ __device__ __forceinline__ void cut_geometry(const CutBox& c, int64_t o, double&
     }
 }
 
+// Inverse-distance weight of neighbour (l, m, n) about the surface point.
+__device__ __forceinline__ double surface_weight(int l, int m, int n, const double dxnd[3], const double xpn[3]) {
+    const double a = __fma_rn((double)l, dxnd[0], -xpn[0]), b = __fma_rn((double)m, dxnd[1], -xpn[1]),
+                 e = __fma_rn((double)n, dxnd[2], -xpn[2]);
+    return rcp_pos(add(__fma_rn(e, e, __fma_rn(b, b, mul(a, a))), kTiny2));
+}
+
 // 1/den of the velocity weights: den = sum wd + 1/dn^2 (the surface point),
 // zero when the cell centre lies on the surface (velocity set to zero).
 __device__ __forceinline__ double vel_iden(const CutBox& c, double dist, double swd) {
     if (fabs(dist) < c.dxmin * 1e-5) return 0.0;
     const double dn = fabs(dist) / c.dxmin;
-    return 1.0 / (swd + 1.0 / (dn * dn));
+    return 1.0 / add(swd, 1.0 / mul(dn, dn));
 }
 
 // Writes the primitives and conserved variables of cut cell (o, t) from the
@@ -97,14 +105,14 @@ __device__ __forceinline__ void cut_finish(const CutBox& c, int64_t t, int64_t o
     const bool interp_spec = !P.species_in_solid;
     double vel[3];
     // the surface value is zero: its term adds 0/(dn*dn) to each sum
-    for (int a = 0; a < 3; ++a) vel[a] = (iden == 0.0) ? 0.0 : (sv[a] + 0.0) * iden;
-    const double pres = have ? sp * iswn : S.p[o + PRES * S.ns];
+    for (int a = 0; a < 3; ++a) vel[a] = (iden == 0.0) ? 0.0 : mul(add(sv[a], 0.0), iden);
+    const double pres = have ? mul(sp, iswn) : S.p[o + PRES * S.ns];
     double temp;
     if (P.conj_ht)
         temp = c.tcht[t];
     else
-        temp = have ? st * iswn : S.p[o + TEMP * S.ns];
-    const double dens = have ? sr * iswn : S.p[o + DENS * S.ns];
+        temp = have ? mul(st, iswn) : S.p[o + TEMP * S.ns];
+    const double dens = have ? mul(sr, iswn) : S.p[o + DENS * S.ns];
     double spec[NS];
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
@@ -112,7 +120,7 @@ __device__ __forceinline__ void cut_finish(const CutBox& c, int64_t t, int64_t o
             spec[s] = 0.0;
             continue;
         }
-        spec[s] = (interp_spec && have) ? ss[s] * iswn : S.p[o + (NFLO + s) * S.ns];
+        spec[s] = (interp_spec && have) ? mul(ss[s], iswn) : S.p[o + (NFLO + s) * S.ns];
     }
     S.p[o + VELX * S.ns] = vel[0];
     S.p[o + VELY * S.ns] = vel[1];
@@ -161,20 +169,19 @@ __device__ __forceinline__ void cutcell_one(const CutBox& c, int64_t t) {
                 const int w = (l + SG) + SW * ((m + SG) + SW * (n + SG));
                 if (!(l == 0 && m == 0 && n == 0)) {
                     const double wd = c_wdir[w];
-                    sv[0] += S.p[q + VELX * S.ns] * wd;
-                    sv[1] += S.p[q + VELY * S.ns] * wd;
-                    sv[2] += S.p[q + VELZ * S.ns] * wd;
-                    swd += wd;
+                    sv[0] = __fma_rn(S.p[q + VELX * S.ns], wd, sv[0]);
+                    sv[1] = __fma_rn(S.p[q + VELY * S.ns], wd, sv[1]);
+                    sv[2] = __fma_rn(S.p[q + VELZ * S.ns], wd, sv[2]);
+                    swd = add(swd, wd);
                 }
-                const double a = l * dxnd[0] - xpn[0], b = m * dxnd[1] - xpn[1], e = n * dxnd[2] - xpn[2];
-                const double wn = rcp_pos(((a * a + b * b) + e * e) + kTiny2);
-                sp += S.p[q + PRES * S.ns] * wn;
-                st += S.p[q + TEMP * S.ns] * wn;
-                sr += S.p[q + DENS * S.ns] * wn;
+                const double wn = surface_weight(l, m, n, dxnd, xpn);
+                sp = __fma_rn(S.p[q + PRES * S.ns], wn, sp);
+                st = __fma_rn(S.p[q + TEMP * S.ns], wn, st);
+                sr = __fma_rn(S.p[q + DENS * S.ns], wn, sr);
                 if (interp_spec) {
 #pragma unroll
                     for (int s = 0; s < NS; ++s)
-                        if (s < P.nspec) ss[s] += S.p[q + (NFLO + s) * S.ns] * wn;
+                        if (s < P.nspec) ss[s] = __fma_rn(S.p[q + (NFLO + s) * S.ns], wn, ss[s]);
                 }
                 swn += wn;
             }
@@ -216,8 +223,7 @@ __device__ __forceinline__ void cut_entries_one(const CutBox& c, int w, const Cu
                 const int slot = (l + SG) + SW * ((m + SG) + SW * (n + SG));
                 const bool centre = l == 0 && m == 0 && n == 0;
                 if (!centre) swd += c_wdir[slot];
-                const double a = l * dxnd[0] - xpn[0], b = m * dxnd[1] - xpn[1], e = n * dxnd[2] - xpn[2];
-                const double wn = rcp_pos(((a * a + b * b) + e * e) + kTiny2);
+                const double wn = surface_weight(l, m, n, dxnd, xpn);
                 offp[ix] = (int)q;
                 wnp[ix] = wn;
                 wdp[ix] = centre ? 0.0 : c_wdir[slot];
@@ -269,32 +275,32 @@ __device__ __forceinline__ void cutcell_cached(const CutBox& c, int w, const Cut
         }
 #pragma unroll
         for (int u = 0; u < CUT_BATCH; ++u) {
-            sv[0] += v[u][0] * wd[u];
-            sv[1] += v[u][1] * wd[u];
-            sv[2] += v[u][2] * wd[u];
-            sp += v[u][3] * wn[u];
-            st += v[u][4] * wn[u];
-            sr += v[u][5] * wn[u];
+            sv[0] = __fma_rn(v[u][0], wd[u], sv[0]);
+            sv[1] = __fma_rn(v[u][1], wd[u], sv[1]);
+            sv[2] = __fma_rn(v[u][2], wd[u], sv[2]);
+            sp = __fma_rn(v[u][3], wn[u], sp);
+            st = __fma_rn(v[u][4], wn[u], st);
+            sr = __fma_rn(v[u][5], wn[u], sr);
             if (interp_spec) {
 #pragma unroll
                 for (int s = 0; s < NS; ++s)
-                    if (s < P.nspec) ss[s] += S.p[q[u] + (NFLO + s) * S.ns] * wn[u];
+                    if (s < P.nspec) ss[s] = __fma_rn(S.p[q[u] + (NFLO + s) * S.ns], wn[u], ss[s]);
             }
         }
     }
     for (; e < kn; ++e, ix += 32) {
         const int64_t q = o + cc.off[ix];
         const double wd = cc.wd[ix], wn = cc.wn[ix];
-        sv[0] += S.p[q + VELX * S.ns] * wd;
-        sv[1] += S.p[q + VELY * S.ns] * wd;
-        sv[2] += S.p[q + VELZ * S.ns] * wd;
-        sp += S.p[q + PRES * S.ns] * wn;
-        st += S.p[q + TEMP * S.ns] * wn;
-        sr += S.p[q + DENS * S.ns] * wn;
+        sv[0] = __fma_rn(S.p[q + VELX * S.ns], wd, sv[0]);
+        sv[1] = __fma_rn(S.p[q + VELY * S.ns], wd, sv[1]);
+        sv[2] = __fma_rn(S.p[q + VELZ * S.ns], wd, sv[2]);
+        sp = __fma_rn(S.p[q + PRES * S.ns], wn, sp);
+        st = __fma_rn(S.p[q + TEMP * S.ns], wn, st);
+        sr = __fma_rn(S.p[q + DENS * S.ns], wn, sr);
         if (interp_spec) {
 #pragma unroll
             for (int s = 0; s < NS; ++s)
-                if (s < P.nspec) ss[s] += S.p[q + (NFLO + s) * S.ns] * wn;
+                if (s < P.nspec) ss[s] = __fma_rn(S.p[q + (NFLO + s) * S.ns], wn, ss[s]);
         }
     }
     cut_finish<NS>(c, t, o, cc.scal[2 * (int64_t)w], kn > 0, cc.scal[2 * (int64_t)w + 1], sv, sp, st, sr, ss);
