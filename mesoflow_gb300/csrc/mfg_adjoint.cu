@@ -39,7 +39,6 @@ namespace mfg {
 
 cudaError_t launch_cutcells_box(const mfg_box& b, const mfg_geom& g, double* tcht_scratch, int* list,
                                 unsigned* count, cudaStream_t st);
-cudaError_t launch_chem_substep(const mfg_box& b, double dt, cudaStream_t st);
 
 namespace {
 
@@ -223,6 +222,36 @@ struct AdjBox {
     Fab lamSb;   // adjoint of the stage state (grown by 3, all components)
     Fab lamAux;  // adjoint of the per-cell scalars (grown by 3, NAUX components)
 };
+
+// One box of the run's device table: the reverse kernels take every box in one
+// launch (a grid dimension is the box), since one 16^3 to 32^3 box leaves most
+// of the GPU idle (a 32^3 level in 16^3 boxes, 10 steps: 7138 launches before).
+// The run's level-wide arrays hold the boxes back to back: valid_fab and
+// grown_fab are a box's part of one with nc components.
+struct WBox {
+    int lo[3], len[3];
+    long long n;           // valid cells
+    long long voff, goff;  // cells of the boxes before this one, valid and grown
+    int ncut;              // cut cells, listed at voff of the cut-cell list
+    Fab snew, sborder;     // the caller's arrays
+};
+
+__device__ __forceinline__ Fab valid_fab(const WBox& w, double* base, int nc) {
+    return dense_fab(base + w.voff * nc, w.lo, w.len);
+}
+__device__ __forceinline__ Fab grown_fab(const WBox& w, double* base, int nc) {
+    const int lo[3] = {w.lo[0] - 3, w.lo[1] - 3, w.lo[2] - 3}, len[3] = {w.len[0] + 6, w.len[1] + 6, w.len[2] + 6};
+    return dense_fab(base + w.goff * nc, lo, len);
+}
+__device__ __forceinline__ Valid valid_of(const WBox& w) {
+    Valid v;
+    for (int d = 0; d < 3; ++d) {
+        v.lo[d] = w.lo[d];
+        v.len[d] = w.len[d];
+    }
+    v.n = w.n;
+    return v;
+}
 
 // d(dsdt)/dF: dsdt(cell) = (F(face lo) - F(face hi))/dx, so the adjoint of
 // face f's flux of state component sc is (lamL(right cell) - lamL(left cell))/dx.
@@ -527,13 +556,15 @@ __global__ void __launch_bounds__(AT, 3) adj_flux_sweep_kernel(const AdjBox* __r
     adj_flux_sweep_body<NS>(boxes[blockIdx.z], d, seg, blockIdx.y, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-// One thread per face of direction d: viscous stress (F_{m_a} -= tau_a,
+// One thread per face (blockIdx.y = direction, blockIdx.z = box): viscous stress (F_{m_a} -= tau_a,
 // F_E -= tau_a facevel_a, tau linear in the lagged velocity gradients,
 // compute_flux_3d.H:293-367) and the LLF eigenvalue
 // lam = max(aL, aR) + max(|vL|, |vR|), aR with the left cell's species
 // (flux_schemes.H:21-43), reversed.
 template <int NS>
-__global__ void __launch_bounds__(AT) adj_face_kernel(AdjBox A, int d) {
+__global__ void __launch_bounds__(AT) adj_face_kernel(const AdjBox* __restrict__ boxes) {
+    const AdjBox& A = boxes[blockIdx.z];
+    const int d = blockIdx.y;
     const RhsBox& B = A.B;
     int len[3];
     for (int e = 0; e < 3; ++e) len[e] = B.hi[e] - B.lo[e] + 1 + (e == d);
@@ -644,7 +675,8 @@ __global__ void __launch_bounds__(AT) adj_face_kernel(AdjBox A, int d) {
 // Per-cell scalars (prim_body) reversed: adjoints of (v, p, rho e_eig, a, gamma)
 // pushed into the conserved state of the cell.
 template <int NS>
-__global__ void __launch_bounds__(AT) adj_aux_kernel(AdjBox A) {
+__global__ void __launch_bounds__(AT) adj_aux_kernel(const AdjBox* __restrict__ boxes) {
+    const AdjBox& A = boxes[blockIdx.z];
     const RhsBox& B = A.B;
     int lo[3], len[3];
     for (int d = 0; d < 3; ++d) {
@@ -738,7 +770,18 @@ __global__ void __launch_bounds__(AT) adj_aux_kernel(AdjBox A) {
 // consumed and distributed to the neighbours with the forward weights.
 // Lists the cut cells (0 < vfrac < 1) of a box; the volume fraction never
 // changes, so one list serves every stage of every step.
-__global__ void adj_cut_list_kernel(CutBox c, int* __restrict__ list, unsigned* __restrict__ count) {
+__global__ void adj_cut_list_kernel(const WBox* __restrict__ boxes, int* __restrict__ lists,
+                                    unsigned* __restrict__ counts) {
+    const WBox& wb = boxes[blockIdx.y];
+    CutBox c;
+    for (int d = 0; d < 3; ++d) {
+        c.lo[d] = wb.lo[d];
+        c.len[d] = wb.len[d];
+    }
+    c.n = wb.n;
+    c.S = wb.snew;
+    int* __restrict__ list = lists + wb.voff;
+    unsigned* __restrict__ count = counts + blockIdx.y;
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     bool cut = false;
     if (t < c.n) {
@@ -757,10 +800,23 @@ __global__ void adj_cut_list_kernel(CutBox c, int* __restrict__ list, unsigned* 
 }
 
 template <int NS>
-__global__ void __launch_bounds__(AT, 4) adj_cut_kernel(CutBox c, Fab G, const int* __restrict__ list, int count) {
+__global__ void __launch_bounds__(AT, 4) adj_cut_kernel(const WBox* __restrict__ boxes, double* sb, double* lamSb,
+                                                        const int* __restrict__ lists, mfg_geom g, double dxmin) {
+    const WBox& wb = boxes[blockIdx.y];
     const int w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= count) return;
-    const int64_t t = list[w];
+    if (w >= wb.ncut) return;
+    const int N = NFLO + c_P.nspec;
+    CutBox c;
+    for (int d = 0; d < 3; ++d) {
+        c.lo[d] = wb.lo[d];
+        c.len[d] = wb.len[d];
+        c.dx[d] = g.dx[d];
+    }
+    c.n = wb.n;
+    c.S = grown_fab(wb, sb, N);
+    c.dxmin = dxmin;
+    const Fab G = grown_fab(wb, lamSb, N);
+    const int64_t t = lists[wb.voff + w];
     int i, j, k;
     cell_of(c, t, i, j, k);
     const Fab& S = c.S;
@@ -862,11 +918,15 @@ __global__ void __launch_bounds__(AT, 4) adj_cut_kernel(CutBox c, Fab G, const i
 //   stage 1: S1 = Sb + dt L;  stage 2: S2 = (S1 + dt L + 3 S_old)/4;
 //   stage 3: S3 = (S_old + 2 (S2 + dt L))/3.
 // L is the masked dsdt (div_3d.H:13-76), so masked components get no adjoint.
-__global__ void adj_stage_kernel(Valid v, Fab lamS, Fab lamOld, Fab lamL, Fab lamSb, Fab sb, int stage, double dt,
-                                 int ncomp) {
+__global__ void adj_stage_kernel(const WBox* __restrict__ boxes, double* pS, double* pOld, double* pL, double* pSb,
+                                 double* psb, int stage, double dt, int ncomp) {
+    const WBox& wb = boxes[blockIdx.z];
+    const Valid v = valid_of(wb);
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int n = blockIdx.y;
     if (t >= v.n || n >= ncomp) return;
+    const Fab lamS = valid_fab(wb, pS, ncomp), lamOld = valid_fab(wb, pOld, ncomp), lamL = valid_fab(wb, pL, ncomp),
+              lamSb = grown_fab(wb, pSb, ncomp), sb = grown_fab(wb, psb, ncomp);
     int i, j, k;
     cell_of(v, t, i, j, k);
     const double a = lamS(i, j, k, n);
@@ -898,8 +958,11 @@ __global__ void adj_stage_kernel(Valid v, Fab lamS, Fab lamOld, Fab lamL, Fab la
 // per launch; the ghost cell's adjoint goes to the cell it was taken from.
 // A velocity inlet's ghost state depends on the inlet velocity only:
 // d(ghost)/d(vel_normal) = (VEL: 1, MOM: dens, RHOE: dens vel) accumulates in gin.
-__global__ void adj_bc_kernel(Fab G, int lo0, int lo1, int lo2, int hi0, int hi1, int hi2, mfg_geom g, int stage,
-                              int nc, double* gin) {
+__global__ void adj_bc_kernel(const WBox* __restrict__ boxes, double* lamSb, mfg_geom g, int stage, int nc, double* gin) {
+    const WBox& wb = boxes[blockIdx.y];
+    const int lo0 = wb.lo[0], lo1 = wb.lo[1], lo2 = wb.lo[2], hi0 = lo0 + wb.len[0] - 1, hi1 = lo1 + wb.len[1] - 1,
+              hi2 = lo2 + wb.len[2] - 1;
+    const Fab G = grown_fab(wb, lamSb, nc);
     const int l0 = hi0 - lo0 + 7, l1 = hi1 - lo1 + 7, l2 = hi2 - lo2 + 7;
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (int64_t)l0 * l1 * l2) return;
@@ -960,9 +1023,9 @@ struct CopyTab {
     Fab dst;  // adjoint of this box's fill source (valid)
 };
 
-__global__ void adj_copy_kernel(const CopyTab* __restrict__ tab, int b, mfg_geom g, const int* __restrict__ owner,
-                                int gran, int m0, int m1, int m2, int nc) {
-    const CopyTab& T = tab[b];
+__global__ void adj_copy_kernel(const CopyTab* __restrict__ tab, mfg_geom g, const int* __restrict__ owner, int gran,
+                                int m0, int m1, int m2, int nc) {
+    const CopyTab& T = tab[blockIdx.y];
     const int l0 = T.hi[0] - T.lo[0] + 7, l1 = T.hi[1] - T.lo[1] + 7, l2 = T.hi[2] - T.lo[2] + 7;
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (int64_t)l0 * l1 * l2) return;
@@ -992,9 +1055,13 @@ __global__ void adj_copy_kernel(const CopyTab* __restrict__ tab, int b, mfg_geom
 // Primitive refresh reversed (mflo_evolve.cpp:114-171), vfrac == 1 cells:
 // DENS, VEL, PRES, TEMP are overwritten from the conserved state.
 template <int NS>
-__global__ void adj_prims_kernel(Valid v, Fab Sc, Fab lam) {
+__global__ void adj_prims_kernel(const WBox* __restrict__ boxes, double* pc, double* plam) {
+    const WBox& wb = boxes[blockIdx.y];
+    const Valid v = valid_of(wb);
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= v.n) return;
+    const int N = NFLO + c_P.nspec;
+    const Fab Sc = valid_fab(wb, pc, N), lam = valid_fab(wb, plam, N);
     int i, j, k;
     cell_of(v, t, i, j, k);
     if (!is_one(Sc(i, j, k, VFRAC))) return;
@@ -1039,9 +1106,12 @@ __global__ void adj_prims_kernel(Valid v, Fab Sc, Fab lam) {
 }
 
 // Species clipping reversed: a clipped species has no dependence on its input.
-__global__ void adj_clip_kernel(Valid v, Fab Sp, Fab lam, int nspec) {
+__global__ void adj_clip_kernel(const WBox* __restrict__ boxes, double* pp, double* plam, int nspec) {
+    const WBox& wb = boxes[blockIdx.y];
+    const Valid v = valid_of(wb);
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= v.n) return;
+    const Fab Sp = valid_fab(wb, pp, NFLO + nspec), lam = valid_fab(wb, plam, NFLO + nspec);
     int i, j, k;
     cell_of(v, t, i, j, k);
     for (int s = 0; s < nspec; ++s)
@@ -1145,9 +1215,13 @@ __device__ __forceinline__ void warp_add(double x, double* dst) {
 // s2 = s0 + dt/4 (f0 + f1), out = s0 + dt (f0/6 + f1/6 + 2 f2/3), T fixed);
 // S3 is the sub-step's input.  Non-species components pass through.
 template <int NS>
-__global__ void adj_chem_kernel(Valid v, Fab S3, Fab lam, double dt, double* gth) {
+__global__ void adj_chem_kernel(const WBox* __restrict__ boxes, double* p3, double* plam, double dt, double* gth) {
+    const WBox& wb = boxes[blockIdx.y];
+    const Valid v = valid_of(wb);
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t - threadIdx.x >= v.n) return;  // whole block past this box
     const DevParams& P = c_P;
+    const Fab S3 = valid_fab(wb, p3, NFLO + P.nspec), lam = valid_fab(wb, plam, NFLO + P.nspec);
     double thb[MAXR];
     for (int r = 0; r < MAXR; ++r) thb[r] = 0.0;
     if (t < v.n && P.chem_on) {
@@ -1290,7 +1364,12 @@ struct Work {
     size_t vtot = 0, gtot = 0;         // cells
     std::vector<size_t> fsoff;         // per box and direction: offset of its face scalars (doubles)
     size_t fstot = 0;
+    int64_t maxvalid = 0, maxgrown = 0, maxface = 0;  // largest box's cells and faces of one direction
+    int maxcut = 0;
     std::vector<double*> owned;
+    double* arena = nullptr;  // one allocation for the run's arrays (owned by `owned`); its rest
+    size_t arena_left = 0;
+    WBox* d_wb = nullptr;
     int* d_owner = nullptr;
     int gran = 1, mlen[3] = {1, 1, 1};
     CopyTab* d_tab = nullptr;  // [nbox] -> lam, [nbox] -> lamOld
@@ -1302,10 +1381,10 @@ struct Work {
     double* d_g = nullptr;  // [J, d/du_in, d/dlog A_r ...]
     int* d_cutlist = nullptr;        // per box (at vcell[b]): its cut cells
     unsigned* d_cutcount = nullptr;  // per box
-    std::vector<int> ncut;
 
     ~Work() {
         for (double* p : owned) cudaFree(p);
+        cudaFree(d_wb);
         cudaFree(d_owner);
         cudaFree(d_tab);
         cudaFree(d_scratch);
@@ -1316,7 +1395,25 @@ struct Work {
         cudaFree(d_cutlist);
         cudaFree(d_cutcount);
     }
+    // Room for the arrays of the run in one allocation (dozens of cudaMalloc and
+    // cudaFree calls otherwise); without it each array is allocated by itself.
+    void reserve(size_t doubles) {
+        if (cudaMalloc(&arena, std::max<size_t>(doubles, 1) * sizeof(double)) != cudaSuccess) {
+            cudaGetLastError();
+            arena = nullptr;
+            return;
+        }
+        owned.push_back(arena);
+        arena_left = doubles;
+    }
+    static size_t padded(size_t doubles) { return (doubles + 31) / 32 * 32; }
     double* alloc(size_t doubles) {
+        if (arena && padded(doubles) <= arena_left) {
+            double* q = arena;
+            arena += padded(doubles);
+            arena_left -= padded(doubles);
+            return q;
+        }
         double* p = nullptr;
         const cudaError_t e = cudaMalloc(&p, std::max<size_t>(doubles, 1) * sizeof(double));
         if (e != cudaSuccess) {
@@ -1355,33 +1452,32 @@ struct Work {
         a.ncomp = N;
         return a;
     }
-    int64_t grown_cells(int b) const {
-        int64_t n = 1;
-        for (int d = 0; d < 3; ++d) n *= boxes[b].hi[d] - boxes[b].lo[d] + 7;
-        return n;
-    }
 };
 
-__global__ void copy_box_kernel(Fab dst, Fab src, Valid v, int nc) {
+// Every box's valid cells (mode 0: buf <- s_new, 1: s_new <- buf) or grown cells
+// (2: buf <- sborder); blockIdx.y = component, blockIdx.z = box.
+__global__ void copy_boxes_kernel(const WBox* __restrict__ boxes, double* buf, int mode, int nc) {
+    const WBox& wb = boxes[blockIdx.z];
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int n = blockIdx.y;
-    if (t >= v.n || n >= nc) return;
+    const int n = blockIdx.y, gr = mode == 2 ? 3 : 0;
     int i, j, k;
-    cell_of(v, t, i, j, k);
-    dst(i, j, k, n) = src(i, j, k, n);
+    if (t >= (int64_t)(wb.len[0] + 2 * gr) * (wb.len[1] + 2 * gr) * (wb.len[2] + 2 * gr)) return;
+    split3(t, wb.len[0] + 2 * gr, wb.len[1] + 2 * gr, i, j, k);
+    i += wb.lo[0] - gr;
+    j += wb.lo[1] - gr;
+    k += wb.lo[2] - gr;
+    const Fab d = mode == 2 ? grown_fab(wb, buf, nc) : valid_fab(wb, buf, nc);
+    const Fab& s = mode == 2 ? wb.sborder : wb.snew;
+    if (mode == 1)
+        s(i, j, k, n) = d(i, j, k, n);
+    else
+        d(i, j, k, n) = s(i, j, k, n);
 }
 
-cudaError_t copy_region(const Fab& dst, const Fab& src, const int lo[3], const int hi[3], int nc, cudaStream_t st) {
-    Valid v;
-    v.n = 1;
-    for (int d = 0; d < 3; ++d) {
-        v.lo[d] = lo[d];
-        v.len[d] = hi[d] - lo[d] + 1;
-        v.n *= v.len[d];
-    }
-    dim3 g(nblk(v.n, 256), nc);
+cudaError_t copy_boxes(const Work& W, double* buf, int mode, cudaStream_t st) {
+    const dim3 g(nblk(mode == 2 ? W.maxgrown : W.maxvalid, 256), W.N, W.nbox);
     ProfScope ps(K_SNAPSHOT, st);
-    copy_box_kernel<<<g, 256, 0, st>>>(dst, src, v, nc);
+    copy_boxes_kernel<<<g, 256, 0, st>>>(W.d_wb, buf, mode, W.N);
     return cudaGetLastError();
 }
 
@@ -1420,8 +1516,6 @@ void snap_views(const Work& W, RhsBox& B, const Snap& sn, int stage, int b) {
 // clipping on, no norms); with snap the intermediates are saved.
 int fwd_step(Work& W, double dt, const Snap* snap, cudaStream_t st) {
     const int N = W.N;
-    Fab none;
-    memset(&none, 0, sizeof(none));
     ADJ_TRY(launch_copy_old(W.boxes.data(), W.nbox, N, st), "forward: phi_old copy");
     for (int stage = 1; stage <= 3; ++stage) {
         ADJ_TRY(launch_fill_patch(W.boxes.data(), W.nbox, W.g, stage == 1 ? 0 : 1, 0.0, st), "forward: fill patch");
@@ -1431,20 +1525,14 @@ int fwd_step(Work& W, double dt, const Snap* snap, cudaStream_t st) {
         if (lv == 0)
             for (int b = 0; b < W.nbox; ++b)
                 ADJ_TRY(launch_cutcells_box(W.boxes[b], W.g, nullptr, W.d_list, W.d_count, st), "forward: cut cells");
+        if (snap) ADJ_TRY(copy_boxes(W, snap->sb[stage - 1], 2, st), "forward: stage snapshot");
         for (int b = 0; b < W.nbox;) {
             const int n = W.grouped ? rhs_group_count(W.boxes.data() + b, W.nbox - b) : 1;
             RhsBox B[kRhsGroup];
             double* scratch = W.d_scratch;
             for (int q = 0; q < n; ++q) {
-                const mfg_box& x = W.boxes[b + q];
-                if (snap) {
-                    const int lo[3] = {x.lo[0] - 3, x.lo[1] - 3, x.lo[2] - 3};
-                    const int hi[3] = {x.hi[0] + 3, x.hi[1] + 3, x.hi[2] + 3};
-                    ADJ_TRY(copy_region(W.gfab(snap->sb[stage - 1], b + q, N), make_fab(x.sborder), lo, hi, N, st),
-                            "forward: stage snapshot");
-                }
-                B[q] = layout_rhs_box(x, W.g, scratch);
-                scratch += rhs_box_scratch_doubles(x);
+                B[q] = layout_rhs_box(W.boxes[b + q], W.g, scratch);
+                scratch += rhs_box_scratch_doubles(W.boxes[b + q]);
                 if (snap) snap_views(W, B[q], *snap, stage, b + q);  // keep the stage's primitives and face scalars
             }
             ADJ_TRY(launch_rhs_boxes(B, n, stage, dt, weno_fast_mode(), st), "forward: right-hand side");
@@ -1458,17 +1546,13 @@ int fwd_step(Work& W, double dt, const Snap* snap, cudaStream_t st) {
                     "forward: bookends");
         return MFG_OK;
     }
-    for (int b = 0; b < W.nbox; ++b) {
-        const mfg_box& x = W.boxes[b];
-        if (snap) ADJ_TRY(copy_region(W.vfab(snap->s3, b), make_fab(x.s_new), x.lo, x.hi, N, st), "forward: snapshot");
-        ADJ_TRY(launch_axpy_valid(x, make_fab(x.s_old), none, 0.0, true, make_fab(x.s_new), N, st),
-                "forward: chemistry copy");
-        ADJ_TRY(launch_chem_substep(x, dt, st), "forward: chemistry");
-        if (snap) ADJ_TRY(copy_region(W.vfab(snap->sc, b), make_fab(x.s_new), x.lo, x.hi, N, st), "forward: snapshot");
-        ADJ_TRY(launch_update_prims(x, nullptr, st), "forward: primitives");
-        if (snap) ADJ_TRY(copy_region(W.vfab(snap->sp, b), make_fab(x.s_new), x.lo, x.hi, N, st), "forward: snapshot");
-        ADJ_TRY(launch_clip_species(x, st), "forward: clipping");
-    }
+    ADJ_TRY(copy_boxes(W, snap->s3, 0, st), "forward: snapshot");
+    ADJ_TRY(launch_copy_old(W.boxes.data(), W.nbox, N, st), "forward: chemistry copy");
+    ADJ_TRY(launch_chem_substep(W.boxes.data(), W.nbox, dt, st), "forward: chemistry");
+    ADJ_TRY(copy_boxes(W, snap->sc, 0, st), "forward: snapshot");
+    ADJ_TRY(launch_update_prims(W.boxes.data(), W.nbox, st), "forward: primitives");
+    ADJ_TRY(copy_boxes(W, snap->sp, 0, st), "forward: snapshot");
+    ADJ_TRY(launch_clip_species(W.boxes.data(), W.nbox, st), "forward: clipping");
     return MFG_OK;
 }
 
@@ -1478,36 +1562,28 @@ int adj_step(Work& W, double dt, const Snap& sn, double* lam, double* lamOld, do
              double* lamAux, cudaStream_t st) {
     const int N = W.N, ns = c_host_params().nspec;
     ADJ_TRY(cudaMemsetAsync(lamOld, 0, W.vtot * N * sizeof(double), st), "reverse: clear");
-    for (int b = 0; b < W.nbox; ++b) {
-        const Valid v = valid_of(W.boxes[b]);
-        {
-            ProfScope ps(K_ADJ_LOCAL, st);
-            adj_clip_kernel<<<nblk(v.n, 256), 256, 0, st>>>(v, W.vfab(sn.sp, b), W.vfab(lam, b), ns);
-        }
-        {
-            ProfScope ps(K_ADJ_LOCAL, st);
-            ADJ_NS(adj_prims_kernel, (nblk(v.n, AT), AT, 0, st), (v, W.vfab(sn.sc, b), W.vfab(lam, b)));
-        }
-        {
-            ProfScope ps(K_ADJ_LOCAL, st);
-            ADJ_NS(adj_chem_kernel, (nblk(v.n, AT), AT, 0, st),
-                   (v, W.vfab(sn.s3, b), W.vfab(lam, b), dt, W.d_g + 2));
-        }
-        ADJ_TRY(cudaGetLastError(), "reverse: clipping, primitives, chemistry");
+    const dim3 gv(nblk(W.maxvalid, 256), W.nbox), gva(nblk(W.maxvalid, AT), W.nbox);
+    {
+        ProfScope ps(K_ADJ_LOCAL, st, 3);
+        adj_clip_kernel<<<gv, 256, 0, st>>>(W.d_wb, sn.sp, lam, ns);
+        ADJ_NS(adj_prims_kernel, (gva, AT, 0, st), (W.d_wb, sn.sc, lam));
+        ADJ_NS(adj_chem_kernel, (gva, AT, 0, st), (W.d_wb, sn.s3, lam, dt, W.d_g + 2));
     }
+    ADJ_TRY(cudaGetLastError(), "reverse: clipping, primitives, chemistry");
     const double dxmin = std::min(W.g.dx[0], std::min(W.g.dx[1], W.g.dx[2]));
+    const int C = NCONS + ns;
+    const bool sweep = adj_flux_sweep();
+    const unsigned nbg = nblk(W.maxgrown, 256), nbf = nblk(W.maxface, AT);
     for (int stage = 3; stage >= 1; --stage) {
         double* sb = sn.sb[stage - 1];
         ADJ_TRY(cudaMemsetAsync(lamSb, 0, W.gtot * N * sizeof(double), st), "reverse: clear");
         ADJ_TRY(cudaMemsetAsync(lamAux, 0, W.gtot * NAUX * sizeof(double), st), "reverse: clear");
-        for (int b = 0; b < W.nbox; ++b) {
-            const Valid v = valid_of(W.boxes[b]);
-            dim3 g(nblk(v.n, 256), N);
+        {
             ProfScope ps(K_ADJ_LOCAL, st);
-            adj_stage_kernel<<<g, 256, 0, st>>>(v, W.vfab(lam, b), W.vfab(lamOld, b), W.vfab(lamL, b),
-                                                W.gfab(lamSb, b, N), W.gfab(sb, b, N), stage, dt, N);
-            ADJ_TRY(cudaGetLastError(), "reverse: stage algebra");
+            adj_stage_kernel<<<dim3(nblk(W.maxvalid, 256), N, W.nbox), 256, 0, st>>>(W.d_wb, lam, lamOld, lamL, lamSb,
+                                                                                     sb, stage, dt, N);
         }
+        ADJ_TRY(cudaGetLastError(), "reverse: stage algebra");
         // forward views of the stage for every box: its state, per-cell primitives
         // and face scalars as the forward computed them
         std::vector<AdjBox> adj(W.nbox);
@@ -1521,71 +1597,47 @@ int adj_step(Work& W, double dt, const Snap& sn, double* lam, double* lamOld, do
             A.lamSb = W.gfab(lamSb, b, N);
             A.lamAux = W.gfab(lamAux, b, NAUX);
         }
-        const int C = NCONS + c_host_params().nspec;
-        const bool sweep = adj_flux_sweep();
-        if (sweep) {  // hyperbolic fluxes of all boxes, one column-sweep launch per direction
-            ADJ_TRY(cudaMemcpyAsync(W.d_adj, adj.data(), W.nbox * sizeof(AdjBox), cudaMemcpyHostToDevice, st),
-                    "reverse: box views");
-            for (int d = 0; d < 3; ++d) {
+        ADJ_TRY(cudaMemcpyAsync(W.d_adj, adj.data(), W.nbox * sizeof(AdjBox), cudaMemcpyHostToDevice, st),
+                "reverse: box views");
+        for (int d = 0; d < 3; ++d) {
+            ProfScope ps(K_ADJ_FLUX, st);
+            if (sweep) {
                 unsigned nbs = 1;
                 for (int b = 0; b < W.nbox; ++b) nbs = std::max(nbs, nblk(sweep_items(adj[b].B, d, kAdjSeg), AT));
-                ProfScope ps(K_ADJ_FLUX, st);
                 ADJ_NS(adj_flux_sweep_kernel, (dim3(nbs, C, W.nbox), AT, 0, st), (W.d_adj, d, kAdjSeg));
-                ADJ_TRY(cudaGetLastError(), "reverse: face fluxes");
+            } else {
+                for (int b = 0; b < W.nbox; ++b)
+                    ADJ_NS(adj_flux_kernel, (dim3(nblk(face_items(adj[b].B, d), AT), C), AT, 0, st), (adj[b], d));
             }
         }
-        for (int b = 0; b < W.nbox; ++b) {
-            const AdjBox& A = adj[b];
-            const mfg_box& x = W.boxes[b];
-            const int64_t ng = W.grown_cells(b);
-            for (int d = 0; d < 3; ++d) {
-                const unsigned nbf = nblk(face_items(A.B, d), AT);
-                if (!sweep) {
-                    ProfScope ps(K_ADJ_FLUX, st);
-                    ADJ_NS(adj_flux_kernel, (dim3(nbf, C), AT, 0, st), (A, d));
-                }
-                {
-                    ProfScope ps(K_ADJ_FACE, st);
-                    ADJ_NS(adj_face_kernel, (nbf, AT, 0, st), (A, d));
-                }
-                ADJ_TRY(cudaGetLastError(), "reverse: face fluxes");
-            }
-            {
-                ProfScope ps(K_ADJ_CELL, st);
-                ADJ_NS(adj_aux_kernel, (nblk(ng, AT), AT, 0, st), (A));
-            }
-            ADJ_TRY(cudaGetLastError(), "reverse: per-cell primitives (adjoint)");
-            CutBox c;
-            memset(&c, 0, sizeof(c));
-            c.n = 1;
-            for (int d = 0; d < 3; ++d) {
-                c.lo[d] = x.lo[d];
-                c.len[d] = x.hi[d] - x.lo[d] + 1;
-                c.n *= c.len[d];
-                c.dx[d] = W.g.dx[d];
-            }
-            c.S = W.gfab(sb, b, N);
-            c.dxmin = dxmin;
-            if (W.ncut[b] > 0) {
-                ProfScope ps(K_ADJ_CUT, st);
-                ADJ_NS(adj_cut_kernel, (nblk(W.ncut[b], AT), AT, 0, st),
-                       (c, W.gfab(lamSb, b, N), W.d_cutlist + W.vcell[b], W.ncut[b]));
-            }
-            ADJ_TRY(cudaGetLastError(), "reverse: cut cells");
-            if (!(W.g.is_periodic[0] && W.g.is_periodic[1] && W.g.is_periodic[2]))
-                for (int s = 3; s >= 1; --s) {
-                    ProfScope ps(K_ADJ_FILL, st);
-                    adj_bc_kernel<<<nblk(ng, 256), 256, 0, st>>>(W.gfab(lamSb, b, N), x.lo[0], x.lo[1], x.lo[2],
-                                                                 x.hi[0], x.hi[1], x.hi[2], W.g, s, N, W.d_g + 1);
-                }
-            ADJ_TRY(cudaGetLastError(), "reverse: physical boundaries");
+        {
+            ProfScope ps(K_ADJ_FACE, st);
+            ADJ_NS(adj_face_kernel, (dim3(nbf, 3, W.nbox), AT, 0, st), (W.d_adj));
         }
+        ADJ_TRY(cudaGetLastError(), "reverse: face fluxes");
+        {
+            ProfScope ps(K_ADJ_CELL, st);
+            ADJ_NS(adj_aux_kernel, (dim3(nblk(W.maxgrown, AT), 1, W.nbox), AT, 0, st), (W.d_adj));
+        }
+        ADJ_TRY(cudaGetLastError(), "reverse: per-cell primitives (adjoint)");
+        if (W.maxcut > 0) {
+            ProfScope ps(K_ADJ_CUT, st);
+            ADJ_NS(adj_cut_kernel, (dim3(nblk(W.maxcut, AT), W.nbox), AT, 0, st),
+                   (W.d_wb, sb, lamSb, W.d_cutlist, W.g, dxmin));
+        }
+        ADJ_TRY(cudaGetLastError(), "reverse: cut cells");
+        if (!(W.g.is_periodic[0] && W.g.is_periodic[1] && W.g.is_periodic[2]))
+            for (int s = 3; s >= 1; --s) {
+                ProfScope ps(K_ADJ_FILL, st);
+                adj_bc_kernel<<<dim3(nbg, W.nbox), 256, 0, st>>>(W.d_wb, lamSb, W.g, s, N, W.d_g + 1);
+            }
+        ADJ_TRY(cudaGetLastError(), "reverse: physical boundaries");
         // the copies return the adjoint to the fill source: S_old in stage 1, else the previous stage
         const CopyTab* tab = W.d_tab + (stage == 1 ? W.nbox : 0);
-        for (int b = 0; b < W.nbox; ++b) {
+        {
             ProfScope ps(K_ADJ_FILL, st);
-            adj_copy_kernel<<<nblk(W.grown_cells(b), 256), 256, 0, st>>>(tab, b, W.g, W.d_owner, W.gran, W.mlen[0],
-                                                                         W.mlen[1], W.mlen[2], N);
+            adj_copy_kernel<<<dim3(nbg, W.nbox), 256, 0, st>>>(tab, W.g, W.d_owner, W.gran, W.mlen[0], W.mlen[1],
+                                                               W.mlen[2], N);
         }
         ADJ_TRY(cudaGetLastError(), "reverse: ghost copies");
     }
@@ -1698,25 +1750,40 @@ extern "C" int mfg_adjoint_objective(const mfg_box* boxes, int nbox, const mfg_g
     ADJ_TRY(cudaMalloc(&W.d_cutlist, std::max<size_t>(W.vtot, 1) * sizeof(int)), "allocation");
     ADJ_TRY(cudaMalloc(&W.d_cutcount, nbox * sizeof(unsigned)), "allocation");
     ADJ_TRY(cudaMemsetAsync(W.d_cutcount, 0, nbox * sizeof(unsigned), st), "clear");
+    std::vector<WBox> wb(nbox);
     for (int b = 0; b < nbox; ++b) {
-        CutBox c;
-        memset(&c, 0, sizeof(c));
-        c.n = 1;
+        WBox& w = wb[b];
+        memset(&w, 0, sizeof(w));
+        w.n = 1;
+        int64_t ng = 1;
         for (int d = 0; d < 3; ++d) {
-            c.lo[d] = boxes[b].lo[d];
-            c.len[d] = boxes[b].hi[d] - boxes[b].lo[d] + 1;
-            c.n *= c.len[d];
+            w.lo[d] = boxes[b].lo[d];
+            w.len[d] = boxes[b].hi[d] - boxes[b].lo[d] + 1;
+            w.n *= w.len[d];
+            ng *= w.len[d] + 6;
         }
-        c.S = make_fab(boxes[b].s_new);
-        adj_cut_list_kernel<<<nblk(c.n, 256), 256, 0, st>>>(c, W.d_cutlist + W.vcell[b], W.d_cutcount + b);
+        for (int d = 0; d < 3; ++d) W.maxface = std::max<int64_t>(W.maxface, w.n / w.len[d] * (w.len[d] + 1));
+        w.voff = (long long)W.vcell[b];
+        w.goff = (long long)W.gcell[b];
+        w.snew = make_fab(boxes[b].s_new);
+        w.sborder = make_fab(boxes[b].sborder);
+        W.maxvalid = std::max<int64_t>(W.maxvalid, w.n);
+        W.maxgrown = std::max(W.maxgrown, ng);
     }
+    ADJ_TRY(cudaMalloc(&W.d_wb, nbox * sizeof(WBox)), "allocation");
+    ADJ_TRY(cudaMemcpyAsync(W.d_wb, wb.data(), nbox * sizeof(WBox), cudaMemcpyHostToDevice, st), "box table");
+    adj_cut_list_kernel<<<dim3(nblk(W.maxvalid, 256), nbox), 256, 0, st>>>(W.d_wb, W.d_cutlist, W.d_cutcount);
     ADJ_TRY(cudaGetLastError(), "cut-cell lists");
     {
         std::vector<unsigned> h(nbox);
         ADJ_TRY(cudaMemcpyAsync(h.data(), W.d_cutcount, nbox * sizeof(unsigned), cudaMemcpyDeviceToHost, st),
                 "cut-cell lists");
         ADJ_TRY(cudaStreamSynchronize(st), "cut-cell lists");
-        W.ncut.assign(h.begin(), h.end());
+        for (int b = 0; b < nbox; ++b) {
+            wb[b].ncut = (int)h[b];
+            W.maxcut = std::max(W.maxcut, (int)h[b]);
+        }
+        ADJ_TRY(cudaMemcpy(W.d_wb, wb.data(), nbox * sizeof(WBox), cudaMemcpyHostToDevice), "box table");
     }
     // owner map of the copies (as the ghost fill's)
     {
@@ -1765,6 +1832,12 @@ extern "C" int mfg_adjoint_objective(const mfg_box* boxes, int nbox, const mfg_g
         seg_keep = need + (size_t)2 * 1024 * 1024 * 1024 < free_b;
     }
     std::vector<double*> ckpt(nseg), zst((keep_all || seg_keep) ? 0 : ce);
+    {
+        const size_t nsnap = keep_all ? nsteps : seg_keep ? ce : 1;
+        const size_t vb = Work::padded(W.vtot * W.N), gb = Work::padded(W.gtot * W.N), xb = Work::padded(W.gtot * NAUX),
+                     fb = Work::padded(W.fstot);
+        W.reserve((ckpt.size() + zst.size() + 4) * vb + nsnap * (3 * (gb + xb + fb) + 3 * vb) + gb + xb);
+    }
     for (auto& p : ckpt)
         if (!(p = W.valid_buf())) return MFG_ERR_CUDA;
     for (auto& p : zst)
@@ -1801,15 +1874,11 @@ extern "C" int mfg_adjoint_objective(const mfg_box* boxes, int nbox, const mfg_g
         ADJ_TRY(cudaMemcpy(W.d_tab, tab.data(), tab.size() * sizeof(CopyTab), cudaMemcpyHostToDevice), "copy table");
     }
     auto save = [&](double* dst) -> int {
-        for (int b = 0; b < nbox; ++b)
-            ADJ_TRY(copy_region(W.vfab(dst, b), make_fab(boxes[b].s_new), boxes[b].lo, boxes[b].hi, W.N, st),
-                    "checkpoint");
+        ADJ_TRY(copy_boxes(W, dst, 0, st), "checkpoint");
         return MFG_OK;
     };
     auto restore = [&](double* src) -> int {
-        for (int b = 0; b < nbox; ++b)
-            ADJ_TRY(copy_region(make_fab(boxes[b].s_new), W.vfab(src, b), boxes[b].lo, boxes[b].hi, W.N, st),
-                    "restore");
+        ADJ_TRY(copy_boxes(W, src, 1, st), "restore");
         return MFG_OK;
     };
     // forward sweep with checkpoints (or with every step's intermediates); with

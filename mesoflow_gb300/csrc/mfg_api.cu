@@ -12,7 +12,6 @@ namespace mfg {
 
 cudaError_t launch_cutcells_box(const mfg_box& b, const mfg_geom& g, double* tcht_scratch, int* list,
                                 unsigned* count, cudaStream_t st);
-cudaError_t launch_chem_substep(const mfg_box& b, double dt, cudaStream_t st);
 cudaError_t launch_resnorm_box(const mfg_box& b, double dt, double* partial, double* acc, cudaStream_t st);
 void fill_release();
 
@@ -453,9 +452,7 @@ int mfg_chem_substep(const mfg_box* boxes, int nbox, const mfg_geom* geom, doubl
     (void)geom;
     int rc = check_boxes(boxes, nbox, false, false, true, true);
     if (rc) return rc;
-    for (int b = 0; b < nbox; ++b)
-        if (launch_chem_substep(boxes[b], dt, (cudaStream_t)stream) != cudaSuccess) return MFG_ERR_CUDA;
-    return MFG_OK;
+    return launch_chem_substep(boxes, nbox, dt, (cudaStream_t)stream) == cudaSuccess ? MFG_OK : MFG_ERR_CUDA;
 }
 
 int mfg_update_primitive_vars(const mfg_box* boxes, int nbox, const mfg_geom* geom, void* stream) {
@@ -465,8 +462,7 @@ int mfg_update_primitive_vars(const mfg_box* boxes, int nbox, const mfg_geom* ge
     cudaStream_t st = (cudaStream_t)stream;
     unsigned before = 0;
     if (cudaStreamSynchronize(st) != cudaSuccess || read_status(&before, false) != cudaSuccess) return MFG_ERR_CUDA;
-    for (int b = 0; b < nbox; ++b)
-        if (launch_update_prims(boxes[b], nullptr, st) != cudaSuccess) return MFG_ERR_CUDA;
+    if (launch_update_prims(boxes, nbox, st) != cudaSuccess) return MFG_ERR_CUDA;
     unsigned after = 0;
     if (cudaStreamSynchronize(st) != cudaSuccess || read_status(&after, false) != cudaSuccess) return MFG_ERR_CUDA;
     return (after & MFG_STATUS_NEG_PRESSURE) ? MFG_ERR_NEG_PRESSURE : MFG_OK;
@@ -503,9 +499,7 @@ int mfg_update_vars_after_chemsolve(const mfg_box* boxes, int nbox, int using_bg
 int mfg_clip_species(const mfg_box* boxes, int nbox, void* stream) {
     int rc = check_boxes(boxes, nbox, false, false, false, true);
     if (rc) return rc;
-    for (int b = 0; b < nbox; ++b)
-        if (launch_clip_species(boxes[b], (cudaStream_t)stream) != cudaSuccess) return MFG_ERR_CUDA;
-    return MFG_OK;
+    return launch_clip_species(boxes, nbox, (cudaStream_t)stream) == cudaSuccess ? MFG_OK : MFG_ERR_CUDA;
 }
 
 int mfg_residual_norms(const mfg_box* boxes, int nbox, double dt, double* out, void* stream) {

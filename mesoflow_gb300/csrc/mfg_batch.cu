@@ -32,7 +32,6 @@ namespace mfg {
 
 cudaError_t launch_cutcells_box(const mfg_box& b, const mfg_geom& g, double* tcht_scratch, int* list,
                                 unsigned* count, cudaStream_t st);
-cudaError_t launch_chem_substep(const mfg_box& b, double dt, cudaStream_t st);
 
 namespace {
 
@@ -1077,9 +1076,9 @@ int step_plain(mfg_boxlist& L, double dt, cudaStream_t st) {
         if (launch_axpy_valid(L.boxes[b], make_fab(L.boxes[b].s_old), none, 0.0, true, make_fab(L.boxes[b].s_new), nc,
                               st) != cudaSuccess)
             return MFG_ERR_CUDA;
-        if (launch_chem_substep(L.boxes[b], dt, st) != cudaSuccess) return MFG_ERR_CUDA;
-        if (launch_update_prims(L.boxes[b], nullptr, st) != cudaSuccess) return MFG_ERR_CUDA;
-        if (launch_clip_species(L.boxes[b], st) != cudaSuccess) return MFG_ERR_CUDA;
+        if (launch_chem_substep(&L.boxes[b], 1, dt, st) != cudaSuccess) return MFG_ERR_CUDA;
+        if (launch_update_prims(&L.boxes[b], 1, st) != cudaSuccess) return MFG_ERR_CUDA;
+        if (launch_clip_species(&L.boxes[b], 1, st) != cudaSuccess) return MFG_ERR_CUDA;
     }
     return MFG_OK;
 }
@@ -1428,7 +1427,7 @@ void amr_chem(mfg_boxlist& L, AmrRun& R, int l, double dtl) {
     const int nc = NFLO + c_host_params().nspec;
     if (R.mode == 0) {
         for (int b = 0; b < L.nbox; ++b)
-            if (L.boxes[b].level == l) amr_note(R, launch_chem_substep(L.boxes[b], dtl, R.st));
+            if (L.boxes[b].level == l) amr_note(R, launch_chem_substep(&L.boxes[b], 1, dtl, R.st));
         return;
     }
     const PhaseTiles& V = level_tiles(L, l)[PH_VALID];
@@ -1499,8 +1498,8 @@ int amr_run(mfg_boxlist& L, double time, double dt0, bool launch, int mode, cuda
     if (!launch) return MFG_OK;
     if (mode == 0) {
         for (int b = 0; b < L.nbox; ++b) {
-            amr_note(R, launch_update_prims(L.boxes[b], nullptr, st));
-            amr_note(R, launch_clip_species(L.boxes[b], st));
+            amr_note(R, launch_update_prims(&L.boxes[b], 1, st));
+            amr_note(R, launch_clip_species(&L.boxes[b], 1, st));
         }
     } else {
         const PhaseTiles& V = L.ph[PH_VALID];

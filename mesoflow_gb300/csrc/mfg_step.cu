@@ -11,13 +11,21 @@ template <int NS>
 __global__ void chem_source_kernel(Valid v, Fab S, Fab D) {
     chem_source_body<NS>(v, S, D, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
+// Boxes of one launch of the chemistry sub-step, primitive refresh and clipping
+// (blockIdx.y).
+constexpr int LOCAL_GROUP = 8;
+struct LocalGroup {
+    Valid v[LOCAL_GROUP];
+    Fab so[LOCAL_GROUP], sn[LOCAL_GROUP];
+};
 template <int NS>
-__global__ void chem_substep_kernel(Valid v, Fab So, Fab Sn, double dt, int ncomp) {
-    chem_substep_body<NS>(v, So, Sn, dt, ncomp, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
+__global__ void chem_substep_kernel(const __grid_constant__ LocalGroup g, double dt, int ncomp) {
+    const int q = blockIdx.y;
+    chem_substep_body<NS>(g.v[q], g.so[q], g.sn[q], dt, ncomp, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 template <int NS>
-__global__ void prims_kernel(Valid v, Fab S) {
-    prims_body<NS>(v, S, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
+__global__ void prims_kernel(const __grid_constant__ LocalGroup g) {
+    prims_body<NS>(g.v[blockIdx.y], g.sn[blockIdx.y], (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 template <int NS>
 __global__ void chem_rk2_kernel(Valid v, Fab So, Fab Sn, double dt, int ncomp) {
@@ -34,8 +42,8 @@ __global__ void vars_after_chem_kernel(Valid v, Fab S, int bg) {
     vars_after_chem_body<NS>(v, S, bg, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-__global__ void clip_kernel(Valid v, Fab S, int nspec) {
-    clip_body(v, S, nspec, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
+__global__ void clip_kernel(const __grid_constant__ LocalGroup g, int nspec) {
+    clip_body(g.v[blockIdx.y], g.sn[blockIdx.y], nspec, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // Block partial sums of ((s_new - s_old)/dt [* vfrac_old])^2 per component;
@@ -229,30 +237,47 @@ cudaError_t launch_chem_source(const mfg_box& b, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_chem_substep(const mfg_box& b, double dt, cudaStream_t st) {
-    Valid v = valid_of(b);
-    Fab So = make_fab(b.s_old), Sn = make_fab(b.s_new);
-    const int ns = c_host_params().nspec, nc = NFLO + ns;
-    ProfScope ps(K_CHEM, st);
-    if (ns <= 1) chem_substep_kernel<1><<<nblocks(v.n), TPB, 0, st>>>(v, So, Sn, dt, nc);
-    else if (ns <= 2) chem_substep_kernel<2><<<nblocks(v.n), TPB, 0, st>>>(v, So, Sn, dt, nc);
-    else if (ns <= 4) chem_substep_kernel<4><<<nblocks(v.n), TPB, 0, st>>>(v, So, Sn, dt, nc);
-    else if (ns <= 8) chem_substep_kernel<8><<<nblocks(v.n), TPB, 0, st>>>(v, So, Sn, dt, nc);
-    else chem_substep_kernel<16><<<nblocks(v.n), TPB, 0, st>>>(v, So, Sn, dt, nc);
+// Calls f(group, grid) for the boxes, LOCAL_GROUP at a time.
+template <class F>
+static cudaError_t for_local_groups(const mfg_box* boxes, int nbox, F&& f) {
+    for (int b = 0; b < nbox; b += LOCAL_GROUP) {
+        const int n = std::min(LOCAL_GROUP, nbox - b);
+        LocalGroup g;
+        int64_t most = 0;
+        for (int q = 0; q < LOCAL_GROUP; ++q) {
+            const mfg_box& x = boxes[b + (q < n ? q : 0)];
+            g.v[q] = valid_of(x);
+            g.so[q] = make_fab(x.s_old);
+            g.sn[q] = make_fab(x.s_new);
+            most = std::max(most, g.v[q].n);
+        }
+        f(g, dim3(nblocks(most), n));
+    }
     return cudaGetLastError();
 }
 
-cudaError_t launch_update_prims(const mfg_box& b, double*, cudaStream_t st) {
-    Valid v = valid_of(b);
-    Fab S = make_fab(b.s_new);
+cudaError_t launch_chem_substep(const mfg_box* boxes, int nbox, double dt, cudaStream_t st) {
+    const int ns = c_host_params().nspec, nc = NFLO + ns;
+    return for_local_groups(boxes, nbox, [&](const LocalGroup& g, dim3 grid) {
+        ProfScope ps(K_CHEM, st);
+        if (ns <= 1) chem_substep_kernel<1><<<grid, TPB, 0, st>>>(g, dt, nc);
+        else if (ns <= 2) chem_substep_kernel<2><<<grid, TPB, 0, st>>>(g, dt, nc);
+        else if (ns <= 4) chem_substep_kernel<4><<<grid, TPB, 0, st>>>(g, dt, nc);
+        else if (ns <= 8) chem_substep_kernel<8><<<grid, TPB, 0, st>>>(g, dt, nc);
+        else chem_substep_kernel<16><<<grid, TPB, 0, st>>>(g, dt, nc);
+    });
+}
+
+cudaError_t launch_update_prims(const mfg_box* boxes, int nbox, cudaStream_t st) {
     const int ns = c_host_params().nspec;
-    ProfScope ps(K_PRIMS, st);
-    if (ns <= 1) prims_kernel<1><<<nblocks(v.n), TPB, 0, st>>>(v, S);
-    else if (ns <= 2) prims_kernel<2><<<nblocks(v.n), TPB, 0, st>>>(v, S);
-    else if (ns <= 4) prims_kernel<4><<<nblocks(v.n), TPB, 0, st>>>(v, S);
-    else if (ns <= 8) prims_kernel<8><<<nblocks(v.n), TPB, 0, st>>>(v, S);
-    else prims_kernel<16><<<nblocks(v.n), TPB, 0, st>>>(v, S);
-    return cudaGetLastError();
+    return for_local_groups(boxes, nbox, [&](const LocalGroup& g, dim3 grid) {
+        ProfScope ps(K_PRIMS, st);
+        if (ns <= 1) prims_kernel<1><<<grid, TPB, 0, st>>>(g);
+        else if (ns <= 2) prims_kernel<2><<<grid, TPB, 0, st>>>(g);
+        else if (ns <= 4) prims_kernel<4><<<grid, TPB, 0, st>>>(g);
+        else if (ns <= 8) prims_kernel<8><<<grid, TPB, 0, st>>>(g);
+        else prims_kernel<16><<<grid, TPB, 0, st>>>(g);
+    });
 }
 
 // Split-chemistry pieces (Source/mflo_splitchem.cpp): kind 0 Advance_chemistry,
@@ -276,11 +301,11 @@ cudaError_t launch_split_chem(const mfg_box& b, int kind, double dt, int bg, cud
     return cudaGetLastError();
 }
 
-cudaError_t launch_clip_species(const mfg_box& b, cudaStream_t st) {
-    Valid v = valid_of(b);
-    ProfScope ps(K_CLIP, st);
-    clip_kernel<<<nblocks(v.n), TPB, 0, st>>>(v, make_fab(b.s_new), c_host_params().nspec);
-    return cudaGetLastError();
+cudaError_t launch_clip_species(const mfg_box* boxes, int nbox, cudaStream_t st) {
+    return for_local_groups(boxes, nbox, [&](const LocalGroup& g, dim3 grid) {
+        ProfScope ps(K_CLIP, st);
+        clip_kernel<<<grid, TPB, 0, st>>>(g, c_host_params().nspec);
+    });
 }
 
 // partial: scratch of (ncomp * 1024) doubles; acc: ncomp doubles (device).
