@@ -382,55 +382,78 @@ __global__ void __launch_bounds__(AT, 4) adj_flux_kernel(AdjBox A, int d) {
     }
 }
 
-// Adjoint of one stencil cell's Euler flux of component c and of its state
-// value (consprim_funcs.H:48-81 reversed), given the summed adjoints fb of the
-// flux and ub of the state value from the WENO5 edges.
-__device__ __forceinline__ void euler_vjp_scatter(const AdjBox& A, int c, int d, int sc, int64_t os, int64_t ox,
-                                                  double u, double fb, double ub) {
-    const RhsBox& B = A.B;
-    const Fab& S = B.sb;
-    const Fab& X = B.aux;
-    const Fab& G = A.lamSb;
-    const Fab& GA = A.lamAux;
-    const double vd = X.p[ox + (AUX_VX + d) * X.ns];
-    double rb = 0.0, vab = 0.0, vdb = 0.0, pb = 0.0, Eb = 0.0;
-    if (c == RHO) {
-        rb = fb * vd;
-        vdb = fb * u;
-    } else if (c <= RHOW) {
-        const double rho = S.p[os + RHO * S.ns], va = X.p[ox + (AUX_VX + c - 1) * X.ns];
-        rb = fb * va * vd;
-        vab = fb * rho * vd;
-        vdb = fb * rho * va;
-        if (c - 1 == d) pb = fb;
-    } else if (c == RHOE) {
-        Eb = fb * vd;
-        pb = fb * vd;
-        vdb = fb * (u + X.p[ox + AUX_PF * X.ns]);
-    } else {
-        ub += fb * vd;
-        vdb = fb * u;
-    }
-    if (c == RHO) ub += rb;
-    if (c == RHOE) ub += Eb;
-    aadd(&G.p[os + sc * G.ns], ub);
-    if (c != RHO) aadd(&G.p[os + RHO * G.ns], rb);
-    if (c != RHOE) aadd(&G.p[os + RHOE * G.ns], Eb);
-    aadd(&GA.p[ox + (AUX_VX + d) * GA.ns], vdb);
-    if (c >= 1 && c <= 3) aadd(&GA.p[ox + (AUX_VX + c - 1) * GA.ns], vab);
-    aadd(&GA.p[ox + AUX_PF * GA.ns], pb);
+// The face's sum of the eigenvalue's adjoint (FS_MH) at offset q.
+__device__ __forceinline__ double& FS_at(const AdjBox& A, int d, int64_t q) {
+    const Fab& F = A.B.fs[d];
+    return F.p[q + FS_MH * F.ns];
 }
 
-// Column-sweep form of adj_flux_kernel: one thread per (segment of seg faces
-// along d in one column, advected component c).  A window of the six stencil
-// cells slides with the face; each cell's state value and Euler flux are
-// evaluated once, the edge adjoints of the faces that use the cell are summed
-// in registers, and the Euler-flux reversal and its atomic scatter run once
-// per cell as it leaves the window (cells at the segment ends also receive
-// the neighbouring segments' sums, so the scatter stays atomic).  Same
-// mathematics as the per-face form; the order of the summation differs.
-template <int NS>
-__device__ __forceinline__ void adj_flux_sweep_body(const AdjBox& A, int d, int seg, int c, int64_t t) {
+// Column-sweep form of adj_flux_kernel in the second differences of the forward
+// sweep (mfg_rhs_body.cuh): one thread per (segment of seg faces along d in one
+// column, advected component c, quantity h: 0 the Euler flux, 1 the state).
+// The two quantities' reversals are independent given the face's adjoint hb
+// and the eigenvalue, so they are threads of their own: half the registers and
+// twice the threads.
+//
+// The correction of a left edge in cell m is P = t_m + W2 gm + W0 gp with gm =
+// t_m - t_{m-1}, gp = t_{m+1} - t_m, W2 twice the far and W0 the near weight;
+// the right edge's has gm, gp exchanged and negated.  The weights' derivative is
+//   dP = sum_k w_k (T_k - P) (-2 ds_k / s_k),
+// T_k the candidates' corrections and s_k the indicators (any common scale),
+// whose reciprocals come with the fixed-point weights; a cell's two edges share
+// the three indicators.  A cell's sums go to its centres (adjoints of s and t),
+// a finished centre's to the two differences beside it (with s' = 3 (eps +
+// beta): s'_C = 3 eps + 4 D-^2 - 5 D- D+ + 4 D+^2, s'_A = s'_C + 6 D- (D- - D+),
+// s'_B = s'_C + 6 D+ (D+ - D-)), those to the cells, and the Euler-flux reversal
+// and its atomic scatter run once per cell as it leaves the window.
+// FP64 issue bounds it: about 60 operations per face, component and quantity,
+// against about 250 in the edge-by-edge form: 85 -> 20 ms of a ten-step gradient
+// on a 32^3 level with ten species.
+struct AdjCtr {
+    WenoIndR w;
+    double sAb, sBb, sCb, tb;
+    bool ready;
+};
+
+// Adjoint of the first-order fallback flux (fsum - lam D W)/2, W = (X + 2Y -
+// Z)/(X + 6Y + 3Z) as in weno_llf_collapsed: W and d(D W)/dD.
+__device__ __forceinline__ void collapsed_weight(double D, double& W, double& dDW) {
+    const double y = D * D, sC = fma(16.0 / 3.0, y, 4.0 * kEpsWeno), sA = fma(8.0, y, sC);
+    const double dB = (4.0 * kEpsWeno) * (4.0 * kEpsWeno), dC = sC * sC, dA = sA * sA;
+    const double cb = (2.0 * 16.0 / 3.0) * sC, ab = (2.0 * 40.0 / 3.0) * sA;  // d/dy of C and A
+    const double X = dC * dA, Y = dB * dA, Z = dB * dC, Xb = cb * dA + dC * ab, Yb = dB * ab, Zb = dB * cb;
+    const double r = 1.0 / (X + 6.0 * Y + 3.0 * Z);
+    W = (X + 2.0 * Y - Z) * r;
+    dDW = W + (2.0 * y) * (((Xb + 2.0 * Yb - Zb) - W * (Xb + 6.0 * Yb + 3.0 * Zb)) * r);
+}
+
+// Adjoint of one cell's value: fb of its Euler flux (h = 0) or of its state.
+__device__ __forceinline__ void flux5_cell_vjp(const Fp& fp, const AdjBox& A, const Flux5Ctx& x, int d, int sc, int h,
+                                               int64_t os, int64_t ox, double fb) {
+    if (fb == 0.0) return;
+    const Fab& G = A.lamSb;
+    if (h) {
+        aadd(&G.p[os + sc * G.ns], fb);
+        return;
+    }
+    if (x.kind == 0) {  // the density flux is the momentum
+        aadd(&G.p[os + (RHOU + d) * G.ns], fb);
+        return;
+    }
+    const Fab& GA = A.lamAux;
+    const double vd = x.v[ox], u = x.u[os], fv = fp.mul(fb, vd);
+    aadd(&G.p[os + sc * G.ns], fv);
+    if (x.kind == 1) {
+        aadd(&GA.p[ox + AUX_PF * GA.ns], fv);
+        aadd(&GA.p[ox + (AUX_VX + d) * GA.ns], fp.mul(fb, fp.add(u, x.p[ox])));
+    } else {
+        if (x.kind == 2) aadd(&GA.p[ox + AUX_PF * GA.ns], fb);
+        aadd(&GA.p[ox + (AUX_VX + d) * GA.ns], fp.mul(fb, u));
+    }
+}
+
+__device__ __forceinline__ void adj_flux_sweep_body(const Fp& fp, const AdjBox& A, int d, int seg, int c, int h,
+                                                    int64_t t) {
     const RhsBox& B = A.B;
     int ta, tb;
     sweep_dirs(d, ta, tb);
@@ -443,117 +466,181 @@ __device__ __forceinline__ void adj_flux_sweep_body(const AdjBox& A, int d, int 
     const int f0 = B.lo[d] + is * seg, f1 = B.lo[d] + min(nfd, (is + 1) * seg);  // faces [f0, f1)
     const DevParams& P = c_P;
     const int sc = (c < NCONS) ? c : c + (NFLO - NCONS);
-    const Fab& S = B.sb;
-    const Fab& X = B.aux;
+    const double adv = (c < NCONS) ? 1.0 : P.advect_flag[c - NCONS];
     const Fab& G = A.lamSb;
-    const Fab& FS = B.fs[d];
-    const int64_t sd = (d == 0) ? 1 : (d == 1) ? S.js : S.ks;
-    const int64_t xd = (d == 0) ? 1 : (d == 1) ? X.js : X.ks;
+    const Flux5Ctx x = flux5_ctx(B, d, c);
+    const int64_t sd = (d == 0) ? 1 : (d == 1) ? B.sb.js : B.sb.ks;
+    const int64_t xd = (d == 0) ? 1 : (d == 1) ? B.aux.js : B.aux.ks;
+    const int64_t fd = (d == 0) ? 1 : (d == 1) ? B.fs[d].js : B.fs[d].ks;
+    ia += B.lo[ta];
+    ib += B.lo[tb];
     Idx3 f;
-    int* fc[3] = {&f.i, &f.j, &f.k};
-    *fc[ta] = B.lo[ta] + ia;
-    *fc[tb] = B.lo[tb] + ib;
-    *fc[d] = f0;
-    // window: position q holds cell (face - 3 + q)
-    double us[6], fl[6], usb[6], flb[6];
-    const int64_t oR0 = S.off(f.i, f.j, f.k), xR0 = X.off(f.i, f.j, f.k);
-    auto load = [&](int q, int64_t os, int64_t ox) {
-        us[q] = S.p[os + sc * S.ns];
-        const double va = (c >= 1 && c <= 3) ? X.p[ox + (AUX_VX + c - 1) * X.ns] : 0.0;
-        fl[q] = euler_flux(c, d, us[q], S.p[os + RHO * S.ns], va, X.p[ox + (AUX_VX + d) * X.ns],
-                           X.p[ox + AUX_PF * X.ns], S.p[os + RHOE * S.ns]);
-        usb[q] = 0.0;
-        flb[q] = 0.0;
+    f.i = (d == 0) ? f0 : ia;
+    f.j = (d == 0) ? ia : (d == 1) ? f0 : ib;
+    f.k = (d == 2) ? f0 : ib;
+    const int64_t ld = (d == 0) ? 1 : (d == 1) ? A.lamL.js : A.lamL.ks;
+    int64_t oc = B.sb.off(f.i, f.j, f.k) - sd, xc = B.aux.off(f.i, f.j, f.k) - xd;  // cell m
+    int64_t qf = B.fs[d].off(f.i, f.j, f.k);                                        // face m + 1
+    int64_t lR = A.lamL.off(f.i, f.j, f.k) + sc * A.lamL.ns;                         // its right cell
+    auto value = [&](int q) {  // the quantity in cell m + q
+        double u, fl;
+        flux5_cell(fp, x, oc + q * sd, xc + q * xd, u, fl);
+        return h ? u : fl;
     };
+    // differences D[q] between cells m-2+q and m-1+q, their adjoints, the direct
+    // adjoints of cells m-2 .. m+2, the centres m-1, m, m+1
+    double v = value(-2), D[4], Db[4] = {0.0, 0.0, 0.0, 0.0}, vb[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, Dlast = 0.0;
 #pragma unroll
-    for (int q = 0; q < 6; ++q) load(q, oR0 + (q - 3) * sd, xR0 + (q - 3) * xd);
-    for (int fd = f0; fd < f1; ++fd) {
-        *fc[d] = fd;
-        const int64_t oR = oR0 + (fd - f0) * sd, oL = oR - sd, xR = xR0 + (fd - f0) * xd;
-        const double Fb = face_bar(B, A.lamL, f, d, sc);
-        if (Fb != 0.0) {
-            if (c == RHOE) {  // heat conduction F_E -= k (T_R - T_L)/dx, on every face
-                const double kb = P.cond_hm * B.idx[d] * Fb;
-                aadd(&G.p[oR + TEMP * G.ns], -kb);
-                aadd(&G.p[oL + TEMP * G.ns], kb);
-            }
-            if (c >= NCONS) {  // species diffusion F_s -= D (c_R - c_L)/dx, on every face
-                const int s = c - NCONS;
-                const double* vf = S.p + VFRAC * S.ns;
-                const double Dh = (P.diff_mode[s] == MFG_TRANSPORT_CONST)
-                                      ? P.diff_hm[s]
-                                      : harmonic_mean(blend(P.diff_mode[s], P.diff_gas[s], P.diff_solid[s], vf[oL]),
-                                                      blend(P.diff_mode[s], P.diff_gas[s], P.diff_solid[s], vf[oR]));
-                const double v = Dh * B.idx[d] * Fb;
-                aadd(&G.p[oR + sc * G.ns], -v);
-                aadd(&G.p[oL + sc * G.ns], v);
-            }
-            const int64_t qf = FS.off(f.i, f.j, f.k);
-            const int flags = (int)__double_as_longlong(FS.p[qf + FS_FLAGS * FS.ns]);
-            const double hb = (c < NCONS) ? Fb : P.advect_flag[c - NCONS] * Fb;
-            if ((flags & 1) && hb != 0.0) {
-                const bool fallback = flags & 2;
-                const double lam = FS.p[qf + FS_LAMBDA * FS.ns];
-                // the same four edge reversals for every lane (with the first-order
-                // fallback the six stencil entries are the two face cells), then the
-                // stencil adjoints are added to the window, collapsed for the fallback
-                double sf[6], su[6];
-#pragma unroll
-                for (int q = 0; q < 6; ++q) {
-                    const int w = fallback ? ((q < 3) ? 2 : 3) : q;
-                    sf[q] = fl[w];
-                    su[q] = us[w];
+    for (int q = 0; q < 4; ++q) {
+        const double w = value(q - 1);
+        D[q] = fp.sub(w, v);
+        v = w;
+    }
+    AdjCtr c0, c1, c2;
+    c0.ready = c1.ready = c2.ready = false;
+    c0.sAb = c0.sBb = c0.sCb = c0.tb = c1.sAb = c1.sBb = c1.sCb = c1.tb = 0.0;
+    double pRb = 0.0, lamP = 0.0;  // adjoint of the right edge of face m; P of the left edge of face m (for lambda)
+    double lamH = 0.0;             // -hb/12 of face m where the eigenvalue's adjoint is due
+    int64_t lamQ = 0;
+    auto centre = [&](AdjCtr& k, int q) {  // centre m-1+q
+        if (k.ready) return;
+        k.w = weno_ind_full<true>(weno_diff((uint64_t)__double_as_longlong(D[q])),
+                                  weno_diff((uint64_t)__double_as_longlong(D[q + 1])));
+        k.ready = true;
+    };
+    // a finished centre's adjoints to its differences D[q], D[q+1]
+    auto reverse_centre = [&](const AdjCtr& k, int q) {
+        const long long any = __double_as_longlong(k.sAb) | __double_as_longlong(k.sBb) | __double_as_longlong(k.sCb) |
+                              __double_as_longlong(k.tb);
+        if ((any << 1) == 0) return;
+        const double ab = fp.add(k.sAb, k.sBb), c8 = __dmul_rn(8.0, fp.add(ab, k.sCb));
+        const double xx = __fma_rn(11.0, ab, __dmul_rn(5.0, k.sCb));
+        Db[q] = __fma_rn(D[q], __fma_rn(12.0, k.sAb, c8), __fma_rn(-D[q + 1], xx, fp.sub(Db[q], k.tb)));
+        Db[q + 1] = __fma_rn(D[q + 1], __fma_rn(12.0, k.sBb, c8), __fma_rn(-D[q], xx, fp.add(Db[q + 1], k.tb)));
+    };
+    auto emit = [&](int q, double left) {  // cell m-2+q, whose left difference's adjoint is `left`
+        const double b = fp.sub(fp.add(vb[q], left), (q < 4) ? Db[q] : 0.0);
+        flux5_cell_vjp(fp, A, x, d, sc, h, oc + (q - 2) * sd, xc + (q - 2) * xd, b);
+    };
+    for (int m = f0 - 1;; ++m) {
+        // face m + 1 of the segment: the adjoint of its left edge (cell m), of its
+        // right edge (cell m + 1), and of its two cells
+        double pLb = 0.0, pRn = 0.0, hb12 = 0.0;
+        if (m + 1 < f1) {
+            double Fb = 0.0;
+            if (m + 1 <= B.hi[d]) Fb = A.lamL.p[lR];
+            if (m >= B.lo[d]) Fb = fp.sub(Fb, A.lamL.p[lR - ld]);
+            Fb = fp.mul(Fb, B.idx[d]);
+            if (Fb != 0.0) {
+                const int64_t oL = oc, oR = oc + sd;
+                if (h && c == RHOE) {  // heat conduction F_E -= k (T_R - T_L)/dx, on every face
+                    const double kb = fp.mul(P.cond_hm * B.idx[d], Fb);
+                    aadd(&G.p[oR + TEMP * G.ns], -kb);
+                    aadd(&G.p[oL + TEMP * G.ns], kb);
                 }
-                double gf[6] = {0, 0, 0, 0, 0, 0}, gu[6] = {0, 0, 0, 0, 0, 0};
-                EdgeGrad g;
-                weno_edge_vjp(sf[0], sf[1], sf[2], sf[3], sf[4], 0.5 * hb, g);
-                gf[0] += g.a; gf[1] += g.b; gf[2] += g.c; gf[3] += g.d; gf[4] += g.e;
-                weno_edge_vjp(sf[5], sf[4], sf[3], sf[2], sf[1], 0.5 * hb, g);
-                gf[5] += g.a; gf[4] += g.b; gf[3] += g.c; gf[2] += g.d; gf[1] += g.e;
-                const double up = weno_edge_vjp(su[0], su[1], su[2], su[3], su[4], 0.5 * lam * hb, g);
-                gu[0] += g.a; gu[1] += g.b; gu[2] += g.c; gu[3] += g.d; gu[4] += g.e;
-                const double um = weno_edge_vjp(su[5], su[4], su[3], su[2], su[1], -0.5 * lam * hb, g);
-                gu[5] += g.a; gu[4] += g.b; gu[3] += g.c; gu[2] += g.d; gu[1] += g.e;
-                if (fallback) {
-                    flb[2] += (gf[0] + gf[1]) + gf[2];
-                    flb[3] += (gf[3] + gf[4]) + gf[5];
-                    usb[2] += (gu[0] + gu[1]) + gu[2];
-                    usb[3] += (gu[3] + gu[4]) + gu[5];
-                } else {
-#pragma unroll
-                    for (int q = 0; q < 6; ++q) {
-                        flb[q] += gf[q];
-                        usb[q] += gu[q];
+                if (h && c >= NCONS) {  // species diffusion F_s -= D (c_R - c_L)/dx, on every face
+                    const int s = c - NCONS;
+                    const double Dh = (P.diff_mode[s] == MFG_TRANSPORT_CONST)
+                                          ? P.diff_hm[s]
+                                          : harmonic_mean(blend(P.diff_mode[s], P.diff_gas[s], P.diff_solid[s], x.vf[oL]),
+                                                          blend(P.diff_mode[s], P.diff_gas[s], P.diff_solid[s], x.vf[oR]));
+                    const double w = fp.mul(Dh * B.idx[d], Fb);
+                    vb[2] = fp.add(vb[2], w);
+                    vb[3] = fp.sub(vb[3], w);
+                }
+                const int flags = (int)__double_as_longlong(x.fs[qf + FS_FLAGS * x.fns]) & 3;
+                const double hb = fp.mul(adv, Fb);
+                if ((flags & 1) && hb != 0.0) {
+                    const double lam = h ? x.fs[qf + FS_LAMBDA * x.fns] : 1.0;
+                    if (!h) {  // half the sum of the two cells' fluxes
+                        const double hh = __dmul_rn(0.5, hb);
+                        vb[2] = fp.add(vb[2], hh);
+                        vb[3] = fp.add(vb[3], hh);
+                    }
+                    if (!(flags & 2)) {
+                        hb12 = __dmul_rn(-1.0 / 12.0, hb);
+                        pLb = fp.mul(hb12, lam);
+                        pRn = h ? -pLb : pLb;
+                    } else if (h) {
+                        double W, dDW;
+                        collapsed_weight(D[2], W, dDW);
+                        const double w = __dmul_rn(-0.5, fp.mul(fp.mul(lam, hb), dDW));
+                        Db[2] = fp.add(Db[2], w);
+                        aadd(&FS_at(A, d, qf), __dmul_rn(-0.5, fp.mul(hb, fp.mul(D[2], W))));
                     }
                 }
-                aadd(&FS.p[qf + FS_MH * FS.ns], 0.5 * hb * (up - um));
             }
         }
-        if (fd + 1 < f1) {  // cell fd - 3 leaves the window; cell fd + 3 enters
-            if (usb[0] != 0.0 || flb[0] != 0.0)
-                euler_vjp_scatter(A, c, d, sc, oR - 3 * sd, xR - 3 * xd, us[0], flb[0], usb[0]);
+        c2.sAb = c2.sBb = c2.sCb = c2.tb = 0.0;
+        double pLval = 0.0;
+        if (pLb != 0.0 || pRb != 0.0 || hb12 != 0.0 || lamH != 0.0) {
+            centre(c0, 0);
+            centre(c1, 1);
+            centre(c2, 2);
+            const WenoWeights w = weno_weights(c0.w.dB, c0.w.eB, c1.w.dC, c1.w.eC, c2.w.dA, c2.w.eA);
+            const double W2L = weight_of(w.farL2), W0L = weight_of(w.nearL), W2R = weight_of(w.farR2),
+                         W0R = weight_of(w.nearR);
+            const double tm = fp.sub(D[1], D[0]), t0 = fp.sub(D[2], D[1]), tp = fp.sub(D[3], D[2]);
+            const double gm = fp.sub(t0, tm), gp = fp.sub(tp, t0);
+            const double eL = __fma_rn(W2L, gm, fp.mul(W0L, gp)), eR = __fma_rn(W2R, gp, fp.mul(W0R, gm));
+            const double a2 = fp.mul(W2L, pLb), a0 = fp.mul(W0L, pLb), b2 = fp.mul(W2R, pRb), b0 = fp.mul(W0R, pRb);
+            // twice w_k (T_k - P) times the edges' adjoints, by indicator
+            const double HB = __fma_rn(a2, __fma_rn(2.0, gm, -eL), __dmul_rn(2.0, fp.mul(b0, fp.sub(eR, gm))));
+            const double HA = __fma_rn(b2, __fma_rn(-2.0, gp, eR), __dmul_rn(2.0, fp.mul(a0, fp.sub(gp, eL))));
+            c0.sBb = __fma_rn(-HB, weight_of(c0.w.rB), c0.sBb);
+            c2.sAb = __fma_rn(-HA, weight_of(c2.w.rA), c2.sAb);
+            c1.sCb = __fma_rn(fp.add(HA, HB), weight_of(c1.w.rC), c1.sCb);
+            const double gmb = fp.sub(a2, b0), gpb = fp.sub(a0, b2);
+            c0.tb = fp.sub(c0.tb, gmb);
+            c2.tb = fp.add(c2.tb, gpb);
+            c1.tb = fp.add(c1.tb, fp.add(fp.add(pLb, pRb), fp.sub(gmb, gpb)));
+            // the eigenvalue's adjoint of face m: (up - um) hb / 2 = -(hb/12) (P_left - P_right)
+            if (h && lamH != 0.0) aadd(&FS_at(A, d, lamQ), fp.mul(lamH, fp.sub(lamP, fp.sub(t0, eR))));
+            pLval = fp.add(t0, eL);
+        }
+        reverse_centre(c0, 0);
+        emit(0, Dlast);
+        if (m + 1 >= f1) break;
+        lamP = pLval;
+        lamH = hb12;
+        lamQ = qf;
+        pRb = pRn;
+        // to cell m + 1
+        Dlast = Db[0];
+        c0 = c1;
+        c1 = c2;
+        c2.ready = false;
 #pragma unroll
-            for (int q = 0; q < 5; ++q) {
-                us[q] = us[q + 1];
-                fl[q] = fl[q + 1];
-                usb[q] = usb[q + 1];
-                flb[q] = flb[q + 1];
-            }
-            load(5, oR + 3 * sd, xR + 3 * xd);
+        for (int q = 0; q < 3; ++q) {
+            D[q] = D[q + 1];
+            Db[q] = Db[q + 1];
         }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) vb[q] = vb[q + 1];
+        vb[4] = 0.0;
+        Db[3] = 0.0;
+        oc += sd;
+        xc += xd;
+        qf += fd;
+        lR += ld;
+        const double w = value(2);
+        D[3] = fp.sub(w, v);
+        v = w;
     }
-    const int64_t oR = oR0 + (f1 - 1 - f0) * sd, xR = xR0 + (f1 - 1 - f0) * xd;
+    // the centres and cells left in the window
+    reverse_centre(c1, 1);
+    reverse_centre(c2, 2);
 #pragma unroll
-    for (int q = 0; q < 6; ++q)
-        if (usb[q] != 0.0 || flb[q] != 0.0)
-            euler_vjp_scatter(A, c, d, sc, oR + (q - 3) * sd, xR + (q - 3) * xd, us[q], flb[q], usb[q]);
+    for (int q = 1; q < 5; ++q) emit(q, Db[q - 1]);
 }
 
-// Every box of a stage in one launch (blockIdx.z = box): the boxes' adjoint
-// accumulations are disjoint, and one box alone leaves too few columns.
-template <int NS>
-__global__ void __launch_bounds__(AT, 3) adj_flux_sweep_kernel(const AdjBox* __restrict__ boxes, int d, int seg) {
-    adj_flux_sweep_body<NS>(boxes[blockIdx.z], d, seg, blockIdx.y, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
+// Every box, direction, component and quantity of a stage in one launch
+// (blockIdx.z = box): the boxes' adjoint accumulations are disjoint, and one
+// box alone leaves too few columns.
+__global__ void __launch_bounds__(AT, 3) adj_flux_sweep_kernel(const AdjBox* __restrict__ boxes, int seg, int C) {
+    const Fp fp;
+    const int h = blockIdx.y & 1, y = blockIdx.y >> 1;
+    adj_flux_sweep_body(fp, boxes[blockIdx.z], y / C, seg, y % C, h, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // One thread per face (blockIdx.y = direction, blockIdx.z = box): viscous stress (F_{m_a} -= tau_a,
@@ -1599,17 +1686,18 @@ int adj_step(Work& W, double dt, const Snap& sn, double* lam, double* lamOld, do
         }
         ADJ_TRY(cudaMemcpyAsync(W.d_adj, adj.data(), W.nbox * sizeof(AdjBox), cudaMemcpyHostToDevice, st),
                 "reverse: box views");
-        for (int d = 0; d < 3; ++d) {
+        if (sweep) {
+            unsigned nbs = 1;
+            for (int b = 0; b < W.nbox; ++b)
+                for (int d = 0; d < 3; ++d) nbs = std::max(nbs, nblk(sweep_items(adj[b].B, d, kAdjSeg), AT));
             ProfScope ps(K_ADJ_FLUX, st);
-            if (sweep) {
-                unsigned nbs = 1;
-                for (int b = 0; b < W.nbox; ++b) nbs = std::max(nbs, nblk(sweep_items(adj[b].B, d, kAdjSeg), AT));
-                ADJ_NS(adj_flux_sweep_kernel, (dim3(nbs, C, W.nbox), AT, 0, st), (W.d_adj, d, kAdjSeg));
-            } else {
-                for (int b = 0; b < W.nbox; ++b)
-                    ADJ_NS(adj_flux_kernel, (dim3(nblk(face_items(adj[b].B, d), AT), C), AT, 0, st), (adj[b], d));
-            }
+            adj_flux_sweep_kernel<<<dim3(nbs, 6 * C, W.nbox), AT, 0, st>>>(W.d_adj, kAdjSeg, C);
         }
+        for (int d = 0; d < 3 && !sweep; ++d)
+            for (int b = 0; b < W.nbox; ++b) {
+                ProfScope ps(K_ADJ_FLUX, st);
+                ADJ_NS(adj_flux_kernel, (dim3(nblk(face_items(adj[b].B, d), AT), C), AT, 0, st), (adj[b], d));
+            }
         {
             ProfScope ps(K_ADJ_FACE, st);
             ADJ_NS(adj_face_kernel, (dim3(nbf, 3, W.nbox), AT, 0, st), (W.d_adj));

@@ -52,7 +52,19 @@ constexpr uint64_t kWenoEps3 = 906694364710971881ull;  // 3e-6 * 2^78
 // one-sided ones, that plus 6 D- (D- - D+) and 6 D+ (D+ - D-).  All three are
 // at least 0.73 max(D-^2, D+^2), so the fixed point relative to the larger
 // difference keeps them to 2^-50 at worst.
-MFG_HD WenoInd weno_ind(const WenoDiff& a, const WenoDiff& b) {
+// RCP: also the reciprocals of the three 3 (eps + beta) as double bits (0 where
+// they leave the exponent range), for the adjoint.
+struct WenoIndR : WenoInd {
+    uint64_t rA, rB, rC;
+};
+
+MFG_HD uint64_t ind_rcp_bits(uint64_t n, int z, int E) {
+    const int e = 3061 - 2 * E + z;  // 3 (eps + beta) = n 2^(2E - 2102 - z), top bit of n set
+    return e < 2 ? 0 : ((uint64_t)(uint32_t)(e - 1) << 52) + ((rcp_fixed(n) + 512) >> 10);
+}
+
+template <bool RCP>
+MFG_HD WenoIndR weno_ind_full(const WenoDiff& a, const WenoDiff& b) {
     const int E = imax(imax(a.e, b.e), kWenoExpFloor);
     const uint64_t ma = a.m >> imin(E - a.e, 63), mb = b.m >> imin(E - b.e, 63);
     const uint64_t E1 = umulhi64(ma, ma), E2 = umulhi64(mb, mb);
@@ -63,15 +75,21 @@ MFG_HD WenoInd weno_ind(const WenoDiff& a, const WenoDiff& b) {
     // each is at least 2^55: the high words are not zero
     const int zA = clz32((uint32_t)(sA >> 32)), zB = clz32((uint32_t)(sB >> 32)), zC = clz32((uint32_t)(sC >> 32));
     const uint64_t nA = sA << zA, nB = sB << zB, nC = sC << zC;
-    WenoInd r;
+    WenoIndR r;
     r.dA = umulhi64(nA, nA);
     r.dB = umulhi64(nB, nB);
     r.dC = umulhi64(nC, nC);
     r.eA = 2 * E - zA;
     r.eB = 2 * E - zB;
     r.eC = 2 * E - zC;
+    if (RCP) {
+        r.rA = ind_rcp_bits(nA, zA, E);
+        r.rB = ind_rcp_bits(nB, zB, E);
+        r.rC = ind_rcp_bits(nC, zC, E);
+    }
     return r;
 }
+MFG_HD WenoInd weno_ind(const WenoDiff& a, const WenoDiff& b) { return weno_ind_full<false>(a, b); }
 
 // w 2^-62 2^k as the bits of a double, truncated (0 reads as 2^(k-62)).
 MFG_HD uint64_t weight_bits(uint64_t w, int k) {
