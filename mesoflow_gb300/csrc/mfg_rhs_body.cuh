@@ -955,10 +955,14 @@ __device__ __forceinline__ void flux5_sweep_body(const Fp& fp, const RhsBox& B, 
             flux5_finish(fp, x, false, 0.0, fp.sub(x.u[oR], x.u[oR - sd]), oR - sd, oR, qf, qf, qr);
         return;
     }
-    // Cells f-1 .. f+1 to start with; the WENO parts are built only when a
-    // face needs them: faces on the solid side of the immersed boundary (no
-    // hyperbolic flux) and first-order fallback faces use the cell values
-    // alone, and the run starts again (three centres) at the next regular face.
+    // Cells f-1 .. f+1 to start with; the WENO parts are built only where a
+    // face of the warp needs them: faces on the solid side of the immersed
+    // boundary (no hyperbolic flux) and first-order fallback faces use the cell
+    // values alone.  A lane at such a face beside a regular one advances its run
+    // with the others, in slots that divergence would leave idle, rather than
+    // start it again (three centres) at its own next regular face (the run is a
+    // function of the cells alone, so the numbers do not depend on it): fluxes of
+    // the 64^3 catalyst step 4.45 -> 4.09 ms.
     WenoRun u, f;
     double uL, fL;
     flux5_cell(fp, x, oR - sd, xR - xd, uL, fL);
@@ -974,7 +978,7 @@ __device__ __forceinline__ void flux5_sweep_body(const Fp& fp, const RhsBox& B, 
         const int flags = (int)__double_as_longlong(x.fs[qf + FS_FLAGS * x.fns]) & 3;
         const double Dun = fp.sub(un, u.v1), Dfn = fp.sub(fn, f.v1);
         double fh = 0.0;
-        if (flags == 1) {
+        if (__any_sync(__activemask(), flags == 1)) {
             if (!primed) {
                 double ua, fa, ub, fb;
                 flux5_cell(fp, x, oR - 3 * sd, xR - 3 * xd, ua, fa);
@@ -985,11 +989,12 @@ __device__ __forceinline__ void flux5_sweep_body(const Fp& fp, const RhsBox& B, 
             }
             const double pLu = u.pL, pLf = f.pL;
             const double pRf = weno_next(fp, f, f.D, Dfn), pRu = weno_next(fp, u, u.D, Dun);
-            fh = weno_llf(fp, x.fs[qf + FS_LAMBDA * x.fns], fp.add(fL, f.v0), pLf, pRf, pLu, pRu);
+            if (flags == 1)
+                fh = weno_llf(fp, x.fs[qf + FS_LAMBDA * x.fns], fp.add(fL, f.v0), pLf, pRf, pLu, pRu);
         } else {
             primed = false;
-            if (flags & 1) fh = weno_llf_collapsed(x.fs[qf + FS_LAMBDA * x.fns], fp.add(fL, f.v0), Du);
         }
+        if (flags == 3) fh = weno_llf_collapsed(x.fs[qf + FS_LAMBDA * x.fns], fp.add(fL, f.v0), Du);
         flux5_finish(fp, x, flags & 1, fh, Du, oR - sd, oR, qf, qf, qr);
         if (fc == f1) break;
         // advance one face
