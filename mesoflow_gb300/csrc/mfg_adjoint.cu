@@ -297,10 +297,7 @@ __global__ void __launch_bounds__(AT, 4) adj_flux_kernel(AdjBox A, int d) {
     if (c >= NCONS) {  // species diffusion F_s -= D (c_R - c_L)/dx, on every face
         const int s = c - NCONS;
         const double* vf = S.p + VFRAC * S.ns;
-        const double Dh = (P.diff_mode[s] == MFG_TRANSPORT_CONST)
-                              ? P.diff_hm[s]
-                              : harmonic_mean(blend(P.diff_mode[s], P.diff_gas[s], P.diff_solid[s], vf[oL]),
-                                              blend(P.diff_mode[s], P.diff_gas[s], P.diff_solid[s], vf[oR]));
+        const double Dh = face_diffusivity(P, s, vf[oL], vf[oR]);
         const double v = Dh * B.idx[d] * Fb;
         aadd(&G.p[oR + sc * G.ns], -v);
         aadd(&G.p[oL + sc * G.ns], v);
@@ -540,10 +537,7 @@ __device__ __forceinline__ void adj_flux_sweep_body(const Fp& fp, const AdjBox& 
                 }
                 if (h && c >= NCONS) {  // species diffusion F_s -= D (c_R - c_L)/dx, on every face
                     const int s = c - NCONS;
-                    const double Dh = (P.diff_mode[s] == MFG_TRANSPORT_CONST)
-                                          ? P.diff_hm[s]
-                                          : harmonic_mean(blend(P.diff_mode[s], P.diff_gas[s], P.diff_solid[s], x.vf[oL]),
-                                                          blend(P.diff_mode[s], P.diff_gas[s], P.diff_solid[s], x.vf[oR]));
+                    const double Dh = face_diffusivity(P, s, x.vf[oL], x.vf[oR]);
                     const double w = fp.mul(Dh * B.idx[d], Fb);
                     vb[2] = fp.add(vb[2], w);
                     vb[3] = fp.sub(vb[3], w);

@@ -297,7 +297,10 @@ int mfg_init(const mfg_params* p) {
     auto hmean = [](double d1, double d2) { return 2.0 * d1 * d2 / (d1 + d2 + 1e-30); };
     h.visc_hm = hmean(p->visc_gas, p->visc_gas);
     h.cond_hm = hmean(p->cond_gas, p->cond_gas);
-    for (int s = 0; s < MFG_MAX_SPECIES; ++s) h.diff_hm[s] = hmean(p->diff_gas[s], p->diff_gas[s]);
+    for (int s = 0; s < MFG_MAX_SPECIES; ++s) {
+        h.diff_hm[s] = hmean(p->diff_gas[s], p->diff_gas[s]);
+        h.diff_hms[s] = hmean(p->diff_solid[s], p->diff_solid[s]);
+    }
     if (p->thermo_kind == MFG_THERMO_MASS_SINGLE) {
         h.g_gm1 = p->gamma_single / (p->gamma_single - 1.0);
         h.astar_fac = (2.0 * (p->gamma_single - 1.0)) / (p->gamma_single + 1.0);

@@ -40,7 +40,7 @@ struct DevParams {
     int diff_mode[MAXS];
     double diff_gas[MAXS], diff_solid[MAXS];
     // face coefficients of constant transport: harmonic_mean(g, g), evaluated once
-    double visc_hm, cond_hm, diff_hm[MAXS];
+    double visc_hm, cond_hm, diff_hm[MAXS], diff_hms[MAXS];  // diff_hms: between solid cells (blended transport)
     // gamma/(gamma-1) and 2(gamma-1)/(gamma+1) of the mass-single family
     double g_gm1, astar_fac, gm1_single, inv_gas_R;
     int order_hyp, do_ns, species_in_solid, conj_ht;

@@ -194,4 +194,18 @@ __device__ __forceinline__ double harmonic_mean(double d1, double d2) {
     return 2.0 * d1 * d2 / (d1 + d2 + 1e-30);
 }
 
+// Diffusivity of species s at the face between cells of volume fractions vL and
+// vR: the harmonic mean of the two cells' coefficients (compute_flux_3d.H:
+// 425-428).  Between two gas or two solid cells it is a constant from mfg_init
+// (the blend gas vf + solid (1 - vf) is the gas or the solid value exactly); the
+// blend and its division, 18 FP64 slots per species and face, remain for faces
+// of cut cells.
+__device__ __forceinline__ double face_diffusivity(const DevParams& P, int s, double vL, double vR) {
+    if (P.diff_mode[s] == MFG_TRANSPORT_CONST || (is_one(vL) && is_one(vR))) return P.diff_hm[s];
+    if (is_zero_bits(vL) && is_zero_bits(vR)) return P.diff_hms[s];
+    const double g = P.diff_gas[s], so = P.diff_solid[s];
+    const double dl = __fma_rn(g, vL, mul(so, sub(1.0, vL))), dr = __fma_rn(g, vR, mul(so, sub(1.0, vR)));
+    return quot_pos(mul(mul(2.0, dl), dr), add(add(dl, dr), 1e-30));
+}
+
 }  // namespace mfg

@@ -442,10 +442,7 @@ __device__ __forceinline__ void face_body_at(const Fp& fp, const RhsBox& B, int 
             if (c == RHOE) F = fp.sub(F, therm);
             if (c >= NCONS) {
                 const int s = c - NCONS;
-                const double Dh = (P.diff_mode[s] == MFG_TRANSPORT_CONST)
-                                      ? P.diff_hm[s]
-                                      : harmonic_mean(blend(P.diff_mode[s], P.diff_gas[s], P.diff_solid[s], vf[oL]),
-                                                      blend(P.diff_mode[s], P.diff_gas[s], P.diff_solid[s], vf[oR]));
+                const double Dh = face_diffusivity(P, s, vf[oL], vf[oR]);
                 F = __fma_rn(-fp.mul(Dh, fp.sub(S.p[oR + sc * S.ns], S.p[oL + sc * S.ns])), B.idx[d], F);
             }
             O.p[qo + c * O.ns] = F;
@@ -559,10 +556,7 @@ __device__ __forceinline__ void flux_body(const RhsBox& B, int d, int c, int64_t
         // species diffusion (compute_flux_3d.H:425-428)
         const int s = c - NCONS;
         const double* vfp = S.p + VFRAC * S.ns;
-        const double Dh = (P.diff_mode[s] == MFG_TRANSPORT_CONST)
-                              ? P.diff_hm[s]
-                              : harmonic_mean(blend(P.diff_mode[s], P.diff_gas[s], P.diff_solid[s], vfp[oL]),
-                                              blend(P.diff_mode[s], P.diff_gas[s], P.diff_solid[s], vfp[oR]));
+        const double Dh = face_diffusivity(P, s, vfp[oL], vfp[oR]);
         F -= (Dh * (u[oR] - u[oL])) * B.idx[d];
     }
     const Fab& O = B.flx[d];
@@ -807,14 +801,8 @@ __device__ __forceinline__ void flux5_finish(const Fp& fp, const Flux5Ctx& x, bo
     if (c == RHOE) F = fp.sub(F, x.fs[qf + FS_THERM * x.fns]);
     if (c >= NCONS) {  // species diffusion (compute_flux_3d.H:425-428)
         const int s = c - NCONS;
-        double Dh = P.diff_hm[s];
-        if (P.diff_mode[s] != MFG_TRANSPORT_CONST) {  // harmonic mean of gas vf + solid (1 - vf)
-            const double g = P.diff_gas[s], so = P.diff_solid[s];
-            const double vfL = x.vf[oL], vfR = x.vf[oR];
-            const double dl = __fma_rn(g, vfL, __dmul_rn(so, __dsub_rn(1.0, vfL)));
-            const double dr = __fma_rn(g, vfR, __dmul_rn(so, __dsub_rn(1.0, vfR)));
-            Dh = __ddiv_rn(__dmul_rn(__dmul_rn(2.0, dl), dr), __dadd_rn(__dadd_rn(dl, dr), 1e-30));
-        }
+        const double Dh = (P.diff_mode[s] == MFG_TRANSPORT_CONST) ? P.diff_hm[s]
+                                                                  : face_diffusivity(P, s, x.vf[oL], x.vf[oR]);
         F = __fma_rn(-fp.mul(Dh, D), x.idx, F);
     }
     x.out[qo] = F;
