@@ -325,10 +325,15 @@ int mfg_init(const mfg_params* p) {
     for (int r = 0; r < MFG_MAX_REACTIONS; ++r) {
         h.A[r] = p->A[r];
         h.Ea[r] = p->Ea[r];
+        if (p->Ea[r] != 0.0) h.arrhenius |= 1u << r;
+        if (std::isfinite(p->A[r]) && std::isfinite(p->Ea[r]) && p->Ea[r] >= 0.0) h.tame |= 1u << r;
         for (int s = 0; s < MFG_MAX_SPECIES; ++s) {
             h.nu[r][s] = p->nu[r][s];
             h.order[r][s] = p->order[r][s];
             if (s < p->nspec && p->order[r][s] > 0.0) h.ord_mask[r] |= 1u << s;
+            if (s < p->nspec && !std::isfinite(p->nu[r][s])) h.tame &= ~(1u << r);
+            if (s < p->nspec && p->order[r][s] == 1.0) h.ord1_mask[r] |= 1u << s;
+            if (s < p->nspec && p->order[r][s] == 2.0) h.ord2_mask[r] |= 1u << s;
             if (s < p->nspec && std::fabs(p->nu[r][s]) > 0.0) h.nu_mask[r] |= 1u << s;
         }
     }

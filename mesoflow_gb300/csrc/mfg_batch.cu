@@ -952,6 +952,10 @@ int ns_bucket(int ns) { return ns <= 1 ? 1 : ns <= 2 ? 2 : ns <= 4 ? 4 : ns <= 8
         case 8: KER<8><<<MFG_UNPACK CFG>>> ARGS; break;                 \
         default: KER<16><<<MFG_UNPACK CFG>>> ARGS; break;               \
     }
+// 9 to 12 species apart: the chemistry's arrays for 16 leave two blocks on an SM
+#define NS_DISPATCH12(KER, CFG, ARGS)                                               \
+    if (c_host_params().nspec > 8 && c_host_params().nspec <= 12) KER<12><<<MFG_UNPACK CFG>>> ARGS; \
+    else NS_DISPATCH(KER, CFG, ARGS)
 
 // ---- batched phases --------------------------------------------------------------
 // The tile lists a phase runs over: every box, or the boxes of one level.
@@ -1045,7 +1049,7 @@ void step_batched(mfg_boxlist& L, double dt, cudaStream_t st, const double* dtp 
     }
     {
         ProfScope ps(K_CHEM, st);
-        NS_DISPATCH(bk_chem, (V.grid, BT, 0, st), (L.d_mbox, V.d, V.n, dt, nc, dtp));
+        NS_DISPATCH12(bk_chem, (V.grid, BT, 0, st), (L.d_mbox, V.d, V.n, dt, nc, dtp));
     }
     {
         ProfScope ps(K_PRIMS, st);
@@ -1433,7 +1437,7 @@ void amr_chem(mfg_boxlist& L, AmrRun& R, int l, double dtl) {
     const PhaseTiles& V = level_tiles(L, l)[PH_VALID];
     if (!V.n) return;
     ProfScope ps(K_CHEM, R.st);
-    NS_DISPATCH(bk_chem, (V.grid, BT, 0, R.st), (L.d_mbox, V.d, V.n, dtl, nc, R.ddt ? R.ddt + l : nullptr));
+    NS_DISPATCH12(bk_chem, (V.grid, BT, 0, R.st), (L.d_mbox, V.d, V.n, dtl, nc, R.ddt ? R.ddt + l : nullptr));
 }
 
 void amr_sync(mfg_boxlist& L, AmrRun& R, int l) {  // reflux of level l, average_down of l+1 onto l

@@ -52,6 +52,9 @@ struct DevParams {
     // sparsity of the reaction table as bit masks over the species (bit s:
     // order[r][s] > 0, resp. nu[r][s] != 0), so the kernels test integers
     unsigned ord_mask[MAXR], nu_mask[MAXR];
+    unsigned ord1_mask[MAXR], ord2_mask[MAXR];  // species of order exactly 1 and 2
+    // reactions with Ea != 0; with A, nu finite and 0 <= Ea finite (rate constant finite at any T > 0)
+    unsigned arrhenius, tame;
     // chemistry sub-step integrator: 0 SSP-RK3 (the reference's default), 1 adaptive ROS2
     int chem_kind, chem_maxsub;
     double chem_rtol, chem_atol;

@@ -264,6 +264,7 @@ cudaError_t launch_chem_substep(const mfg_box* boxes, int nbox, double dt, cudaS
         else if (ns <= 2) chem_substep_kernel<2><<<grid, TPB, 0, st>>>(g, dt, nc);
         else if (ns <= 4) chem_substep_kernel<4><<<grid, TPB, 0, st>>>(g, dt, nc);
         else if (ns <= 8) chem_substep_kernel<8><<<grid, TPB, 0, st>>>(g, dt, nc);
+        else if (ns <= 12) chem_substep_kernel<12><<<grid, TPB, 0, st>>>(g, dt, nc);
         else chem_substep_kernel<16><<<grid, TPB, 0, st>>>(g, dt, nc);
     });
 }
@@ -367,6 +368,7 @@ cudaError_t launch_post_step(const mfg_box* boxes, int n, double dt, bool chem, 
     else if (ns <= 2) { MFG_POST(2) }
     else if (ns <= 4) { MFG_POST(4) }
     else if (ns <= 8) { MFG_POST(8) }
+    else if (ns <= 12 && kind == 2) { MFG_POST_K(12, 2); }  // the reactions' arrays for 16 species spill
     else { MFG_POST(16) }
 #undef MFG_POST
 #undef MFG_POST_K
