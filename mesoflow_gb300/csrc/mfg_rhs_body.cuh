@@ -720,7 +720,8 @@ struct Flux5Ctx {
     int64_t rns, rsc;
     int kind;       // 0 density, 1 energy, 2 momentum along d, 3 other
     int c;
-    double idx;
+    double half;    // 1/2, times the advection flag of a species
+    double idx, kd; // 1/dx along d, and that times the diffusivity where it is constant
 };
 
 __device__ __forceinline__ Flux5Ctx flux5_ctx(const RhsBox& B, int d, int c) {
@@ -741,6 +742,8 @@ __device__ __forceinline__ Flux5Ctx flux5_ctx(const RhsBox& B, int d, int c) {
     x.kind = (c == RHO) ? 0 : (c == RHOE) ? 1 : (c == 1 + d) ? 2 : 3;
     x.c = c;
     x.idx = B.idx[d];
+    x.half = (c < NCONS) ? 0.5 : __dmul_rn(0.5, c_P.advect_flag[c - NCONS]);
+    x.kd = (c < NCONS) ? 0.0 : __dmul_rn(c_P.diff_hm[c - NCONS], x.idx);
     return x;
 }
 
@@ -761,19 +764,36 @@ __device__ __forceinline__ void flux5_cell(const Fp& fp, const Flux5Ctx& x, int6
         f = fp.mul(u, x.v[ox]);
 }
 
-// Local Lax-Friedrichs flux of a regular face from the corrections of its two
-// edges (f: of the Euler flux, u: of the state) and fsum = f_L + f_R.
-__device__ __forceinline__ double weno_llf(const Fp& fp, double lam, double fsum, double pLf, double pRf, double pLu,
-                                           double pRu) {
-    const double S = __fma_rn(lam, fp.sub(pLu, pRu), fp.add(pLf, pRf));
-    return __fma_rn(-1.0 / 12.0, S, __dmul_rn(0.5, fsum));
+// Twice the local Lax-Friedrichs flux of a regular face: fsum = f_L + f_R, C
+// the sum of the two edges' corrections of the Euler flux, U the difference of
+// those of the state.
+__device__ __forceinline__ double weno_llf(double lam, double fsum, double C, double U) {
+    return __fma_rn(-1.0 / 6.0, __fma_rn(lam, U, C), fsum);
+}
+
+// C and U of one face between the cells L and R, with t the cells' second
+// differences, g = t_R - t_L, gL and gR the third differences on its two sides
+// and the edges' corrections
+//   P_L = t_L + farL2 gL + nearL g,   P_R = t_R - nearR g - farR2 gR:
+// the two near weights share their third difference and t_L - t_R is -g, so
+// they are added in fixed point, with one conversion and one multiply-add for
+// both (P_L and P_R apart: two more FP64 operations for C, three for U).
+// sumL = t_L + farL2 gL for C, farL2 gL for U.
+template <bool STATE>
+__device__ __forceinline__ double weno_pair(const Fp& fp, double sumL, int64_t qL, const WenoWeights& wR, double g,
+                                            double gR, double tR) {
+    const int64_t q = STATE ? (qL + wR.qR) - ((int64_t)1 << 62) : qL - wR.qR;
+    const double m = weight_of(signed_weight_bits(q)), far = weight_of(wR.farR2);
+    if (STATE) return __fma_rn(far, gR, __fma_rn(m, g, sumL));
+    return __fma_rn(-far, gR, __fma_rn(m, g, fp.add(sumL, tR)));
 }
 
 // First-order stencil near the immersed boundary (compute_flux_3d.H:233-249):
 // the six cells collapse to (L, L, L, R, R, R).  Of the second differences
 // only t_{f-1} = D and t_f = -D with D = R - L remain, both edges have the
 // same weight products, the corrections of the Euler flux cancel and those of
-// the state add up: flux = (f_L + f_R)/2 - lam D (X + 2Y - Z) / (2 (X + 6Y + 3Z)).
+// the state add up: flux = (f_L + f_R)/2 - lam D (X + 2Y - Z) / (2 (X + 6Y + 3Z));
+// returned: twice that.
 __device__ __forceinline__ double weno_llf_collapsed(double lam, double fsum, double D) {
     const double D2 = __dmul_rn(D, D);
     const double sC = __fma_rn(16.0 / 3.0, D2, 4.0 * kEpsWeno), sA = __fma_rn(8.0, D2, sC);
@@ -781,29 +801,32 @@ __device__ __forceinline__ double weno_llf_collapsed(double lam, double fsum, do
     const double X = __dmul_rn(dC, dA), Y = __dmul_rn(dB, dA), Z = __dmul_rn(dB, dC);
     const double p = __fma_rn(2.0, Y, X), q = __fma_rn(2.0, Y, Z);
     const double w = quot_pos(__dsub_rn(p, Z), __fma_rn(3.0, q, X));
-    return __dmul_rn(0.5, __fma_rn(-__dmul_rn(lam, D), w, fsum));
+    return __fma_rn(-__dmul_rn(lam, D), w, fsum);
 }
 
 // Complete flux of one face (the sweep and the per-face form share it, so
-// they agree bitwise), stored: fh is the hyperbolic flux where active, D = u_R
-// - u_L, oL/oR the face's cells, qf, qo, qr its offsets in the face scalars,
+// they agree bitwise), stored: fh2 is twice the hyperbolic flux where active
+// (the half, the advection flag and the viscous term take one operation), D =
+// u_R - u_L, oL/oR the face's cells, qf, qo, qr its offsets in the face scalars,
 // the flux scratch and the caller's flux array.
-__device__ __forceinline__ void flux5_finish(const Fp& fp, const Flux5Ctx& x, bool active, double fh, double D,
+__device__ __forceinline__ void flux5_finish(const Fp& fp, const Flux5Ctx& x, bool active, double fh2, double D,
                                              int64_t oL, int64_t oR, int64_t qf, int64_t qo, int64_t qr) {
     const DevParams& P = c_P;
     const int c = x.c;
     double F = 0.0;
     if (active) {
-        F = (c < NCONS) ? fh : __dmul_rn(P.advect_flag[c - NCONS], fh);
-        if (c >= RHOU && c <= RHOW) F = fp.sub(F, x.fs[qf + (FS_VIS + c - 1) * x.fns]);
-        if (c == RHOE) F = fp.sub(F, x.fs[qf + FS_VISE * x.fns]);
+        if (c >= RHOU && c <= RHOE)
+            F = __fma_rn(x.half, fh2, -x.fs[qf + (c == RHOE ? FS_VISE : FS_VIS + c - 1) * x.fns]);
+        else
+            F = fp.mul(x.half, fh2);
     }
     if (c == RHOE) F = fp.sub(F, x.fs[qf + FS_THERM * x.fns]);
     if (c >= NCONS) {  // species diffusion (compute_flux_3d.H:425-428)
         const int s = c - NCONS;
-        const double Dh = (P.diff_mode[s] == MFG_TRANSPORT_CONST) ? P.diff_hm[s]
-                                                                  : face_diffusivity(P, s, x.vf[oL], x.vf[oR]);
-        F = __fma_rn(-fp.mul(Dh, D), x.idx, F);
+        const double k = (P.diff_mode[s] == MFG_TRANSPORT_CONST)
+                             ? x.kd
+                             : fp.mul(face_diffusivity(P, s, x.vf[oL], x.vf[oR]), x.idx);
+        F = __fma_rn(-k, D, F);
     }
     x.out[qo] = F;
     if (x.reg) {
@@ -832,7 +855,7 @@ __device__ __forceinline__ void flux5_face_body(const Fp& fp, const RhsBox& B, i
         double ru[6], rf[6];
 #pragma unroll
         for (int q = 0; q < 6; ++q) flux5_cell(fp, x, oR + (q - 3) * sd, xR + (q - 3) * xd, ru[q], rf[q]);
-        double pL[2], pR[2];  // corrections of the flux and of the state
+        double cu[2];  // C of the Euler flux, U of the state
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const double* r = h ? ru : rf;
@@ -846,11 +869,11 @@ __device__ __forceinline__ void flux5_face_body(const Fp& fp, const RhsBox& B, i
                           i3 = weno_ind(dd[3], dd[4]);
             const WenoWeights wl = weno_weights(i0.dB, i0.eB, i1.dC, i1.eC, i2.dA, i2.eA);
             const WenoWeights wr = weno_weights(i1.dB, i1.eB, i2.dC, i2.eC, i3.dA, i3.eA);
-            pL[h] = __fma_rn(weight_of(wl.nearL), g1, __fma_rn(weight_of(wl.farL2), g0, tt[1]));
-            pR[h] = __fma_rn(-weight_of(wr.nearR), g1, __fma_rn(-weight_of(wr.farR2), g2, tt[2]));
+            cu[h] = h ? weno_pair<true>(fp, fp.mul(weight_of(wl.farL2), g0), wl.qL, wr, g1, g2, tt[2])
+                      : weno_pair<false>(fp, __fma_rn(weight_of(wl.farL2), g0, tt[1]), wl.qL, wr, g1, g2, tt[2]);
             if (h) D = dd[2];
         }
-        fh = weno_llf(fp, x.fs[qf + FS_LAMBDA * x.fns], fp.add(rf[2], rf[3]), pL[0], pR[0], pL[1], pR[1]);
+        fh = weno_llf(x.fs[qf + FS_LAMBDA * x.fns], fp.add(rf[2], rf[3]), cu[0], cu[1]);
     } else if (flags & 1) {
         double uL, uR, fL, fR;
         flux5_cell(fp, x, oR - sd, xR - xd, uL, fL);
@@ -867,23 +890,25 @@ __device__ __forceinline__ void flux5_face_body(const Fp& fp, const RhsBox& B, i
 // Carried from face to face for one of the two reconstructed quantities (the
 // state or its Euler flux): v0, v1 = cells f, f+1; D = v1 - v0; t_f and g =
 // t_f - t_{f-1}; the indicators of the centres f-1 (B) and f (B, C); the left
-// edge's correction at this face.
+// cell's part of C or U at this face (weno_pair) and its near weight.
 struct WenoRun {
     double v0, v1, D;
-    double t0, g, pL;
+    double t0, g, sumL;
+    int64_t qL;
     uint64_t dBm, dB0, dC0;
     int eBm, eB0, eC0;
 };
 
-// Adds centre f+1 (Dn = v_{f+2} - v_{f+1}): returns the right edge's
-// correction at face f and moves the indicators, t, g and the left edge's
-// correction of the run to face f+1.
+// Adds centre f+1 (Dn = v_{f+2} - v_{f+1}): returns C or U of face f and moves
+// the run to face f+1.
+template <bool STATE>
 __device__ __forceinline__ double weno_next(const Fp& fp, WenoRun& r, double D, double Dn) {
     const WenoInd c = weno_ind(D, Dn);
     const WenoWeights w = weno_weights(r.dBm, r.eBm, r.dC0, r.eC0, c.dA, c.eA);
     const double t = fp.sub(Dn, D), gp = fp.sub(t, r.t0);
-    r.pL = __fma_rn(weight_of(w.nearL), gp, __fma_rn(weight_of(w.farL2), r.g, r.t0));
-    const double pR = __fma_rn(-weight_of(w.nearR), r.g, __fma_rn(-weight_of(w.farR2), gp, r.t0));
+    const double res = weno_pair<STATE>(fp, r.sumL, r.qL, w, r.g, gp, r.t0);
+    r.sumL = STATE ? fp.mul(weight_of(w.farL2), r.g) : __fma_rn(weight_of(w.farL2), r.g, r.t0);
+    r.qL = w.qL;
     r.t0 = t;
     r.g = gp;
     r.dBm = r.dB0;
@@ -892,23 +917,26 @@ __device__ __forceinline__ double weno_next(const Fp& fp, WenoRun& r, double D, 
     r.eB0 = c.eB;
     r.dC0 = c.dC;
     r.eC0 = c.eC;
-    return pR;
+    return res;
 }
 
 // Starts the run at face f: va .. vL = cells f-3, f-2, f-1.
+template <bool STATE>
 __device__ __forceinline__ void weno_prime(const Fp& fp, WenoRun& r, double va, double vb, double vL) {
     const double d0 = fp.sub(vb, va), d1 = fp.sub(vL, vb), d2 = fp.sub(r.v0, vL);
     const WenoInd c0 = weno_ind(d0, d1), c1 = weno_ind(d1, d2);
     const double ta = fp.sub(d1, d0);
     r.t0 = fp.sub(d2, d1);
     r.g = fp.sub(r.t0, ta);
+    r.sumL = 0.0;
+    r.qL = 0;
     r.dBm = c0.dB;
     r.eBm = c0.eB;
     r.dB0 = c1.dB;
     r.eB0 = c1.eB;
     r.dC0 = c1.dC;
     r.eC0 = c1.eC;
-    weno_next(fp, r, d2, r.D);
+    weno_next<STATE>(fp, r, d2, r.D);
 }
 
 __device__ __forceinline__ void flux5_sweep_body(const Fp& fp, const RhsBox& B, int d, int c, int64_t t,
@@ -971,14 +999,12 @@ __device__ __forceinline__ void flux5_sweep_body(const Fp& fp, const RhsBox& B, 
                 double ua, fa, ub, fb;
                 flux5_cell(fp, x, oR - 3 * sd, xR - 3 * xd, ua, fa);
                 flux5_cell(fp, x, oR - 2 * sd, xR - 2 * xd, ub, fb);
-                weno_prime(fp, u, ua, ub, uL);
-                weno_prime(fp, f, fa, fb, fL);
+                weno_prime<true>(fp, u, ua, ub, uL);
+                weno_prime<false>(fp, f, fa, fb, fL);
                 primed = true;
             }
-            const double pLu = u.pL, pLf = f.pL;
-            const double pRf = weno_next(fp, f, f.D, Dfn), pRu = weno_next(fp, u, u.D, Dun);
-            if (flags == 1)
-                fh = weno_llf(fp, x.fs[qf + FS_LAMBDA * x.fns], fp.add(fL, f.v0), pLf, pRf, pLu, pRu);
+            const double C = weno_next<false>(fp, f, f.D, Dfn), U = weno_next<true>(fp, u, u.D, Dun);
+            if (flags == 1) fh = weno_llf(x.fs[qf + FS_LAMBDA * x.fns], fp.add(fL, f.v0), C, U);
         } else {
             primed = false;
         }

@@ -105,13 +105,21 @@ MFG_HD uint64_t weight_bits(uint64_t w, int k) {
     return ((uint64_t)(uint32_t)(e - z - 1) << 52) + (n >> 11);
 }
 
+// A signed number of 2^-62 as the bits of a double.
+MFG_HD uint64_t signed_weight_bits(int64_t v) {
+    const uint64_t neg = (uint64_t)v >> 63;
+    return weight_bits(neg ? 0 - (uint64_t)v : (uint64_t)v, 0) | (neg << 63);
+}
+
 // Weights of the two edges in cell m from the centres m-1 (dB), m (dC), m+1
 // (dA).  With X = C A, Y = B A, Z = B C the left edge of face m+1 has the
 // weights X, 6 Y, 3 Z over their sum for the far, middle and near candidate,
 // the right edge of face m has Z, 6 Y, 3 X.  Returned: twice the far weight
-// and the near weight of each edge, as double bits.
+// and the near weight of each edge, as double bits, and the near weights in
+// units of 2^-62 (to be added before they are converted).
 struct WenoWeights {
     uint64_t farL2, nearL, farR2, nearR;
+    int64_t qL, qR;
 };
 
 MFG_HD WenoWeights weno_weights(uint64_t dB, int eB, uint64_t dC, int eC, uint64_t dA, int eA) {
@@ -126,9 +134,11 @@ MFG_HD WenoWeights weno_weights(uint64_t dB, int eB, uint64_t dC, int eC, uint64
     const uint64_t rL = rcp_fixed(sL << zL), rR = rcp_fixed(sR << zR);
     WenoWeights w;
     w.farL2 = weight_bits(umulhi64(X << zL, rL), 1);
-    w.nearL = weight_bits(umulhi64(Z3 << zL, rL), 0);
+    w.qL = (int64_t)umulhi64(Z3 << zL, rL);
+    w.nearL = weight_bits((uint64_t)w.qL, 0);
     w.farR2 = weight_bits(umulhi64(Z << zR, rR), 1);
-    w.nearR = weight_bits(umulhi64(X3 << zR, rR), 0);
+    w.qR = (int64_t)umulhi64(X3 << zR, rR);
+    w.nearR = weight_bits((uint64_t)w.qR, 0);
     return w;
 }
 

@@ -45,6 +45,20 @@ extern "C" void weights(const double* d, double* w, int n) {
         w[4 * i + 3] = val(r.nearR);
     }
 }
+// d: 5 differences per face; w: far weight of its left edge (twice), the near weights' sum less one and
+// difference, far weight of its right edge (twice)
+extern "C" void pairs(const double* d, double* w, int n) {
+    for (int i = 0; i < n; ++i) {
+        WenoInd c[4];
+        for (int q = 0; q < 4; ++q) c[q] = weno_ind(weno_diff(bits(d[5 * i + q])), weno_diff(bits(d[5 * i + q + 1])));
+        const WenoWeights l = weno_weights(c[0].dB, c[0].eB, c[1].dC, c[1].eC, c[2].dA, c[2].eA);
+        const WenoWeights r = weno_weights(c[1].dB, c[1].eB, c[2].dC, c[2].eC, c[3].dA, c[3].eA);
+        w[4 * i] = val(l.farL2);
+        w[4 * i + 1] = val(signed_weight_bits((l.qL + r.qR) - ((int64_t)1 << 62)));
+        w[4 * i + 2] = val(signed_weight_bits(l.qL - r.qR));
+        w[4 * i + 3] = val(r.farR2);
+    }
+}
 """
 
 
@@ -87,16 +101,20 @@ def reference(f, u, lam):
 
 
 def kernel_form(lib, f, u, lam):
-    def corrections(v):
+    def parts(v):
         d = [v[i + 1] - v[i] for i in range(5)]
         t = [d[i + 1] - d[i] for i in range(4)]
         g = [t[i + 1] - t[i] for i in range(3)]
-        wl, wr = fixed_weights(lib, d[:4]), fixed_weights(lib, d[1:])
-        return t[1] + 2 * wl[0] * g[0] + wl[1] * g[1], t[2] - 2 * wr[2] * g[2] - wr[3] * g[1]
+        a = np.ascontiguousarray(np.stack(d, axis=1))
+        w = np.empty((a.shape[0], 4))
+        lib.pairs(a.ctypes.data_as(C.c_void_p), w.ctypes.data_as(C.c_void_p), C.c_int(a.shape[0]))
+        return t, g, w.T
 
-    fl, fr = corrections(f)
-    ul, ur = corrections(u)
-    return 0.5 * (f[2] + f[3]) - ((fl + fr) + lam * (ul - ur)) / 12
+    t, g, w = parts(f)
+    c = ((t[1] + w[0] * g[0]) + t[2]) + w[2] * g[1] - w[3] * g[2]  # sum of the two edges' corrections
+    t, g, w = parts(u)
+    d = w[0] * g[0] + w[1] * g[1] + w[3] * g[2]                     # difference of the state's
+    return 0.5 * ((f[2] + f[3]) - (c + lam * d) / 6)
 
 
 def collapsed_form(f, u, lam):
