@@ -123,6 +123,55 @@ __device__ __forceinline__ int floor_div(int a, int r) { return a >= 0 ? a / r :
 __device__ __forceinline__ double dmin_(double a, double b) { return (b < a) ? b : a; }  // std::min
 __device__ __forceinline__ double dmax_(double a, double b) { return (a < b) ? b : a; }  // std::max
 
+// min(|a|, |b|) as the comparison b < a selects, on the integer pipe (the order
+// of non-negative doubles is that of their bits; a NaN b is not selected, a NaN
+// a is kept).
+__device__ __forceinline__ double min_abs(double a, double b) {
+    const long long m = 0x7fffffffffffffffll, inf = 0x7ff0000000000000ll;
+    const long long ia = __double_as_longlong(a) & m, ib = __double_as_longlong(b) & m;
+    return __longlong_as_double((ib < ia && ia <= inf) ? ib : ia);
+}
+
+// Largest and smallest of u0 and the 27 values around it, as comparisons in
+// turn select them: NaN neighbours are passed over.  The doubles are compared
+// as integers (54 comparisons of doubles would hold the FP64 pipe longer than
+// the rest of the interpolation); a NaN among them, which sorts beyond an
+// infinity, takes the comparisons themselves.
+__device__ __forceinline__ long long order_key(double x) {
+    const long long b = __double_as_longlong(x);
+    return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+__device__ __forceinline__ double from_key(long long k) {
+    return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
+}
+__device__ __noinline__ void bounds27_nan(const double* q, int64_t js, int64_t ks, double u0, double& umin,
+                                          double& umax) {
+    umin = umax = u0;
+    for (int kk = -1; kk <= 1; ++kk)
+        for (int jj = -1; jj <= 1; ++jj)
+            for (int ii = -1; ii <= 1; ++ii) {
+                const double x = q[ii + jj * js + kk * ks];
+                umin = dmin_(umin, x);
+                umax = dmax_(umax, x);
+            }
+}
+__device__ __forceinline__ void bounds27(const double* q, int64_t js, int64_t ks, double u0, double& umin,
+                                         double& umax) {
+    long long lo = order_key(u0), hi = lo;
+    for (int kk = -1; kk <= 1; ++kk)
+        for (int jj = -1; jj <= 1; ++jj)
+#pragma unroll
+            for (int ii = -1; ii <= 1; ++ii) {
+                const long long x = order_key(q[ii + jj * js + kk * ks]);
+                lo = x < lo ? x : lo;
+                hi = x > hi ? x : hi;
+            }
+    const long long inf = 0x7ff0000000000000ll;
+    if (hi > inf || lo < ~inf) return bounds27_nan(q, js, ks, u0, umin, umax);
+    umin = from_key(lo);
+    umax = from_key(hi);
+}
+
 // cell_cons_interp (AMReX CellConservativeLinear without cross-component
 // limiting) from the coarse patch u of a box of level l (coarse level geometry
 // Gc, ratio r), for coarse cell ic and component c: MC-limited central slopes,
@@ -160,33 +209,31 @@ __device__ double cc_slopes(const MBox& b, const LevelG& Gc, int r, const int ic
         }
         const double df = __dmul_rn(2.0, __dsub_rn(up, u0));
         const double db = __dmul_rn(2.0, __dsub_rn(u0, um));
-        double sx = (__dmul_rn(df, db) >= 0.0) ? dmin_(fabs(df), fabs(db)) : 0.0;
-        sx = __dmul_rn(copysign(1.0, dc), dmin_(sx, fabs(dc)));
-        sl[d] = sx;
+        const double p = __dmul_rn(df, db);
+        const double sx = min_abs((is_negative(p) || is_nan(p)) ? 0.0 : min_abs(df, db), dc);
+        sl[d] = __double_as_longlong(dc) < 0 ? -sx : sx;
     }
     double alpha = 1.0;
-    if (sl[0] != 0.0 || sl[1] != 0.0 || sl[2] != 0.0) {
+    if (!is_zero_bits(sl[0]) || !is_zero_bits(sl[1]) || !is_zero_bits(sl[2])) {
         // (|s| (r-1)) / (2r); for r a power of two the division is the exact
         // multiplication by 1/(2r)
-        const double f = (double)(r - 1), g = (double)(2 * r);
-        const bool pow2 = (r & (r - 1)) == 0;
-        const double ig = 1.0 / g;
         double t[3];
+        if (r == 2) {
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const double x = __dmul_rn(fabs(sl[d]), f);
-            t[d] = pow2 ? __dmul_rn(x, ig) : __ddiv_rn(x, g);
+            for (int d = 0; d < 3; ++d) t[d] = __dmul_rn(fabs(sl[d]), 0.25);
+        } else {
+            const double f = (double)(r - 1), g = (double)(2 * r);
+            const bool pow2 = (r & (r - 1)) == 0;
+            const double ig = 1.0 / g;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const double x = __dmul_rn(fabs(sl[d]), f);
+                t[d] = pow2 ? __dmul_rn(x, ig) : __ddiv_rn(x, g);
+            }
         }
         const double dumax = __dadd_rn(__dadd_rn(t[0], t[1]), t[2]);
-        double umax = u0, umin = u0;
-        for (int kk = -1; kk <= 1; ++kk)
-            for (int jj = -1; jj <= 1; ++jj)
-#pragma unroll
-                for (int ii = -1; ii <= 1; ++ii) {
-                    const double x = u.p[q0 + ii + jj * u.js + kk * u.ks];
-                    umin = dmin_(umin, x);
-                    umax = dmax_(umax, x);
-                }
+        double umax, umin;
+        bounds27(u.p + q0, u.js, u.ks, u0, umin, umax);
         if (__dmul_rn(dumax, alpha) > __dsub_rn(umax, u0)) alpha = __ddiv_rn(__dsub_rn(umax, u0), dumax);
         if (__dmul_rn(dumax, alpha) > __dsub_rn(u0, umin)) alpha = __ddiv_rn(__dsub_rn(u0, umin), dumax);
     }
@@ -207,7 +254,9 @@ struct IEnt {
 
 // Ghost cells of the fine boxes that the fine level does not cover, by
 // cell_cons_interp: one thread per (listed coarse cell, component) computes the
-// slopes once and writes the masked children.
+// slopes once and writes the masked children.  FP64 issue bounds it: 4.8 ->
+// 2.4 ms of a three-level catalyst step with the comparisons on integer keys and
+// the children sharing their offsets.
 __global__ void __launch_bounds__(BT) bk_cp_interp(const IEnt* __restrict__ ent, int ne,
                                                    const MBox* __restrict__ boxes, const LevelG* __restrict__ lev) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -219,6 +268,24 @@ __global__ void __launch_bounds__(BT) bk_cp_interp(const IEnt* __restrict__ ent,
     const int ic[3] = {E.i, E.j, E.k};
     double sa[3];
     const double u0 = cc_slopes(b, lev[b.level - 1], r, ic, c, sa);
+    if (r == 2) {  // offsets -1/4 and 1/4, a direction's two products shared by its children
+        double px[2], py[2], pz[2];
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+            const double off = m ? 0.25 : -0.25;
+            px[m] = __dadd_rn(u0, __dmul_rn(off, sa[0]));
+            py[m] = __dmul_rn(off, sa[1]);
+            pz[m] = __dmul_rn(off, sa[2]);
+        }
+        const unsigned mask = (unsigned)E.mask;
+        double* q = b.sb.p + b.sb.off(ic[0] * 2, ic[1] * 2, ic[2] * 2) + (int64_t)c * b.sb.ns;
+#pragma unroll
+        for (int m = 0; m < 8; ++m) {
+            const int mi = m & 1, mj = (m >> 1) & 1, mk = m >> 2;
+            if ((mask >> m) & 1u) q[mi + mj * b.sb.js + mk * b.sb.ks] = __dadd_rn(__dadd_rn(px[mi], py[mj]), pz[mk]);
+        }
+        return;
+    }
     // child offsets ((m + 0.5) / r - 0.5, m = 0..r-1; the division is exact as
     // a multiplication for r a power of two)
     double offs[4];
@@ -277,6 +344,15 @@ __global__ void __launch_bounds__(BT) bk_fill_copy(const MBox* __restrict__ boxe
     TILE_END
 }
 
+// Directions in which cells lo .. hi reach beyond the domain's non-periodic
+// boundary: a box has cells for the boundary's stage n (outside in n
+// directions) only if it reaches out in n of them.
+__device__ __forceinline__ int outside_dims(const LevelG& G, const int lo[3], const int hi[3], int grow) {
+    int n = 0;
+    for (int d = 0; d < 3; ++d) n += !G.per[d] && (lo[d] - grow < G.dlo[d] || hi[d] + grow > G.dhi[d]);
+    return n;
+}
+
 // Physical boundary of one cell (i, j, k) of the array S outside the domain of
 // G in `stage` non-periodic directions (faces 1, edges 2, corners 3), from S
 // itself.
@@ -313,26 +389,42 @@ __device__ __forceinline__ void bc_cell(const Fab& S, const LevelG& G, int i, in
     } else if (kind == MFG_BC_FOEXTRAP) {
         sv[ds] = lo ? G.dlo[ds] : G.dhi[ds];
         const long long qs = S.off(sv[0], sv[1], sv[2]);
-        for (int c = 0; c < nc; ++c) S.p[qd + c * S.ns] = S.p[qs + c * S.ns];
+        for (int c = 0; c < nc; c += 4) {  // four loads in flight
+            double x[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) x[u] = (c + u < nc) ? S.p[qs + (c + u) * S.ns] : 0.0;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (c + u < nc) S.p[qd + (c + u) * S.ns] = x[u];
+        }
     } else {
         sv[ds] = lo ? (2 * G.dlo[ds] - iv[ds] - 1) : (2 * G.dhi[ds] - iv[ds] + 1);
         const long long qs = S.off(sv[0], sv[1], sv[2]);
-        for (int c = 0; c < nc; ++c) {
-            const double x = S.p[qs + c * S.ns];
-            S.p[qd + c * S.ns] = odd_at_wall(c) ? -x : x;
+        for (int c = 0; c < nc; c += 4) {
+            double x[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) x[u] = (c + u < nc) ? S.p[qs + (c + u) * S.ns] : 0.0;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (c + u < nc) S.p[qd + (c + u) * S.ns] = odd_at_wall(c + u) ? -x[u] : x[u];
         }
     }
 }
 
+// Tiles of boxes that do not reach the boundary are passed over.
 template <int NS>
 __global__ void __launch_bounds__(BT) bk_fill_bc(const MBox* __restrict__ boxes, const LevelG* __restrict__ lev,
                                                  const Tile* __restrict__ tiles, int ntiles, int stage, int nc) {
-    TILE_LOOP
-    const MBox& b = boxes[tl.box];
-    int i, j, k;
-    grown_of(b, t, i, j, k);
-    bc_cell<NS>(b.sb, lev[b.level], i, j, k, stage, nc);
-    TILE_END
+    for (int ti = blockIdx.x; ti < ntiles; ti += gridDim.x) {
+        const Tile tl = tiles[ti];
+        const MBox& b = boxes[tl.box];
+        if (outside_dims(lev[b.level], b.lo, b.hi, MFG_NGROW) < stage) continue;
+        for (long long t = tl.start + threadIdx.x; t < tl.end; t += blockDim.x) {
+            int i, j, k;
+            grown_of(b, t, i, j, k);
+            bc_cell<NS>(b.sb, lev[b.level], i, j, k, stage, nc);
+        }
+    }
 }
 
 __device__ __forceinline__ void cp_of(const MBox& b, long long t, int& i, int& j, int& k) {
@@ -371,11 +463,24 @@ __global__ void __launch_bounds__(BT) bk_cp_fill(const MBox* __restrict__ boxes,
     const MBox& o = boxes[ob];
     const TCoef cf = coef[ev];
     const long long q0 = o.sold.off(w[0], w[1], w[2]), q1 = o.snew.off(w[0], w[1], w[2]);
-    const long long qd = b.cp.off(i, j, k);
-    for (int c = 0; c < nc; ++c) {
-        const double x0 = o.sold.p[q0 + c * o.sold.ns], x1 = o.snew.p[q1 + c * o.snew.ns];
-        b.cp.p[qd + c * b.cp.ns] =
-            cf.kind == 0 ? x0 : cf.kind == 1 ? x1 : __dadd_rn(__dmul_rn(cf.a, x0), __dmul_rn(cf.b, x1));
+    double* qd = b.cp.p + b.cp.off(i, j, k);
+    if (cf.kind < 2) {
+        const Fab& S = cf.kind ? o.snew : o.sold;
+        copy_comps(qd, b.cp.ns, S.p + (cf.kind ? q1 : q0), S.ns, nc);
+        continue;
+    }
+    const double *s0 = o.sold.p + q0, *s1 = o.snew.p + q1;
+    const int64_t n0 = o.sold.ns, n1 = o.snew.ns, nd = b.cp.ns;
+    for (int c = 0; c < nc; c += 4) {  // eight loads in flight
+        double x0[4], x1[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            x0[u] = (c + u < nc) ? __ldg(s0 + (c + u) * n0) : 0.0;
+            x1[u] = (c + u < nc) ? __ldg(s1 + (c + u) * n1) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (c + u < nc) qd[(c + u) * nd] = __dadd_rn(__dmul_rn(cf.a, x0[u]), __dmul_rn(cf.b, x1[u]));
     }
     TILE_END
 }
@@ -383,12 +488,16 @@ __global__ void __launch_bounds__(BT) bk_cp_fill(const MBox* __restrict__ boxes,
 template <int NS>
 __global__ void __launch_bounds__(BT) bk_cp_bc(const MBox* __restrict__ boxes, const LevelG* __restrict__ lev,
                                                const Tile* __restrict__ tiles, int ntiles, int stage, int nc) {
-    TILE_LOOP
-    const MBox& b = boxes[tl.box];
-    int i, j, k;
-    cp_of(b, t, i, j, k);
-    bc_cell<NS>(b.cp, lev[b.level - 1], i, j, k, stage, nc);
-    TILE_END
+    for (int ti = blockIdx.x; ti < ntiles; ti += gridDim.x) {
+        const Tile tl = tiles[ti];
+        const MBox& b = boxes[tl.box];
+        if (outside_dims(lev[b.level - 1], b.cplo, b.cphi, 0) < stage) continue;
+        for (long long t = tl.start + threadIdx.x; t < tl.end; t += blockDim.x) {
+            int i, j, k;
+            cp_of(b, t, i, j, k);
+            bc_cell<NS>(b.cp, lev[b.level - 1], i, j, k, stage, nc);
+        }
+    }
 }
 
 // Flux registers (AMReX FluxRegister).  One thread per (register cell, advected
