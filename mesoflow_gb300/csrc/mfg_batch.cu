@@ -619,13 +619,17 @@ __global__ void __launch_bounds__(BT) bk_cut_list(const CutBox* __restrict__ cb,
     TILE_END
 }
 
+constexpr int CUT_BT = 128;  // small blocks: the cells of one level spread over more SMs
 template <int NS>
-__global__ void __launch_bounds__(BT) bk_cut(const CutBox* __restrict__ cb, const int2* __restrict__ list,
-                                             const unsigned* __restrict__ count) {
+__global__ void __launch_bounds__(CUT_BT) bk_cut(const CutBox* __restrict__ cb, const int2* __restrict__ list,
+                                                 const unsigned* __restrict__ count) {
     const unsigned n = *count;
+    if (blockIdx.x * blockDim.x >= n) return;
+    __shared__ CutShared<CUT_BT> sm;
+    cut_shared_init(sm);
     for (unsigned w = blockIdx.x * blockDim.x + threadIdx.x; w < n; w += gridDim.x * blockDim.x) {
         const int2 e = list[w];
-        cutcell_one<NS>(cb[e.x], e.y);
+        cutcell_one<NS>(cb[e.x], e.y, sm);
     }
 }
 
@@ -1100,7 +1104,7 @@ void b_cutcells(mfg_boxlist& L, const PhaseTiles& T, cudaStream_t st) {
     ProfScope ps(K_CUT, st);
     cudaMemsetAsync(L.d_count, 0, sizeof(unsigned), st);
     bk_cut_list<<<T.grid, BT, 0, st>>>(L.d_cut, T.d, T.n, L.d_cutlist, L.d_count);
-    NS_DISPATCH(bk_cut, (L.cut_grid, BT, 0, st), (L.d_cut, L.d_cutlist, L.d_count));
+    NS_DISPATCH(bk_cut, (L.cut_grid, CUT_BT, 0, st), (L.d_cut, L.d_cutlist, L.d_count));
 }
 
 void b_rhs(mfg_boxlist& L, const TSet& TS, int stage, double dt, cudaStream_t st, const double* dtp = nullptr) {

@@ -111,8 +111,11 @@ __global__ void __launch_bounds__(TPB) cutcell_kernel(const __grid_constant__ Cu
     const unsigned n = *g.count[blockIdx.y];
     const int* __restrict__ list = g.list[blockIdx.y];
     const CutBox& c = g.c[blockIdx.y];
+    if (blockIdx.x * blockDim.x >= n) return;
+    __shared__ CutShared<TPB> sm;
+    cut_shared_init(sm);
     for (unsigned w = blockIdx.x * blockDim.x + threadIdx.x; w < n; w += gridDim.x * blockDim.x)
-        cutcell_one<NS>(c, list[w]);
+        cutcell_one<NS>(c, list[w], sm);
 }
 
 __device__ __forceinline__ int vf_kind(double v) { return is_one(v) ? 2 : (v > 0.0 && v < 1.0) ? 1 : 0; }

@@ -142,49 +142,124 @@ __device__ __forceinline__ void cut_finish(const CutBox& c, int64_t t, int64_t o
     S.p[o + RHOE * S.ns] = add(mul(dens, e), mul(mul(0.5, dens), ke));
 }
 
+// The vfrac == 1 cells of a cut cell's 5^3 neighbourhood as a bit set, in
+// neighbour order (bit = (l + 2) + 5 ((m + 2) + 5 (n + 2))).
+struct CutMask {
+    unsigned long long lo, hi;  // bits 0..63, 64..124
+};
+__device__ __forceinline__ CutMask cut_mask(const double* V, int64_t o, int64_t js, int64_t ks) {
+    CutMask k = {0, 0};
+#pragma unroll 1
+    for (int n = 0; n < SW; ++n) {  // 25 loads in flight
+        const double* q = V + o + (n - SG) * ks;
+        unsigned plane = 0;
+#pragma unroll
+        for (int m = 0; m < SW; ++m)
+#pragma unroll
+            for (int l = 0; l < SW; ++l)
+                if (is_one(q[(l - SG) + (m - SG) * js])) plane |= 1u << (l + SW * m);
+        const int at = SW * SW * n;
+        if (at < 64) k.lo |= (unsigned long long)plane << at;
+        if (at + SW * SW > 64) k.hi |= at < 64 ? (unsigned long long)plane >> (64 - at) : (unsigned long long)plane << (at - 64);
+    }
+    return k;
+}
+// Takes the first neighbour out of the set: its index 0..124.
+__device__ __forceinline__ int cut_next(CutMask& k) {
+    if (k.lo) {
+        const int b = __ffsll((long long)k.lo) - 1;
+        k.lo &= k.lo - 1;
+        return b;
+    }
+    const int b = __ffsll((long long)k.hi) - 1;
+    k.hi &= k.hi - 1;
+    return 64 + b;
+}
+
+// Shared memory of a block's on-the-fly cut cells: per thread the parts of the
+// surface distance of the five positions in each direction ((l dx - xp)^2, m dy
+// - yp, n dz - zp), and the Dirichlet weights (constant memory serves one
+// address at a time).
+template <int NT>
+struct CutShared {
+    double part[3 * SW][NT];
+    double wdir[SW * SW * SW];
+};
+template <int NT>
+__device__ __forceinline__ void cut_shared_init(CutShared<NT>& sm) {  // every thread of the block
+    for (int q = threadIdx.x; q < SW * SW * SW; q += NT) sm.wdir[q] = c_wdir[q];
+    __syncthreads();
+}
+template <int NT>
+__device__ __forceinline__ void cut_parts(CutShared<NT>& sm, const double dxnd[3], const double xpn[3]) {
+#pragma unroll
+    for (int q = 0; q < SW; ++q) {
+        const double a = __fma_rn((double)(q - SG), dxnd[0], -xpn[0]);
+        sm.part[q][threadIdx.x] = mul(a, a);
+        sm.part[SW + q][threadIdx.x] = __fma_rn((double)(q - SG), dxnd[1], -xpn[1]);
+        sm.part[2 * SW + q][threadIdx.x] = __fma_rn((double)(q - SG), dxnd[2], -xpn[2]);
+    }
+}
+// surface_weight of neighbour (l, m, n) + 2 from the parts: the same operations.
+template <int NT>
+__device__ __forceinline__ double cut_weight(const CutShared<NT>& sm, int l, int m, int n) {
+    const double b = sm.part[SW + m][threadIdx.x], e = sm.part[2 * SW + n][threadIdx.x];
+    return rcp_pos(add(__fma_rn(e, e, __fma_rn(b, b, sm.part[l][threadIdx.x])), kTiny2));
+}
+// index 0..124 = l + 5 (m + 5 n)
+__device__ __forceinline__ void cut_split(int idx, int& l, int& m, int& n) {
+    n = (idx * 41) >> 10;
+    const int r = idx - 25 * n;
+    m = (r * 13) >> 6;
+    l = r - 5 * m;
+}
+
 // On-the-fly form: velocity by inverse-distance weighting with a zero
 // Dirichlet value at the surface point; pressure, temperature, density and
 // species by inverse-distance weighting about the surface point (zero normal
-// gradient), over the vfrac == 1 cells of the 5^3 neighbourhood.
-template <int NS>
-__device__ __forceinline__ void cutcell_one(const CutBox& c, int64_t t) {
+// gradient), over the vfrac == 1 cells of the 5^3 neighbourhood.  Every lane
+// walks its own set of fluid neighbours: a loop over the 125 positions runs
+// the body, FP64 issue of 24 slots with ten species, for nearly all of them
+// since some lane of the warp has each (cut cells of a three-level catalyst step
+// 3.55 -> 2.55 ms).
+template <int NS, int NT>
+__device__ __forceinline__ void cutcell_one(const CutBox& c, int64_t t, CutShared<NT>& sm) {
     int i, j, k;
     cell_of(c, t, i, j, k);
     const Fab& S = c.S;
     const int64_t o = S.off(i, j, k);
     const DevParams& P = c_P;
-    const double* V = S.p + VFRAC * S.ns;
     double dist, xpn[3], dxnd[3];
     cut_geometry(c, o, dist, xpn, dxnd);
+    cut_parts(sm, dxnd, xpn);
     double sv[3] = {0.0, 0.0, 0.0}, swd = 0.0;
     double sp = 0.0, st = 0.0, sr = 0.0, ss[NS], swn = 0.0;
 #pragma unroll
     for (int s = 0; s < NS; ++s) ss[s] = 0.0;
     const bool interp_spec = !P.species_in_solid;
-    for (int n = -SG; n <= SG; ++n)
-        for (int m = -SG; m <= SG; ++m)
-            for (int l = -SG; l <= SG; ++l) {
-                const int64_t q = o + l + m * S.js + n * S.ks;
-                if (!is_one(V[q])) continue;
-                const int w = (l + SG) + SW * ((m + SG) + SW * (n + SG));
-                if (!(l == 0 && m == 0 && n == 0)) {
-                    const double wd = c_wdir[w];
-                    sv[0] = __fma_rn(S.p[q + VELX * S.ns], wd, sv[0]);
-                    sv[1] = __fma_rn(S.p[q + VELY * S.ns], wd, sv[1]);
-                    sv[2] = __fma_rn(S.p[q + VELZ * S.ns], wd, sv[2]);
-                    swd = add(swd, wd);
-                }
-                const double wn = surface_weight(l, m, n, dxnd, xpn);
-                sp = __fma_rn(S.p[q + PRES * S.ns], wn, sp);
-                st = __fma_rn(S.p[q + TEMP * S.ns], wn, st);
-                sr = __fma_rn(S.p[q + DENS * S.ns], wn, sr);
-                if (interp_spec) {
+    CutMask nb = cut_mask(S.p + VFRAC * S.ns, o, S.js, S.ks);
+    while (nb.lo | nb.hi) {
+        const int w = cut_next(nb);
+        int l, m, n;
+        cut_split(w, l, m, n);
+        const int64_t q = o + (l - SG) + (m - SG) * S.js + (n - SG) * S.ks;
+        // a cut cell is not its own fluid neighbour: its vfrac is below one
+        const double wd = sm.wdir[w];
+        sv[0] = __fma_rn(S.p[q + VELX * S.ns], wd, sv[0]);
+        sv[1] = __fma_rn(S.p[q + VELY * S.ns], wd, sv[1]);
+        sv[2] = __fma_rn(S.p[q + VELZ * S.ns], wd, sv[2]);
+        swd = add(swd, wd);
+        const double wn = cut_weight(sm, l, m, n);
+        sp = __fma_rn(S.p[q + PRES * S.ns], wn, sp);
+        st = __fma_rn(S.p[q + TEMP * S.ns], wn, st);
+        sr = __fma_rn(S.p[q + DENS * S.ns], wn, sr);
+        if (interp_spec) {
 #pragma unroll
-                    for (int s = 0; s < NS; ++s)
-                        if (s < P.nspec) ss[s] = __fma_rn(S.p[q + (NFLO + s) * S.ns], wn, ss[s]);
-                }
-                swn += wn;
-            }
+            for (int s = 0; s < NS; ++s)
+                if (s < P.nspec) ss[s] = __fma_rn(S.p[q + (NFLO + s) * S.ns], wn, ss[s]);
+        }
+        swn = add(swn, wn);
+    }
     const bool have = swn > 0.0;
     cut_finish<NS>(c, t, o, vel_iden(c, dist, swd), have, have ? 1.0 / swn : 0.0, sv, sp, st, sr, ss);
 }
