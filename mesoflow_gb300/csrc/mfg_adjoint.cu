@@ -427,7 +427,7 @@ __device__ __forceinline__ void collapsed_weight(double D, double& W, double& dD
 // Adjoint of one cell's value: fb of its Euler flux (h = 0) or of its state.
 __device__ __forceinline__ void flux5_cell_vjp(const Fp& fp, const AdjBox& A, const Flux5Ctx& x, int d, int sc, int h,
                                                int64_t os, int64_t ox, double fb) {
-    if (fb == 0.0) return;
+    if (is_zero_bits(fb)) return;
     const Fab& G = A.lamSb;
     if (h) {
         aadd(&G.p[os + sc * G.ns], fb);
@@ -528,7 +528,7 @@ __device__ __forceinline__ void adj_flux_sweep_body(const Fp& fp, const AdjBox& 
             if (m + 1 <= B.hi[d]) Fb = A.lamL.p[lR];
             if (m >= B.lo[d]) Fb = fp.sub(Fb, A.lamL.p[lR - ld]);
             Fb = fp.mul(Fb, B.idx[d]);
-            if (Fb != 0.0) {
+            if (!is_zero_bits(Fb)) {
                 const int64_t oL = oc, oR = oc + sd;
                 if (h && c == RHOE) {  // heat conduction F_E -= k (T_R - T_L)/dx, on every face
                     const double kb = fp.mul(P.cond_hm * B.idx[d], Fb);
@@ -544,7 +544,7 @@ __device__ __forceinline__ void adj_flux_sweep_body(const Fp& fp, const AdjBox& 
                 }
                 const int flags = (int)__double_as_longlong(x.fs[qf + FS_FLAGS * x.fns]) & 3;
                 const double hb = fp.mul(adv, Fb);
-                if ((flags & 1) && hb != 0.0) {
+                if ((flags & 1) && !is_zero_bits(hb)) {
                     const double lam = h ? x.fs[qf + FS_LAMBDA * x.fns] : 1.0;
                     if (!h) {  // half the sum of the two cells' fluxes
                         const double hh = __dmul_rn(0.5, hb);
@@ -567,7 +567,7 @@ __device__ __forceinline__ void adj_flux_sweep_body(const Fp& fp, const AdjBox& 
         }
         c2.sAb = c2.sBb = c2.sCb = c2.tb = 0.0;
         double pLval = 0.0;
-        if (pLb != 0.0 || pRb != 0.0 || hb12 != 0.0 || lamH != 0.0) {
+        if (!(is_zero_bits(pLb) && is_zero_bits(pRb) && is_zero_bits(hb12) && is_zero_bits(lamH))) {
             centre(c0, 0);
             centre(c1, 1);
             centre(c2, 2);
@@ -589,7 +589,7 @@ __device__ __forceinline__ void adj_flux_sweep_body(const Fp& fp, const AdjBox& 
             c2.tb = fp.add(c2.tb, gpb);
             c1.tb = fp.add(c1.tb, fp.add(fp.add(pLb, pRb), fp.sub(gmb, gpb)));
             // the eigenvalue's adjoint of face m: (up - um) hb / 2 = -(hb/12) (P_left - P_right)
-            if (h && lamH != 0.0) aadd(&FS_at(A, d, lamQ), fp.mul(lamH, fp.sub(lamP, fp.sub(t0, eR))));
+            if (h && !is_zero_bits(lamH)) aadd(&FS_at(A, d, lamQ), fp.mul(lamH, fp.sub(lamP, fp.sub(t0, eR))));
             pLval = fp.add(t0, eL);
         }
         reverse_centre(c0, 0);
