@@ -1220,12 +1220,8 @@ template <int NS>
 __device__ void rate_constants(double T, double* kr, double* eT) {
     const DevParams& P = c_P;
     for (int r = 0; r < P.nreact; ++r) {
-        kr[r] = P.A[r];
-        eT[r] = 0.0;
-        if (P.Ea[r] != 0.0) {
-            kr[r] = P.A[r] * exp(-P.Ea[r] / (kRU * T));
-            eT[r] = P.Ea[r] / (kRU * T * T);
-        }
+        kr[r] = rate_constant(P, r, T);
+        eT[r] = ((P.arrhenius >> r) & 1u) ? P.Ea[r] / (kRU * T * T) : 0.0;
     }
 }
 

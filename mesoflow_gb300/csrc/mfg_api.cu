@@ -326,6 +326,10 @@ int mfg_init(const mfg_params* p) {
         h.A[r] = p->A[r];
         h.Ea[r] = p->Ea[r];
         if (p->Ea[r] != 0.0) h.arrhenius |= 1u << r;
+        if (mid_positive(p->Ea[r])) {
+            h.ea[r] = exp_scale(p->Ea[r], kRU);
+            h.ea_mask |= 1u << r;
+        }
         if (std::isfinite(p->A[r]) && std::isfinite(p->Ea[r]) && p->Ea[r] >= 0.0) h.tame |= 1u << r;
         for (int s = 0; s < MFG_MAX_SPECIES; ++s) {
             h.nu[r][s] = p->nu[r][s];

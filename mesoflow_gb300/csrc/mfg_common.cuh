@@ -1,5 +1,6 @@
 // Common device-side definitions of the GB300 mesoflow RHS library.
 #pragma once
+#include "mfg_fixed.cuh"
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string.h>
@@ -55,6 +56,9 @@ struct DevParams {
     unsigned ord1_mask[MAXR], ord2_mask[MAXR];  // species of order exactly 1 and 2
     // reactions with Ea != 0; with A, nu finite and 0 <= Ea finite (rate constant finite at any T > 0)
     unsigned arrhenius, tame;
+    // Ea/RU of the reactions (mask) whose exponential is evaluated in fixed point
+    ExpScale ea[MAXR];
+    unsigned ea_mask;
     // chemistry sub-step integrator: 0 SSP-RK3 (the reference's default), 1 adaptive ROS2
     int chem_kind, chem_maxsub;
     double chem_rtol, chem_atol;

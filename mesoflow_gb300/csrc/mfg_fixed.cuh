@@ -9,6 +9,7 @@
 // kernels leave idle, and its result is rounded once, from 59 or more correct
 // bits (the FP64 sequences round three to five times).
 #pragma once
+#include <math.h>
 #include <stdint.h>
 #include <string.h>
 
@@ -173,6 +174,84 @@ MFG_HD double limited_half(double d1, double d2) {
     if ((int64_t)(b1 ^ b2) < 0 || el < 2) h = 0;
     if (eh == 0x7ff) h = 0x7ff8000000000000ull;
     return double_of(h);
+}
+
+// exp(-E/T) for E, T > 0 (the Arrhenius factor, E = Ea/RU), after the
+// table-driven scheme of P. T. P. Tang (1989): with y = E log2(e) / T = n + j/64
+// + r, exp(-E/T) = 2^-n 2^(-j/64) 2^-r, the last factor by its Taylor series
+// (r < 2^-6: six terms leave 2^-58).  y has 59 correct bits, which the FP64
+// form, a rounded product and a rounded quotient in front of the exponential,
+// does not reach: its error is y 2^-53 and more.  About 300 cycles of the
+// integer pipe against about 1900 of the FP64 pipe.
+// E log2(e) as m 2^(e - 63), top bit of m set, comes from the host.
+struct ExpScale {
+    uint64_t m;
+    int e;
+};
+inline ExpScale exp_scale(double num, double den) {  // host: E = num / den, both positive, finite, normal
+    int xn, xd;
+    const uint64_t n = (uint64_t)ldexp(frexp(num, &xn), 64), d = (uint64_t)ldexp(frexp(den, &xd), 53);
+    const uint64_t log2e = 0xb8aa3b295c17f0bcull;  // 2^63 log2(e)
+    const unsigned __int128 q = (unsigned __int128)n * log2e / d;
+    int top = 127;
+    while (!(uint64_t)(q >> top)) --top;
+    return ExpScale{(uint64_t)(q >> (top - 63)), top + xn - xd - 74};
+}
+
+#define MFG_EXP2_TABLE /* 2^(-j/64) 2^63 */ \
+    0x8000000000000000ull, 0x7e9f06067a4360baull, 0x7d41d96db915019dull, 0x7be86fb985689ddcull, \
+    0x7a92be8a92436616ull, 0x7940bb9e2cffd89dull, 0x77f25ccdee6d7ae6ull, 0x76a7980f6cca15c2ull, \
+    0x75606373ee921c97ull, 0x741cb5281e25ee34ull, 0x72dc8373be41a454ull, 0x719fc4b95f452d29ull, \
+    0x70666f76154a7089ull, 0x6f307a412f074892ull, 0x6dfddbcbed791babull, 0x6cce8ae13c57ebdbull, \
+    0x6ba27e656b4eb57aull, 0x6a79ad55e7f6fd10ull, 0x69540ec8f895722dull, 0x683199ed779592caull, \
+    0x6712460a8fc24072ull, 0x65f60a7f79393e2eull, 0x64dcdec3371793d1ull, 0x63c6ba6455dcd8aeull, \
+    0x62b39508aa836d6full, 0x61a3666d124bb204ull, 0x6096266533384a2bull, 0x5f8bccdb3d398841ull, \
+    0x5e8451cfac061b5full, 0x5d7fad59099f22feull, 0x5c7dd7a3b17dcf75ull, 0x5b7ec8f19468bbc9ull, \
+    0x5a827999fcef3242ull, 0x5988e20954889245ull, 0x5891fac0e95612c8ull, 0x579dbc56b48521baull, \
+    0x56ac1f752150a563ull, 0x55bd1cdad49f699cull, 0x54d0ad5a753e077cull, 0x53e6c9da74b29ab5ull, \
+    0x52ff6b54d8a89c75ull, 0x521a8ad704f3404full, 0x513821818624b40cull, 0x50582887dcb8a7e1ull, \
+    0x4f7a993048d088d7ull, 0x4e9f6cd3967fdba8ull, 0x4dc69cdceaa72a9cull, 0x4cf022c9905bfd32ull, \
+    0x4c1bf828c6dc54b8ull, 0x4b4a169b900c2d00ull, 0x4a7a77d47f7b84b1ull, 0x49ad159789f37496ull, \
+    0x48e1e9b9d588e19bull, 0x4818ee218a3358eeull, 0x47521cc5a2e6a9e0ull, 0x468d6fadbf2dd4f3ull, \
+    0x45cae0f1f545eb73ull, 0x450a6abaa4b77ecdull, 0x444c0740496d4294ull, 0x438fb0cb4f468808ull, \
+    0x42d561b3e6243d8aull, 0x421d1461d66f2023ull, 0x4166c34c5615d0ecull, 0x40b268f9de0183baull,
+#ifdef __CUDACC__
+__device__ static const uint64_t kExp2Device[64] = {MFG_EXP2_TABLE};
+#endif
+#ifndef __CUDA_ARCH__
+static const uint64_t kExp2Host[64] = {MFG_EXP2_TABLE};
+#endif
+MFG_HD uint64_t exp2_entry(int j) {
+#ifdef __CUDA_ARCH__
+    return __ldg((const unsigned long long*)kExp2Device + j);
+#else
+    return kExp2Host[j];
+#endif
+}
+
+// T mid-range positive (mid_positive); false where the factor leaves the range
+// of normal numbers.
+MFG_HD bool exp_neg_over(const ExpScale& E, double T, double* out) {
+    const uint64_t b = bits_of(T);
+    const uint64_t rT = rcp_fixed(((b & kMantMask) | kMantOne) << 11);  // 2^126 / mantissa
+    const uint64_t p = umulhi64(E.m, rT);                              // in [2^61, 2^63)
+    const int s = 62 - E.e + ((int)(b >> 52) - 1023);                  // y = p 2^-s
+    const uint64_t n = s < 64 ? p >> imax(s, 53) : 0;
+    if (s < 53 || n > 1000) return false;                              // y >= 2^9 or 1001
+    const uint64_t f = s <= 63 ? (p << (63 - s)) & 0x7fffffffffffffffull : s < 127 ? p >> (s - 63) : 0;  // 2^63 frac(y)
+    const uint64_t z = umulhi64((f & 0x01ffffffffffffffull) << 1, 0xb17217f7d1cf79acull);  // r ln 2, 2^64
+    uint64_t t = 0x002d82d82d82d82eull;  // 2^63 / 6!
+    t = 0x0111111111111111ull - umulhi64(z, t);  // 2^63 / 5!
+    t = 0x0555555555555555ull - umulhi64(z, t);  // 2^63 / 4!
+    t = 0x1555555555555555ull - umulhi64(z, t);  // 2^63 / 3!
+    t = 0x4000000000000000ull - umulhi64(z, t);  // 2^63 / 2!
+    t = 0x8000000000000000ull - umulhi64(z, t);  // 2^63 / 1!
+    t = 0x8000000000000000ull - umulhi64(z, t);
+    const uint64_t w = umulhi64(exp2_entry((int)(f >> 57)), t);  // 2^-(j/64 + r) 2^62, in (2^61, 2^62]
+    const int up = (int)(w >> 62);                        // 1 only for exactly 1
+    const uint64_t m = w << (1 - up);                     // top bit at 62
+    *out = double_of(((uint64_t)(uint32_t)(1023 - 1 - 1 + up - (int)n) << 52) + ((m + 512) >> 10));
+    return true;
 }
 
 }  // namespace mfg

@@ -40,9 +40,14 @@ __device__ __forceinline__ double order_power(const DevParams& P, int r, int s, 
     return pow(c, P.order[r][s]);
 }
 
-// Rate constant of one reaction: A_r, or A_r exp(-Ea_r/(RU T)) when Ea_r != 0.
+// Rate constant of one reaction: A_r, or A_r exp(-Ea_r/(RU T)) when Ea_r != 0,
+// the exponential in fixed point (bookends of the 64^3 catalyst step 586 -> 515
+// us) but for negative or tiny Ea, T outside the mid range and factors below
+// 2^-1000.
 __device__ __forceinline__ double rate_constant(const DevParams& P, int r, double temp) {
     if (!((P.arrhenius >> r) & 1u)) return P.A[r];
+    double f;
+    if (((P.ea_mask >> r) & 1u) && mid_positive(temp) && exp_neg_over(P.ea[r], temp, &f)) return P.A[r] * f;
     return P.A[r] * exp(-P.Ea[r] / (kRU * temp));
 }
 

@@ -25,6 +25,11 @@ extern "C" void run(int what, const double* a, const double* b, double* o, int n
         o[i] = what == 0 ? rcp_mid(a[i]) : what == 1 ? rsqrt_mid(a[i]) : what == 2 ? limited_half(a[i], b[i])
                                                                         : (double)mid_positive(a[i]);
 }
+// exp(-(a/den)/b); -1 where the fixed point is not taken
+extern "C" void arrhenius(const double* a, double den, const double* b, double* o, int n) {
+    for (int i = 0; i < n; ++i)
+        if (!mid_positive(a[i]) || !mid_positive(b[i]) || !exp_neg_over(exp_scale(a[i], den), b[i], o + i)) o[i] = -1.0;
+}
 """
 
 
@@ -46,6 +51,7 @@ def run(tmp_path_factory):
         lib.run(C.c_int(what), p[0], p[1], p[2], C.c_int(a.size))
         return o
 
+    call.lib = lib
     return call
 
 
@@ -109,3 +115,25 @@ def test_ausm_split_forms():
         tol = 16 * 4 * 2.0 ** -53
         assert np.all(np.abs(sign * 0.25 * m4 - mach) <= tol * np.maximum(1.0, np.abs(M)))
         assert np.all(np.abs((sign * alpha * mq + 0.25 * g) - pres) <= tol)
+
+
+@pytest.mark.skipif(np.finfo(L).nmant < 63, reason="needs extended precision")
+@pytest.mark.parametrize("lo,hi", [(1e-12, 1e-3), (1e-3, 1e2), (1e2, 1e5), (1e5, 3e6)])
+def test_arrhenius_factor(run, lo, hi):
+    """exp(-x), x = Ea/(RU T): y = x log2(e) has 58.5 bits (the reciprocal's 59
+    and two truncations), which the exponential turns into x 2^-58; the series,
+    its table and its products leave 2^-57; one rounding."""
+    rng = np.random.default_rng(7)
+    n, RU = 200000, 8.31446261815324
+    Ea = np.exp(rng.uniform(np.log(lo), np.log(hi), n))
+    T = rng.uniform(150.0, 4000.0, n)
+    T[:100] = 2.0 ** rng.integers(6, 12, 100)
+    T[100:200] = np.nextafter(T[:100], 0.0)
+    o = np.empty(n)
+    p = [v.ctypes.data_as(C.c_void_p) for v in (Ea, T, o)]
+    run.lib.arrhenius(p[0], C.c_double(RU), p[1], p[2], C.c_int(n))
+    x = L(Ea) / L(RU) / L(T)
+    taken = o >= 0.0
+    assert np.all(taken[x < 354.0]) and not np.any(taken[x > 710.0])
+    want = np.exp(-x[taken])
+    assert np.all(np.abs(L(o[taken]) - want) <= (2.0 ** -53 + 2.0 ** -57 + x[taken] * 2.0 ** -58) * want)
