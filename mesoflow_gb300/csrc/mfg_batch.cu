@@ -657,10 +657,15 @@ __global__ void __launch_bounds__(BT) bk_face_high(const RhsBox* __restrict__ B,
     TILE_END
 }
 
-template <bool FAST>
 __global__ void __launch_bounds__(BT) bk_flux(const RhsBox* __restrict__ B, const Tile* __restrict__ tiles, int ntiles) {
     TILE_LOOP
-    flux_body<FAST>(B[tl.box], tl.part >> 5, tl.part & 31, t);
+    flux_body(B[tl.box], tl.part >> 5, tl.part & 31, t);
+    TILE_END
+}
+__global__ void __launch_bounds__(BT) bk_flux4(const RhsBox* __restrict__ B, const Tile* __restrict__ tiles, int ntiles) {
+    const Fp fp;
+    TILE_LOOP
+    flux4_body(fp, B[tl.box], tl.part >> 5, tl.part & 31, t);
     TILE_END
 }
 
@@ -1153,10 +1158,10 @@ void b_rhs(mfg_boxlist& L, const TSet& TS, int stage, double dt, cudaStream_t st
             bk_flux_sweep<<<T.grid, SWEEP_BT, 0, st>>>(L.d_rhs, T.d, T.n);
         else if (flux_kind(L) == 1)
             bk_flux5_face<<<T.grid, SWEEP_BT, 0, st>>>(L.d_rhs, T.d, T.n);
-        else if (weno_fast_mode())
-            bk_flux<true><<<T.grid, BT, 0, st>>>(L.d_rhs, T.d, T.n);
+        else if (ord == 4 && c_host_params().do_ns)
+            bk_flux4<<<T.grid, BT, 0, st>>>(L.d_rhs, T.d, T.n);
         else
-            bk_flux<false><<<T.grid, BT, 0, st>>>(L.d_rhs, T.d, T.n);
+            bk_flux<<<T.grid, BT, 0, st>>>(L.d_rhs, T.d, T.n);
     }
     {
         const PhaseTiles& T = TS[PH_UPDATE];
@@ -2089,8 +2094,10 @@ int mfg_boxlist_autotune(mfg_boxlist* L, double dt, double* results, void* strea
                                 bk_flux_sweep<<<P.grid, SWEEP_BT, 0, st>>>(L->d_rhs, P.d, P.n);
                             else if (flux_kind(*L) == 1)
                                 bk_flux5_face<<<P.grid, SWEEP_BT, 0, st>>>(L->d_rhs, P.d, P.n);
+                            else if (ord == 4 && c_host_params().do_ns)
+                                bk_flux4<<<P.grid, BT, 0, st>>>(L->d_rhs, P.d, P.n);
                             else
-                                bk_flux<true><<<P.grid, BT, 0, st>>>(L->d_rhs, P.d, P.n);
+                                bk_flux<<<P.grid, BT, 0, st>>>(L->d_rhs, P.d, P.n);
                             break;
                         case PH_UPDATE: bk_update<<<P.grid, BT, 0, st>>>(L->d_rhs, P.d, P.n, 0, dt, nullptr); break;
                     }

@@ -64,10 +64,8 @@ __device__ __forceinline__ double euler_flux(int c, int d, double u_c, double rh
 // stencil values ordered from the far upwind cell (a) to the far downwind
 // cell (e); the right-biased edge passes them mirrored.  MIR selects the
 // operand order of the reference's third candidate polynomial for the mirrored
-// call.  FAST normalises the three nonlinear weights with one division
-// (w_k/(eps+b_k)^2 / sum = w_k e_k / sum w_j e_j, e_k = prod_{j!=k} (eps+b_j)^2)
-// instead of four; the result differs from the reference by a few ulp.
-template <bool MIR, bool FAST>
+// call.
+template <bool MIR>
 __device__ __forceinline__ double weno_edge(double a, double b, double c, double d, double e) {
     double t = (a - 2.0 * b) + c;
     double t2 = (a - 4.0 * b) + 3.0 * c;
@@ -80,15 +78,6 @@ __device__ __forceinline__ double weno_edge(double a, double b, double c, double
     double v2 = MIR ? (11.0 * c - 7.0 * b) + 2.0 * a : (2.0 * a - 7.0 * b) + 11.0 * c;
     double v1 = (-b + 5.0 * c) + 2.0 * d;
     double v0 = (2.0 * c + 5.0 * d) - e;
-    if (FAST) {
-        double d2 = (kEpsWeno + b2) * (kEpsWeno + b2);
-        double d1 = (kEpsWeno + b1) * (kEpsWeno + b1);
-        double d0 = (kEpsWeno + b0) * (kEpsWeno + b0);
-        double e2 = d1 * d0, e1 = 6.0 * (d2 * d0), e0 = 3.0 * (d2 * d1);
-        double num = (e2 * v2 + e1 * v1) + e0 * v0;
-        double den = (e2 + e1) + e0;
-        return num / (6.0 * den);
-    }
     double a2 = 1.0 / ((kEpsWeno + b2) * (kEpsWeno + b2));
     double a1 = 6.0 * (1.0 / ((kEpsWeno + b1) * (kEpsWeno + b1)));
     double a0 = 3.0 * (1.0 / ((kEpsWeno + b0) * (kEpsWeno + b0)));
@@ -98,10 +87,9 @@ __device__ __forceinline__ double weno_edge(double a, double b, double c, double
 
 // Face value pair of the stencil s[0..5] = cells i-3 .. i+2 of face i:
 // up = left-biased value (cells i-3..i+1), um = right-biased (cells i-2..i+2).
-template <bool FAST>
 __device__ __forceinline__ void weno_face(const double s[6], double& up, double& um) {
-    up = weno_edge<false, FAST>(s[0], s[1], s[2], s[3], s[4]);
-    um = weno_edge<true, FAST>(s[5], s[4], s[3], s[2], s[1]);
+    up = weno_edge<false>(s[0], s[1], s[2], s[3], s[4]);
+    um = weno_edge<true>(s[5], s[4], s[3], s[2], s[1]);
 }
 
 // Sound speed sqrt(gamma p / rho), p = kap rho e (get_max_eigenvalue,
@@ -480,7 +468,8 @@ __device__ __forceinline__ void face_body(const Fp& fp, const RhsBox& B, int d, 
 // ---------------------------------------------------------------------------
 // flux_kernel: per (face, component) along d
 // ---------------------------------------------------------------------------
-template <bool FAST>
+// WENO5 in the reference's candidate form (four divisions per edge), and the
+// species convection without Navier-Stokes terms.
 __device__ __forceinline__ void flux_body(const RhsBox& B, int d, int c, int64_t t) {
     int lo[3] = {B.lo[0], B.lo[1], B.lo[2]}, len[3];
     for (int e = 0; e < 3; ++e) len[e] = B.hi[e] - B.lo[e] + 1 + (e == d);
@@ -501,39 +490,29 @@ __device__ __forceinline__ void flux_body(const RhsBox& B, int d, int c, int64_t
 
     double F = 0.0;
     if (P.do_ns) {
-        if (active) {  // orders 4 and 5 (the face kernels write the fluxes of orders 1 and 2)
-            const int ord = P.order_hyp;
-            double fh;
-            {
-                const Fab& X = B.aux;
-                const int64_t xd = (d == 0) ? 1 : (d == 1) ? X.js : X.ks;
-                const int64_t xR = X.off(f.i, f.j, f.k);
-                const double lam = FS.p[qf + FS_LAMBDA * FS.ns];
-                double us[6], fl[6];
+        if (active) {
+            const Fab& X = B.aux;
+            const int64_t xd = (d == 0) ? 1 : (d == 1) ? X.js : X.ks;
+            const int64_t xR = X.off(f.i, f.j, f.k);
+            const double lam = FS.p[qf + FS_LAMBDA * FS.ns];
+            double us[6], fl[6];
 #pragma unroll
-                for (int q = 0; q < 6; ++q) {
-                    int qq = q - 3;
-                    if (fallback) qq = (q < 3) ? -1 : 0;  // first-order stencil (:233-249)
-                    const int64_t os = oR + qq * sd, ox = xR + qq * xd;
-                    us[q] = u[os];
-                    const double rho = S.p[os + RHO * S.ns];
-                    const double vd = X.p[ox + (AUX_VX + d) * X.ns];
-                    const double va = (c >= 1 && c <= 3) ? X.p[ox + (AUX_VX + c - 1) * X.ns] : 0.0;
-                    const double p = X.p[ox + AUX_PF * X.ns];
-                    const double E = S.p[os + RHOE * S.ns];
-                    fl[q] = euler_flux(c, d, us[q], rho, va, vd, p, E);
-                }
-                if (ord == 5) {
-                    double fp, fm, up, um;
-                    weno_face<FAST>(fl, fp, fm);
-                    weno_face<FAST>(us, up, um);
-                    fh = 0.5 * (fp + lam * up) + 0.5 * (fm - lam * um);
-                } else {
-                    // central_with_diss_flux(ul, ur, ulm1, urp1): uim1=ul, ui=ur, uim2=ulm1, uip1=urp1
-                    fh = kTwelveth * (((7.0 * fl[3] + 7.0 * fl[2]) - fl[1]) - fl[4]);
-                    fh -= ((kTwelveth * (((3.0 * us[3] - 3.0 * us[2]) - us[4]) + us[3])) * lam) * P.dissfactor;
-                }
+            for (int q = 0; q < 6; ++q) {
+                int qq = q - 3;
+                if (fallback) qq = (q < 3) ? -1 : 0;  // first-order stencil (:233-249)
+                const int64_t os = oR + qq * sd, ox = xR + qq * xd;
+                us[q] = u[os];
+                const double rho = S.p[os + RHO * S.ns];
+                const double vd = X.p[ox + (AUX_VX + d) * X.ns];
+                const double va = (c >= 1 && c <= 3) ? X.p[ox + (AUX_VX + c - 1) * X.ns] : 0.0;
+                const double p = X.p[ox + AUX_PF * X.ns];
+                const double E = S.p[os + RHOE * S.ns];
+                fl[q] = euler_flux(c, d, us[q], rho, va, vd, p, E);
             }
+            double fp, fm, up, um;
+            weno_face(fl, fp, fm);
+            weno_face(us, up, um);
+            const double fh = 0.5 * (fp + lam * up) + 0.5 * (fm - lam * um);
             F = (c < NCONS) ? fh : P.advect_flag[c - NCONS] * fh;
             if (c >= RHOU && c <= RHOW) F -= FS.p[qf + (FS_VIS + c - 1) * FS.ns];
             if (c == RHOE) F -= FS.p[qf + FS_VISE * FS.ns];
@@ -720,7 +699,7 @@ struct Flux5Ctx {
     int64_t rns, rsc;
     int kind;       // 0 density, 1 energy, 2 momentum along d, 3 other
     int c;
-    double half;    // 1/2, times the advection flag of a species
+    double half;    // scale of the flux sum: 1/2 (order 4: 1/12), times the advection flag of a species
     double idx, kd; // 1/dx along d, and that times the diffusivity where it is constant
 };
 
@@ -805,9 +784,9 @@ __device__ __forceinline__ double weno_llf_collapsed(double lam, double fsum, do
 }
 
 // Complete flux of one face (the sweep and the per-face form share it, so
-// they agree bitwise), stored: fh2 is twice the hyperbolic flux where active
-// (the half, the advection flag and the viscous term take one operation), D =
-// u_R - u_L, oL/oR the face's cells, qf, qo, qr its offsets in the face scalars,
+// they agree bitwise), stored: fh2 times x.half is the hyperbolic flux where
+// active (the half, the advection flag and the viscous term take one operation),
+// D = u_R - u_L, oL/oR the face's cells, qf, qo, qr its offsets in the face scalars,
 // the flux scratch and the caller's flux array.
 __device__ __forceinline__ void flux5_finish(const Fp& fp, const Flux5Ctx& x, bool active, double fh2, double D,
                                              int64_t oL, int64_t oR, int64_t qf, int64_t qo, int64_t qr) {
@@ -884,6 +863,44 @@ __device__ __forceinline__ void flux5_face_body(const Fp& fp, const RhsBox& B, i
         D = fp.sub(x.u[oR], x.u[oR - sd]);
     }
     flux5_finish(fp, x, flags & 1, fh, D, oR - sd, oR, qf, B.flx[d].off(f.i, f.j, f.k),
+                 x.reg ? B.uflux[d].off(f.i, f.j, f.k) : 0);
+}
+
+// Order 4, central with dissipation (the reference's central_with_diss_flux:
+// (7 (f_L + f_R) - f_LL - f_RR - lam dissfactor (3 u_R - 3 u_L - u_RR + u_R))
+// / 12): one thread per (face, component), the four cells it reads as the
+// order-5 sweep takes them (one or two FP64 operations each, against six cells
+// of the general Euler flux before), half, flag and viscous term in one
+// multiply-add: about 16 FP64 operations against 60 (right-hand side of 57x64x33 cells
+// 287 -> 217 us).
+__device__ __forceinline__ void flux4_body(const Fp& fp, const RhsBox& B, int d, int c, int64_t t) {
+    int len[3];
+    for (int e = 0; e < 3; ++e) len[e] = B.hi[e] - B.lo[e] + 1 + (e == d);
+    if (t >= (int64_t)len[0] * len[1] * len[2]) return;
+    const Idx3 f = delinear(t, B.lo, len);
+    Flux5Ctx x = flux5_ctx(B, d, c);
+    x.half = (c < NCONS) ? kTwelveth : __dmul_rn(kTwelveth, c_P.advect_flag[c - NCONS]);
+    const int64_t sd = (d == 0) ? 1 : (d == 1) ? B.sb.js : B.sb.ks;
+    const int64_t xd = (d == 0) ? 1 : (d == 1) ? B.aux.js : B.aux.ks;
+    const int64_t oR = B.sb.off(f.i, f.j, f.k), xR = B.aux.off(f.i, f.j, f.k);
+    const int64_t qf = B.fs[d].off(f.i, f.j, f.k);
+    const int flags = (int)__double_as_longlong(x.fs[qf + FS_FLAGS * x.fns]);
+    double S = 0.0, D;
+    if (flags & 1) {
+        const double lam = __dmul_rn(x.fs[qf + FS_LAMBDA * x.fns], c_P.dissfactor);
+        double u[4], fl[4];  // cells LL, L, R, RR
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int at = (flags & 2) ? (q < 2 ? -1 : 0) : q - 2;  // first-order stencil (:233-249)
+            flux5_cell(fp, x, oR + at * sd, xR + at * xd, u[q], fl[q]);
+        }
+        D = fp.sub(u[2], u[1]);
+        S = __fma_rn(-lam, __fma_rn(3.0, D, fp.sub(u[2], u[3])),
+                     fp.sub(__fma_rn(7.0, fp.add(fl[2], fl[1]), -fl[0]), fl[3]));
+    } else {
+        D = fp.sub(x.u[oR], x.u[oR - sd]);
+    }
+    flux5_finish(fp, x, flags & 1, S, D, oR - sd, oR, qf, B.flx[d].off(f.i, f.j, f.k),
                  x.reg ? B.uflux[d].off(f.i, f.j, f.k) : 0);
 }
 

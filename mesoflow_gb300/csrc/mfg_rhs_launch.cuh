@@ -91,9 +91,15 @@ __global__ void __launch_bounds__(LIST_TPB, NS <= 2 ? 5 : 4) face_list_kernel(co
     if (w < B.fcount[d]) face_body<NS, false>(fp, B, d, B.flist[face_list_off(B, d) + w]);
 }
 // Direction and box of the flux launches: blockIdx.z = 3 box + direction.
-template <bool FAST, int G>
+template <int G>
+__global__ void __launch_bounds__(TPB) flux4_kernel(const __grid_constant__ RhsGroup<G> g) {
+    const Fp fp;
+    flux4_body(fp, g.b[G == 1 ? 0 : blockIdx.z / 3], blockIdx.z % 3, blockIdx.y,
+               (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
+}
+template <int G>
 __global__ void __launch_bounds__(TPB) flux_kernel(const __grid_constant__ RhsGroup<G> g) {
-    flux_body<FAST>(g.b[G == 1 ? 0 : blockIdx.z / 3], blockIdx.z % 3, blockIdx.y,
+    flux_body(g.b[G == 1 ? 0 : blockIdx.z / 3], blockIdx.z % 3, blockIdx.y,
                     (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 constexpr int SWEEP_TPB = 128;
@@ -176,10 +182,10 @@ cudaError_t launch_group_ns(const RhsGroup<G>& g, int n, int stage, double dt, b
             } else {
                 flux5_face_kernel<G><<<dim3(blocks_for(nf, SWEEP_TPB), C, 3 * n), SWEEP_TPB, 0, st>>>(g);
             }
-        } else if (fast) {
-            flux_kernel<true, G><<<dim3(blocks_for(nf), C, 3 * n), TPB, 0, st>>>(g);
+        } else if (ord == 4 && P.do_ns) {
+            flux4_kernel<G><<<dim3(blocks_for(nf), C, 3 * n), TPB, 0, st>>>(g);
         } else {
-            flux_kernel<false, G><<<dim3(blocks_for(nf), C, 3 * n), TPB, 0, st>>>(g);
+            flux_kernel<G><<<dim3(blocks_for(nf), C, 3 * n), TPB, 0, st>>>(g);
         }
     }
     ProfScope ps(K_UPDATE, st);
