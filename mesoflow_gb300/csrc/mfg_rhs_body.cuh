@@ -198,19 +198,22 @@ __device__ __forceinline__ void ausm_split(const Fp& fp, double M, double sign, 
 // active and the pass is the split form of orders 1/2 with Navier-Stokes
 // terms (face_split_kernel); the flux branch and the first-order fallback
 // test (used only by the flux branch and the stored face scalars of orders
-// 4/5) are compiled out, the remaining arithmetic is the same.
+// 4/5) are compiled out, the remaining arithmetic is the same.  ACTIVE: the
+// caller knows that it is active.
 //
 // FP64 issue bounds the flux branch of orders 1/2.  Its reciprocals, square
 // roots and limiters run in fixed point on the integer pipe (mfg_fixed.cuh),
 // its sums and products as register-operand multiply-adds (Fp), and every
 // rounding is explicit, so the one-pass and the listed form agree bitwise.
-// About 170 FP64 operations per face of one species at 70 cycles (205 at 82
+// About 150 FP64 operations per face of one species at 70 cycles (205 at 82
 // with the refined reciprocals there): face passes of a 256^3 sphere-pack step
-// 50.4 -> 38.0 ms; the listed form keeps the FP64 pipe 83% busy.
+// 50.4 -> 38.0 ms, and 36.5 with the factors of four of the splits, the viscosity
+// and the conductivity inside multiply-adds; the listed form keeps the FP64 pipe
+// 83% busy.
 //
 // HIGH: orders 4 and 5, else 1 and 2 (the caller has the order from the host,
 // so each kernel holds the registers of its own branch).
-template <int NS, bool HIGH, bool SOLID_SIDE = false>
+template <int NS, bool HIGH, bool SOLID_SIDE = false, bool ACTIVE = false>
 __device__ __forceinline__ void face_body_at(const Fp& fp, const RhsBox& B, int d, const Idx3& f) {
     const DevParams& P = c_P;
     const Fab& S = B.sb;
@@ -229,13 +232,13 @@ __device__ __forceinline__ void face_body_at(const Fp& fp, const RhsBox& B, int 
         for (int q = -3; q <= 2; ++q) fallback |= below_one(vf[oR + q * sd]);
     }
     // face volume fraction 0.5 (a + b) >= 0.5, i.e. a + b >= 1 (the halving is exact)
-    const bool active = !SOLID_SIDE && P.do_ns && nonneg_ge(fp.add(vf[oL], vf[oR]), 1.0);
+    const bool active = ACTIVE || (!SOLID_SIDE && P.do_ns && nonneg_ge(fp.add(vf[oL], vf[oR]), 1.0));
 
     double lam = 0.0;                        // orders 4, 5: LLF eigenvalue
     double uL[NCONS + NS], uR[NCONS + NS];   // orders 1, 2: advected face states, E + p for the energy
-    double wL = 0.0, wR = 0.0, ph = 0.0;     // orders 1, 2: mass-flux weights, interface pressure
-    double vis[3] = {0.0, 0.0, 0.0}, vise2 = 0.0;  // viscous stresses; twice the viscous work
-    double therm = 0.0;                      // heat conduction
+    double wL = 0.0, wR = 0.0, ph4 = 0.0;    // orders 1, 2: mass-flux weights, four times the interface pressure
+    double vis[3] = {0.0, 0.0, 0.0}, vise2 = 0.0;  // viscous stresses over mu; twice the viscous work over mu
+    double mu = 0.0, kc = 0.0, therm = 0.0;  // viscosity, conductivity; heat conduction over k
 
     if (active) {
         if (HIGH) {
@@ -351,19 +354,21 @@ __device__ __forceinline__ void face_body_at(const Fp& fp, const RhsBox& B, int 
             // a_1/2^2) with rho_1/2 = (rho_L + rho_R)/2, as 4 M_1/2 less
             // (-qs)^+ (p_R - p_L) / (fa (rho_L + rho_R) a_1/2^2)
             const double pd = fp.mul(fp.mul(pos_part(-qs), fp.sub(pR, pL)), fp.mul(iah, iah));
-            const double Mh = __dmul_rn(0.25, __fma_rn(-pd, face_rcp(fr), fp.sub(m4L, m4R)));
-            double modM = fabs(Mh);
-            if (nonneg_le(modM, 0.3)) modM = __dmul_rn(__fma_rn(Mh, Mh, 0.3 * 0.3), 1.0 / (2.0 * 0.3));
+            // M_1/2, its modulus with the parabola below 0.3, and the pressure
+            // splits, each times four (exact scales, taken back where they cost nothing)
+            const double M4 = __fma_rn(-pd, face_rcp(fr), fp.sub(m4L, m4R));
+            double mod4 = fabs(M4);
+            if (nonneg_le(mod4, 4.0 * 0.3)) mod4 = __dmul_rn(__fma_rn(M4, M4, 16.0 * (0.3 * 0.3)), 0.25 * (1.0 / (2.0 * 0.3)));
             // alpha = 3/16 (-4 + 5 fa^2) as (15/16 fa) fa - 3/4
-            const double alpha = __fma_rn(__dmul_rn(15.0 / 16.0, fa), fa, -0.75);
-            const double PLp = __fma_rn(alpha, mqL, __dmul_rn(0.25, gL)), PRm = __fma_rn(-alpha, mqR, __dmul_rn(0.25, gR));
-            const double pu = fp.mul(fp.mul(fp.mul(PLp, PRm), fp.mul(fr, ah)), fp.sub(vR, vL));
-            ph = __fma_rn(-0.75, pu, __fma_rn(PLp, pL, fp.mul(PRm, pR)));
+            const double a4 = __fma_rn(__dmul_rn(15.0 / 4.0, fa), fa, -3.0);
+            const double PL4 = __fma_rn(a4, mqL, gL), PR4 = __fma_rn(-a4, mqR, gR);
+            const double pu16 = fp.mul(fp.mul(fp.mul(PL4, PR4), fp.mul(fr, ah)), fp.sub(vR, vL));
+            ph4 = __fma_rn(-3.0 / 16.0, pu16, __fma_rn(PL4, pL, fp.mul(PR4, pR)));
             // mass-flux weights with the wave speed folded in: the flux of a
             // component (M/2 (fL + fR) - |M|/2 (fR - fL)) a_half is wL fL + wR fR
             // with wL = (M + |M|) a_half / 2, wR = (M - |M|) a_half / 2
-            const double ahh = __dmul_rn(0.5, ah);
-            const double cmh = fp.mul(Mh, ahh), cmod = fp.mul(modM, ahh);
+            const double ah8 = __dmul_rn(0.125, ah);
+            const double cmh = fp.mul(M4, ah8), cmod = fp.mul(mod4, ah8);
             wL = fp.add(cmh, cmod);
             wR = fp.sub(cmh, cmod);
         }
@@ -386,27 +391,27 @@ __device__ __forceinline__ void face_body_at(const Fp& fp, const RhsBox& B, int 
         const double s1 = fp.sub(fp.add(Vt1[oL + st1], Vt1[oR + st1]), fp.add(Vt1[oL - st1], Vt1[oR - st1]));
         const double s2 = fp.sub(fp.add(Vt2[oL + st2], Vt2[oR + st2]), fp.add(Vt2[oL - st2], Vt2[oR - st2]));
         // viscosity always from cells (i,j,k) and (i-1,j,k) (compute_flux_3d.H:179)
-        const double mu = (P.visc_mode == MFG_TRANSPORT_CONST)
-                              ? P.visc_hm
-                              : harmonic_mean(blend(P.visc_mode, P.visc_gas, P.visc_solid, vf[oR]),
-                                              blend(P.visc_mode, P.visc_gas, P.visc_solid, vf[oR - 1]));
-        const double taud = fp.mul(mu, __fma_rn(fp.sub(vdR, vdL), B.i43[d],
-                                                __fma_rn(s1, B.iq23[t1], fp.mul(s2, B.iq23[t2]))));
-        const double tau1 = fp.mul(mu, __fma_rn(fp.sub(v1R, v1L), B.idx[d], fp.mul(e1, B.iq[t1])));
-        const double tau2 = fp.mul(mu, __fma_rn(fp.sub(v2R, v2L), B.idx[d], fp.mul(e2, B.iq[t2])));
-        // twice the viscous work sum_a tau_{d a} v_a of the energy flux
+        mu = (P.visc_mode == MFG_TRANSPORT_CONST)
+                 ? P.visc_hm
+                 : harmonic_mean(blend(P.visc_mode, P.visc_gas, P.visc_solid, vf[oR]),
+                                 blend(P.visc_mode, P.visc_gas, P.visc_solid, vf[oR - 1]));
+        const double taud = __fma_rn(fp.sub(vdR, vdL), B.i43[d], __fma_rn(s1, B.iq23[t1], fp.mul(s2, B.iq23[t2])));
+        const double tau1 = __fma_rn(fp.sub(v1R, v1L), B.idx[d], fp.mul(e1, B.iq[t1]));
+        const double tau2 = __fma_rn(fp.sub(v2R, v2L), B.idx[d], fp.mul(e2, B.iq[t2]));
+        // over mu, which the flux takes in its multiply-adds; twice the viscous
+        // work sum_a tau_{d a} v_a of the energy flux
         vise2 = __fma_rn(taud, fp.add(vdL, vdR), __fma_rn(tau1, fp.add(v1L, v1R), fp.mul(tau2, fp.add(v2L, v2R))));
 #pragma unroll
         for (int a = 0; a < 3; ++a) vis[a] = (a == d) ? taud : (a == t1) ? tau1 : tau2;
     }
     if (P.do_ns) {
         // heat conduction (compute_flux_3d.H:373-374), conductivity from (i,j,k),(i-1,j,k)
-        const double kc = (P.cond_mode == MFG_TRANSPORT_CONST)
-                              ? P.cond_hm
-                              : harmonic_mean(blend(P.cond_mode, P.cond_gas, P.cond_solid, vf[oR]),
-                                              blend(P.cond_mode, P.cond_gas, P.cond_solid, vf[oR - 1]));
+        kc = (P.cond_mode == MFG_TRANSPORT_CONST)
+                 ? P.cond_hm
+                 : harmonic_mean(blend(P.cond_mode, P.cond_gas, P.cond_solid, vf[oR]),
+                                 blend(P.cond_mode, P.cond_gas, P.cond_solid, vf[oR - 1]));
         const double* T = S.p + TEMP * S.ns;
-        therm = fp.mul(kc, fp.mul(fp.sub(T[oR], T[oL]), B.idx[d]));
+        therm = fp.mul(fp.sub(T[oR], T[oL]), B.idx[d]);
     }
     if (!HIGH && (SOLID_SIDE || P.do_ns)) {
         // AUSM+-up: the face thread holds the face states and the scheme scalars,
@@ -422,12 +427,12 @@ __device__ __forceinline__ void face_body_at(const Fp& fp, const RhsBox& B, int 
             double F = 0.0;
             if (active) {
                 F = __fma_rn(wR, uR[c], fp.mul(wL, uL[c]));
-                if (c == 1 + d) F = fp.add(F, ph);
+                if (c == 1 + d) F = __fma_rn(0.25, ph4, F);
                 if (c >= NCONS && !is_one(P.advect_flag[c - NCONS])) F = fp.mul(P.advect_flag[c - NCONS], F);
-                if (c >= RHOU && c <= RHOW) F = fp.sub(F, vis[c - 1]);
-                if (c == RHOE) F = __fma_rn(-0.5, vise2, F);
+                if (c >= RHOU && c <= RHOW) F = __fma_rn(-mu, vis[c - 1], F);
+                if (c == RHOE) F = __fma_rn(__dmul_rn(-0.5, mu), vise2, F);
             }
-            if (c == RHOE) F = fp.sub(F, therm);
+            if (c == RHOE) F = __fma_rn(-kc, therm, F);
             if (c >= NCONS) {
                 const int s = c - NCONS;
                 const double Dh = face_diffusivity(P, s, vf[oL], vf[oR]);
@@ -446,23 +451,23 @@ __device__ __forceinline__ void face_body_at(const Fp& fp, const RhsBox& B, int 
     double* q = F.p + F.off(f.i, f.j, f.k);
     q[FS_FLAGS * F.ns] = __longlong_as_double((active ? 1 : 0) | ((P.do_ns && fallback) ? 2 : 0));  // bit pattern
     q[FS_MH * F.ns] = 0.0;
-    q[FS_THERM * F.ns] = therm;
+    q[FS_THERM * F.ns] = fp.mul(kc, therm);
     if (active) {
         q[FS_LAMBDA * F.ns] = lam;
 #pragma unroll
-        for (int a = 0; a < 3; ++a) q[(FS_VIS + a) * F.ns] = vis[a];
-        q[FS_VISE * F.ns] = __dmul_rn(0.5, vise2);
+        for (int a = 0; a < 3; ++a) q[(FS_VIS + a) * F.ns] = fp.mul(mu, vis[a]);
+        q[FS_VISE * F.ns] = fp.mul(__dmul_rn(0.5, mu), vise2);
     }
 }
 
 // Face t (linear index over growHi(bx, d, 1)) of direction d.
-template <int NS, bool HIGH>
+template <int NS, bool HIGH, bool ACTIVE = false>
 __device__ __forceinline__ void face_body(const Fp& fp, const RhsBox& B, int d, int64_t t) {
     int lo[3] = {B.lo[0], B.lo[1], B.lo[2]}, len[3];
     for (int e = 0; e < 3; ++e) len[e] = B.hi[e] - B.lo[e] + 1 + (e == d);
     const int64_t nf = (int64_t)len[0] * len[1] * len[2];
     if (t >= nf) return;
-    face_body_at<NS, HIGH>(fp, B, d, delinear(t, lo, len));
+    face_body_at<NS, HIGH, false, ACTIVE>(fp, B, d, delinear(t, lo, len));
 }
 
 // ---------------------------------------------------------------------------

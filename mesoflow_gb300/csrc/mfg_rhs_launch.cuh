@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(LIST_TPB, NS <= 2 ? 5 : 4) face_list_kernel(co
     const int d = blockIdx.y;
     const unsigned w = blockIdx.x * blockDim.x + threadIdx.x;
     const Fp fp;
-    if (w < B.fcount[d]) face_body<NS, false>(fp, B, d, B.flist[face_list_off(B, d) + w]);
+    if (w < B.fcount[d]) face_body<NS, false, true>(fp, B, d, B.flist[face_list_off(B, d) + w]);
 }
 // Direction and box of the flux launches: blockIdx.z = 3 box + direction.
 template <int G>
