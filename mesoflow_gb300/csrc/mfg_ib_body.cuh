@@ -34,9 +34,9 @@ struct CutBox {
     double* tcht;  // conjugate-heat-transfer temperature average per valid cell (or null)
 };
 
-// Stored entries of the cut cells of one box.  Cut cells sit in the list in
-// decreasing order of their fluid-neighbour count, so the 32 cells of a warp
-// loop about as often; entry e of list position w lives at
+// Stored entries of the cut cells of one box.  Cut cells sit in the list by
+// bricks of the box and in decreasing order of their fluid-neighbour count, so
+// the 32 cells of a warp lie near each other and loop about as often; entry e of list position w lives at
 // base[w / 32] + 32 e + w % 32, so a warp's loads of entry e are contiguous.
 struct CutCacheView {
     const int* list;       // cell index by list position
