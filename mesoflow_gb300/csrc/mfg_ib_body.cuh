@@ -80,13 +80,6 @@ __device__ __forceinline__ void cut_geometry(const CutBox& c, int64_t o, double&
     }
 }
 
-// Inverse-distance weight of neighbour (l, m, n) about the surface point.
-__device__ __forceinline__ double surface_weight(int l, int m, int n, const double dxnd[3], const double xpn[3]) {
-    const double a = __fma_rn((double)l, dxnd[0], -xpn[0]), b = __fma_rn((double)m, dxnd[1], -xpn[1]),
-                 e = __fma_rn((double)n, dxnd[2], -xpn[2]);
-    return rcp_pos(add(__fma_rn(e, e, __fma_rn(b, b, mul(a, a))), kTiny2));
-}
-
 // 1/den of the velocity weights: den = sum wd + 1/dn^2 (the surface point),
 // zero when the cell centre lies on the surface (velocity set to zero).
 __device__ __forceinline__ double vel_iden(const CutBox& c, double dist, double swd) {
@@ -200,7 +193,7 @@ __device__ __forceinline__ void cut_parts(CutShared<NT>& sm, const double dxnd[3
         sm.part[2 * SW + q][threadIdx.x] = __fma_rn((double)(q - SG), dxnd[2], -xpn[2]);
     }
 }
-// surface_weight of neighbour (l, m, n) + 2 from the parts: the same operations.
+// Inverse-distance weight of neighbour (l, m, n) + 2 about the surface point.
 template <int NT>
 __device__ __forceinline__ double cut_weight(const CutShared<NT>& sm, int l, int m, int n) {
     const double b = sm.part[SW + m][threadIdx.x], e = sm.part[2 * SW + n][threadIdx.x];
@@ -279,32 +272,36 @@ __device__ __forceinline__ int cut_count_one(const CutBox& c, int64_t t) {
 }
 
 // Stores the entries of the cut cell at list position w (cell cc.list[w]).
+// FULL: all of them; else the weights about the surface point and the sums'
+// reciprocals alone (offsets and Dirichlet weights depend on which cells are
+// gas only).  As in cutcell_one, every lane walks its own neighbours.
+template <bool FULL, int NT>
 __device__ __forceinline__ void cut_entries_one(const CutBox& c, int w, const CutCacheView& cc, int* offp,
-                                                double* wnp, double* wdp, double* scal) {
+                                                double* wnp, double* wdp, double* scal, CutShared<NT>& sm) {
     int i, j, k;
     cell_of(c, cc.list[w], i, j, k);
     const Fab& S = c.S;
     const int64_t o = S.off(i, j, k);
-    const double* V = S.p + VFRAC * S.ns;
     double dist, xpn[3], dxnd[3];
     cut_geometry(c, o, dist, xpn, dxnd);
+    cut_parts(sm, dxnd, xpn);
     double swd = 0.0, swn = 0.0;
     int64_t ix = cc.base[w >> 5] + (w & 31);
-    for (int n = -SG; n <= SG; ++n)
-        for (int m = -SG; m <= SG; ++m)
-            for (int l = -SG; l <= SG; ++l) {
-                const int64_t q = l + m * S.js + n * S.ks;
-                if (!is_one(V[o + q])) continue;
-                const int slot = (l + SG) + SW * ((m + SG) + SW * (n + SG));
-                const bool centre = l == 0 && m == 0 && n == 0;
-                if (!centre) swd += c_wdir[slot];
-                const double wn = surface_weight(l, m, n, dxnd, xpn);
-                offp[ix] = (int)q;
-                wnp[ix] = wn;
-                wdp[ix] = centre ? 0.0 : c_wdir[slot];
-                ix += 32;
-                swn += wn;
-            }
+    CutMask nb = cut_mask(S.p + VFRAC * S.ns, o, S.js, S.ks);
+    while (nb.lo | nb.hi) {
+        const int slot = cut_next(nb);
+        int l, m, n;
+        cut_split(slot, l, m, n);
+        const double wn = cut_weight(sm, l, m, n), wd = sm.wdir[slot];
+        swd = add(swd, wd);
+        wnp[ix] = wn;
+        if (FULL) {
+            offp[ix] = (int)((l - SG) + (m - SG) * S.js + (n - SG) * S.ks);
+            wdp[ix] = wd;
+        }
+        ix += 32;
+        swn = add(swn, wn);
+    }
     scal[2 * (int64_t)w] = vel_iden(c, dist, swd);
     scal[2 * (int64_t)w + 1] = swn > 0.0 ? 1.0 / swn : 0.0;
 }
