@@ -344,85 +344,27 @@ __global__ void __launch_bounds__(BT) bk_fill_copy(const MBox* __restrict__ boxe
     TILE_END
 }
 
-// Directions in which cells lo .. hi reach beyond the domain's non-periodic
-// boundary: a box has cells for the boundary's stage n (outside in n
-// directions) only if it reaches out in n of them.
-__device__ __forceinline__ int outside_dims(const LevelG& G, const int lo[3], const int hi[3], int grow) {
-    int n = 0;
-    for (int d = 0; d < 3; ++d) n += !G.per[d] && (lo[d] - grow < G.dlo[d] || hi[d] + grow > G.dhi[d]);
-    return n;
-}
-
-// Physical boundary of one cell (i, j, k) of the array S outside the domain of
-// G in `stage` non-periodic directions (faces 1, edges 2, corners 3), from S
-// itself.
-template <int NS>
-__device__ __forceinline__ void bc_cell(const Fab& S, const LevelG& G, int i, int j, int k, int stage, int nc) {
-    const int iv[3] = {i, j, k};
-    bool out[3];
-    int nout = 0;
-    for (int d = 0; d < 3; ++d) {
-        out[d] = !G.per[d] && (iv[d] < G.dlo[d] || iv[d] > G.dhi[d]);
-        nout += out[d];
-    }
-    if (nout != stage) return;
-    const DevParams& P = c_P;
-    int dext = -1, dlast = -1;
-    for (int d = 0; d < 3; ++d) {
-        if (!out[d]) continue;
-        dlast = d;
-        const int kind = (iv[d] < G.dlo[d]) ? P.bc_lo[d] : P.bc_hi[d];
-        if (kind == MFG_BC_EXT_DIR) dext = d;
-    }
-    const int ds = (dext >= 0) ? dext : dlast;
-    const bool lo = iv[ds] < G.dlo[ds];
-    const int kind = lo ? P.bc_lo[ds] : P.bc_hi[ds];
-    int sv[3] = {i, j, k};
-    const long long qd = S.off(i, j, k);
-    if (dext >= 0) {
-        sv[ds] = lo ? G.dlo[ds] : G.dhi[ds];
-        const long long qs = S.off(sv[0], sv[1], sv[2]);
-        double s_int[NFLO + MAXS], s_ext[NFLO + MAXS];
-        for (int c = 0; c < nc; ++c) s_int[c] = S.p[qs + c * S.ns];
-        external_state<NS>(lo ? P.ext_lo[ds] : P.ext_hi[ds], ds, s_int, s_ext, nc);
-        for (int c = 0; c < nc; ++c) S.p[qd + c * S.ns] = s_ext[c];
-    } else if (kind == MFG_BC_FOEXTRAP) {
-        sv[ds] = lo ? G.dlo[ds] : G.dhi[ds];
-        const long long qs = S.off(sv[0], sv[1], sv[2]);
-        for (int c = 0; c < nc; c += 4) {  // four loads in flight
-            double x[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) x[u] = (c + u < nc) ? S.p[qs + (c + u) * S.ns] : 0.0;
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (c + u < nc) S.p[qd + (c + u) * S.ns] = x[u];
-        }
-    } else {
-        sv[ds] = lo ? (2 * G.dlo[ds] - iv[ds] - 1) : (2 * G.dhi[ds] - iv[ds] + 1);
-        const long long qs = S.off(sv[0], sv[1], sv[2]);
-        for (int c = 0; c < nc; c += 4) {
-            double x[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) x[u] = (c + u < nc) ? S.p[qs + (c + u) * S.ns] : 0.0;
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (c + u < nc) S.p[qd + (c + u) * S.ns] = odd_at_wall(c + u) ? -x[u] : x[u];
-        }
-    }
+// Whether cells lo .. hi (and grow more) reach beyond the domain's non-periodic
+// boundary.
+__device__ __forceinline__ bool reaches_out(const LevelG& G, const int lo[3], const int hi[3], int grow) {
+    bool any = false;
+    for (int d = 0; d < 3; ++d) any |= !G.per[d] && (lo[d] - grow < G.dlo[d] || hi[d] + grow > G.dhi[d]);
+    return any;
 }
 
 // Tiles of boxes that do not reach the boundary are passed over.
 template <int NS>
 __global__ void __launch_bounds__(BT) bk_fill_bc(const MBox* __restrict__ boxes, const LevelG* __restrict__ lev,
-                                                 const Tile* __restrict__ tiles, int ntiles, int stage, int nc) {
+                                                 const Tile* __restrict__ tiles, int ntiles, int nc) {
     for (int ti = blockIdx.x; ti < ntiles; ti += gridDim.x) {
         const Tile tl = tiles[ti];
         const MBox& b = boxes[tl.box];
-        if (outside_dims(lev[b.level], b.lo, b.hi, MFG_NGROW) < stage) continue;
+        const LevelG& G = lev[b.level];
+        if (!reaches_out(G, b.lo, b.hi, MFG_NGROW)) continue;
         for (long long t = tl.start + threadIdx.x; t < tl.end; t += blockDim.x) {
             int i, j, k;
             grown_of(b, t, i, j, k);
-            bc_cell<NS>(b.sb, lev[b.level], i, j, k, stage, nc);
+            bc_fill<NS>(b.sb, G.dlo, G.dhi, G.per, i, j, k, nc);
         }
     }
 }
@@ -487,15 +429,16 @@ __global__ void __launch_bounds__(BT) bk_cp_fill(const MBox* __restrict__ boxes,
 
 template <int NS>
 __global__ void __launch_bounds__(BT) bk_cp_bc(const MBox* __restrict__ boxes, const LevelG* __restrict__ lev,
-                                               const Tile* __restrict__ tiles, int ntiles, int stage, int nc) {
+                                               const Tile* __restrict__ tiles, int ntiles, int nc) {
     for (int ti = blockIdx.x; ti < ntiles; ti += gridDim.x) {
         const Tile tl = tiles[ti];
         const MBox& b = boxes[tl.box];
-        if (outside_dims(lev[b.level - 1], b.cplo, b.cphi, 0) < stage) continue;
+        const LevelG& G = lev[b.level - 1];
+        if (!reaches_out(G, b.cplo, b.cphi, 0)) continue;
         for (long long t = tl.start + threadIdx.x; t < tl.end; t += blockDim.x) {
             int i, j, k;
             cp_of(b, t, i, j, k);
-            bc_cell<NS>(b.cp, lev[b.level - 1], i, j, k, stage, nc);
+            bc_fill<NS>(b.cp, G.dlo, G.dhi, G.per, i, j, k, nc);
         }
     }
 }
@@ -1122,10 +1065,8 @@ void b_fill(mfg_boxlist& L, const PhaseTiles& T, int src, cudaStream_t st, int i
         ProfScope ps(K_FILL_COPY, st);
         bk_fill_copy<<<T.grid, BT, 0, st>>>(L.d_mbox, L.d_lev, L.d_owner, T.d, T.n, src, nc, interp);
     }
-    for (int s = 1; s <= 3; ++s) {
-        ProfScope ps(K_FILL_BC, st);
-        NS_DISPATCH(bk_fill_bc, (T.grid, BT, 0, st), (L.d_mbox, L.d_lev, T.d, T.n, s, nc));
-    }
+    ProfScope ps(K_FILL_BC, st);
+    NS_DISPATCH(bk_fill_bc, (T.grid, BT, 0, st), (L.d_mbox, L.d_lev, T.d, T.n, nc));
 }
 
 void b_cutcells(mfg_boxlist& L, const PhaseTiles& T, cudaStream_t st) {
@@ -1505,9 +1446,9 @@ void amr_fill(mfg_boxlist& L, AmrRun& R, int l, int src, int ev) {
             ProfScope ps(K_AMR_PATCH, st);
             bk_cp_fill<<<C.grid, BT, 0, st>>>(L.d_mbox, L.d_lev, L.d_owner, C.d, C.n, L.d_coef, ev, nc);
         }
-        for (int s = 1; s <= 3; ++s) {
+        {
             ProfScope ps(K_AMR_PATCH, st);
-            NS_DISPATCH(bk_cp_bc, (C.grid, BT, 0, st), (L.d_mbox, L.d_lev, C.d, C.n, s, nc));
+            NS_DISPATCH(bk_cp_bc, (C.grid, BT, 0, st), (L.d_mbox, L.d_lev, C.d, C.n, nc));
         }
         const int ni = L.nient[l];
         ProfScope ps(K_AMR_INTERP, st);

@@ -1,12 +1,12 @@
 // Single-level ghost fill of every box's Sborder (FillPatchSingleLevel with
 // the case's physical boundary functor): copy of valid data from the owning
-// box (periodic images included), then the physical boundaries in the order
-// faces -> edges -> corners.  A cell outside the domain in the set D of
+// box (periodic images included), then the physical boundaries with the result
+// of filling faces, then edges, then corners.  A cell outside the domain in the set D of
 // non-periodic directions takes its value from the cell one step inward
 // along d*: the highest direction of D whose boundary is ext_dir (the user
 // functor runs after the extrapolation rules and checks x, y, z in turn,
 // Source/mflo_bcfill.H:236-320), otherwise the highest direction of D.
-// The physical-boundary launches cover only the blocks ("slabs") of the
+// The physical-boundary launch covers only the blocks ("slabs") of the
 // grown boxes that lie outside the domain, listed once per box layout, not
 // every grown cell of every box.
 #include <algorithm>
@@ -34,7 +34,7 @@ struct FillGeom {
 };
 
 // A block of a box's grown region outside the domain: its cells leave the
-// domain through the same directions (the bc_kernel stage = their number).
+// domain through the same directions.
 struct BcSlab {
     int box;
     int lo[3], len[3];
@@ -76,62 +76,16 @@ __global__ void copy_kernel(const FillBox* __restrict__ boxes, FillGeom G, const
     copy_comps(b.sb.p + b.sb.off(i, j, k), b.sb.ns, o.src.p + o.src.off(w[0], w[1], w[2]), o.src.ns, ncomp);
 }
 
-// One launch per stage over the slabs of that stage only (blockIdx.y = slab).
+// Every slab in one launch (blockIdx.y = slab).
+constexpr int BC_TPB = 128;
 template <int NS>
-__global__ void bc_kernel(const FillBox* __restrict__ boxes, const BcSlab* __restrict__ slabs, FillGeom G, int stage,
-                          int ncomp) {
+__global__ void __launch_bounds__(BC_TPB) bc_kernel(const FillBox* __restrict__ boxes, const BcSlab* __restrict__ slabs, FillGeom G, int ncomp) {
     const BcSlab& sl = slabs[blockIdx.y];
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (int64_t)sl.len[0] * sl.len[1] * sl.len[2]) return;
-    const FillBox& b = boxes[sl.box];
     int i, j, k;
     split3(t, sl.len[0], sl.len[1], i, j, k);
-    i += sl.lo[0];
-    j += sl.lo[1];
-    k += sl.lo[2];
-    const int iv[3] = {i, j, k};
-    bool out[3];
-    int nout = 0;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        out[d] = !G.per[d] && (iv[d] < G.dlo[d] || iv[d] > G.dhi[d]);
-        nout += out[d];
-    }
-    if (nout != stage) return;
-    const DevParams& P = c_P;
-    int dext = -1, dlast = -1;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        if (!out[d]) continue;
-        dlast = d;
-        const int kind = (iv[d] < G.dlo[d]) ? P.bc_lo[d] : P.bc_hi[d];
-        if (kind == MFG_BC_EXT_DIR) dext = d;
-    }
-    const int ds = (dext >= 0) ? dext : dlast;
-    const bool lo = iv[ds] < G.dlo[ds];
-    const int kind = lo ? P.bc_lo[ds] : P.bc_hi[ds];
-    int sv[3] = {i, j, k};
-    const Fab& S = b.sb;
-    const int64_t qd = S.off(i, j, k);
-    if (dext >= 0) {
-        sv[ds] = lo ? G.dlo[ds] : G.dhi[ds];
-        const int64_t qs = S.off(sv[0], sv[1], sv[2]);
-        double s_int[NFLO + MAXS], s_ext[NFLO + MAXS];
-        for (int c = 0; c < ncomp; ++c) s_int[c] = S.p[qs + c * S.ns];
-        external_state<NS>(lo ? P.ext_lo[ds] : P.ext_hi[ds], ds, s_int, s_ext, ncomp);
-        for (int c = 0; c < ncomp; ++c) S.p[qd + c * S.ns] = s_ext[c];
-    } else if (kind == MFG_BC_FOEXTRAP) {
-        sv[ds] = lo ? G.dlo[ds] : G.dhi[ds];
-        const int64_t qs = S.off(sv[0], sv[1], sv[2]);
-        for (int c = 0; c < ncomp; ++c) S.p[qd + c * S.ns] = S.p[qs + c * S.ns];
-    } else {  // wall: reflect_even, reflect_odd for momenta and velocities
-        sv[ds] = lo ? (2 * G.dlo[ds] - iv[ds] - 1) : (2 * G.dhi[ds] - iv[ds] + 1);
-        const int64_t qs = S.off(sv[0], sv[1], sv[2]);
-        for (int c = 0; c < ncomp; ++c) {
-            const double x = S.p[qs + c * S.ns];
-            S.p[qd + c * S.ns] = odd_at_wall(c) ? -x : x;
-        }
-    }
+    bc_fill<NS>(boxes[sl.box].sb, G.dlo, G.dhi, G.per, i + sl.lo[0], j + sl.lo[1], k + sl.lo[2], ncomp);
 }
 
 // Owner map cache (host-built, device-resident); rebuilt when the box layout changes.
@@ -143,10 +97,10 @@ struct OwnerCache {
     FillBox* d_boxes = nullptr;
     size_t bcap = 0;
     std::vector<char> table;
-    BcSlab* d_slabs = nullptr;  // grouped by stage 1, 2, 3
+    BcSlab* d_slabs = nullptr;
     size_t scap = 0;
-    int nslab[3] = {0, 0, 0}, soff[3] = {0, 0, 0};
-    int64_t smax[3] = {0, 0, 0};  // largest slab of each stage (cells)
+    int nslab = 0;
+    int64_t smax = 0;  // largest slab (cells)
 } g_fill;
 
 int igcd(int a, int b) {
@@ -208,8 +162,9 @@ cudaError_t ensure_owner(const mfg_box* boxes, int nbox, const mfg_geom& g) {
         return e;
     // Slabs: per direction the grown extent splits into below / inside /
     // above the domain (one range when periodic); every combination with at
-    // least one outside range is a slab of the stage = number of those.
-    std::vector<BcSlab> sl[3];
+    // least one outside range is a slab.
+    std::vector<BcSlab> all;
+    g_fill.smax = 0;
     for (int b = 0; b < nbox; ++b) {
         int rlo[3][3], rhi[3][3], rout[3][3], nr[3];
         for (int d = 0; d < 3; ++d) {
@@ -243,17 +198,12 @@ cudaError_t ensure_owner(const mfg_box* boxes, int nbox, const mfg_geom& g) {
                         x.lo[d] = rlo[d][r[d]];
                         x.len[d] = rhi[d][r[d]] - rlo[d][r[d]] + 1;
                     }
-                    if (nout) sl[nout - 1].push_back(x);
+                    if (!nout) continue;
+                    all.push_back(x);
+                    g_fill.smax = std::max<int64_t>(g_fill.smax, (int64_t)x.len[0] * x.len[1] * x.len[2]);
                 }
     }
-    std::vector<BcSlab> all;
-    for (int q = 0; q < 3; ++q) {
-        g_fill.soff[q] = (int)all.size();
-        g_fill.nslab[q] = (int)sl[q].size();
-        g_fill.smax[q] = 0;
-        for (const BcSlab& x : sl[q]) g_fill.smax[q] = std::max<int64_t>(g_fill.smax[q], (int64_t)x.len[0] * x.len[1] * x.len[2]);
-        all.insert(all.end(), sl[q].begin(), sl[q].end());
-    }
+    g_fill.nslab = (int)all.size();
     if (all.size() > g_fill.scap) {
         if (g_fill.d_slabs) cudaFree(g_fill.d_slabs);
         g_fill.d_slabs = nullptr;
@@ -331,19 +281,16 @@ cudaError_t launch_fill_patch(const mfg_box* boxes, int nbox, const mfg_geom& g,
         copy_kernel<<<grid, TPB, 0, st>>>(tab, G, g_fill.d_owner, nc);
     }
     const int ns = c_host_params().nspec;
-    for (int s = 1; s <= 3; ++s) {
-        // faces, then edges, then corners; at most 65535 slabs per launch
-        for (int s0 = 0; s0 < g_fill.nslab[s - 1]; s0 += 65535) {
-            const int cnt = std::min(65535, g_fill.nslab[s - 1] - s0);
-            const BcSlab* sl = g_fill.d_slabs + g_fill.soff[s - 1] + s0;
-            dim3 gb((unsigned)((g_fill.smax[s - 1] + TPB - 1) / TPB), (unsigned)cnt);
-            ProfScope ps(K_FILL_BC, st);
-            if (ns <= 1) bc_kernel<1><<<gb, TPB, 0, st>>>(tab, sl, G, s, nc);
-            else if (ns <= 2) bc_kernel<2><<<gb, TPB, 0, st>>>(tab, sl, G, s, nc);
-            else if (ns <= 4) bc_kernel<4><<<gb, TPB, 0, st>>>(tab, sl, G, s, nc);
-            else if (ns <= 8) bc_kernel<8><<<gb, TPB, 0, st>>>(tab, sl, G, s, nc);
-            else bc_kernel<16><<<gb, TPB, 0, st>>>(tab, sl, G, s, nc);
-        }
+    for (int s0 = 0; s0 < g_fill.nslab; s0 += 65535) {  // at most 65535 slabs per launch
+        const int cnt = std::min(65535, g_fill.nslab - s0);
+        const BcSlab* sl = g_fill.d_slabs + s0;
+        const dim3 gb((unsigned)((g_fill.smax + BC_TPB - 1) / BC_TPB), (unsigned)cnt);
+        ProfScope ps(K_FILL_BC, st);
+        if (ns <= 1) bc_kernel<1><<<gb, BC_TPB, 0, st>>>(tab, sl, G, nc);
+        else if (ns <= 2) bc_kernel<2><<<gb, BC_TPB, 0, st>>>(tab, sl, G, nc);
+        else if (ns <= 4) bc_kernel<4><<<gb, BC_TPB, 0, st>>>(tab, sl, G, nc);
+        else if (ns <= 8) bc_kernel<8><<<gb, BC_TPB, 0, st>>>(tab, sl, G, nc);
+        else bc_kernel<16><<<gb, BC_TPB, 0, st>>>(tab, sl, G, nc);
     }
     return cudaGetLastError();
 }
