@@ -224,23 +224,24 @@ __global__ void cut_level_vf_kernel(const LevelCutBox* __restrict__ tab) {
     vf_compare(in, v, L.vf + t, L.dirty);
 }
 
-// cut_refresh_kernel for every box of the level (blockIdx.y).
-__global__ void __launch_bounds__(TPB) cut_level_refresh_kernel(const LevelCutBox* __restrict__ tab) {
+// What a box's change asks for (blockIdx.y = box), in one launch: the weights
+// refreshed as cut_refresh_kernel does, or, where its entry is out of use, its
+// cut cells listed afresh (grid-stride over the box; one atomic per warp).
+__global__ void __launch_bounds__(TPB) cut_level_change_kernel(const LevelCutBox* __restrict__ tab,
+                                                               unsigned* __restrict__ cnt, int* __restrict__ lists,
+                                                               int64_t cap) {
     const LevelCutBox& L = tab[blockIdx.y];
-    if (*L.dirty != VF_MOVED || blockIdx.x * TPB >= L.ncut) return;
-    __shared__ CutShared<TPB> sm;
-    cut_shared_init(sm);
-    for (unsigned w = blockIdx.x * TPB + threadIdx.x; w < L.ncut; w += gridDim.x * TPB)
-        cut_entries_one<false>(L.c, (int)w, L.v, nullptr, const_cast<double*>(L.v.wn), nullptr,
-                               const_cast<double*>(L.v.scal), sm);
-}
-
-// For a box whose entry is out of use: its cut cells listed afresh
-// (grid-stride over the box; one atomic per warp).
-__global__ void cut_level_list_kernel(const LevelCutBox* __restrict__ tab, unsigned* __restrict__ cnt,
-                                      int* __restrict__ lists, int64_t cap) {
-    const LevelCutBox& L = tab[blockIdx.y];
-    if (!(*L.dirty & VF_OTHER)) return;
+    const unsigned flag = *L.dirty;
+    if (!flag) return;
+    if (flag == VF_MOVED) {
+        if (blockIdx.x * TPB >= L.ncut) return;
+        __shared__ CutShared<TPB> sm;
+        cut_shared_init(sm);
+        for (unsigned w = blockIdx.x * TPB + threadIdx.x; w < L.ncut; w += gridDim.x * TPB)
+            cut_entries_one<false>(L.c, (int)w, L.v, nullptr, const_cast<double*>(L.v.wn), nullptr,
+                                   const_cast<double*>(L.v.scal), sm);
+        return;
+    }
     const CutBox& c = L.c;
     int* list = lists + (int64_t)blockIdx.y * cap;
     for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < c.n; base += (int64_t)gridDim.x * blockDim.x) {
@@ -658,16 +659,16 @@ int launch_cutcells_level(const mfg_box* boxes, int nbox, const mfg_geom& g, cud
         return 0;
     }
     const int ns = c_host_params().nspec;
-    ProfScope ps(K_CUT, st, 5 + (nbox + CUT_GROUP - 1) / CUT_GROUP);
+    ProfScope ps(K_CUT, st, 3 + (T->ngroups > 0) + (nbox + CUT_GROUP - 1) / CUT_GROUP);
     cut_level_reset_kernel<<<(nbox + 127) / 128, 128, 0, st>>>(T->d_tab, nbox, g_level.d_cnt);
     cut_level_vf_kernel<<<dim3((unsigned)((T->maxgrown + 255) / 256), (unsigned)nbox), 256, 0, st>>>(T->d_tab);
     const unsigned per = (unsigned)std::max<int64_t>(1, std::min<int64_t>((T->cap + TPB - 1) / TPB, 152));
-    cut_level_refresh_kernel<<<dim3(per, (unsigned)nbox), TPB, 0, st>>>(T->d_tab);
-    cut_level_list_kernel<<<dim3(8, (unsigned)nbox), TPB, 0, st>>>(T->d_tab, g_level.d_cnt, g_level.d_lists, T->cap);
-    const unsigned nb = std::max(1u, (unsigned)(((uint64_t)T->ngroups * 32 + TPB - 1) / TPB));
+    cut_level_change_kernel<<<dim3(per, (unsigned)nbox), TPB, 0, st>>>(T->d_tab, g_level.d_cnt, g_level.d_lists,
+                                                                        T->cap);
+    const unsigned nb = (unsigned)(((uint64_t)T->ngroups * 32 + TPB - 1) / TPB);
 #define MFG_LEVEL_LAUNCH(K)                                                                                 \
     do {                                                                                                    \
-        cutcell_level_kernel<K><<<nb, TPB, 0, st>>>(T->d_tab, T->d_groups, T->ngroups);                   \
+        if (nb) cutcell_level_kernel<K><<<nb, TPB, 0, st>>>(T->d_tab, T->d_groups, T->ngroups);             \
         for (int b = 0; b < nbox; b += CUT_GROUP) {                                                         \
             const int n = std::min(CUT_GROUP, nbox - b);                                                    \
             CutGroup cg;                                                                                    \
