@@ -705,14 +705,8 @@ __global__ void __launch_bounds__(BT) bk_timestep(const MBox* __restrict__ boxes
             ws = fmax(ws, w1);
             md = fmax(md, m1);
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            ws = fmax(ws, __shfl_down_sync(0xffffffffu, ws, o));
-            md = fmax(md, __shfl_down_sync(0xffffffffu, md, o));
-        }
-        if ((threadIdx.x & 31) == 0) {
-            atomic_max_nonneg(&R->acc[2 * b.level], ws);
-            atomic_max_nonneg(&R->acc[2 * b.level + 1], md);
-        }
+        warp_max_nonneg(&R->acc[2 * b.level], ws);
+        warp_max_nonneg(&R->acc[2 * b.level + 1], md);
     }
 }
 

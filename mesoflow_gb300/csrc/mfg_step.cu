@@ -175,14 +175,8 @@ __global__ void timestep_kernel(const __grid_constant__ StepGroup g, double* acc
         cell_of(v, t, i, j, k);
         timestep_cell<NS>(g.s[blockIdx.y], i, j, k, ws, md);
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        ws = fmax(ws, __shfl_down_sync(0xffffffffu, ws, o));
-        md = fmax(md, __shfl_down_sync(0xffffffffu, md, o));
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomic_max_nonneg(acc2, ws);
-        atomic_max_nonneg(acc2 + 1, md);
-    }
+    warp_max_nonneg(acc2, ws);
+    warp_max_nonneg(acc2 + 1, md);
 }
 
 // Contiguous copies of several arrays in one launch (blockIdx.y = array), four

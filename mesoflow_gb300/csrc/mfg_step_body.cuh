@@ -465,9 +465,20 @@ __device__ __forceinline__ void prims_body(const Valid& v, const Fab& S, int64_t
         if ((wrote >> n) & 1u) S(i, j, k, n) = u[n];
 }
 
-__device__ __forceinline__ void atomic_max_nonneg(double* a, double v) {
+// The warp's largest v (>= +0, or NaN, which counts only when every lane has
+// one, as with fmax) into *a.  Integer reductions, since a comparison of doubles
+// is an instruction of the FP64 pipe; and *a only grows, so a warp that is not
+// above what it reads there has nothing to add: one atomic per warp on one
+// address bound the pass (256^3 sphere-pack step: 1.55 -> 1.23 ms).
+__device__ __forceinline__ void warp_max_nonneg(double* a, double v) {
+    const unsigned all = 0xffffffffu;
+    const bool nan = is_nan(v);
+    const unsigned hi = nan ? 0u : (unsigned)__double2hiint(v), lo = nan ? 0u : (unsigned)__double2loint(v);
+    const unsigned mh = __reduce_max_sync(all, hi), ml = __reduce_max_sync(all, hi == mh ? lo : 0u);
+    const unsigned long long m = __all_sync(all, nan) ? 0x7fffffffffffffffull : ((unsigned long long)mh << 32) | ml;
+    unsigned long long* p = reinterpret_cast<unsigned long long*>(a);
     // IEEE order of non-negative doubles equals the order of their bit patterns
-    atomicMax(reinterpret_cast<unsigned long long*>(a), (unsigned long long)__double_as_longlong(v));
+    if ((threadIdx.x & 31) == 0 && m > *reinterpret_cast<volatile unsigned long long*>(p)) atomicMax(p, m);
 }
 
 // One cell's wave speed |u| + do_ns c and largest species diffusivity
