@@ -412,16 +412,12 @@ struct AdjCtr {
     bool ready;
 };
 
-// Adjoint of the first-order fallback flux (fsum - lam D W)/2, W = (X + 2Y -
-// Z)/(X + 6Y + 3Z) as in weno_llf_collapsed: W and d(D W)/dD.
+// Adjoint of the first-order fallback flux (fsum - lam D W)/2 (weno_collapsed):
+// W and d(D W)/dD.
 __device__ __forceinline__ void collapsed_weight(double D, double& W, double& dDW) {
-    const double y = D * D, sC = fma(16.0 / 3.0, y, 4.0 * kEpsWeno), sA = fma(8.0, y, sC);
-    const double dB = (4.0 * kEpsWeno) * (4.0 * kEpsWeno), dC = sC * sC, dA = sA * sA;
-    const double cb = (2.0 * 16.0 / 3.0) * sC, ab = (2.0 * 40.0 / 3.0) * sA;  // d/dy of C and A
-    const double X = dC * dA, Y = dB * dA, Z = dB * dC, Xb = cb * dA + dC * ab, Yb = dB * ab, Zb = dB * cb;
-    const double r = 1.0 / (X + 6.0 * Y + 3.0 * Z);
-    W = (X + 2.0 * Y - Z) * r;
-    dDW = W + (2.0 * y) * (((Xb + 2.0 * Yb - Zb) - W * (Xb + 6.0 * Yb + 3.0 * Zb)) * r);
+    const WenoCollapsed c = weno_collapsed(weno_diff((uint64_t)__double_as_longlong(D)));
+    W = weight_of(weight_bits(c.W, 0));
+    dDW = __fma_rn(-4.0, weight_of(weno_collapsed_slope(c)), W);
 }
 
 // Adjoint of one cell's value: fb of its Euler flux (h = 0) or of its state.

@@ -772,20 +772,11 @@ __device__ __forceinline__ double weno_pair(const Fp& fp, double sumL, int64_t q
     return __fma_rn(-far, gR, __fma_rn(m, g, fp.add(sumL, tR)));
 }
 
-// First-order stencil near the immersed boundary (compute_flux_3d.H:233-249):
-// the six cells collapse to (L, L, L, R, R, R).  Of the second differences
-// only t_{f-1} = D and t_f = -D with D = R - L remain, both edges have the
-// same weight products, the corrections of the Euler flux cancel and those of
-// the state add up: flux = (f_L + f_R)/2 - lam D (X + 2Y - Z) / (2 (X + 6Y + 3Z));
-// returned: twice that.
-__device__ __forceinline__ double weno_llf_collapsed(double lam, double fsum, double D) {
-    const double D2 = __dmul_rn(D, D);
-    const double sC = __fma_rn(16.0 / 3.0, D2, 4.0 * kEpsWeno), sA = __fma_rn(8.0, D2, sC);
-    const double dB = (4.0 * kEpsWeno) * (4.0 * kEpsWeno), dC = __dmul_rn(sC, sC), dA = __dmul_rn(sA, sA);
-    const double X = __dmul_rn(dC, dA), Y = __dmul_rn(dB, dA), Z = __dmul_rn(dB, dC);
-    const double p = __fma_rn(2.0, Y, X), q = __fma_rn(2.0, Y, Z);
-    const double w = quot_pos(__dsub_rn(p, Z), __fma_rn(3.0, q, X));
-    return __fma_rn(-__dmul_rn(lam, D), w, fsum);
+// Twice the flux of a first-order face near the immersed boundary
+// (compute_flux_3d.H:233-249), weno_collapsed.
+__device__ __forceinline__ double weno_llf_collapsed(const Fp& fp, double lam, double fsum, double D) {
+    const double W = weight_of(weight_bits(weno_collapsed(weno_diff((uint64_t)__double_as_longlong(D))).W, 0));
+    return __fma_rn(-fp.mul(lam, D), W, fsum);
 }
 
 // Complete flux of one face (the sweep and the per-face form share it, so
@@ -863,7 +854,7 @@ __device__ __forceinline__ void flux5_face_body(const Fp& fp, const RhsBox& B, i
         flux5_cell(fp, x, oR - sd, xR - xd, uL, fL);
         flux5_cell(fp, x, oR, xR, uR, fR);
         D = fp.sub(uR, uL);
-        fh = weno_llf_collapsed(x.fs[qf + FS_LAMBDA * x.fns], fp.add(fL, fR), D);
+        fh = weno_llf_collapsed(fp, x.fs[qf + FS_LAMBDA * x.fns], fp.add(fL, fR), D);
     } else {
         D = fp.sub(x.u[oR], x.u[oR - sd]);
     }
@@ -1030,7 +1021,7 @@ __device__ __forceinline__ void flux5_sweep_body(const Fp& fp, const RhsBox& B, 
         } else {
             primed = false;
         }
-        if (flags == 3) fh = weno_llf_collapsed(x.fs[qf + FS_LAMBDA * x.fns], fp.add(fL, f.v0), Du);
+        if (flags == 3) fh = weno_llf_collapsed(fp, x.fs[qf + FS_LAMBDA * x.fns], fp.add(fL, f.v0), Du);
         flux5_finish(fp, x, flags & 1, fh, Du, oR - sd, oR, qf, qf, qr);
         if (fc == f1) break;
         // advance one face

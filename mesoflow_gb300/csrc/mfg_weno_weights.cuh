@@ -142,4 +142,45 @@ MFG_HD WenoWeights weno_weights(uint64_t dB, int eB, uint64_t dC, int eC, uint64
     return w;
 }
 
+// Weight of the first-order stencil (L, L, L, R, R, R) near the immersed
+// boundary.  Its second differences are D and -D with D = R - L, both edges have
+// the weight products X = c^2 b^2, Y = a^2 b^2, Z = a^2 c^2 of a = 3 eps, c = a +
+// 4 D^2, b = a + 10 D^2, and the flux is (f_L + f_R)/2 - lam D W/2 with
+//   W = (X + 2 Y - Z)/(X + 6 Y + 3 Z) = (1 + 2 u^2 - v^2)/(1 + 6 u^2 + 3 v^2),
+// u = a/c, v = a/b, in [1/5, 1]: three reciprocals and eight products of the
+// integer pipe, 2^-55 accurate, where the FP64 form took 25 operations beside the
+// 19 of a regular face, in most warps near a boundary: fluxes of the 64^3
+// catalyst step 3.65 -> 2.77 ms.
+struct WenoCollapsed {
+    uint64_t U, V;     // u, v: 2^62
+    uint64_t den, rd;  // the denominator normalised (top bit 63), 2^126 over it
+    int zd;            // its shift from units of 2^60
+    uint64_t W;        // 2^62
+};
+MFG_HD WenoCollapsed weno_collapsed(const WenoDiff& d) {
+    const int E = imax(d.e, kWenoExpFloor);
+    const uint64_t m = d.m >> imin(E - d.e, 63), e2 = umulhi64(m, m), a = kWenoEps3 >> imin(2 * (E - kWenoExpFloor), 63);
+    const uint64_t c = 4 * e2 + a, b = 10 * e2 + a;  // at least 2^57
+    const int zc = clz32((uint32_t)(c >> 32)), zb = clz32((uint32_t)(b >> 32));
+    WenoCollapsed r;
+    r.U = umulhi64(a << zc, rcp_fixed(c << zc));
+    r.V = umulhi64(a << zb, rcp_fixed(b << zb));
+    const uint64_t one = 1ull << 60, u2 = umulhi64(r.U, r.U), v2 = umulhi64(r.V, r.V);
+    const uint64_t num = one + 2 * u2 - v2, den = one + 6 * u2 + 3 * v2;  // den <= 10 2^60, num <= den
+    r.zd = clz32((uint32_t)(den >> 32));
+    r.den = den << r.zd;
+    r.rd = rcp_fixed(r.den);
+    r.W = umulhi64(num << r.zd, r.rd);
+    return r;
+}
+// D dW/dD = -4 ((2 A - B) - W (6 A + 3 B))/den with A = u^2 (1 - u), B = v^2 (1 -
+// v): the quotient without the factor, as double bits.
+MFG_HD uint64_t weno_collapsed_slope(const WenoCollapsed& r) {
+    const uint64_t one = 1ull << 62;
+    const uint64_t A = umulhi64(umulhi64(r.U, r.U) << 2, one - r.U), B = umulhi64(umulhi64(r.V, r.V) << 2, one - r.V);  // 2^60
+    const int64_t q = (int64_t)(2 * A) - (int64_t)B - (int64_t)(umulhi64(r.W, 6 * A + 3 * B) << 2);
+    const uint64_t neg = (uint64_t)q >> 63;
+    return weight_bits(umulhi64((neg ? 0 - (uint64_t)q : (uint64_t)q) << r.zd, r.rd), 0) | (neg << 63);
+}
+
 }  // namespace mfg

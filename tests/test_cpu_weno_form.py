@@ -45,6 +45,14 @@ extern "C" void weights(const double* d, double* w, int n) {
         w[4 * i + 3] = val(r.nearR);
     }
 }
+// weight W of the first-order stencil with the jump d, and D dW/dD over -4
+extern "C" void collapsed(const double* d, double* w, double* q, int n) {
+    for (int i = 0; i < n; ++i) {
+        const WenoCollapsed c = weno_collapsed(weno_diff(bits(d[i])));
+        w[i] = val(weight_bits(c.W, 0));
+        q[i] = val(weno_collapsed_slope(c));
+    }
+}
 // d: 5 differences per face; w: far weight of its left edge (twice), the near weights' sum less one and
 // difference, far weight of its right edge (twice)
 extern "C" void pairs(const double* d, double* w, int n) {
@@ -117,12 +125,17 @@ def kernel_form(lib, f, u, lam):
     return 0.5 * ((f[2] + f[3]) - (c + lam * d) / 6)
 
 
-def collapsed_form(f, u, lam):
+def collapsed_weight(lib, d):
+    d = np.ascontiguousarray(d)
+    w, q = np.empty_like(d), np.empty_like(d)
+    p = [x.ctypes.data_as(C.c_void_p) for x in (d, w, q)]
+    lib.collapsed(p[0], p[1], p[2], C.c_int(d.size))
+    return w, q
+
+
+def collapsed_form(lib, f, u, lam):
     d = u[3] - u[2]
-    sc = 16.0 / 3.0 * d * d + 4e-6
-    sa = 8.0 * d * d + sc
-    x, y, z = sc * sc * (sa * sa), 4e-6 ** 2 * (sa * sa), 4e-6 ** 2 * (sc * sc)
-    return 0.5 * ((f[2] + f[3]) - lam * d * ((x + 2 * y - z) / (x + 6 * y + 3 * z)))
+    return 0.5 * ((f[2] + f[3]) - lam * d * collapsed_weight(lib, d)[0])
 
 
 def stencils(kind, rng):
@@ -168,7 +181,7 @@ def test_flux_form(lib, kind):
     s = np.abs(f).max(0) + lam * np.abs(u).max(0)
     assert np.all(np.abs(kernel_form(lib, f, u, lam) - ref) <= 20 * EPS * s)
     if kind == "collapsed":
-        assert np.all(np.abs(collapsed_form(f, u, lam) - ref) <= 20 * EPS * s)
+        assert np.all(np.abs(collapsed_form(lib, f, u, lam) - ref) <= 20 * EPS * s)
 
 
 def test_weights_follow_infinite_and_nan_differences(lib):
@@ -177,3 +190,21 @@ def test_weights_follow_infinite_and_nan_differences(lib):
     bad = np.array([[np.nan, 1.0, 2.0, 3.0], [1.0, np.inf, 2.0, 3.0], [0.0, 0.0, -np.inf, 1e308]])
     w = fixed_weights(lib, list(bad.T))
     assert np.all(np.isfinite(w))
+
+
+def test_collapsed_weight(lib):
+    """W and d(D W)/dD: u and v carry 2^-57 (a reciprocal of 59 bits, a product
+    and the truncated indicators), their squares and the sums at most eight times
+    that, the last reciprocal 2^-59 and the truncated double 2^-52: 2^-51 in all."""
+    rng = np.random.default_rng(5)
+    d = np.concatenate([10.0 ** rng.uniform(-12, 12, N), 10.0 ** rng.uniform(-5, -1, N), [0.0, -0.0, 1e300, -1e-300]])
+    d *= rng.choice([-1.0, 1.0], d.size)
+    w, q = collapsed_weight(lib, d)
+    y, a = L(d) * L(d), L(3e-6)
+    u, v = a / (a + 4 * y), a / (a + 10 * y)
+    den = 1 + 6 * u * u + 3 * v * v
+    W = (1 + 2 * u * u - v * v) / den
+    A, B = u * u * (1 - u), v * v * (1 - v)
+    slope = W - 4 * ((2 * A - B) - W * (6 * A + 3 * B)) / den
+    assert np.all(np.abs(L(w) - W) <= 2.0 ** -51 * W)
+    assert np.all(np.abs((L(w) - 4 * L(q)) - slope) <= 2.0 ** -49)
