@@ -29,6 +29,25 @@ MFG_HD uint64_t umulhi64(uint64_t a, uint64_t b) {
 #endif
 }
 
+// High half of a product and of a square without the low partial product, whose
+// place a constant takes: within 1 and 1.5 units of the exact value (the exact
+// high half is within 1), in three and two 32-bit products instead of four.
+MFG_HD uint32_t umulhi32(uint32_t a, uint32_t b) {
+#ifdef __CUDA_ARCH__
+    return __umulhi(a, b);
+#else
+    return (uint32_t)(((uint64_t)a * b) >> 32);
+#endif
+}
+MFG_HD uint64_t mulhi_near(uint64_t a, uint64_t b) {
+    const uint32_t ah = (uint32_t)(a >> 32), al = (uint32_t)a, bh = (uint32_t)(b >> 32), bl = (uint32_t)b;
+    return (uint64_t)ah * bh + ((uint64_t)umulhi32(ah, bl) + umulhi32(al, bh) + 1u);
+}
+MFG_HD uint64_t sqhi_near(uint64_t a) {
+    const uint32_t ah = (uint32_t)(a >> 32), al = (uint32_t)a;
+    return (uint64_t)ah * ah + (2 * (uint64_t)umulhi32(ah, al) + 1u);
+}
+
 MFG_HD int clz32(uint32_t x) {  // x != 0
 #ifdef __CUDA_ARCH__
     return __clz((int)x);

@@ -67,8 +67,8 @@ template <bool RCP>
 MFG_HD WenoIndR weno_ind_full(const WenoDiff& a, const WenoDiff& b) {
     const int E = imax(imax(a.e, b.e), kWenoExpFloor);
     const uint64_t ma = a.m >> imin(E - a.e, 63), mb = b.m >> imin(E - b.e, 63);
-    const uint64_t E1 = umulhi64(ma, ma), E2 = umulhi64(mb, mb);
-    uint64_t X = umulhi64(ma, mb);
+    const uint64_t E1 = sqhi_near(ma), E2 = sqhi_near(mb);
+    uint64_t X = mulhi_near(ma, mb);
     if ((a.sign ^ b.sign) >> 31) X = 0 - X;
     const uint64_t sC = ((E1 + E2) << 2) - 5 * X + (kWenoEps3 >> imin(2 * (E - kWenoExpFloor), 63));
     const uint64_t sA = sC + 6 * (E1 - X), sB = sC + 6 * (E2 - X);
@@ -76,9 +76,9 @@ MFG_HD WenoIndR weno_ind_full(const WenoDiff& a, const WenoDiff& b) {
     const int zA = clz32((uint32_t)(sA >> 32)), zB = clz32((uint32_t)(sB >> 32)), zC = clz32((uint32_t)(sC >> 32));
     const uint64_t nA = sA << zA, nB = sB << zB, nC = sC << zC;
     WenoIndR r;
-    r.dA = umulhi64(nA, nA);
-    r.dB = umulhi64(nB, nB);
-    r.dC = umulhi64(nC, nC);
+    r.dA = sqhi_near(nA);
+    r.dB = sqhi_near(nB);
+    r.dC = sqhi_near(nC);
     r.eA = 2 * E - zA;
     r.eB = 2 * E - zB;
     r.eC = 2 * E - zC;
@@ -125,19 +125,19 @@ struct WenoWeights {
 MFG_HD WenoWeights weno_weights(uint64_t dB, int eB, uint64_t dC, int eC, uint64_t dA, int eA) {
     const int em = imin(imin(eA, eB), eC);
     // common exponent of the three products; four bits of headroom for the sums
-    const uint64_t X = umulhi64(dC, dA) >> imin(2 * (eB - em) + 4, 63);
-    const uint64_t Y = umulhi64(dB, dA) >> imin(2 * (eC - em) + 4, 63);
-    const uint64_t Z = umulhi64(dB, dC) >> imin(2 * (eA - em) + 4, 63);
+    const uint64_t X = mulhi_near(dC, dA) >> imin(2 * (eB - em) + 4, 63);
+    const uint64_t Y = mulhi_near(dB, dA) >> imin(2 * (eC - em) + 4, 63);
+    const uint64_t Z = mulhi_near(dB, dC) >> imin(2 * (eA - em) + 4, 63);
     const uint64_t X3 = 3 * X, Z3 = 3 * Z, Y6 = 6 * Y;
     const uint64_t sL = X + Y6 + Z3, sR = Z + Y6 + X3;
     const int zL = clz32((uint32_t)(sL >> 32)), zR = clz32((uint32_t)(sR >> 32));
     const uint64_t rL = rcp_fixed(sL << zL), rR = rcp_fixed(sR << zR);
     WenoWeights w;
-    w.farL2 = weight_bits(umulhi64(X << zL, rL), 1);
-    w.qL = (int64_t)umulhi64(Z3 << zL, rL);
+    w.farL2 = weight_bits(mulhi_near(X << zL, rL), 1);
+    w.qL = (int64_t)mulhi_near(Z3 << zL, rL);
     w.nearL = weight_bits((uint64_t)w.qL, 0);
-    w.farR2 = weight_bits(umulhi64(Z << zR, rR), 1);
-    w.qR = (int64_t)umulhi64(X3 << zR, rR);
+    w.farR2 = weight_bits(mulhi_near(Z << zR, rR), 1);
+    w.qR = (int64_t)mulhi_near(X3 << zR, rR);
     w.nearR = weight_bits((uint64_t)w.qR, 0);
     return w;
 }
