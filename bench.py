@@ -237,9 +237,9 @@ def run_reference(a):
     return 0
 
 
-def algorithmic(kind, case, a, nlaunch_per_step):
-    """Algorithmic bytes per launch of a kernel kind (unique compulsory
-    traffic), for one box of max_grid^3 cells."""
+def algorithmic(kind, case, a):
+    """Algorithmic bytes of one pass of a kernel kind over one box of max_grid^3
+    cells (unique compulsory traffic; one direction of the face and flux passes)."""
     B = a.max_grid
     N = case.ncomp
     Cadv = 5 + case.params.nspec
@@ -615,16 +615,18 @@ def main():
             "algorithmic_bytes_per_cell_update": abytes_cell, "algorithmic_bytes_per_step": abytes_cell * cells,
             "step_ms": step_ms, "traffic_source": traffic["source"] if traffic else None}
 
-    # the dominant kernel on its own: its byte model per launch over its launch time
+    # the dominant pass on its own: the byte model of its stages over all
+    # boxes (and directions, of the face and flux passes) over its time; a launch
+    # covers several boxes and all directions, so both are divided by the launches
     dom = max(kernels, key=lambda k: kernels[k]["ms"])
-    avg_ms = kernels[dom]["ms"] / kernels[dom]["launches"]
-    # the face pass of orders 1/2 covers the three directions of a box in one
-    # timed entry (split + list kernels); the per-direction figures scale by 3
-    dirs = 3 if (dom == "face" and a.order <= 2) else 1
-    kbytes = dirs * algorithmic(dom, case, a, kernels[dom]["launches"])
+    nl = kernels[dom]["launches"]
+    avg_ms = kernels[dom]["ms"] / nl
+    dirs = 3 if dom in ("face", "flux") else 1
+    stages = 1 if dom in ("post", "copy", "chem", "timestep") else 3
+    kbytes = stages * len(case.boxes) * dirs * algorithmic(dom, case, a) / nl
     kach = kbytes / (avg_ms / 1e3) / 1e9
     kroof = {"kernel": dom, "achieved": kach, "peak": hbm, "unit": "GB/s", "frac": kach / hbm,
-             "model_bytes_per_launch": kbytes, "avg_launch_ms": avg_ms, "directions_per_launch": dirs,
+             "model_bytes_per_launch": kbytes, "avg_launch_ms": avg_ms, "launches_per_step": nl,
              "share_of_step": kernels[dom]["ms"] / tot if tot else None,
              "note": "bytes of a per-kernel traffic model (inputs and outputs of the kernel, intermediates included), "
                      "not the step's algorithmic bytes"}
