@@ -131,7 +131,10 @@ MFG_HD WenoWeights weno_weights(uint64_t dB, int eB, uint64_t dC, int eC, uint64
     const uint64_t X3 = 3 * X, Z3 = 3 * Z, Y6 = 6 * Y;
     const uint64_t sL = X + Y6 + Z3, sR = Z + Y6 + X3;
     const int zL = clz32((uint32_t)(sL >> 32)), zR = clz32((uint32_t)(sR >> 32));
-    const uint64_t rL = rcp_fixed(sL << zL), rR = rcp_fixed(sR << zR);
+    // both reciprocals from that of the product: three products for one reciprocal
+    const uint64_t nL = sL << zL, nR = sR << zR, P = mulhi_near(nL, nR);
+    const int zP = (int)(~P >> 63);  // P in [2^62, 2^64)
+    const uint64_t rP = rcp_fixed(P << zP), rL = mulhi_near(nR, rP) << zP, rR = mulhi_near(nL, rP) << zP;
     WenoWeights w;
     w.farL2 = weight_bits(mulhi_near(X << zL, rL), 1);
     w.qL = (int64_t)mulhi_near(Z3 << zL, rL);
