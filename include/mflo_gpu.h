@@ -320,9 +320,10 @@ int mfg_set_weno_mode(int fast);
  * them in device memory (synchronizes twice; 24 B per cut cell plus 20 B per
  * fluid neighbour, about 0.3 KiB per cut cell in a sphere pack), and
  * every later call checks the box's grown volume fraction against a stored
- * copy on the device (exact) before using them: a changed geometry falls back
- * to recomputation in the same call and is dropped from the cache.  Results
- * are bitwise the same either way.  enable = 0 frees the cache.  Synchronizes. */
+ * copy on the device (exact) before using them: values that moved between the
+ * same gas, cut and solid cells refresh the weights on the device, a changed
+ * geometry falls back to recomputation in the same call and is out of use until
+ * it is built anew.  Results are bitwise the same either way.  enable = 0 frees the cache.  Synchronizes. */
 int mfg_set_cutcell_cache(int enable);
 
 /* Form of the face pass of orders 1 and 2 with Navier-Stokes terms

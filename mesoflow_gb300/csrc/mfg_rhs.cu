@@ -3,7 +3,7 @@
 // Structure (per RK stage; each kernel one launch for a group of boxes,
 // mfg_rhs_launch.cuh):
 //   prim_kernel   per cell of grow(bx,3): velocities, pressure, eigen-pressure
-//                 energy, own sound speed and gamma, computed once per cell
+//                 energy, own sound speed and gamma - 1, computed once per cell
 //                 instead of once per face use (the reference re-derives them
 //                 inside every face's geteulerflux / get_max_eigenvalue).
 //   face_kernel   per face of growHi(bx,d,1): scheme scalars (LLF eigenvalue,
@@ -14,14 +14,16 @@
 //                 face_list_kernel runs the flux branch over those lists, each
 //                 for the three directions in one launch, so no lane of a warp
 //                 idles on a solid-side face.
-//   flux_kernel   per (face, component): the hyperbolic flux of one
-//                 component (WENO5-JS / MUSCL+AUSM+-up / central), species
-//                 diffusion, and the viscous terms, written once per face and
-//                 read by both neighbouring cells.
-//   flux5_sweep_kernel  WENO5 with Navier-Stokes terms in the one-division
-//                 mode: per (column segment along d, component), the per-cell
-//                 parts of the reconstruction computed once per cell and kept
-//                 in registers while the thread walks the faces.
+//   flux5_sweep_kernel  WENO5 with Navier-Stokes terms: per (column segment
+//                 along d, component), the per-cell parts of the reconstruction
+//                 computed once per cell and kept in registers while the thread
+//                 walks the faces; species diffusion and viscous terms included,
+//                 written once per face and read by both neighbouring cells.
+//                 flux5_face_kernel is the per-face form for small launches.
+//   flux4_kernel  per (face, component): the central scheme with dissipation.
+//   flux_kernel   per (face, component): WENO5 in the reference's operation
+//                 order (mfg_set_weno_mode 0), and the species convection
+//                 without Navier-Stokes terms.
 //   update_kernel per (cell, component): flux divergence, IB masking, NaN
 //                 status, and the RK3 stage algebra.
 // Semantics: compute_flux (Source/Src_3d/compute_flux_3d.H:88-430),

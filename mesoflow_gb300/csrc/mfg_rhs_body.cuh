@@ -867,8 +867,8 @@ __device__ __forceinline__ void flux5_face_body(const Fp& fp, const RhsBox& B, i
 // / 12): one thread per (face, component), the four cells it reads as the
 // order-5 sweep takes them (one or two FP64 operations each, against six cells
 // of the general Euler flux before), half, flag and viscous term in one
-// multiply-add: about 16 FP64 operations against 60 (right-hand side of 57x64x33 cells
-// 287 -> 217 us).
+// multiply-add: about 16 FP64 operations against 60 (right-hand side of 57x64x33
+// cells 287 -> 217 us).
 __device__ __forceinline__ void flux4_body(const Fp& fp, const RhsBox& B, int d, int c, int64_t t) {
     int len[3];
     for (int e = 0; e < 3; ++e) len[e] = B.hi[e] - B.lo[e] + 1 + (e == d);

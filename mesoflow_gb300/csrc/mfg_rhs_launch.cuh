@@ -103,9 +103,9 @@ __global__ void __launch_bounds__(TPB) flux_kernel(const __grid_constant__ RhsGr
                     (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 constexpr int SWEEP_TPB = 128;
-// Four blocks per SM (128 registers, 20 bytes spilled): 16 warps keep the FP64
-// and integer pipes busier than 12 (168 registers): 24.6 against 25.7 ms per
-// 128^3 Taylor-Green step.
+// Four blocks per SM (128 registers): 16 warps keep the FP64 and integer pipes
+// busier than 12 (168 registers): 24.6 against 25.7 ms per 128^3 Taylor-Green
+// step when that was measured, 16 ms with the operations cut since.
 template <int G>
 __global__ void __launch_bounds__(SWEEP_TPB, 4) flux5_sweep_kernel(const __grid_constant__ RhsGroup<G> g, int seg) {
     const Fp fp;
@@ -121,8 +121,8 @@ __global__ void __launch_bounds__(SWEEP_TPB, 4) flux5_face_kernel(const __grid_c
 // The column segments of a launch must fill the GPU: segments of 32, 16, 8 or 4
 // faces (longer ones share more per-cell work), else the per-face form of the
 // same arithmetic, which does about twice the work per face.  A 16^3 box with
-// 12 advected components takes the per-face form: 58 us per right-hand side,
-// against 67 and 84 with half and a quarter of this bound.
+// 13 advected components takes the per-face form: 58 us per right-hand side (50
+// since), against 67 and 84 with half and a quarter of this bound.
 constexpr int64_t SWEEP_MIN_THREADS = 152 * 2 * SWEEP_TPB * 2;
 template <int G>
 __global__ void __launch_bounds__(TPB) update_kernel(const __grid_constant__ RhsGroup<G> g, int stage, double dt) {
