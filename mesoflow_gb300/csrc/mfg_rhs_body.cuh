@@ -178,20 +178,22 @@ __device__ __forceinline__ bool surely_below(double v, double a2) {
 }
 
 // The two sides' shares of an AUSM+-up face (flux_schemes.H:107-181, beta =
-// 1/8) at the Mach number M, sign = +1 for the left side and -1 for the right:
-// four times the Mach split, sign ((M + sign)^2 + (M^2 - 1)^2/2) below |M| = 1
-// and 2 (M + sign |M|) above, and the pressure split, (M + sign)^2 (2 - sign M)/4
-// + sign alpha M (M^2 - 1)^2 below and (M + sign |M|)/(2 M) above.  q = M^2 - 1.
-// The supersonic branches are exactly 4 M or 0, and 1 or 0; the |M| <= 1 tests
-// run on the integer pipe.
-__device__ __forceinline__ void ausm_split(const Fp& fp, double M, double sign, double q, double& m4, double& g,
-                                           double& mq2) {
+// 1/8) at the Mach number M, sign = +1 for the left side and -1 for the right; q
+// = M^2 - 1, and the |M| <= 1 tests run on the integer pipe.  Four times the
+// pressure split: (M + sign)^2 (2 - sign M) + 4 sign alpha M (M^2 - 1)^2 below
+// |M| = 1, as g and M q^2, and exactly 4 or 0 above.
+__device__ __forceinline__ void ausm_split(const Fp& fp, double M, double sign, double q, double& g, double& mq2) {
     const double a = __fma_rn(sign, fp.one, M);
-    const double sq = fp.mul(a, a), q2 = fp.mul(q, q);
     const bool sub = abs_le(M, 1.0), on = sign > 0.0 ? is_positive(M) : is_negative(M);
-    m4 = sub ? __fma_rn(0.5, q2, sq) : (on ? __dmul_rn(4.0 * sign, M) : 0.0);
-    g = sub ? fp.mul(sq, __fma_rn(-sign, M, 2.0)) : (on ? 4.0 : 0.0);
-    mq2 = sub ? fp.mul(M, q2) : 0.0;
+    g = sub ? fp.mul(fp.mul(a, a), __fma_rn(-sign, M, 2.0)) : (on ? 4.0 : 0.0);
+    mq2 = sub ? fp.mul(M, fp.mul(q, q)) : 0.0;
+}
+// Four times one side's Mach split: sign ((M + sign)^2 + (M^2 - 1)^2/2) below
+// |M| = 1, 4 M or 0 above (without the sign).
+__device__ __forceinline__ double ausm_mach4(const Fp& fp, double M, double sign, double q) {
+    const double a = __fma_rn(sign, fp.one, M);
+    const bool on = sign > 0.0 ? is_positive(M) : is_negative(M);
+    return abs_le(M, 1.0) ? __fma_rn(0.5, fp.mul(q, q), fp.mul(a, a)) : (on ? __dmul_rn(4.0 * sign, M) : 0.0);
 }
 
 // Face f of direction d.  SOLID_SIDE: the caller knows the face is not
@@ -290,16 +292,17 @@ __device__ __forceinline__ void face_body_at(const Fp& fp, const RhsBox& B, int 
             const double k2R = fp.mul(
                 __fma_rn(uR[RHOU], uR[RHOU], __fma_rn(uR[RHOV], uR[RHOV], fp.mul(uR[RHOW], uR[RHOW]))), irR);
             // kappa = gamma - 1 of both states as one division each, or as its
-            // numerator and denominator: 2 (gamma - 1)/(gamma + 1) = 2 n/(2 d + n)
+            // numerator and denominator: 2 (gamma - 1)/(gamma + 1) = n/(d + n/2),
+            // with reciprocals of the integer pipe
             double kL = P.gm1_single, kR = P.gm1_single, afL = P.astar_fac, afR = P.astar_fac;
             if (P.thermo_kind != MFG_THERMO_MASS_SINGLE) {
                 double n, dn;
                 thermo_ratio<NS>(rL, uL + NCONS, n, dn);
-                kL = quot_pos(n, dn);
-                afL = quot_pos(2.0 * n, __fma_rn(2.0, dn, n));
+                kL = fp.mul(n, face_rcp(dn));
+                afL = fp.mul(n, face_rcp(__fma_rn(0.5, n, dn)));
                 thermo_ratio<NS>(rR, uR + NCONS, n, dn);
-                kR = quot_pos(n, dn);
-                afR = quot_pos(2.0 * n, __fma_rn(2.0, dn, n));
+                kR = fp.mul(n, face_rcp(dn));
+                afR = fp.mul(n, face_rcp(__fma_rn(0.5, n, dn)));
             }
             const double pL = fp.mul(__fma_rn(-0.5, k2L, uL[RHOE]), kL), pR = fp.mul(__fma_rn(-0.5, k2R, uR[RHOE]), kR);
             const double vL = fp.mul((d == 0) ? uL[RHOU] : (d == 1) ? uL[RHOV] : uL[RHOW], irL);
@@ -340,13 +343,21 @@ __device__ __forceinline__ void face_body_at(const Fp& fp, const RhsBox& B, int 
             }
             const double ML = fp.mul(vL, iah), MR = fp.mul(vR, iah);
             const double qL = __fma_rn(ML, ML, -fp.one), qR = __fma_rn(MR, MR, -fp.one);
-            double m4L, m4R, gL, gR, mqL, mqR;
-            ausm_split(fp, ML, 1.0, qL, m4L, gL, mqL);
-            ausm_split(fp, MR, -1.0, qR, m4R, gR, mqR);
+            double gL, gR, mqL, mqR;
+            ausm_split(fp, ML, 1.0, qL, gL, mqL);
+            ausm_split(fp, MR, -1.0, qR, gR, mqR);
             // mean Mach number Mb^2 = (ML^2 + MR^2)/2 = 1 + (qL + qR)/2
-            const double qs = fp.add(qL, qR);
+            const double qs = fp.add(qL, qR), Mb2 = __fma_rn(0.5, qs, 1.0);
+            // four times M_1/2: with both sides subsonic the splits' sum in closed
+            // form, (ML + MR) (2 + (ML - MR) Mb^2), which does not cancel at low Mach
+            // numbers as the difference of two terms near one does
+            double mm4;
+            if (abs_le(ML, 1.0) && abs_le(MR, 1.0))
+                mm4 = fp.mul(fp.add(ML, MR), __fma_rn(fp.sub(ML, MR), Mb2, 2.0));
+            else
+                mm4 = fp.sub(ausm_mach4(fp, ML, 1.0, qL), ausm_mach4(fp, MR, -1.0, qR));
             // M_o = sqrt(min(1, max(Mb^2, 0.3^2))) as x rsqrt(x) on the clamped x
-            const double xmo = min_nonneg(1.0, max_nonneg(pos_part(__fma_rn(0.5, qs, 1.0)), 0.3 * 0.3));
+            const double xmo = min_nonneg(1.0, max_nonneg(pos_part(Mb2), 0.3 * 0.3));
             const double Mo = fp.mul(xmo, face_rsqrt(xmo));
             const double fa = fp.mul(Mo, __fma_rn(-Mo, fp.one, 2.0));
             const double fr = fp.mul(fa, rsum);
@@ -356,7 +367,7 @@ __device__ __forceinline__ void face_body_at(const Fp& fp, const RhsBox& B, int 
             const double pd = fp.mul(fp.mul(pos_part(-qs), fp.sub(pR, pL)), fp.mul(iah, iah));
             // M_1/2, its modulus with the parabola below 0.3, and the pressure
             // splits, each times four (exact scales, taken back where they cost nothing)
-            const double M4 = __fma_rn(-pd, face_rcp(fr), fp.sub(m4L, m4R));
+            const double M4 = __fma_rn(-pd, face_rcp(fr), mm4);
             double mod4 = fabs(M4);
             if (nonneg_le(mod4, 4.0 * 0.3)) mod4 = __dmul_rn(__fma_rn(M4, M4, 16.0 * (0.3 * 0.3)), 0.25 * (1.0 / (2.0 * 0.3)));
             // alpha = 3/16 (-4 + 5 fa^2) as (15/16 fa) fa - 3/4
