@@ -209,7 +209,7 @@ __device__ __forceinline__ double ausm_mach4(const Fp& fp, double M, double sign
 // rounding is explicit, so the one-pass and the listed form agree bitwise.
 // About 150 FP64 operations per face of one species at 70 cycles (205 at 82
 // with the refined reciprocals there): face passes of a 256^3 sphere-pack step
-// 50.4 -> 38.0 ms, and 36.5 with the factors of four of the splits, the viscosity
+// 50.4 -> 38.0 ms, and 36.8 with the factors of four of the splits, the viscosity
 // and the conductivity inside multiply-adds; the listed form keeps the FP64 pipe
 // 83% busy.
 //
