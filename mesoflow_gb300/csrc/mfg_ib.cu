@@ -53,7 +53,8 @@ __constant__ double c_wdir[125];
 namespace {
 
 constexpr int TPB = 128;
-// An entry's flag.  VF_MOVED: some value differs from the copy in this call;
+// An entry's flag.  VF_MOVED: some value differs from the copy in this call (or
+// did in an earlier one of the box alone: a refresh then changes nothing);
 // VF_OTHER: since the entry was built some cell changed between gas, cut and
 // solid (kept until the entry is dropped).
 constexpr unsigned VF_MOVED = 1u, VF_OTHER = 2u;
@@ -105,12 +106,15 @@ struct CutGroup {
     CutBox c[CUT_GROUP];
     const int* list[CUT_GROUP];
     const unsigned* count[CUT_GROUP];
+    unsigned* moved[CUT_GROUP];  // change flags whose VF_MOVED the launch clears, or null
 };
 template <int NS>
 __global__ void __launch_bounds__(TPB) cutcell_kernel(const __grid_constant__ CutGroup g) {
     const unsigned n = *g.count[blockIdx.y];
     const int* __restrict__ list = g.list[blockIdx.y];
     const CutBox& c = g.c[blockIdx.y];
+    // the last launch of a level's pass, and no block of it reads the flag
+    if (g.moved[blockIdx.y] && blockIdx.x == 0 && threadIdx.x == 0) *g.moved[blockIdx.y] &= VF_OTHER;
     if (blockIdx.x * blockDim.x >= n) return;
     __shared__ CutShared<TPB> sm;
     cut_shared_init(sm);
@@ -201,18 +205,12 @@ struct LevelCutBox {
     int glo[3], glen[3];  // grown box
 };
 
-// Clears every box's VF_MOVED and rebuilt-list count.
-__global__ void cut_level_reset_kernel(const LevelCutBox* __restrict__ tab, int nbox, unsigned* __restrict__ cnt) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b < nbox) {
-        *tab[b].dirty &= VF_OTHER;
-        cnt[b] = 0;
-    }
-}
-
-// Grown volume fraction against the stored copy (blockIdx.y = box).
-__global__ void cut_level_vf_kernel(const LevelCutBox* __restrict__ tab) {
+// Grown volume fraction against the stored copy (blockIdx.y = box); clears the
+// box's rebuilt-list count.  VF_MOVED is clear from the last pass (or, after a
+// pass of the box alone, asks for a refresh that changes nothing).
+__global__ void cut_level_vf_kernel(const LevelCutBox* __restrict__ tab, unsigned* __restrict__ cnt) {
     const LevelCutBox& L = tab[blockIdx.y];
+    if (blockIdx.x == 0 && threadIdx.x == 0) cnt[blockIdx.y] = 0;
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const bool in = t < (int64_t)L.glen[0] * L.glen[1] * L.glen[2];
     double v = 0.0;
@@ -659,9 +657,9 @@ int launch_cutcells_level(const mfg_box* boxes, int nbox, const mfg_geom& g, cud
         return 0;
     }
     const int ns = c_host_params().nspec;
-    ProfScope ps(K_CUT, st, 3 + (T->ngroups > 0) + (nbox + CUT_GROUP - 1) / CUT_GROUP);
-    cut_level_reset_kernel<<<(nbox + 127) / 128, 128, 0, st>>>(T->d_tab, nbox, g_level.d_cnt);
-    cut_level_vf_kernel<<<dim3((unsigned)((T->maxgrown + 255) / 256), (unsigned)nbox), 256, 0, st>>>(T->d_tab);
+    ProfScope ps(K_CUT, st, 2 + (T->ngroups > 0) + (nbox + CUT_GROUP - 1) / CUT_GROUP);
+    cut_level_vf_kernel<<<dim3((unsigned)((T->maxgrown + 255) / 256), (unsigned)nbox), 256, 0, st>>>(T->d_tab,
+                                                                                                        g_level.d_cnt);
     const unsigned per = (unsigned)std::max<int64_t>(1, std::min<int64_t>((T->cap + TPB - 1) / TPB, 152));
     cut_level_change_kernel<<<dim3(per, (unsigned)nbox), TPB, 0, st>>>(T->d_tab, g_level.d_cnt, g_level.d_lists,
                                                                         T->cap);
@@ -677,6 +675,7 @@ int launch_cutcells_level(const mfg_box* boxes, int nbox, const mfg_geom& g, cud
                 cg.c[q] = tab[w].c;                                                                         \
                 cg.list[q] = g_level.d_lists + (int64_t)w * T->cap;                                         \
                 cg.count[q] = g_level.d_cnt + w;                                                            \
+                cg.moved[q] = tab[w].dirty;                                                                 \
             }                                                                                               \
             cutcell_kernel<K><<<dim3(152, n), TPB, 0, st>>>(cg);                                            \
         }                                                                                                   \
@@ -727,6 +726,7 @@ cudaError_t launch_cutcells_box(const mfg_box& b, const mfg_geom& g, double* tch
         cg.c[q] = c;
         cg.list[q] = list;
         cg.count[q] = count;
+        cg.moved[q] = nullptr;
     }
     if (ns <= 1) cutcell_kernel<1><<<ng, TPB, 0, st>>>(cg);
     else if (ns <= 2) cutcell_kernel<2><<<ng, TPB, 0, st>>>(cg);
