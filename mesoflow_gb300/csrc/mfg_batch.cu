@@ -620,7 +620,7 @@ __global__ void __launch_bounds__(SWEEP_BT, 4) bk_flux_sweep(const RhsBox* __res
     flux5_sweep_body(fp, B[tl.box], tl.part >> 5, tl.part & 31, t);
     TILE_END
 }
-__global__ void __launch_bounds__(SWEEP_BT, 2) bk_flux5_face(const RhsBox* __restrict__ B,
+__global__ void __launch_bounds__(SWEEP_BT, 3) bk_flux5_face(const RhsBox* __restrict__ B,
                                                              const Tile* __restrict__ tiles, int ntiles) {
     const Fp fp;
     TILE_LOOP

@@ -24,6 +24,8 @@ struct Fp {
         one = __hiloint2double(__shfl_sync(0xffffffffu, 0x3ff00000, 0), 0);
         nz = __hiloint2double(__shfl_sync(0xffffffffu, (int)0x80000000, 0), 0);
     }
+    // the constants as immediates, for code that part of a warp runs
+    __device__ __forceinline__ explicit Fp(int) : one(1.0), nz(-0.0) {}
     __device__ __forceinline__ double add(double a, double b) const { return __fma_rn(a, one, b); }
     __device__ __forceinline__ double sub(double a, double b) const { return __fma_rn(b, -one, a); }
     __device__ __forceinline__ double mul(double a, double b) const { return __fma_rn(a, b, nz); }
@@ -665,9 +667,12 @@ __device__ __forceinline__ void update_body(const Fp& fp, const RhsBox& B, int s
 // (each candidate polynomial written about the mean, with w2 + w1 + w0 = 1),
 // so the local Lax-Friedrichs flux needs the fluxes' mean and the corrections
 // only: the state's mean cancels.  Rounding errors of the reconstruction then
-// scale with the differences instead of the values (two to five times smaller
-// against 80-bit arithmetic than the candidate form on smooth, noisy and
-// discontinuous data).
+// scale with the differences instead of the values: two to five times smaller
+// against 80-bit arithmetic than the candidate form where the values are at least
+// as large.  Beside a front, where the differences are 2^6 and more times the
+// face's values, they would be larger than the flux in the end, and the face takes
+// the candidates (weno_front, weno_front_llf): the test, on the integer pipe, costs
+// 3% of the 128^3 Taylor-Green step and 4% of a 64^3 right-hand side.
 //   The right edge of face m and the left edge of face m + 1 lie in cell m and
 // see the same five cells, so they share the products of their weights.
 //   The weights are ratios of positive numbers: mfg_weno_weights.cuh forms
@@ -790,6 +795,22 @@ __device__ __forceinline__ double weno_llf_collapsed(const Fp& fp, double lam, d
     return __fma_rn(-fp.mul(lam, D), W, fsum);
 }
 
+// Twice the local Lax-Friedrichs flux of a regular face beside a front
+// (weno_front): both edges of the state and of its Euler flux as weighted
+// candidates, from the six cells read again (os, ox: the face's right cell; sd,
+// xd: the strides along d).
+__device__ __forceinline__ double weno_front_llf(const Fp& op, const Flux5Ctx& x, int64_t os, int64_t sd, int64_t ox,
+                                                 int64_t xd, double lam) {
+    double us[6], fl[6];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) flux5_cell(op, x, os + (q - 3) * sd, ox + (q - 3) * xd, us[q], fl[q]);
+    const double up = weno_front_edge(us[0], us[1], us[2], us[3], us[4]);
+    const double um = weno_front_edge(us[5], us[4], us[3], us[2], us[1]);
+    const double fp = weno_front_edge(fl[0], fl[1], fl[2], fl[3], fl[4]);
+    const double fm = weno_front_edge(fl[5], fl[4], fl[3], fl[2], fl[1]);
+    return mul(op.add(__fma_rn(lam, up, fp), __fma_rn(-lam, um, fm)), 1.0 / 6.0);  // the edges come six times
+}
+
 // Complete flux of one face (the sweep and the per-face form share it, so
 // they agree bitwise), stored: fh2 times x.half is the hyperbolic flux where
 // active (the half, the advection flag and the viscous term take one operation),
@@ -842,6 +863,7 @@ __device__ __forceinline__ void flux5_face_body(const Fp& fp, const RhsBox& B, i
 #pragma unroll
         for (int q = 0; q < 6; ++q) flux5_cell(fp, x, oR + (q - 3) * sd, xR + (q - 3) * xd, ru[q], rf[q]);
         double cu[2];  // C of the Euler flux, U of the state
+        int top[2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const double* r = h ? ru : rf;
@@ -857,9 +879,13 @@ __device__ __forceinline__ void flux5_face_body(const Fp& fp, const RhsBox& B, i
             const WenoWeights wr = weno_weights(i1.dB, i1.eB, i2.dC, i2.eC, i3.dA, i3.eA);
             cu[h] = h ? weno_pair<true>(fp, fp.mul(weight_of(wl.farL2), g0), wl.qL, wr, g1, g2, tt[2])
                       : weno_pair<false>(fp, __fma_rn(weight_of(wl.farL2), g0, tt[1]), wl.qL, wr, g1, g2, tt[2]);
+            top[h] = imax(imax(i0.eB, i1.eB), imax(i2.eB, i3.eB));
             if (h) D = dd[2];
         }
-        fh = weno_llf(x.fs[qf + FS_LAMBDA * x.fns], fp.add(rf[2], rf[3]), cu[0], cu[1]);
+        const double lam = x.fs[qf + FS_LAMBDA * x.fns];
+        fh = weno_front(top[0], top[1], x.kind == 2, rf[2], rf[3], ru[2], ru[3], lam)
+                 ? weno_front_llf(fp, x, oR, sd, xR, xd, lam)
+                 : weno_llf(lam, fp.add(rf[2], rf[3]), cu[0], cu[1]);
     } else if (flags & 1) {
         double uL, uR, fL, fR;
         flux5_cell(fp, x, oR - sd, xR - xd, uL, fL);
@@ -920,14 +946,16 @@ struct WenoRun {
     double t0, g, sumL;
     int64_t qL;
     uint64_t dBm, dB0, dC0;
-    int eBm, eB0, eC0;
+    int eBm, eB0, eC0, eBp;  // eBp: of centre f-2
 };
 
-// Adds centre f+1 (Dn = v_{f+2} - v_{f+1}): returns C or U of face f and moves
-// the run to face f+1.
+// Adds centre f+1 (Dn = v_{f+2} - v_{f+1}): returns C or U of face f, in top the
+// largest eB of its four centres (weno_front), and moves the run to face f+1.
 template <bool STATE>
-__device__ __forceinline__ double weno_next(const Fp& fp, WenoRun& r, double D, double Dn) {
+__device__ __forceinline__ double weno_next(const Fp& fp, WenoRun& r, double D, double Dn, int& top) {
     const WenoInd c = weno_ind(D, Dn);
+    top = imax(imax(r.eBp, r.eBm), imax(r.eB0, c.eB));
+    r.eBp = r.eBm;
     const WenoWeights w = weno_weights(r.dBm, r.eBm, r.dC0, r.eC0, c.dA, c.eA);
     const double t = fp.sub(Dn, D), gp = fp.sub(t, r.t0);
     const double res = weno_pair<STATE>(fp, r.sumL, r.qL, w, r.g, gp, r.t0);
@@ -954,18 +982,19 @@ __device__ __forceinline__ void weno_prime(const Fp& fp, WenoRun& r, double va, 
     r.g = fp.sub(r.t0, ta);
     r.sumL = 0.0;
     r.qL = 0;
+    r.eBp = 0;
     r.dBm = c0.dB;
     r.eBm = c0.eB;
     r.dB0 = c1.dB;
     r.eB0 = c1.eB;
     r.dC0 = c1.dC;
     r.eC0 = c1.eC;
-    weno_next<STATE>(fp, r, d2, r.D);
+    int top;
+    weno_next<STATE>(fp, r, d2, r.D, top);
 }
 
-__device__ __forceinline__ void flux5_sweep_body(const Fp& fp, const RhsBox& B, int d, int c, int64_t t,
-                                                 int seglen = SWEEP_SEG) {
-    if (t >= sweep_items(B, d, seglen)) return;
+// Column segment t of a sweep: its first face f (indices) and its number of faces.
+__device__ __forceinline__ int sweep_segment(const RhsBox& B, int d, int64_t t, int seglen, Idx3& f) {
     int ta, tb;
     sweep_dirs(d, ta, tb);
     const int na = B.hi[ta] - B.lo[ta] + 1, nb = B.hi[tb] - B.lo[tb] + 1;
@@ -976,10 +1005,43 @@ __device__ __forceinline__ void flux5_sweep_body(const Fp& fp, const RhsBox& B, 
     const int nseg = sweep_nseg(B, d, seglen);
     const int per = (nf + nseg - 1) / nseg;
     const int f0 = B.lo[d] + seg * per;
-    const int f1 = min(B.lo[d] + nf - 1, f0 + per - 1);
-    if (f0 > f1) return;
     const int ia = B.lo[ta] + (int)(col % na), ib = B.lo[tb] + (int)(col / na);
-    const int i = (d == 0) ? f0 : ia, j = (d == 0) ? ia : (d == 1) ? f0 : ib, k = (d == 2) ? f0 : ib;
+    f.i = (d == 0) ? f0 : ia;
+    f.j = (d == 0) ? ia : (d == 1) ? f0 : ib;
+    f.k = (d == 2) ? f0 : ib;
+    return min(per, B.lo[d] + nf - f0);
+}
+
+// The faces of a column segment that are beside a front (bit q: the face q before
+// the last), done again by the candidates.  Apart from the walk and not inlined:
+// it shares no registers with it (inside the loop the kernel spilled 200 bytes,
+// after it 50, the batched one 500 against 270), and few segments come here.
+__device__ __noinline__ void flux5_fronts(const RhsBox& B, int d, int c, int64_t t, int seglen, unsigned fronts) {
+    const Fp fp(0);  // few lanes of a warp are here: no shuffle
+    Idx3 f;
+    int n = sweep_segment(B, d, t, seglen, f);
+    const Flux5Ctx x = flux5_ctx(B, d, c);
+    const int64_t sd = (d == 0) ? 1 : (d == 1) ? B.sb.js : B.sb.ks;
+    const int64_t xd = (d == 0) ? 1 : (d == 1) ? B.aux.js : B.aux.ks;
+    const int64_t fd = (d == 0) ? 1 : (d == 1) ? B.fs[d].js : B.fs[d].ks;
+    const int64_t rd = (d == 0) ? 1 : (d == 1) ? B.uflux[d].js : B.uflux[d].ks;
+    const int64_t o0 = B.sb.off(f.i, f.j, f.k), a0 = B.aux.off(f.i, f.j, f.k), q0 = B.fs[d].off(f.i, f.j, f.k);
+    const int64_t r0 = x.reg ? B.uflux[d].off(f.i, f.j, f.k) : 0;
+    for (; fronts; fronts &= fronts - 1) {
+        const int m = n - __ffs(fronts);
+        const int64_t o = o0 + m * sd, q = q0 + m * fd;
+        const double fh = weno_front_llf(fp, x, o, sd, a0 + m * xd, xd, x.fs[q + FS_LAMBDA * x.fns]);
+        flux5_finish(fp, x, true, fh, fp.sub(x.u[o], x.u[o - sd]), o - sd, o, q, q, r0 + m * rd);
+    }
+}
+
+__device__ __forceinline__ void flux5_sweep_body(const Fp& fp, const RhsBox& B, int d, int c, int64_t t,
+                                                 int seglen = SWEEP_SEG) {
+    if (t >= sweep_items(B, d, seglen)) return;
+    Idx3 f0;
+    int left = sweep_segment(B, d, t, seglen, f0);  // faces to do
+    if (left <= 0) return;
+    const int i = f0.i, j = f0.j, k = f0.k;
     const Flux5Ctx x = flux5_ctx(B, d, c);
     const int64_t sd = (d == 0) ? 1 : (d == 1) ? B.sb.js : B.sb.ks;
     const int64_t xd = (d == 0) ? 1 : (d == 1) ? B.aux.js : B.aux.ks;
@@ -991,7 +1053,7 @@ __device__ __forceinline__ void flux5_sweep_body(const Fp& fp, const RhsBox& B, 
     int64_t qf = B.fs[d].off(i, j, k);
     int64_t qr = x.reg ? B.uflux[d].off(i, j, k) : 0;
     if (c >= NCONS && c_P.advect_flag[c - NCONS] == 0.0) {  // not advected: diffusion only
-        for (int fc = f0; fc <= f1; ++fc, oR += sd, qf += fd, qr += rd)
+        for (; left > 0; --left, oR += sd, qf += fd, qr += rd)
             flux5_finish(fp, x, false, 0.0, fp.sub(x.u[oR], x.u[oR - sd]), oR - sd, oR, qf, qf, qr);
         return;
     }
@@ -1012,7 +1074,8 @@ __device__ __forceinline__ void flux5_sweep_body(const Fp& fp, const RhsBox& B, 
     u.D = fp.sub(u.v1, u.v0);
     f.D = fp.sub(f.v1, f.v0);
     bool primed = false;
-    for (int fc = f0;; ++fc) {
+    unsigned fronts = 0;  // faces beside a front, done again below (a segment has up to 32)
+    for (;;) {
         double un, fn;  // cell f+2, loaded before this face's arithmetic
         flux5_cell(fp, x, oR + 2 * sd, xR + 2 * xd, un, fn);
         const int flags = (int)__double_as_longlong(x.fs[qf + FS_FLAGS * x.fns]) & 3;
@@ -1027,14 +1090,20 @@ __device__ __forceinline__ void flux5_sweep_body(const Fp& fp, const RhsBox& B, 
                 weno_prime<false>(fp, f, fa, fb, fL);
                 primed = true;
             }
-            const double C = weno_next<false>(fp, f, f.D, Dfn), U = weno_next<true>(fp, u, u.D, Dun);
-            if (flags == 1) fh = weno_llf(x.fs[qf + FS_LAMBDA * x.fns], fp.add(fL, f.v0), C, U);
+            int topf, topu;
+            const double C = weno_next<false>(fp, f, f.D, Dfn, topf), U = weno_next<true>(fp, u, u.D, Dun, topu);
+            if (flags == 1) {
+                const double lam = x.fs[qf + FS_LAMBDA * x.fns];
+                fh = weno_llf(lam, fp.add(fL, f.v0), C, U);
+                if (weno_front(topf, topu, x.kind == 2, fL, f.v0, uL, u.v0, lam)) fronts |= 1u;
+            }
         } else {
             primed = false;
         }
         if (flags == 3) fh = weno_llf_collapsed(fp, x.fs[qf + FS_LAMBDA * x.fns], fp.add(fL, f.v0), Du);
         flux5_finish(fp, x, flags & 1, fh, Du, oR - sd, oR, qf, qf, qr);
-        if (fc == f1) break;
+        if (--left == 0) break;
+        fronts <<= 1;
         // advance one face
         oR += sd;
         xR += xd;
@@ -1050,6 +1119,7 @@ __device__ __forceinline__ void flux5_sweep_body(const Fp& fp, const RhsBox& B, 
         u.D = Dun;
         f.D = Dfn;
     }
+    if (fronts) flux5_fronts(B, d, c, t, seglen, fronts);
 }
 
 // Work items of each phase for one box.

@@ -6,15 +6,24 @@
 // takes 18 cycles of the integer pipe, which the order-5 flux kernels leave
 // idle.  The weights are ratios of positive numbers, so they need no signs, no
 // special values and no rounding modes, and fixed point gives them with errors
-// of 2^-50 or less relative to their sum (the FP64 form reached 2^-50 at best,
-// since it formed the indicators from rounded second differences): indicators,
-// squares, products, sums and reciprocals run here, beside the FP64 pipe that
-// forms the differences and applies the weights.
+// of 2^-50 or less of their sum: indicators, squares, products, sums and
+// reciprocals run here, beside the FP64 pipe that forms the differences and
+// applies the weights.
+//
+// Such a weight is absolute: one of 1e-12, that of the stencil across a front,
+// keeps 22 bits, and the corrections of the second-difference form are as large
+// as the differences and cancel.  Where the stencil's differences are far above
+// the values at the face the flux takes the weights in FP64 instead
+// (weno_front, weno_front_edge).
 //
 // Everything is integer arithmetic but the 23-bit seed of the reciprocal, so
 // every kernel that uses it gets the same bits.
 #pragma once
+#ifdef __CUDACC__
+#include "mfg_common.cuh"
+#else
 #include "mfg_fixed.cuh"
+#endif
 
 namespace mfg {
 
@@ -143,6 +152,67 @@ MFG_HD WenoWeights weno_weights(uint64_t dB, int eB, uint64_t dC, int eC, uint64
     w.qR = (int64_t)mulhi_near(X3 << zR, rR);
     w.nearR = weight_bits((uint64_t)w.qR, 0);
     return w;
+}
+
+// Whether a face is beside a front: some difference of its stencil, of the state
+// or of the Euler flux, large enough for the weights to depend on it (above the
+// exponent floor) and far above the face's own values lam max(|u_L|, |u_R|) (with
+// PRESSURE, the momentum along the sweep: and max(|f_L|, |f_R|), whose pressure
+// that does not bound).  The fixed-point form's error is about 2^-54 of the
+// differences, the FP64 candidates' 2^-51 of the values at the face: they meet
+// near a ratio of 2^6.  Against 113-bit arithmetic, largest error over the face's
+// values: a state of 1e-9 two faces from one of 1e3, 1e-6 in fixed point and 3e-16
+// here; of 0.01 beside 1 (differences of 2^7), 2.6e-16 and 3.2e-16.
+// topf, topu: the largest eB of the stencil's four centres: 3 (eps + beta) is 3 to
+// 25 times the square of a difference (0.97 for the first one), so a difference's
+// square counts to within 1.6 to 4.6 bits; the values' high words add as
+// logarithms do, to within a bit.  A ratio between 2^5.5 and 2^7.5 is the first to
+// count.  Infinities, NaN and values above 2^880 count too.
+constexpr int kFrontTop = 9;
+MFG_HD int hi_abs(double x) { return (int)(bits_of(x) >> 32) & 0x7fffffff; }
+MFG_HD bool weno_front(int topf, int topu, bool pressure, double fL, double fR, double uL, double uR, double lam) {
+    const int one = 0x3ff00000, most = 1900 << 20, least = 2 * kWenoExpFloor - 2;
+    const int l = hi_abs(lam) - one;
+    int mu = imin(imax(hi_abs(uL), hi_abs(uR)), most), mf = imin((int)((unsigned)mu + (unsigned)l), most);
+    if (pressure) {
+        mf = imin(imax(mf, imax(hi_abs(fL), hi_abs(fR))), most);
+        mu = imin(mf - l, most);
+    }
+    return topf > imax((mf >> 19) + kFrontTop, least) || topu > imax((mu >> 19) + kFrontTop, least);
+}
+
+// Six times one WENO5-JS edge of the cells a .. e, far upwind to far downwind
+// (flux_schemes.H:373-446), as the mean of the candidates with positive FP64
+// weights: its error is relative to the parts that make it up, whatever the
+// cells beyond a front hold.  Explicit roundings: the sweep and the per-face
+// form call it with the same cells and get the same bits.
+struct Rn {
+#ifdef __CUDA_ARCH__
+    static MFG_HD double fma(double a, double b, double c) { return __fma_rn(a, b, c); }
+    static MFG_HD double mul(double a, double b) { return __dmul_rn(a, b); }
+    static MFG_HD double add(double a, double b) { return __dadd_rn(a, b); }
+    static MFG_HD double rcp(double x) { return rcp_pos(x); }
+#else
+    static MFG_HD double fma(double a, double b, double c) { return __builtin_fma(a, b, c); }
+    static MFG_HD double mul(double a, double b) { return a * b; }
+    static MFG_HD double add(double a, double b) { return a + b; }
+    static MFG_HD double rcp(double x) { return 1.0 / x; }
+#endif
+};
+// Weight of one candidate, not normalised: linear / (eps + 13/12 t^2 + q^2/4)^2.
+MFG_HD double weno_front_weight(double t, double q, double linear) {
+    const double s = Rn::fma(Rn::mul(0.25, q), q, Rn::fma(Rn::mul(13.0 / 12.0, t), t, 1e-6));
+    const double r = Rn::rcp(s);
+    return Rn::mul(linear, Rn::mul(r, r));
+}
+MFG_HD double weno_front_edge(double a, double b, double c, double d, double e) {
+    const double w2 = weno_front_weight(Rn::add(Rn::fma(-2.0, b, a), c), Rn::fma(3.0, c, Rn::fma(-4.0, b, a)), 1.0);
+    const double w1 = weno_front_weight(Rn::add(Rn::fma(-2.0, c, b), d), Rn::add(b, -d), 6.0);
+    const double w0 = weno_front_weight(Rn::add(Rn::fma(-2.0, d, c), e), Rn::add(Rn::fma(3.0, c, Rn::mul(-4.0, d)), e), 3.0);
+    const double v2 = Rn::fma(11.0, c, Rn::fma(-7.0, b, Rn::mul(2.0, a)));
+    const double v1 = Rn::fma(2.0, d, Rn::fma(5.0, c, -b));
+    const double v0 = Rn::fma(5.0, d, Rn::fma(2.0, c, -e));
+    return Rn::mul(Rn::fma(w0, v0, Rn::fma(w1, v1, Rn::mul(w2, v2))), Rn::rcp(Rn::add(Rn::add(w2, w1), w0)));
 }
 
 // Weight of the first-order stencil (L, L, L, R, R, R) near the immersed
