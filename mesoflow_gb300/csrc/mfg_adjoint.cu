@@ -412,6 +412,19 @@ struct AdjCtr {
     bool ready;
 };
 
+// Beside a front (front_above: the stencil's differences far above the edge's two
+// cells c, d) the edge of the cells a .. e takes the FP64 weights of weno_edge_vjp,
+// as the forward flux does: the fixed-point ones are good to a fraction of the
+// largest difference only.  pb: the adjoint of its correction P = 3 (c + d) - 6
+// edge; returns P.  Not inlined: few edges come here.
+__device__ __noinline__ double front_edge_vjp(double a, double b, double c, double d, double e, double pb,
+                                              EdgeGrad& g) {
+    const double edge = weno_edge_vjp(a, b, c, d, e, -6.0 * pb, g);
+    g.c += 3.0 * pb;
+    g.d += 3.0 * pb;
+    return 3.0 * (c + d) - 6.0 * edge;
+}
+
 // Adjoint of the first-order fallback flux (fsum - lam D W)/2 (weno_collapsed):
 // W and d(D W)/dD.
 __device__ __forceinline__ void collapsed_weight(double D, double& W, double& dDW) {
@@ -482,12 +495,15 @@ __device__ __forceinline__ void adj_flux_sweep_body(const Fp& fp, const AdjBox& 
     };
     // differences D[q] between cells m-2+q and m-1+q, their adjoints, the direct
     // adjoints of cells m-2 .. m+2, the centres m-1, m, m+1
-    double v = value(-2), D[4], Db[4] = {0.0, 0.0, 0.0, 0.0}, vb[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, Dlast = 0.0;
+    double v = value(-2);
+    int mag[4];  // high words of the magnitudes of cells m-1 .. m+2
+    double D[4], Db[4] = {0.0, 0.0, 0.0, 0.0}, vb[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, Dlast = 0.0;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const double w = value(q - 1);
         D[q] = fp.sub(w, v);
         v = w;
+        mag[q] = hi_abs(v);
     }
     AdjCtr c0, c1, c2;
     c0.ready = c1.ready = c2.ready = false;
@@ -567,6 +583,24 @@ __device__ __forceinline__ void adj_flux_sweep_body(const Fp& fp, const AdjBox& 
             centre(c0, 0);
             centre(c1, 1);
             centre(c2, 2);
+            // the edges beside a front, by themselves
+            const int top = imax(imax(c0.w.eB, c1.w.eB), c2.w.eB);
+            const bool frontL = front_above(top, imax(mag[1], mag[2])), frontR = front_above(top, imax(mag[0], mag[1]));
+            double PR = 0.0;
+            if (frontL || frontR) {
+                const double x0 = value(-2), x1 = value(-1), x2 = value(0), x3 = value(1), x4 = value(2);
+                EdgeGrad g;
+                if (frontL) {
+                    pLval = front_edge_vjp(x0, x1, x2, x3, x4, pLb, g);
+                    vb[0] += g.a, vb[1] += g.b, vb[2] += g.c, vb[3] += g.d, vb[4] += g.e;
+                    pLb = 0.0;
+                }
+                if (frontR) {
+                    PR = front_edge_vjp(x4, x3, x2, x1, x0, pRb, g);
+                    vb[4] += g.a, vb[3] += g.b, vb[2] += g.c, vb[1] += g.d, vb[0] += g.e;
+                    pRb = 0.0;
+                }
+            }
             const WenoWeights w = weno_weights(c0.w.dB, c0.w.eB, c1.w.dC, c1.w.eC, c2.w.dA, c2.w.eA);
             const double W2L = weight_of(w.farL2), W0L = weight_of(w.nearL), W2R = weight_of(w.farR2),
                          W0R = weight_of(w.nearR);
@@ -585,8 +619,8 @@ __device__ __forceinline__ void adj_flux_sweep_body(const Fp& fp, const AdjBox& 
             c2.tb = fp.add(c2.tb, gpb);
             c1.tb = fp.add(c1.tb, fp.add(fp.add(pLb, pRb), fp.sub(gmb, gpb)));
             // the eigenvalue's adjoint of face m: (up - um) hb / 2 = -(hb/12) (P_left - P_right)
-            if (h && !is_zero_bits(lamH)) aadd(&FS_at(A, d, lamQ), fp.mul(lamH, fp.sub(lamP, fp.sub(t0, eR))));
-            pLval = fp.add(t0, eL);
+            if (h && !is_zero_bits(lamH)) aadd(&FS_at(A, d, lamQ), fp.mul(lamH, fp.sub(lamP, frontR ? PR : fp.sub(t0, eR))));
+            if (!frontL) pLval = fp.add(t0, eL);
         }
         reverse_centre(c0, 0);
         emit(0, Dlast);
@@ -607,6 +641,8 @@ __device__ __forceinline__ void adj_flux_sweep_body(const Fp& fp, const AdjBox& 
         }
 #pragma unroll
         for (int q = 0; q < 4; ++q) vb[q] = vb[q + 1];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) mag[q] = mag[q + 1];
         vb[4] = 0.0;
         Db[3] = 0.0;
         oc += sd;
@@ -616,6 +652,7 @@ __device__ __forceinline__ void adj_flux_sweep_body(const Fp& fp, const AdjBox& 
         const double w = value(2);
         D[3] = fp.sub(w, v);
         v = w;
+        mag[3] = hi_abs(v);
     }
     // the centres and cells left in the window
     reverse_centre(c1, 1);

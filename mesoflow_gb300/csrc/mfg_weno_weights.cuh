@@ -168,17 +168,20 @@ MFG_HD WenoWeights weno_weights(uint64_t dB, int eB, uint64_t dC, int eC, uint64
 // square counts to within 1.6 to 4.6 bits; the values' high words add as
 // logarithms do, to within a bit.  A ratio between 2^5.5 and 2^7.5 is the first to
 // count.  Infinities, NaN and values above 2^880 count too.
-constexpr int kFrontTop = 9;
+constexpr int kFrontTop = 9, kFrontMost = 1900 << 20;
+// Whether a stencil's differences (largest eB of its centres) are far above a value (high word of |v|).
+MFG_HD bool front_above(int top, int value) {
+    return top > imax((imin(value, kFrontMost) >> 19) + kFrontTop, 2 * kWenoExpFloor - 2);
+}
 MFG_HD int hi_abs(double x) { return (int)(bits_of(x) >> 32) & 0x7fffffff; }
 MFG_HD bool weno_front(int topf, int topu, bool pressure, double fL, double fR, double uL, double uR, double lam) {
-    const int one = 0x3ff00000, most = 1900 << 20, least = 2 * kWenoExpFloor - 2;
-    const int l = hi_abs(lam) - one;
-    int mu = imin(imax(hi_abs(uL), hi_abs(uR)), most), mf = imin((int)((unsigned)mu + (unsigned)l), most);
+    const int l = hi_abs(lam) - 0x3ff00000;
+    int mu = imin(imax(hi_abs(uL), hi_abs(uR)), kFrontMost), mf = (int)((unsigned)mu + (unsigned)l);
     if (pressure) {
-        mf = imin(imax(mf, imax(hi_abs(fL), hi_abs(fR))), most);
-        mu = imin(mf - l, most);
+        mf = imin(imax(mf, imax(hi_abs(fL), hi_abs(fR))), kFrontMost);
+        mu = mf - l;
     }
-    return topf > imax((mf >> 19) + kFrontTop, least) || topu > imax((mu >> 19) + kFrontTop, least);
+    return front_above(topf, mf) || front_above(topu, mu);
 }
 
 // Six times one WENO5-JS edge of the cells a .. e, far upwind to far downwind
