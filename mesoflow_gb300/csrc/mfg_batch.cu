@@ -1070,39 +1070,42 @@ void b_cutcells(mfg_boxlist& L, const PhaseTiles& T, cudaStream_t st) {
     NS_DISPATCH(bk_cut, (L.cut_grid, CUT_BT, 0, st), (L.d_cut, L.d_cutlist, L.d_count));
 }
 
+// The kernels of a right-hand side, one phase each: a step and the search over
+// tiles run the same ones.
+void b_prim(mfg_boxlist& L, const PhaseTiles& T, cudaStream_t st) {  // orders 4 and 5
+    ProfScope ps(K_PRIM, st);
+    NS_DISPATCH(bk_prim, (T.grid, BT, 0, st), (L.d_rhs, T.d, T.n));
+}
+void b_face(mfg_boxlist& L, const PhaseTiles& T, cudaStream_t st) {
+    ProfScope ps(K_FACE, st);
+    if (c_host_params().order_hyp >= 4) {
+        NS_DISPATCH(bk_face_high, (T.grid, BT, 0, st), (L.d_rhs, T.d, T.n));
+    } else {
+        NS_DISPATCH(bk_face, (T.grid, BT, 0, st), (L.d_rhs, T.d, T.n));
+    }
+}
+void b_flux(mfg_boxlist& L, const PhaseTiles& T, cudaStream_t st) {
+    ProfScope ps(K_FLUX, st);
+    if (flux_kind(L) == 2)
+        bk_flux_sweep<<<T.grid, SWEEP_BT, 0, st>>>(L.d_rhs, T.d, T.n);
+    else if (flux_kind(L) == 1)
+        bk_flux5_face<<<T.grid, SWEEP_BT, 0, st>>>(L.d_rhs, T.d, T.n);
+    else if (c_host_params().order_hyp == 4 && c_host_params().do_ns)
+        bk_flux4<<<T.grid, BT, 0, st>>>(L.d_rhs, T.d, T.n);
+    else
+        bk_flux<<<T.grid, BT, 0, st>>>(L.d_rhs, T.d, T.n);
+}
+void b_update(mfg_boxlist& L, const PhaseTiles& T, int stage, double dt, cudaStream_t st, const double* dtp) {
+    ProfScope ps(K_UPDATE, st);
+    bk_update<<<T.grid, BT, 0, st>>>(L.d_rhs, T.d, T.n, stage, dt, dtp);
+}
+
 void b_rhs(mfg_boxlist& L, const TSet& TS, int stage, double dt, cudaStream_t st, const double* dtp = nullptr) {
     const int ord = c_host_params().order_hyp;
-    if (ord >= 4) {
-        const PhaseTiles& T = TS[PH_GROWN];
-        ProfScope ps(K_PRIM, st);
-        NS_DISPATCH(bk_prim, (T.grid, BT, 0, st), (L.d_rhs, T.d, T.n));
-    }
-    {
-        const PhaseTiles& T = TS[PH_FACE];
-        ProfScope ps(K_FACE, st);
-        if (ord >= 4) {
-            NS_DISPATCH(bk_face_high, (T.grid, BT, 0, st), (L.d_rhs, T.d, T.n));
-        } else {
-            NS_DISPATCH(bk_face, (T.grid, BT, 0, st), (L.d_rhs, T.d, T.n));
-        }
-    }
-    if (!(c_host_params().do_ns && ord <= 2)) {
-        const PhaseTiles& T = TS[PH_FLUX];
-        ProfScope ps(K_FLUX, st);
-        if (flux_kind(L) == 2)
-            bk_flux_sweep<<<T.grid, SWEEP_BT, 0, st>>>(L.d_rhs, T.d, T.n);
-        else if (flux_kind(L) == 1)
-            bk_flux5_face<<<T.grid, SWEEP_BT, 0, st>>>(L.d_rhs, T.d, T.n);
-        else if (ord == 4 && c_host_params().do_ns)
-            bk_flux4<<<T.grid, BT, 0, st>>>(L.d_rhs, T.d, T.n);
-        else
-            bk_flux<<<T.grid, BT, 0, st>>>(L.d_rhs, T.d, T.n);
-    }
-    {
-        const PhaseTiles& T = TS[PH_UPDATE];
-        ProfScope ps(K_UPDATE, st);
-        bk_update<<<T.grid, BT, 0, st>>>(L.d_rhs, T.d, T.n, stage, dt, dtp);
-    }
+    if (ord >= 4) b_prim(L, TS[PH_GROWN], st);
+    b_face(L, TS[PH_FACE], st);
+    if (!(c_host_params().do_ns && ord <= 2)) b_flux(L, TS[PH_FLUX], st);
+    b_update(L, TS[PH_UPDATE], stage, dt, st, dtp);
 }
 
 // dtp (optional): device address of dt (mfg_boxlist_evolve's loop).
@@ -1988,9 +1991,10 @@ int mfg_boxlist_step_amr(mfg_boxlist* L, double time, double dt0, int mode, void
 }
 
 // Measured search over tile size and grid size for each batched phase: every
-// candidate runs the phase alone (the phases are idempotent on their inputs:
-// fill, cut cells, face scalars, fluxes, and the update with stage 0, which only
-// recomputes dsdt) and the fastest by CUDA events is kept.  results[] (optional,
+// candidate runs the phase alone, by the step's own launches and in its order, so
+// that each phase reads what the one before wrote (the phases are idempotent on
+// their inputs: fill, cut cells, face scalars, fluxes, and the update with stage
+// 0, which only recomputes dsdt), and the fastest by CUDA events is kept.  results[] (optional,
 // 3 doubles per phase: tile items, grid blocks, ms) reports the choice.
 int mfg_boxlist_autotune(mfg_boxlist* L, double dt, double* results, void* stream) {
     if (!L) return MFG_ERR_ARG;
@@ -2004,6 +2008,7 @@ int mfg_boxlist_autotune(mfg_boxlist* L, double dt, double* results, void* strea
     const int ord = c_host_params().order_hyp;
     for (int p = 0; p < PH_COUNT; ++p) {
         if (p == PH_FLUX && c_host_params().do_ns && ord <= 2) continue;
+        if (p == PH_FACE && ord >= 4) b_prim(*L, L->ph[PH_GROWN], st);  // what the face and flux phases read
         float best = 1e30f;
         int bt = L->ph[p].tile_items, bg = L->ph[p].grid_cap, bf = L->flux_form;
         const int nforms = (p == PH_FLUX && flux_sweep_mode()) ? 2 : 1;
@@ -2020,21 +2025,9 @@ int mfg_boxlist_autotune(mfg_boxlist* L, double dt, double* results, void* strea
                     switch (p) {
                         case PH_GROWN: b_fill(*L, P, 1, st); break;
                         case PH_VALID: b_cutcells(*L, P, st); break;
-                        case PH_FACE: {
-                            NS_DISPATCH(bk_face, (P.grid, BT, 0, st), (L->d_rhs, P.d, P.n));
-                            break;
-                        }
-                        case PH_FLUX:
-                            if (flux_kind(*L) == 2)
-                                bk_flux_sweep<<<P.grid, SWEEP_BT, 0, st>>>(L->d_rhs, P.d, P.n);
-                            else if (flux_kind(*L) == 1)
-                                bk_flux5_face<<<P.grid, SWEEP_BT, 0, st>>>(L->d_rhs, P.d, P.n);
-                            else if (ord == 4 && c_host_params().do_ns)
-                                bk_flux4<<<P.grid, BT, 0, st>>>(L->d_rhs, P.d, P.n);
-                            else
-                                bk_flux<<<P.grid, BT, 0, st>>>(L->d_rhs, P.d, P.n);
-                            break;
-                        case PH_UPDATE: bk_update<<<P.grid, BT, 0, st>>>(L->d_rhs, P.d, P.n, 0, dt, nullptr); break;
+                        case PH_FACE: b_face(*L, P, st); break;
+                        case PH_FLUX: b_flux(*L, P, st); break;
+                        case PH_UPDATE: b_update(*L, P, 0, dt, st, nullptr); break;
                     }
                     cudaEventRecord(e1, st);
                     cudaEventSynchronize(e1);
