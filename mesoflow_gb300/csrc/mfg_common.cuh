@@ -188,10 +188,11 @@ __device__ __forceinline__ double rcp_pos(double x) {
     return fma(r, fma(e, e, e), r);
 }
 
-// n / x for a positive, finite, normal x: the hardware approximation r0 of 1/x
-// (relative error e <= 2^-23) corrected by 1/x = r0 (1 + e + e^2 + O(e^3)),
-// e = 1 - x r0, applied to n r0: four FP64 operations, within about one ulp.
-__device__ __forceinline__ double quot_pos(double n, double x) {
+// n / x for a finite normal x and a finite n whose product with 1/x is one too:
+// the hardware approximation r0 of 1/x (relative error e <= 2^-23) corrected by
+// 1/x = r0 (1 + e + e^2 + O(e^3)), e = 1 - x r0, applied to n r0: four FP64
+// operations, within about one ulp.
+__device__ __forceinline__ double quot_mid(double n, double x) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
     const double e = __fma_rn(-x, r, 1.0);
@@ -199,17 +200,25 @@ __device__ __forceinline__ double quot_pos(double n, double x) {
     return __fma_rn(q, __fma_rn(e, e, e), q);
 }
 
-// Square root of x >= 0, normal or zero (NaN below zero): the hardware
-// approximation y of 1/sqrt(x) (relative error about 2^-22) corrected by
-// sqrt(x) = x y (1 + e/2 + 3 e^2/8 + O(e^3)), e = 1 - x y^2: five FP64
-// operations, within about one ulp.
-__device__ __forceinline__ double sqrt_nonneg(double x) {
+// n / x: that for magnitudes of x between 2^-500 and 2^500 and of n below 2^500,
+// the division itself for everything else, so infinities, zeros and subnormal
+// numbers give what it gives.
+__device__ __forceinline__ double quot(double n, double x) {
+    const unsigned hn = (unsigned)__double2hiint(n) & 0x7fffffffu, hx = (unsigned)__double2hiint(x) & 0x7fffffffu;
+    return (hx - (523u << 20) < (1000u << 20) && hn < (1523u << 20)) ? quot_mid(n, x) : __ddiv_rn(n, x);
+}
+
+// Square root of x: for a positive normal number the hardware approximation y of
+// 1/sqrt(x) (relative error about 2^-22) corrected by sqrt(x) = x y (1 + e/2 + 3
+// e^2/8 + O(e^3)), e = 1 - x y^2: five FP64 operations, within about one ulp.  The
+// library's for zeros, subnormal and negative numbers, infinity and NaN.
+__device__ __forceinline__ double sqrt_fast(double x) {
+    if ((unsigned)__double2hiint(x) - 0x00100000u >= 0x7fe00000u) return __dsqrt_rn(x);
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
     const double t = __dmul_rn(x, y);
     const double e = __fma_rn(-t, y, 1.0);
-    const double r = __fma_rn(t, __dmul_rn(e, __fma_rn(0.375, e, 0.5)), t);
-    return is_zero_bits(x) ? x : r;
+    return __fma_rn(t, __dmul_rn(e, __fma_rn(0.375, e, 0.5)), t);
 }
 
 // Copies nc components of one cell, src and dst component strides ss and ds,

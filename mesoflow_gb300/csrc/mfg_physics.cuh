@@ -111,7 +111,7 @@ __device__ __forceinline__ double thermo_kappa(double rho, const double* spec) {
     if (c_P.thermo_kind == MFG_THERMO_MASS_SINGLE) return c_P.gm1_single;
     double n, d;
     thermo_ratio<NS>(rho, spec, n, d);
-    return quot_pos(n, d);
+    return quot(n, d);
 }
 
 // Pressure from (rho e, rho, species).
@@ -134,7 +134,7 @@ __device__ __forceinline__ void thermo_pt(double rhoe, double rho, double irho, 
     }
     double n, d;
     thermo_ratio<NS>(rho, spec, n, d);
-    T = quot_pos(rhoe, d);
+    T = quot(rhoe, d);
     p = n * T;
 }
 
@@ -205,7 +205,7 @@ __device__ __forceinline__ double face_diffusivity(const DevParams& P, int s, do
     if (is_zero_bits(vL) && is_zero_bits(vR)) return P.diff_hms[s];
     const double g = P.diff_gas[s], so = P.diff_solid[s];
     const double dl = __fma_rn(g, vL, mul(so, sub(1.0, vL))), dr = __fma_rn(g, vR, mul(so, sub(1.0, vR)));
-    return quot_pos(mul(mul(2.0, dl), dr), add(add(dl, dr), 1e-30));
+    return quot_mid(mul(mul(2.0, dl), dr), add(add(dl, dr), 1e-30));  // the divisor is at least 1e-30
 }
 
 }  // namespace mfg

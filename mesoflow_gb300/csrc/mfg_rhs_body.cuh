@@ -98,7 +98,7 @@ __device__ __forceinline__ void weno_face(const double s[6], double& up, double&
 // flux_schemes.H:21-43).  Explicit roundings: equal states give equal speeds
 // wherever it is compiled (the adjoint compares the two sides of a face).
 __device__ __forceinline__ double eig_speed(double gam, double kap, double rhoe, double irho) {
-    return sqrt_nonneg(__dmul_rn(__dmul_rn(gam, __dmul_rn(kap, rhoe)), irho));
+    return sqrt_fast(__dmul_rn(__dmul_rn(gam, __dmul_rn(kap, rhoe)), irho));
 }
 
 // ---------------------------------------------------------------------------
