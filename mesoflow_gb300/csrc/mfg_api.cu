@@ -291,9 +291,11 @@ int mfg_init(const mfg_params* p) {
     for (int s = 0; s <= p->ngas && s <= MFG_MAX_SPECIES; ++s) {
         if (s == p->ngas && p->thermo_kind != MFG_THERMO_BG_GAS) break;
         h.cv[s] = R / (p->gamma[s] - 1.0);
-        h.igm1[s] = 1.0 / (p->gamma[s] - 1.0);
+        h.igd[s] = 1.0 / (p->gamma[s] - 1.0);
+        h.ig_min = s ? std::min(h.ig_min, h.igd[s]) : h.igd[s];
         if (s < p->ngas && p->molwt[s] != 0.0) h.cvmass[s] = R / (p->gamma[s] - 1.0) / p->molwt[s];
     }
+    for (int s = 0; s <= MFG_MAX_SPECIES; ++s) h.igd[s] -= h.ig_min;
     auto hmean = [](double d1, double d2) { return 2.0 * d1 * d2 / (d1 + d2 + 1e-30); };
     h.visc_hm = hmean(p->visc_gas, p->visc_gas);
     h.cond_hm = hmean(p->cond_gas, p->cond_gas);

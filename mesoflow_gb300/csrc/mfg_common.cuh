@@ -33,7 +33,7 @@ struct DevParams {
     double molwt[MAXS];
     double gamma[MAXS + 1];
     double cv[MAXS + 1];       // R/(gamma_k - 1) per gas species (+ background gas)
-    double igm1[MAXS + 1];     // 1/(gamma_k - 1)
+    double ig_min, igd[MAXS + 1];  // smallest 1/(gamma_k - 1) of the gases, and each one's excess over it
     double cvmass[MAXS];       // R/(gamma_k - 1)/W_k (mass-cv energy form)
     double advect_flag[MAXS];
     int visc_mode, cond_mode;
