@@ -1,6 +1,7 @@
-"""Rounding errors against extended precision: the pressure of a mixture has an rms
-error no larger than the reference's own order of operations in double precision
-(the oracle's)."""
+"""Rounding errors against extended precision: the pressure of a mixture, and
+fluxes whose exact value is plain (order 1 along lines of
+constant state), have an rms error no larger than the reference's own order of
+operations in double precision (the oracle's)."""
 import ctypes as C
 
 import numpy as np
@@ -79,3 +80,27 @@ def test_pressure(name):
     ref = pressure(P, S[:, G:-G, G:-G, G:-G])
     print(name, rms(o, ref) / 2.0 ** -53, rms(k, ref) / 2.0 ** -53)
     assert rms(k, ref) <= rms(o, ref)
+
+
+def rhs(P):
+    return lambda lib, oracle, d, g: lib.oracle_compute_dsdt(C.byref(P), C.byref(g), d, 1) if oracle else \
+        lib.mfg_compute_dsdt_flow(d, 1, C.byref(g), 0.0, 1e-6, None)
+
+
+@pytest.mark.parametrize("name", ["five", "one"])
+@pytest.mark.parametrize("d", [0, 1, 2])
+def test_order1_momentum_of_constant_lines(name, d):
+    """Both sides of a face alike: the flux of the normal momentum is rho v^2 + p."""
+    P, rng = params(name, 1), np.random.default_rng(3)
+    shape = tuple(q + 2 * G for q in N[::-1])
+    S = state(P, shape, rng, [100.0 * rng.standard_normal(shape) for _ in range(3)])
+    ax = 3 - d
+    S = np.repeat(np.take(S, [0], axis=ax), S.shape[ax], axis=ax)
+    S[abi.VELX:abi.VELZ + 1] = 0.0  # no viscous terms
+    o, k = run(P, S, N, rhs(P))
+    one = tuple(slice(0, 1) if a == ax - 1 else slice(G, -G) for a in range(3))
+    ref = pressure(P, S)[one] + L(S[abi.RHOU + d][one]) ** 2 / S[abi.RHO][one]
+    x, y = (np.take(np.asarray(v.flux[0][d][abi.RHOU + d].cpu() if v is k else v.flux[0][d][abi.RHOU + d]), [1], axis=ax - 1)
+            for v in (o, k))
+    print(name, d, rms(x, ref) / 2.0 ** -53, rms(y, ref) / 2.0 ** -53)
+    assert rms(y, ref) <= rms(x, ref)
