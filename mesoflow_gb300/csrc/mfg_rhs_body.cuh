@@ -908,11 +908,13 @@ __device__ __forceinline__ void flux5_face_body(const Fp& fp, const RhsBox& B, i
 
 // Order 4, central with dissipation (the reference's central_with_diss_flux:
 // (7 (f_L + f_R) - f_LL - f_RR - lam dissfactor (3 u_R - 3 u_L - u_RR + u_R))
-// / 12): one thread per (face, component), the four cells it reads as the
-// order-5 sweep takes them (one or two FP64 operations each, against six cells
-// of the general Euler flux before), half, flag and viscous term in one
-// multiply-add: about 16 FP64 operations against 60 (right-hand side of 57x64x33
-// cells 287 -> 217 us).
+// / 12, its twelfth rounded to ten digits): one thread per (face, component), the
+// four cells it reads as the order-5 sweep takes them (one or two FP64 operations
+// each, against six cells of the general Euler flux before), half, flag and viscous
+// term in one multiply-add: about 16 FP64 operations against 60 (right-hand side of
+// 57x64x33 cells 287 -> 217 us).  The outer cells are added to the dissipation before
+// they leave seven times the inner sum: one rounding of that size, where the terms in
+// turn had two to four.
 __device__ __forceinline__ void flux4_body(const Fp& fp, const RhsBox& B, int d, int c, int64_t t) {
     int len[3];
     for (int e = 0; e < 3; ++e) len[e] = B.hi[e] - B.lo[e] + 1 + (e == d);
@@ -935,8 +937,8 @@ __device__ __forceinline__ void flux4_body(const Fp& fp, const RhsBox& B, int d,
             flux5_cell(fp, x, oR + at * sd, xR + at * xd, u[q], fl[q]);
         }
         D = fp.sub(u[2], u[1]);
-        S = __fma_rn(-lam, __fma_rn(3.0, D, fp.sub(u[2], u[3])),
-                     fp.sub(__fma_rn(7.0, fp.add(fl[2], fl[1]), -fl[0]), fl[3]));
+        const double outer = __fma_rn(lam, __fma_rn(3.0, D, fp.sub(u[2], u[3])), fp.add(fl[0], fl[3]));
+        S = __fma_rn(7.0, fp.add(fl[1], fl[2]), -outer);
     } else {
         D = fp.sub(x.u[oR], x.u[oR - sd]);
     }

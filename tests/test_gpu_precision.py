@@ -1,5 +1,5 @@
 """Rounding errors against extended precision: the pressure of a mixture, and
-fluxes whose exact value is plain (order 1 along lines of
+fluxes whose exact value is plain (order 4 of a gas at rest, order 1 along lines of
 constant state), have an rms error no larger than the reference's own order of
 operations in double precision (the oracle's)."""
 import ctypes as C
@@ -85,6 +85,25 @@ def test_pressure(name):
 def rhs(P):
     return lambda lib, oracle, d, g: lib.oracle_compute_dsdt(C.byref(P), C.byref(g), d, 1) if oracle else \
         lib.mfg_compute_dsdt_flow(d, 1, C.byref(g), 0.0, 1e-6, None)
+
+
+@pytest.mark.parametrize("name", ["five", "one"])
+def test_order4_momentum_at_rest(name):
+    P, rng = params(name, 4), np.random.default_rng(2)
+    shape = tuple(q + 2 * G for q in N[::-1])
+    S = state(P, shape, rng, [np.zeros(shape)] * 3)
+    o, k = run(P, S, N, rhs(P))
+    p = pressure(P, S)
+    for d in range(3):
+        ax = 2 - d
+        f = [np.moveaxis(p[tuple(slice(None) if a == ax else slice(G, -G) for a in range(3))], ax, -1)[..., G - 2 + q:]
+             for q in range(4)]
+        m = N[d] + 1
+        ref = L(0.08333333333) * (7 * (f[1][..., :m] + f[2][..., :m]) - f[0][..., :m] - f[3][..., :m])
+        x, y = (np.moveaxis(np.asarray(v.flux[0][d][abi.RHOU + d].cpu() if v is k else v.flux[0][d][abi.RHOU + d]), ax, -1)
+                for v in (o, k))
+        print(name, d, rms(x, ref) / 2.0 ** -53, rms(y, ref) / 2.0 ** -53)
+        assert rms(y, ref) <= rms(x, ref)
 
 
 @pytest.mark.parametrize("name", ["five", "one"])
