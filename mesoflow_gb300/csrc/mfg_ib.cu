@@ -624,14 +624,19 @@ CutLevelTable* level_prepare(const std::vector<LevelCutBox>& tab) {
 // itself, so those boxes give that path's results by construction).  Returns 1
 // when done, -1 on a CUDA error, and 0, having launched nothing, where the
 // per-box path must run: cache off, conjugate heat transfer (its
-// neighbour-temperature scratch is per box), a box without an entry, or a
-// table to build during capture.
+// neighbour-temperature scratch is per box), a box without an entry, boxes that
+// share an array (tiles: an array has one entry, and the second box's replaces the
+// first's), or a table to build during capture.
 int launch_cutcells_level(const mfg_box* boxes, int nbox, const mfg_geom& g, cudaStream_t st) {
     if (nbox < 1 || !g_cache.enabled || c_host_params().conj_ht) return 0;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return 0;
     const double dxmin = fmin(g.dx[0], fmin(g.dx[1], g.dx[2]));
     if (ensure_wdir(g, dxmin, st) != cudaSuccess) return -1;
+    std::vector<const double*> arrays(nbox);
+    for (int b = 0; b < nbox; ++b) arrays[b] = boxes[b].sborder.p;
+    std::sort(arrays.begin(), arrays.end());
+    if (std::adjacent_find(arrays.begin(), arrays.end()) != arrays.end()) return 0;
     std::vector<LevelCutBox> tab(nbox);
     std::vector<int> slots(nbox);
     for (int b = 0; b < nbox; ++b) {
