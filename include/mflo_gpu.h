@@ -321,9 +321,9 @@ int mfg_set_weno_mode(int fast);
  * fluid neighbour, about 0.3 KiB per cut cell in a sphere pack), and
  * every later call checks the box's grown volume fraction against a stored
  * copy on the device (exact) before using them: values that moved between the
- * same gas, cut and solid cells refresh the weights on the device, a changed
- * geometry falls back to recomputation in the same call and is out of use until
- * it is built anew.  Results are bitwise the same either way.  enable = 0 frees the cache.  Synchronizes. */
+ * same gas, cut and solid cells refresh the weights on the device, another
+ * geometry falls back to recomputation in the same call, until the stored one
+ * comes back or is built anew.  Results are bitwise the same either way.  enable = 0 frees the cache.  Synchronizes. */
 int mfg_set_cutcell_cache(int enable);
 
 /* Form of the face pass of orders 1 and 2 with Navier-Stokes terms

@@ -32,9 +32,9 @@
 //   another state of the same geometry): the entries' weights are recomputed
 //   in place, then applied;
 //   another gas, cut or solid cell anywhere: the list is rebuilt and the
-//   weights computed on the fly in the same call, and the entry is out of use
-//   until cutcache_sweep (called where the host synchronizes anyway) drops it
-//   and the next call builds it anew.
+//   weights computed on the fly in the same call; the entry waits for its own
+//   geometry to come back (mfg_cut_flags.h), or cutcache_sweep (called where the
+//   host synchronizes anyway) drops it and the next call builds it anew.
 // No host round trip is needed, no stale weight is ever applied, and all paths
 // give bitwise equal results.  (Dropping an entry at every drift cost a host
 // sort and a dozen allocations per box in each of a state's first steps: the
@@ -44,6 +44,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "mfg_cut_flags.h"
 #include "mfg_ib_body.cuh"
 
 namespace mfg {
@@ -53,12 +54,6 @@ __constant__ double c_wdir[125];
 namespace {
 
 constexpr int TPB = 128;
-// An entry's flag.  VF_MOVED: some value differs from the copy in this call (or
-// did in an earlier one of the box alone: a refresh then changes nothing);
-// VF_OTHER: since the entry was built some cell changed between gas, cut and
-// solid (kept until the entry is dropped).
-constexpr unsigned VF_MOVED = 1u, VF_OTHER = 2u;
-
 // Conjugate heat transfer: mean temperature of the 26 neighbours, read before
 // any cut cell is updated (ib_utils.H:345-364).
 __global__ void cht_avg_kernel(CutBox c) {
@@ -77,10 +72,10 @@ __global__ void cht_avg_kernel(CutBox c) {
 }
 
 // Appends the linear index of every cut cell (0 < vfrac < 1) of the box to
-// list; with a non-null flag, only when it has VF_OTHER.
+// list; with a non-null flag, only when the entry cannot be applied.
 __global__ void cut_list_kernel(CutBox c, int* __restrict__ list, unsigned* __restrict__ count,
                                 const unsigned* __restrict__ flag) {
-    if (flag && !(*flag & VF_OTHER)) return;
+    if (flag && vf_apply(*flag)) return;
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     bool cut = false;
     if (t < c.n) {
@@ -106,15 +101,16 @@ struct CutGroup {
     CutBox c[CUT_GROUP];
     const int* list[CUT_GROUP];
     const unsigned* count[CUT_GROUP];
-    unsigned* moved[CUT_GROUP];  // change flags whose VF_MOVED the launch clears, or null
+    unsigned* flag[CUT_GROUP];  // the entries' flags, which the launch closes (vf_after), or null
 };
 template <int NS>
 __global__ void __launch_bounds__(TPB) cutcell_kernel(const __grid_constant__ CutGroup g) {
     const unsigned n = *g.count[blockIdx.y];
     const int* __restrict__ list = g.list[blockIdx.y];
     const CutBox& c = g.c[blockIdx.y];
-    // the last launch of a level's pass, and no block of it reads the flag
-    if (g.moved[blockIdx.y] && blockIdx.x == 0 && threadIdx.x == 0) *g.moved[blockIdx.y] &= VF_OTHER;
+    // the last launch of a pass, and no block of it reads the flag
+    unsigned* flag = g.flag[blockIdx.y];
+    if (flag && blockIdx.x == 0 && threadIdx.x == 0) *flag = vf_after(*flag);
     if (blockIdx.x * blockDim.x >= n) return;
     __shared__ CutShared<TPB> sm;
     cut_shared_init(sm);
@@ -122,20 +118,10 @@ __global__ void __launch_bounds__(TPB) cutcell_kernel(const __grid_constant__ Cu
         cutcell_one<NS>(c, list[w], sm);
 }
 
-__device__ __forceinline__ int vf_kind(double v) { return is_one(v) ? 2 : (v > 0.0 && v < 1.0) ? 1 : 0; }
-
-// One grown cell's volume fraction against the copy, which takes the new value;
-// the warp's flag bits are raised by one lane.
+// One grown cell's volume fraction against the copy (vf_change); the warp's flag
+// bits are raised by one lane.
 __device__ __forceinline__ void vf_compare(bool in, double v, double* copy, unsigned* flag) {
-    unsigned f = 0;
-    if (in) {
-        const double old = *copy;
-        if (__double_as_longlong(v) != __double_as_longlong(old)) {
-            f = VF_MOVED | (vf_kind(v) != vf_kind(old) ? VF_OTHER : 0u);
-            *copy = v;
-        }
-    }
-    f = __reduce_or_sync(0xffffffffu, f);
+    const unsigned f = __reduce_or_sync(0xffffffffu, in ? vf_change(v, copy) : 0u);
     if (f && (threadIdx.x & 31) == 0) atomicOr(flag, f);
 }
 
@@ -153,8 +139,6 @@ __global__ void cut_vf_kernel(Fab S, int lo0, int lo1, int lo2, int l0, int l1, 
     }
     if (mode == 1) vf_compare(in, v, vf + t, flag);
 }
-
-__global__ void cut_flag_reset_kernel(unsigned* flag) { *flag &= VF_OTHER; }
 
 __global__ void cut_count_kernel(CutBox c, const int* __restrict__ list, unsigned n, int* __restrict__ kc) {
     const unsigned w = blockIdx.x * blockDim.x + threadIdx.x;
@@ -175,7 +159,7 @@ __global__ void cut_entries_kernel(CutBox c, CutCacheView cc, unsigned n, int* o
 // written afresh by a loop over the 125 positions).
 __global__ void __launch_bounds__(TPB) cut_refresh_kernel(CutBox c, CutCacheView cc, unsigned n,
                                                           const unsigned* __restrict__ flag) {
-    if (*flag != VF_MOVED || blockIdx.x * TPB >= n) return;
+    if (!vf_refresh(*flag) || blockIdx.x * TPB >= n) return;
     __shared__ CutShared<TPB> sm;
     cut_shared_init(sm);
     for (unsigned w = blockIdx.x * TPB + threadIdx.x; w < n; w += gridDim.x * TPB)
@@ -183,12 +167,12 @@ __global__ void __launch_bounds__(TPB) cut_refresh_kernel(CutBox c, CutCacheView
                                const_cast<double*>(cc.scal), sm);
 }
 
-// Stored entries, unless the entry is out of use.  The grid stride is a
+// Stored entries, unless they do not fit this pass's geometry.  The grid stride is a
 // multiple of 32, so a warp always holds one group of 32 list positions.
 template <int NS>
 __global__ void __launch_bounds__(TPB) cutcell_cached_kernel(CutBox c, CutCacheView cc, unsigned ncut,
                                                              const unsigned* __restrict__ flag) {
-    if (*flag & VF_OTHER) return;
+    if (!vf_apply(*flag)) return;
     for (unsigned w = blockIdx.x * blockDim.x + threadIdx.x; w < ncut; w += gridDim.x * blockDim.x)
         cutcell_cached<NS>(c, (int)w, cc);
 }
@@ -206,8 +190,7 @@ struct LevelCutBox {
 };
 
 // Grown volume fraction against the stored copy (blockIdx.y = box); clears the
-// box's rebuilt-list count.  VF_MOVED is clear from the last pass (or, after a
-// pass of the box alone, asks for a refresh that changes nothing).
+// box's rebuilt-list count.
 __global__ void cut_level_vf_kernel(const LevelCutBox* __restrict__ tab, unsigned* __restrict__ cnt) {
     const LevelCutBox& L = tab[blockIdx.y];
     if (blockIdx.x == 0 && threadIdx.x == 0) cnt[blockIdx.y] = 0;
@@ -223,23 +206,22 @@ __global__ void cut_level_vf_kernel(const LevelCutBox* __restrict__ tab, unsigne
 }
 
 // What a box's change asks for (blockIdx.y = box), in one launch: the weights
-// refreshed as cut_refresh_kernel does, or, where its entry is out of use, its
+// refreshed as cut_refresh_kernel does, or, where its entry does not fit, its
 // cut cells listed afresh (grid-stride over the box; one atomic per warp).
 __global__ void __launch_bounds__(TPB) cut_level_change_kernel(const LevelCutBox* __restrict__ tab,
                                                                unsigned* __restrict__ cnt, int* __restrict__ lists,
                                                                int64_t cap) {
     const LevelCutBox& L = tab[blockIdx.y];
     const unsigned flag = *L.dirty;
-    if (!flag) return;
-    if (flag == VF_MOVED) {
+    if (vf_refresh(flag)) {
         if (blockIdx.x * TPB >= L.ncut) return;
         __shared__ CutShared<TPB> sm;
         cut_shared_init(sm);
         for (unsigned w = blockIdx.x * TPB + threadIdx.x; w < L.ncut; w += gridDim.x * TPB)
             cut_entries_one<false>(L.c, (int)w, L.v, nullptr, const_cast<double*>(L.v.wn), nullptr,
                                    const_cast<double*>(L.v.scal), sm);
-        return;
     }
+    if (vf_apply(flag)) return;
     const CutBox& c = L.c;
     int* list = lists + (int64_t)blockIdx.y * cap;
     for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < c.n; base += (int64_t)gridDim.x * blockDim.x) {
@@ -271,7 +253,7 @@ __global__ void __launch_bounds__(TPB) cutcell_level_kernel(const LevelCutBox* _
     if (gw >= ngroups) return;
     const int2 bg = groups[gw];
     const LevelCutBox& L = tab[bg.x];
-    if (*L.dirty & VF_OTHER) return;
+    if (!vf_apply(*L.dirty)) return;
     const unsigned w = 32u * (unsigned)bg.y + (threadIdx.x & 31);
     if (w < L.ncut) cutcell_cached<NS>(L.c, (int)w, L.v);
 }
@@ -490,14 +472,14 @@ CutEntry* find_entry(const mfg_box& b, const CutBox& c, const mfg_geom& g, cudaS
 
 }  // namespace
 
-// Drops the entries that are out of use (another geometry); the host has
-// synchronized the stream before.
+// Drops the entries that did not fit in their last pass (another geometry); the
+// host has synchronized the stream before.
 void cutcache_sweep() {
     if (g_cache.map.empty() || !g_cache.dirty) return;
     std::vector<unsigned> h(g_cache.nslots);
     if (cudaMemcpy(h.data(), g_cache.dirty, h.size() * sizeof(unsigned), cudaMemcpyDeviceToHost) != cudaSuccess) return;
     for (auto it = g_cache.map.begin(); it != g_cache.map.end();) {
-        if (it->second.slot >= 0 && (h[it->second.slot] & VF_OTHER)) {
+        if (it->second.slot >= 0 && (h[it->second.slot] & (VF_OTHER | VF_LEFT))) {
             free_entry(it->second);
             it = g_cache.map.erase(it);
         } else {
@@ -617,11 +599,12 @@ CutLevelTable* level_prepare(const std::vector<LevelCutBox>& tab) {
 
 }  // namespace
 
-// All boxes of a level in five launches (flags cleared, volume fractions
-// compared, moved boxes' weights refreshed, lists of boxes out of use rebuilt,
-// stored entries applied) plus the on-the-fly launch for sixteen boxes at a
-// time, which works only where a box is out of use (the cache-off kernel
-// itself, so those boxes give that path's results by construction).  Returns 1
+// All boxes of a level in three launches (volume fractions compared; moved boxes'
+// weights refreshed or other geometries' cells listed; stored entries applied, none
+// without a stored cell) plus the on-the-fly launch for sixteen boxes at a
+// time, which works only where a box's entry does not fit (the cache-off kernel
+// itself, so those boxes give that path's results by construction) and closes the
+// flags.  Returns 1
 // when done, -1 on a CUDA error, and 0, having launched nothing, where the
 // per-box path must run: cache off, conjugate heat transfer (its
 // neighbour-temperature scratch is per box), a box without an entry, boxes that
@@ -680,7 +663,7 @@ int launch_cutcells_level(const mfg_box* boxes, int nbox, const mfg_geom& g, cud
                 cg.c[q] = tab[w].c;                                                                         \
                 cg.list[q] = g_level.d_lists + (int64_t)w * T->cap;                                         \
                 cg.count[q] = g_level.d_cnt + w;                                                            \
-                cg.moved[q] = tab[w].dirty;                                                                 \
+                cg.flag[q] = tab[w].dirty;                                                                 \
             }                                                                                               \
             cutcell_kernel<K><<<dim3(152, n), TPB, 0, st>>>(cg);                                            \
         }                                                                                                   \
@@ -702,7 +685,7 @@ cudaError_t launch_cutcells_box(const mfg_box& b, const mfg_geom& g, double* tch
     const unsigned nb = (unsigned)((c.n + TPB - 1) / TPB);
     const int ns = c_host_params().nspec;
     CutEntry* ce = find_entry(b, c, g, st);
-    ProfScope ps(K_CUT, st, (ce ? 6 : 2) + (c_host_params().conj_ht ? 1 : 0));
+    ProfScope ps(K_CUT, st, (ce ? 5 : 2) + (c_host_params().conj_ht ? 1 : 0));
     if (c_host_params().conj_ht) cht_avg_kernel<<<nb, TPB, 0, st>>>(c);
     cudaMemsetAsync(count, 0, sizeof(unsigned), st);
     const unsigned ng = (unsigned)std::min<int64_t>(std::max<int64_t>(nb, 1), 152 * 8);
@@ -711,7 +694,6 @@ cudaError_t launch_cutcells_box(const mfg_box& b, const mfg_geom& g, double* tch
         flag = g_cache.dirty + ce->slot;
         const int l0 = c.len[0] + 6, l1 = c.len[1] + 6, l2 = c.len[2] + 6;
         const int64_t ngc = (int64_t)l0 * l1 * l2;
-        cut_flag_reset_kernel<<<1, 1, 0, st>>>(flag);
         cut_vf_kernel<<<(unsigned)((ngc + 255) / 256), 256, 0, st>>>(c.S, b.lo[0] - 3, b.lo[1] - 3, b.lo[2] - 3, l0,
                                                                       l1, l2, ce->vf, flag, 1);
         cut_refresh_kernel<<<ng, TPB, 0, st>>>(c, ce->view(), ce->ncut, flag);
@@ -723,7 +705,7 @@ cudaError_t launch_cutcells_box(const mfg_box& b, const mfg_geom& g, double* tch
         else cutcell_cached_kernel<16><<<ng, TPB, 0, st>>>(MFG_CUT_ARGS);
 #undef MFG_CUT_ARGS
     }
-    // the on-the-fly form: without an entry, or where the entry is out of use
+    // the on-the-fly form: without an entry, or where it does not fit
     // (a fixed grid walks the list, whose length stays on the device)
     cut_list_kernel<<<nb, TPB, 0, st>>>(c, list, count, flag);
     CutGroup cg;
@@ -731,7 +713,7 @@ cudaError_t launch_cutcells_box(const mfg_box& b, const mfg_geom& g, double* tch
         cg.c[q] = c;
         cg.list[q] = list;
         cg.count[q] = count;
-        cg.moved[q] = nullptr;
+        cg.flag[q] = flag;
     }
     if (ns <= 1) cutcell_kernel<1><<<ng, TPB, 0, st>>>(cg);
     else if (ns <= 2) cutcell_kernel<2><<<ng, TPB, 0, st>>>(cg);
