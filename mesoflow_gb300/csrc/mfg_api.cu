@@ -304,7 +304,6 @@ int mfg_init(const mfg_params* p) {
         h.diff_hms[s] = hmean(p->diff_solid[s], p->diff_solid[s]);
     }
     if (p->thermo_kind == MFG_THERMO_MASS_SINGLE) {
-        h.g_gm1 = p->gamma_single / (p->gamma_single - 1.0);
         h.astar_fac = (2.0 * (p->gamma_single - 1.0)) / (p->gamma_single + 1.0);
         h.gm1_single = p->gamma_single - 1.0;
         h.inv_gas_R = 1.0 / p->gas_R;

@@ -42,8 +42,8 @@ struct DevParams {
     double diff_gas[MAXS], diff_solid[MAXS];
     // face coefficients of constant transport: harmonic_mean(g, g), evaluated once
     double visc_hm, cond_hm, diff_hm[MAXS], diff_hms[MAXS];  // diff_hms: between solid cells (blended transport)
-    // gamma/(gamma-1) and 2(gamma-1)/(gamma+1) of the mass-single family
-    double g_gm1, astar_fac, gm1_single, inv_gas_R;
+    // 2(gamma-1)/(gamma+1), gamma-1 and 1/R of the mass-single family
+    double astar_fac, gm1_single, inv_gas_R;
     int order_hyp, do_ns, species_in_solid, conj_ht;
     double dissfactor, solid_temp, cfl;
     int chem_on, nreact;
@@ -236,9 +236,5 @@ __device__ __forceinline__ void copy_comps(double* dst, int64_t ds, const double
     }
     for (; c < nc; ++c) dst[c * ds] = __ldg(src + c * ss);
 }
-
-// The same refinement for a finite, normal x of either sign (the hardware
-// approximation and the correction are odd in x).
-__device__ __forceinline__ double rcp_nonzero(double x) { return rcp_pos(x); }
 
 }  // namespace mfg

@@ -213,9 +213,6 @@ __global__ void axpy_kernel(Valid v, Fab dst, Fab src, double a, int copy_first,
 
 inline unsigned nblocks(int64_t n) { return (unsigned)((n + TPB - 1) / TPB); }
 
-template <template <int> class K>
-struct Dispatch;
-
 }  // namespace
 
 cudaError_t launch_chem_source(const mfg_box& b, cudaStream_t st) {
