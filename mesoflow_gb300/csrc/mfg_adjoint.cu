@@ -1609,7 +1609,7 @@ constexpr int kAdjSeg = 16;  // faces per column segment of the batched adjoint 
 struct Snap {
     double* sb[3];   // stage states after the cut cells (grown)
     double* aux[3];  // per-cell primitives of each stage (grown, NAUX components)
-    double* fs[3];   // face scalars of each stage (NFS per face, three directions)
+    double* fs[3];   // face scalars of each stage (FS_USED per face, three directions)
     double* s3;      // flow result = chemistry input (valid)
     double* sc;      // chemistry result (valid)
     double* sp;      // after the primitive refresh, before clipping (valid)
@@ -1846,7 +1846,7 @@ extern "C" int mfg_adjoint_objective(const mfg_box* boxes, int nbox, const mfg_g
         W.gcell[b] = W.gtot;
         for (int d = 0; d < 3; ++d) {
             W.fsoff.push_back(W.fstot);
-            W.fstot += face_doubles(n, d, NFS);
+            W.fstot += face_doubles(n, d, FS_USED);
         }
         W.vtot += (size_t)n[0] * n[1] * n[2];
         W.gtot += (size_t)(n[0] + 6) * (n[1] + 6) * (n[2] + 6);

@@ -17,7 +17,8 @@ enum FsComp {
     FS_VIS,        // 3: viscous momentum terms tau_{d,a}
     FS_VISE = FS_VIS + 3,   // viscous work sum_a tau_{d,a} * facevel_a
     FS_THERM = FS_VISE + 1, // heat-conduction term k dT/dn
-    NFS = 14                // the rest is spare: the box-size limit of the allocation-free entry point follows from it
+    FS_USED = FS_THERM + 1,
+    NFS = 14                // of the scratch layout; the rest is spare: the box-size limit of the allocation-free entry point follows from it
 };
 
 // Kernel kinds of the launch counter / event profiler (mfg_prof.cu).
