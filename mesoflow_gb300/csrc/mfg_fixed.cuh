@@ -76,6 +76,9 @@ MFG_HD double double_of(uint64_t u) {
 #endif
 }
 
+// High word of |x|: the order of magnitudes as integers.
+MFG_HD int hi_abs(double x) { return (int)(bits_of(x) >> 32) & 0x7fffffff; }
+
 // Bits of the float32 1/f, f in (1, 2), and 1/sqrt(f), f in (1, 4), relative
 // error below 2^-22.
 MFG_HD uint32_t rcp_seed_bits(uint32_t fbits) {

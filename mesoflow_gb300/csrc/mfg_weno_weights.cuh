@@ -173,7 +173,6 @@ constexpr int kFrontTop = 9, kFrontMost = 1900 << 20;
 MFG_HD bool front_above(int top, int value) {
     return top > imax((imin(value, kFrontMost) >> 19) + kFrontTop, 2 * kWenoExpFloor - 2);
 }
-MFG_HD int hi_abs(double x) { return (int)(bits_of(x) >> 32) & 0x7fffffff; }
 MFG_HD bool weno_front(int topf, int topu, bool pressure, double fL, double fR, double uL, double uR, double lam) {
     const int l = hi_abs(lam) - 0x3ff00000;
     int mu = imin(imax(hi_abs(uL), hi_abs(uR)), kFrontMost), mf = (int)((unsigned)mu + (unsigned)l);
