@@ -667,7 +667,7 @@ __device__ __forceinline__ void update_body(const Fp& fp, const RhsBox& B, int s
 // one thread walks a segment of faces along d for one component, keeping the
 // per-cell parts of the reconstruction in registers.  FP64 issue bounds it
 // (GB300 issues 2 FP64 operations per SM and cycle), so the form below is the
-// one with the fewest FP64 operations, about 23 per (face, component).
+// one with the fewest FP64 operations, about 19 per (face, component).
 //
 // The WENO5-JS edges (flux_schemes.H:373-446) in second differences.  With
 // cell differences D and t_m = v_{m-1} - 2 v_m + v_{m+1}, the linear weights
@@ -692,8 +692,9 @@ __device__ __forceinline__ void update_body(const Fp& fp, const RhsBox& B, int s
 // and quantity, in the shadow of about 800 on the FP64 pipe).
 // Fluxes of a 64^3 box with 10 components, per right-hand side: 2.34 ms in the
 // candidate form (130 FP64 operations per face and component, one division per
-// edge), 1.29 ms in second differences with FP64 weights (75 operations),
-// 0.57 ms with the fixed-point weights (23 operations).
+// edge), 1.29 ms in second differences with FP64 weights (75 operations), 0.57 ms
+// with the fixed-point weights (23), 0.42 ms with the near weights added in fixed
+// point and fewer integer products (19), 0.44 ms with the faces beside fronts.
 // ---------------------------------------------------------------------------
 constexpr int SWEEP_SEG = 32;  // longest face segment per thread (batched launches)
 
