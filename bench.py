@@ -429,7 +429,7 @@ def run_adjoint(a):
 
     cells = n ** 3
     runs = [("forward", forward), (f"adjoint_checkpoint{a.checkpoint}", adjoint(a.checkpoint))]
-    keep_bytes = nsteps * cells * 8 * 345 * 1.1  # snapshots of every step: about 345 doubles per cell and step
+    keep_bytes = nsteps * cells * 8 * 290 * 1.1  # snapshots of every step: about 290 doubles per cell and step
     if keep_bytes < 0.8 * total_mem:
         runs.append(("adjoint_keep_all", adjoint(0)))
     res, mem, Js = {}, {}, {}
