@@ -683,8 +683,9 @@ __device__ __forceinline__ void update_body(const Fp& fp, const RhsBox& B, int s
 // against 80-bit arithmetic than the candidate form where the values are at least
 // as large.  Beside a front, where the differences are 2^6 and more times the
 // face's values, they would be larger than the flux in the end, and the face takes
-// the candidates (weno_front, weno_front_llf): the test, on the integer pipe, costs
-// 3% of the 128^3 Taylor-Green step and 4% of a 64^3 right-hand side.
+// the candidates (weno_front, weno_front_llf): the test, on the integer pipe, and
+// the faces it finds cost 2.5% of the 128^3 Taylor-Green step and 4% of a 64^3
+// right-hand side.
 //   The right edge of face m and the left edge of face m + 1 lie in cell m and
 // see the same five cells, so they share the products of their weights.
 //   The weights are ratios of positive numbers: mfg_weno_weights.cuh forms
